@@ -166,11 +166,19 @@ int lq_int4_kv_append(const lq_int4_cache* cache, const void* k, const int64_t k
                       const int64_t v_stride[4], int32_t dtype, const int64_t* positions, int32_t q_len,
                       void* cuda_stream);
 
+/* What the elements of a decode mask are: additive biases, or keep flags (zero: the token is masked out). */
+#define LQ_MASK_ADD_F32 0
+#define LQ_MASK_ADD_BF16 1
+#define LQ_MASK_ADD_F16 2
+#define LQ_MASK_KEEP_U8 3   /* also bool */
+#define LQ_MASK_KEEP_I32 4
+#define LQ_MASK_KEEP_I64 5
+
 /* q_len = 1 GQA attention over rows [0, seq_len) of the cache, split over the context.
- * q: [B, Hq, D] (stride of the length-1 query axis is irrelevant); mask: optional device fp32
- * additive bias, element (b, n) at mask[b * mask_stride_b + n * mask_stride_k], tokens
- * n >= mask_k_len are masked out; the bias is added to scores already scaled by
- * log2(e)/sqrt(D) (one unit = a factor of two).  out: [B, Hq, D] in `dtype`.
+ * q: [B, Hq, D] (stride of the length-1 query axis is irrelevant); mask: optional device mask,
+ * element (b, n) at mask[b * mask_stride_b + n * mask_stride_k], of the kind mask_kind (0: fp32
+ * additive bias); tokens n >= mask_k_len are masked out; a bias is added to scores already scaled
+ * by log2(e)/sqrt(D) (one unit = a factor of two).  out: [B, Hq, D] in `dtype`.
  * splits = 0 lets the library choose; workspace (see lq_int4_decode_workspace_bytes) is needed
  * whenever more than one split is used and must start zeroed once (the kernel restores the
  * zero state of the part it uses as counters before it finishes).
@@ -183,7 +191,7 @@ typedef struct lq_int4_decode_args {
   int32_t dtype;        /* of q and out                                                         */
   int32_t q_heads;
   int32_t seq_len;
-  const float* mask; int64_t mask_stride_b; int64_t mask_stride_k; int32_t mask_k_len;
+  const void* mask; int64_t mask_stride_b; int64_t mask_stride_k; int32_t mask_k_len;
   int32_t splits;       /* 0: the library picks; otherwise used as given, capped at the tile count and at 128 */
   void* workspace; size_t workspace_bytes;
   /* Fused append (optional): when k_new != NULL the row seq_len - 1 of every (batch, kv head) is
@@ -199,6 +207,7 @@ typedef struct lq_int4_decode_args {
    * [1, capacity] is clamped and sets bit 1 of lq_device_status.  No reference counterpart: the
    * reference reads the length on the host each step (int4_8b_attention.py:667).               */
   const uint64_t* seq_len_counter;
+  int32_t mask_kind;    /* LQ_MASK_* */
 } lq_int4_decode_args;
 
 int lq_int4_decode_attn(const lq_int4_decode_args* args, void* cuda_stream);

@@ -99,7 +99,7 @@ class Int4DecodeArgs(C.Structure):
         ("workspace", C.c_void_p), ("workspace_bytes", C.c_size_t),
         ("k_new", C.c_void_p), ("k_new_stride", C.c_int64 * 3),
         ("v_new", C.c_void_p), ("v_new_stride", C.c_int64 * 3),
-        ("seq_len_counter", C.c_void_p),
+        ("seq_len_counter", C.c_void_p), ("mask_kind", C.c_int32),
     ]
 
 
@@ -155,6 +155,25 @@ def lib() -> C.CDLL:
         raise RuntimeError(f"{LIB_PATH}: ABI version {l.lq_abi_version()} != 1; rebuild the library")
     _lib = l
     return l
+
+
+_native = None
+
+
+def native():
+    """The call path in C++ (csrc/lq_torch.cpp): the functions of the host mirrors that sit on every decode step fill the
+    argument block and launch there.  Each returns None when the call is not the ordinary case; the caller
+    then goes through the ctypes binding above, which also raises the errors."""
+    global _native
+    if _native is None:
+        lib()
+        try:
+            from . import _native as module
+        except ImportError as exc:
+            raise RuntimeError(f"{PKG / '_native.so'} cannot be imported ({exc}): build it with `python -m layer_quant_b200.build`") from exc
+        module.bind(str(LIB_PATH))
+        _native = module
+    return _native
 
 
 def check(rc: int) -> None:

@@ -93,6 +93,21 @@ __device__ __forceinline__ uint32_t int4_code(float x, float scale) {
   return static_cast<uint32_t>(q) & 15u;
 }
 
+// Bias of token n in sequence b: the mask in the caller's own type, read where it is used (a 2-D tokenizer mask costs no
+// conversion pass); tokens past the mask are masked out.
+__device__ __forceinline__ float mask_bias(const lq_int4_decode_args& a, int b, int n) {
+  if (n >= a.mask_k_len) return -INFINITY;
+  const int64_t i = b * a.mask_stride_b + n * a.mask_stride_k;
+  switch (a.mask_kind) {
+    case LQ_MASK_ADD_F32: return static_cast<const float*>(a.mask)[i];
+    case LQ_MASK_ADD_BF16: return load_as_float(a.mask, i, LQ_BF16);
+    case LQ_MASK_ADD_F16: return load_as_float(a.mask, i, LQ_F16);
+    case LQ_MASK_KEEP_U8: return static_cast<const uint8_t*>(a.mask)[i] ? 0.0f : -INFINITY;
+    case LQ_MASK_KEEP_I32: return static_cast<const int32_t*>(a.mask)[i] ? 0.0f : -INFINITY;
+    default: return static_cast<const long long*>(a.mask)[i] ? 0.0f : -INFINITY;
+  }
+}
+
 struct AppendParams {
   lq_int4_cache c;
   const void* k; const void* v;
@@ -457,7 +472,7 @@ __global__ void __launch_bounds__(kDecodeThreads, 1) int4_decode_kernel(const De
         bias[ps] = 0.0f;
         if (HAS_MASK) {
           const int n = tok0 + t;
-          bias[ps] = n < a.mask_k_len ? a.mask[b * a.mask_stride_b + n * a.mask_stride_k] : -INFINITY;
+          bias[ps] = mask_bias(a, b, n);
         }
       }
 #pragma unroll
@@ -486,7 +501,7 @@ __global__ void __launch_bounds__(kDecodeThreads, 1) int4_decode_kernel(const De
       float bias = 0.0f;
       if (HAS_MASK) {
         const int n = rl.seq_len - 1;
-        bias = n < a.mask_k_len ? a.mask[b * a.mask_stride_b + n * a.mask_stride_k] : -INFINITY;
+        bias = mask_bias(a, b, n);
       }
       process_token(warp == 0 && tg == 0, kc, vc, ksc, vsc, bias);
     }
@@ -787,7 +802,9 @@ LQ_EXPORT int lq_int4_decode_attn(const lq_int4_decode_args* args, void* cuda_st
                "lq_int4_decode_attn: packed batch/head strides must be multiples of 16 bytes");
   LQ_CHECK_ARG(c.ks_stride[0] % 4 == 0 && c.ks_stride[1] % 4 == 0 && c.vs_stride[0] % 4 == 0 && c.vs_stride[1] % 4 == 0,
                "lq_int4_decode_attn: scale batch/head strides must be multiples of 4 elements");
-  if (a.mask) LQ_CHECK_ARG(a.mask_k_len >= 0, "lq_int4_decode_attn: mask_k_len=%d", a.mask_k_len);
+  if (a.mask)
+    LQ_CHECK_ARG(a.mask_k_len >= 0 && a.mask_kind >= LQ_MASK_ADD_F32 && a.mask_kind <= LQ_MASK_KEEP_I64,
+                 "lq_int4_decode_attn: mask_k_len=%d, mask_kind=%d", a.mask_k_len, a.mask_kind);
 
   DecodeParams p;
   p.a = a;

@@ -442,7 +442,7 @@ __global__ void __launch_bounds__(kThreadsM, (R * (QB > 0 ? QB : 1) <= 4 && !QSP
       float bias = 0.0f;
       if (HAS_MASK) {
         const int n = tok_first + rr;
-        bias = ((FULL || rr < valid) && n < a.mask_k_len) ? a.mask[b * a.mask_stride_b + n * a.mask_stride_k] : -INFINITY;
+        bias = (FULL || rr < valid) ? mask_bias(a, b, n) : -INFINITY;
       }
       // both columns of the token at once: packed fp32x2 FMA / MUL (sm_100), same rounding per component
       float2 sum2 = make_float2(0.0f, 0.0f);

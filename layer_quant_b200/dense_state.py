@@ -28,6 +28,9 @@ def selective_state_update(state, x, dt, A, B, C, D=None, z=None, dt_bias=None, 
     ``dt = softplus(dt + dt_bias)``, ``state = state * exp(A dt) + B dt x``, ``y = <state, C> + D x``
     and, with z, ``y * z * sigmoid(z)``.
     """
+    y = _lib.native().dense_update(state, x, dt, A, B, C, D, z, dt_bias, dt_softplus, out)
+    if y is not None:
+        return y
     squeeze = state.dim() == 3
     if squeeze:
         state, x, dt, A = state.unsqueeze(1), x.unsqueeze(1), dt.unsqueeze(1), A.unsqueeze(0)
@@ -76,6 +79,9 @@ def causal_conv1d_update(x, conv_state, weight, bias=None, activation=None, *, o
     product with the channel's weights (+ bias), through SiLU when asked."""
     if activation not in (None, "silu", "swish"):
         raise NotImplementedError("activation must be None, silu, or swish")
+    y = _lib.native().conv1d_update(x, conv_state, weight, bias, activation is not None, out)
+    if y is not None:
+        return y
     unsqueeze = x.dim() == 3
     if unsqueeze:
         if x.shape[2] != 1:

@@ -151,6 +151,9 @@ def _pack_kv_into_cache(cache: Int4KVLayerCache, key_states: torch.Tensor, value
     """Quantise ``key_states`` / ``value_states`` [B, Hkv, q_len, D] and write them to cache rows
     ``positions`` (int64 [q_len], shared by the batch).  ``known_len`` = max(positions) + 1 when the
     caller already has it (saves the read-back the reference does at :515)."""
+    if _lib.native().pack_kv(cache, key_states, value_states, positions, group_size) is not None:
+        cache.length = max(cache.length, known_len if known_len is not None else int(positions.max().item()) + 1)
+        return
     batch, kv_heads, q_len, head_dim = key_states.shape
     if value_states.shape != key_states.shape or value_states.dtype != key_states.dtype:
         raise ValueError("key_states and value_states must agree in shape and dtype")
@@ -187,19 +190,10 @@ def _decode_attention_mask(attention_mask: torch.Tensor | None, batch: int, seq_
     raise ValueError(f"INT4 decode attention only supports 2D or 4D attention_mask, got {attention_mask.dim()}D")
 
 
-_WORKSPACES: dict[tuple[int, int], torch.Tensor] = {}
-
-
 def _workspace(device: torch.device, nbytes: int) -> torch.Tensor:
     """Zero-initialised scratch for the split merge, one per (device, stream), grown on demand.
     The kernel leaves its ticket counters at zero, so the buffer is cleared only when created."""
-    key = (device.index if device.index is not None else torch.cuda.current_device(),
-           torch.cuda.current_stream(device).cuda_stream)
-    ws = _WORKSPACES.get(key)
-    if ws is None or ws.numel() < nbytes:
-        ws = torch.zeros(max(nbytes, 1 << 20), dtype=torch.uint8, device=device)
-        _WORKSPACES[key] = ws
-    return ws
+    return _lib.native().workspace_for(device.index if device.index is not None else torch.cuda.current_device(), nbytes)
 
 
 def _decode_args(query_states, cache, seq_len, group_size, mask, k_new=None, v_new=None, splits=0, out=None,
@@ -223,7 +217,8 @@ def _decode_args(query_states, cache, seq_len, group_size, mask, k_new=None, v_n
     a.seq_len = seq_len
     if mask is not None:
         a.mask = mask.data_ptr()
-        a.mask_stride_b, a.mask_stride_k, a.mask_k_len = mask.stride(0), mask.stride(3), mask.shape[-1]
+        a.mask_stride_b = mask.stride(0) if mask.shape[0] == batch else 0
+        a.mask_stride_k, a.mask_k_len = mask.stride(3), mask.shape[-1]
     if k_new is not None:
         a.k_new, a.v_new = k_new.data_ptr(), v_new.data_ptr()
         for i, ax in enumerate((0, 1, 3)):
@@ -268,13 +263,16 @@ class Int4DecodePlan:
             raise ValueError(f"Fused INT4 decode attention expects q_len=1, got {query_states.shape[2]}")
         self.args, self.out, self._keep = _decode_args(query_states, cache, seq_len, group_size, mask, k_new, v_new, splits,
                                                        out, seq_len_counter)
-        self._ref = ct.byref(self.args)
-        self._fn = _lib.lib().lq_int4_decode_attn
+        self._launch = _lib.native().int4_plan_launch
+        self._address = ct.addressof(self.args)
         self.device = self.out.device
+        self._device_index = self.device.index
         self.seq_len_counter = seq_len_counter
 
     def launch(self) -> torch.Tensor:
-        _lib.check(self._fn(self._ref, _lib.stream_ptr(self.device)))
+        rc = self._launch(self._address, self._device_index)
+        if rc:
+            _lib.check(rc)
         return self.out
 
 
@@ -287,6 +285,10 @@ def _decode_attention(query_states: torch.Tensor, cache: Int4KVLayerCache, seq_l
                       group_size: int, attention_mask: torch.Tensor | None = None, *, splits: int = 0) -> torch.Tensor:
     """softmax(q K^T / sqrt(D) [+ mask]) V over cache rows [0, seq_len) for one query token.
     query_states [B, Hq, 1, D] -> [B, Hq, D] in the query's dtype."""
+    out = _lib.native().decode_attn(query_states, cache, seq_len, num_key_value_groups, group_size, attention_mask, None, None,
+                                    splits, None)
+    if out is not None:
+        return out
     batch, n_heads, q_len, head_dim = query_states.shape
     if q_len != 1:
         raise ValueError(f"Fused INT4 decode attention expects q_len=1, got {q_len}")
@@ -301,6 +303,10 @@ def _append_decode_attention(query_states, key_states, value_states, cache, seq_
     """Decode step in one launch: quantise the new K/V row [B, Hkv, 1, D] into cache row
     ``seq_len - 1`` and attend over rows [0, seq_len).  Equals ``_pack_kv_into_cache`` followed by
     ``_decode_attention``."""
+    out = _lib.native().decode_attn(query_states, cache, seq_len, 0, group_size, attention_mask, key_states, value_states, splits, None)
+    if out is not None:
+        cache.length = max(cache.length, seq_len)
+        return out
     batch, n_heads, q_len, head_dim = query_states.shape
     if q_len != 1 or key_states.shape[2] != 1:
         raise ValueError(f"Fused INT4 decode attention expects q_len=1, got {q_len}")
@@ -322,6 +328,9 @@ def _prefill_attention(query_states: torch.Tensor, cache: Int4KVLayerCache, num_
     query's dtype.  Positional arguments as the reference's ``_prefill_attention`` (:594-625, the launcher of its
     unused ``_int4_prefill_attention_kernel``, :114-251), which is ``first_len = 1``: a prompt from position 0;
     larger values (keyword-only, not in the reference) continue an existing context."""
+    result = _lib.native().prefill_attn(query_states, cache, num_key_value_groups, group_size, first_len, out)
+    if result is not None:
+        return result
     batch, n_heads, q_len, head_dim = query_states.shape
     if n_heads != cache.k_packed.shape[1] * num_key_value_groups:
         raise ValueError(f"{n_heads} query heads != {cache.k_packed.shape[1]} kv heads x {num_key_value_groups}")
@@ -374,6 +383,9 @@ def _graph_decode_step(query_states, key_states, value_states, cache, group_size
         raise NotImplementedError("recorded decode steps take no attention_mask: a mask's length changes every step")
     advance_seq_len(cache.length_counter)  # the new token's position + 1
     capacity = cache.k_packed.shape[2]
+    out = _lib.native().decode_attn(query_states, cache, capacity, 0, group_size, None, key_states, value_states, 0, cache.length_counter)
+    if out is not None:
+        return out
     a, out, keep = _decode_args(query_states, cache, capacity, group_size, None, key_states, value_states,
                                 seq_len_counter=cache.length_counter)
     _lib.check(_lib.lib().lq_int4_decode_attn(ct.byref(a), _lib.stream_ptr(out.device)))

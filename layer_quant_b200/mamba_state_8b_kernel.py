@@ -28,15 +28,13 @@ Differences a caller can see, all opt-out:
   ``patch_nemotron_h_mamba_decode_state_kernel`` (or ``RNG_STREAM`` is set): that reproduces the
   reference's ``tl.rand(seed, step * numel + index)`` numbers and rounding rule bit for bit at
   about a quarter of the speed (one Philox block per value instead of one per 16 values).
-* Repeated calls with the same operand tensors (the decode loop) reuse the argument block prepared
-  by the first call; only the output pointer and the step change.
 * A decode step never recompiles anything (the reference re-JITs each step because its RNG offset
   is a compile-time constant).
 """
 from __future__ import annotations
 
 import ctypes as ct
-from dataclasses import dataclass, field
+from dataclasses import dataclass
 from types import SimpleNamespace
 
 import torch
@@ -80,10 +78,6 @@ class MambaStateKernelCache:
     # Whether this cache's update advances ``step_counter`` afterwards.  When the caches of one model share a counter
     # (prepare_graph_decode), only the last layer's update does, once per decode step.
     advances_counter: bool = True
-    # Not in the reference: the argument block prepared by the last mx_state_selective_update call on this cache
-    # and the operand signature it was prepared for.
-    _plan: object = field(default=None, repr=False, compare=False)
-    _plan_key: object = field(default=None, repr=False, compare=False)
 
     @property
     def state_shape(self) -> tuple[int, int, int, int]:
@@ -201,6 +195,10 @@ def allocate_state_kernel_cache(ssm_state_4d: torch.Tensor, group_size: int = MX
     if ssm_state_4d.ndim != 4:
         raise ValueError(f"Expected ssm_state [B,H,P,N], got {tuple(ssm_state_4d.shape)}")
     layout = layout or DEFAULT_STATE_LAYOUT
+    if layout in _LAYOUTS:
+        got = _lib.native().mx_quantize(ssm_state_4d, format_bits, layout == "packed")
+        if got is not None:
+            return MambaStateKernelCache(*got, format_bits=format_bits, layout=layout)
     q, e, m = _quantize_initial_state_mx(ssm_state_4d, format_bits=format_bits, block_size=16, pair_size=2,
                                          mantissa_max=mmax, layout=layout)
     return MambaStateKernelCache(q_state=q, shared_exp=e, micro_exp=m, format_bits=format_bits, layout=layout)
@@ -283,8 +281,10 @@ class MxUpdatePlan:
             if step_counter.dtype != torch.int64 or step_counter.numel() != 1:
                 raise ValueError("step_counter must be a 1-element int64 CUDA tensor")
             r.step_counter = step_counter.data_ptr()
-        self._fn = _lib.lib().lq_mx_state_update
-        self._ref = ct.byref(a)
+        self._launch = _lib.native().mx_plan_run
+        self._address = ct.addressof(a)
+        self._device_index = self.device.index
+        self._counts_on_device = step_counter is not None
         self._out_sig = (self.out.data_ptr(), self.out.stride(), self.out.dtype)
 
     def rebind_out(self, out: torch.Tensor) -> None:
@@ -300,15 +300,13 @@ class MxUpdatePlan:
         a.out_dtype = _lib.dtype_code(out)
 
     def run(self) -> torch.Tensor:
-        r = self.args.rounding
-        step = int(self.cache.step)
-        r.step = step
-        r.rng_offset = (step * self.numel) & 0xFFFFFFFFFFFFFFFF
-        rc = self._fn(self._ref, _lib.stream_ptr(self.device))
+        cache = self.cache
+        step = int(cache.step)
+        rc = self._launch(self._address, self._device_index, step)
         if rc:
             _lib.check(rc)
-        if not r.step_counter:
-            self.cache.step = step + 1
+        if not self._counts_on_device:
+            cache.step = step + 1
         return self.out
 
 
@@ -350,42 +348,17 @@ def mx_state_selective_update(
     ``h_out`` (fp32 [B,H,P,N]) receives the updated state before requantisation; ``out`` is
     written instead of a fresh tensor.  :class:`MxUpdatePlan` prepares the same call once for
     loops that repeat it."""
-    # the reference's own checks, in its order (:615-621)
-    if cache.q_state.ndim != 4:
-        raise ValueError(f"Expected q_state [B,H,P,N], got {tuple(cache.q_state.shape)}")
-    if x.shape != cache.state_shape[:3]:
-        raise ValueError(f"Expected x shape {cache.state_shape[:3]}, got {tuple(x.shape)}")
-    if B.ndim != 3 or C.ndim != 3:
-        raise ValueError("Expected B and C with shape [batch, ngroups, dstate] for decode update.")
-    # The decode loop calls this with the same tensors every step: the prepared argument block of the previous call is
-    # reused when every operand still has the same address and strides (and x / B the same shape and type: with the
-    # state's shape they fix every other operand's shape).
-    key = (x.data_ptr(), x.stride(), x.shape, x.dtype, dt.data_ptr(), dt.stride(), dt.dtype, A.data_ptr(), A.stride(), A.dtype,
-           B.data_ptr(), B.stride(), B.shape, B.dtype, C.data_ptr(), C.stride(), C.dtype, _sig(D), _sig(z), _sig(dt_bias),
-           _sig(rand_words), _sig(h_out), cache.q_state.data_ptr(), cache.shared_exp.data_ptr(), cache.micro_exp.data_ptr(),
-           None if cache.step_counter is None else cache.step_counter.data_ptr(),
-           dt_softplus, stochastic, seed, rng_stream or RNG_STREAM, cache.layout, cache.format_bits, cache.layer)
-    plan = cache._plan if cache._plan_key == key else None
-    if out is None:
-        out = torch.empty_like(x)
-    if plan is None:
-        plan = MxUpdatePlan(cache, x, dt, A, B, C, D=D, z=z, dt_bias=dt_bias, dt_softplus=dt_softplus, stochastic=stochastic,
-                            seed=seed, rng_stream=rng_stream, rand_words=rand_words, h_out=h_out, out=out,
-                            step_counter=cache.step_counter)
-        cache._plan, cache._plan_key = plan, key
-    else:
-        if out.shape != x.shape:
-            raise ValueError(f"Expected out shape {tuple(x.shape)}, got {tuple(out.shape)}")
-        plan.rebind_out(out)
-    y = plan.run()
+    if rand_words is None and h_out is None:
+        y = _lib.native().mx_update(cache, x, dt, A, B, C, D, z, dt_bias, dt_softplus, stochastic, seed, rng_stream or RNG_STREAM, out)
+        if y is not None:
+            return y
+    # anything out of the ordinary: the reference's own checks in its order (:615-621), errors included
+    y = MxUpdatePlan(cache, x, dt, A, B, C, D=D, z=z, dt_bias=dt_bias, dt_softplus=dt_softplus, stochastic=stochastic,
+                     seed=seed, rng_stream=rng_stream, rand_words=rand_words, h_out=h_out, out=out,
+                     step_counter=cache.step_counter).run()
     if cache.step_counter is not None and cache.advances_counter:
         advance_step_counter(cache.step_counter)
     return y
-
-
-def _sig(t):
-    """What a prepared argument block depends on in an optional operand: address, strides, type."""
-    return None if t is None else (t.data_ptr(), t.stride(), t.dtype)
 
 
 def prepare_graph_decode(model, shared: bool = True) -> None:

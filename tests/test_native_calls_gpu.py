@@ -1,0 +1,90 @@
+"""The C++ call path of the host mirrors against the general path through ctypes: the same launch, so the same bits."""
+import pytest
+import torch
+
+from tests.util import dev
+
+pytestmark = pytest.mark.gpu
+
+
+def _cache(m, b, hkv, tlen, gs, g):
+    cache = m._allocate_layer_cache(b, hkv, 256, 128, 128 // gs, dev())
+    k, v = (torch.randn(b, hkv, tlen, 128, generator=g, device=dev()) for _ in range(2))
+    m._pack_kv_into_cache(cache, k, v, torch.arange(tlen, device=dev()), gs)
+    return cache
+
+
+@pytest.mark.parametrize("kind", ["bool", "uint8", "int32", "int64", "int64_wide", "bool4", "f32_4", "bf16_4", "f16_4", "f32_4_one", "f32_2"])
+def test_masks_are_read_in_their_own_type(kind):
+    """Every mask the kernel reads directly equals the fp32 bias that the host conversion makes of it."""
+    from layer_quant_b200 import int4_8b_attention as m
+    g = torch.Generator(device=dev()).manual_seed(3)
+    b, tlen, gs = 3, 130, 32
+    cache = _cache(m, b, 2, tlen, gs, g)
+    q = torch.randn(b, 8, 1, 128, generator=g, device=dev()).to(torch.bfloat16)
+    keep = torch.rand(b, tlen + 7, generator=g, device=dev()) < 0.7
+    keep[:, -1] = True
+    bias = torch.randn(b, 1, 2, tlen + 7, generator=g, device=dev())
+    mask = {"bool": keep[:, :tlen], "uint8": keep[:, :tlen].to(torch.uint8), "int32": keep[:, :tlen].int(), "int64": keep[:, :tlen].long(),
+            "int64_wide": keep.long(), "bool4": keep[:, None, None, :], "f32_4": bias, "bf16_4": bias.bfloat16(), "f16_4": bias.half(),
+            "f32_4_one": bias[:1], "f32_2": keep.float()}[kind]
+    out = m._decode_attention(q, cache, tlen, 4, gs, attention_mask=mask)
+    general = m._launch_decode(q, cache, tlen, gs, m._decode_attention_mask(mask, b, tlen, dev()))
+    assert torch.equal(out, general)
+
+
+@pytest.mark.parametrize("case", ["plain", "z", "given_out", "step_counter", "no_D", "fp32_operands", "half_up", "layered4", "reference_layout"])
+def test_state_update_equals_the_prepared_call(case):
+    from layer_quant_b200 import mamba_state_8b_kernel as m
+    g = torch.Generator(device=dev()).manual_seed(5)
+    b, h, p, n, grp = 2, 4, 16, 128, 2
+    dtype = torch.float32 if case == "fp32_operands" else torch.bfloat16
+    r = lambda *s: torch.randn(*s, generator=g, device=dev()).to(dtype)
+    state = torch.randn(b, h, p, n, generator=g, device=dev())
+    x, dt, B, C = r(b, h, p), r(b, h)[:, :, None].expand(b, h, p), r(b, grp, n), r(b, grp, n)
+    A = -torch.rand(h, generator=g, device=dev())[:, None, None].expand(h, p, n)
+    D, bias = (None if case == "no_D" else r(h)[:, None].expand(h, p)), r(h)[:, None].expand(h, p)
+    kw = dict(D=D, z=r(b, h, p) if case == "z" else None, dt_bias=bias, dt_softplus=True, stochastic=case != "half_up", seed=2**63 + 5,
+              rng_stream="layered4" if case == "layered4" else "layered")
+    ys, caches = [], []
+    for prepared in (False, True):
+        cache = m.allocate_state_kernel_cache(state, layout="reference" if case == "reference_layout" else "packed")
+        cache.step, cache.layer = 7, 3
+        if case == "step_counter":
+            cache.step_counter = torch.full((1,), 2, dtype=torch.int64, device=dev())
+        out = torch.empty_like(x) if case == "given_out" else None
+        if prepared:
+            y = m.MxUpdatePlan(cache, x, dt, A, B, C, out=out, step_counter=cache.step_counter, **kw).run()
+        else:
+            y = m.mx_state_selective_update(cache, x, dt, A, B, C, out=out, **kw)
+            assert out is None or y is out
+            assert cache.step == (7 if case == "step_counter" else 8)
+            assert case != "step_counter" or cache.step_counter.item() == 3
+        ys.append(y)
+        caches.append(cache)
+    assert torch.equal(*ys)
+    for name in ("q_state", "shared_exp", "micro_exp"):
+        assert torch.equal(getattr(caches[0], name), getattr(caches[1], name))
+
+
+def test_errors_come_from_the_general_path():
+    from layer_quant_b200 import dense_state, int4_8b_attention as ia, mamba_state_8b_kernel as mk
+    d = dev()
+    cache = mk.allocate_state_kernel_cache(torch.zeros(1, 2, 16, 128, device=d))
+    x, A, B = torch.zeros(1, 2, 8, device=d), torch.zeros(2, 16, 128, device=d), torch.zeros(1, 1, 128, device=d)
+    with pytest.raises(ValueError, match="Expected x shape"):
+        mk.mx_state_selective_update(cache, x, x, A, B, B)
+    x = torch.zeros(1, 2, 16, device=d)
+    with pytest.raises(ValueError, match="unknown rng_stream"):
+        mk.mx_state_selective_update(cache, x, x, A, B, B, rng_stream="other")
+    assert cache.step == 0
+    kv = ia._allocate_layer_cache(1, 2, 16, 128, 4, torch.device(d))
+    q = torch.zeros(1, 8, 1, 128, device=d, dtype=torch.bfloat16)
+    with pytest.raises(ValueError, match="outside"):
+        ia._decode_attention(q, kv, 17, 4, 32)
+    with pytest.raises(ValueError, match="query heads"):
+        ia._decode_attention(q, kv, 4, 2, 32)
+    with pytest.raises(ValueError, match="only supports 2D or 4D"):
+        ia._decode_attention(q, kv, 4, 4, 32, attention_mask=torch.zeros(1, 1, 4, device=d))
+    with pytest.raises(ValueError, match="do not match state"):
+        dense_state.selective_state_update(torch.zeros(1, 2, 16, 128, device=d), x[:, :, :8], x, A, B, B)
