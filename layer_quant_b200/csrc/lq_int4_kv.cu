@@ -601,6 +601,7 @@ __global__ void __launch_bounds__(kDecodeThreads, 1) int4_decode_kernel(const De
 }  // namespace lq
 
 #include "lq_int4_mma.cuh"
+#include "lq_int4_prefill.cuh"
 
 namespace lq {
 
@@ -874,6 +875,25 @@ static int launch_prefill_gs(const DecodeParams& p, cudaStream_t st) {
   }
 }
 
+// 16-bit queries: the tcgen05 kernel, whatever the sizes.  An fp32 query needs a third product for its low half, for which there is
+// no room in tensor memory: it stays on the mma.sync kernel.
+static int launch_prefill_tc(const lq_int4_prefill_args& a, int ratio, cudaStream_t st) {
+  const auto log2_of = [](int v) { int l = 0; while ((1 << l) < v) ++l; return l; };
+  prefill::Params p;
+  p.a = a;
+  p.ratio_log2 = log2_of(ratio);
+  p.gs_log2 = log2_of(a.cache.group_size);
+  const int pos_per_cta = prefill::kCtaRows / ratio;
+  p.nqb = (a.q_len + pos_per_cta - 1) / pos_per_cta;
+  p.kv_len = a.first_len + a.q_len - 1;
+  const int64_t grid = static_cast<int64_t>(p.nqb) * a.cache.batch * a.cache.kv_heads;
+  LQ_CHECK_ARG(grid <= 0x7FFFFFFFLL, "lq_int4_prefill_attn: batch * kv heads * query blocks too large for one launch");
+  LQ_SET_SMEM_ONCE(prefill::int4_prefill_kernel, prefill::kSmemBytes);
+  prefill::int4_prefill_kernel<<<static_cast<unsigned>(grid), prefill::kThreads, prefill::kSmemBytes, st>>>(p);
+  LQ_CHECK_CUDA(cudaGetLastError());
+  return LQ_OK;
+}
+
 LQ_EXPORT int lq_int4_prefill_attn(const lq_int4_prefill_args* args, void* cuda_stream) {
   LQ_CHECK_ARG(args != nullptr, "lq_int4_prefill_attn: null args");
   const lq_int4_prefill_args& a = *args;
@@ -901,6 +921,8 @@ LQ_EXPORT int lq_int4_prefill_attn(const lq_int4_prefill_args* args, void* cuda_
   const int ratio = a.q_heads / c.kv_heads;
   if (ratio != 1 && ratio != 2 && ratio != 4 && ratio != 8)
     return fail(LQ_ERR_UNSUPPORTED, "lq_int4_prefill_attn: %d query heads per kv head (supported: 1, 2, 4, 8)", ratio);
+  if (a.dtype != LQ_F32 && (c.group_size == 32 || c.group_size == 64 || c.group_size == 128))
+    return launch_prefill_tc(a, ratio, static_cast<cudaStream_t>(cuda_stream));
   DecodeParams p;
   p.a = lq_int4_decode_args{};
   p.a.cache = c;

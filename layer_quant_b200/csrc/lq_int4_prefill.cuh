@@ -1,0 +1,527 @@
+// Causal attention of many query positions over the packed INT4 KV cache on the 5th-generation tensor cores.  sm_100a.
+//
+// One CTA = 256 (position, query head) rows of one (batch, kv head): the query heads that share a kv head are rows of the
+// same tile, so a cache tile is unpacked once for 256 / R positions.  Thirteen warps:
+//   0 .. 7    softmax, two groups of 128 rows, one row per thread (= one TMEM lane)
+//   8 .. 11   unpack 64-token tiles of K and V from global memory to fp16 in shared memory, two stages each
+//   12        issues the tcgen05.mma of both groups: O += P V of a tile, then S of the group's next tile into the columns
+//             that P has just been read from (the tensor pipe takes one thread's products in order)
+// Registers: launched with 128 a thread; the softmax groups raise theirs to 168, the other two groups go down to 88.
+// TMEM (512 columns, 256 per group): O 128, Q 64 (fp16, A operand), S 64; P replaces S (A operand).
+//
+// Precision.  A dequantised value n * scale (n in [-8, 7]) is held as two fp16 numbers: the leading 8 bits of the scale
+// times n, exact in fp16, and the rest of the scale times n, rounded to fp16: 2^-20 relative in all.  P is split
+// the same way (2^-22).  Q is exact in fp16 for 16-bit queries.  S = Q Khi + Q Klo, O = Phi Vhi + Plo Vhi + Phi Vlo: five
+// products per tile pair, all in fp32 accumulators.  (The mma.sync kernel keeps 16 bits of P * v_scale.)
+// Range.  Powers of two are taken out of every row of Q and of the K and V scales of every 16 tokens, so the
+// fp16 operands sit at the top of their range; the exponents come back for free, in the factor and the offset of the
+// exp2 argument.  With p' = 2^(s + Ev - m) the V exponent Ev is part of the running maximum m.
+//
+// What bounds it: the five products take 5/2 of the tensor time of a bf16 attention.  Per 256 x 64 tile that is 2620 cycles;
+// shared memory moves 230 KB meanwhile (1800 cycles), which is why Q is an operand in TMEM, and the exp2 take 1024.
+#pragma once
+
+#include "lq_common.cuh"
+
+namespace lq {
+namespace prefill {
+
+constexpr int kTok = 64;                      // tokens per tile
+constexpr int kGroupRows = 128;               // rows of a softmax group
+constexpr int kCtaRows = 2 * kGroupRows;
+constexpr int kThreads = 512;                 // four warp groups; warps 13 .. 15 only fill the last one
+constexpr int kWorkers = 416;
+constexpr int kPart = kTok * 128 * 2;         // 16 KB: fp16 [64 tokens][128 dims], as two 128-byte-swizzled halves of 64 dims
+constexpr int kStageBytes = 2 * kPart;        // hi and lo part
+constexpr int kSmemBytes = 4 * kStageBytes + 1024;  // K stages 0, 1, V stages 0, 1; alignment of the swizzle atoms
+constexpr uint32_t kColO = 0, kColQ = 128, kColS = 192, kColsPerGroup = 256;
+constexpr float kSlack = 8.0f;                // the running maximum is raised when a score exceeds it by more (log2 units)
+
+struct Params {
+  lq_int4_prefill_args a;
+  int32_t ratio_log2;   // query heads per kv head
+  int32_t gs_log2;      // group size
+  int32_t nqb;          // row blocks per (batch, kv head)
+  int32_t kv_len;       // rows of the cache that hold tokens: first_len + q_len - 1
+};
+
+// ---- tcgen05 ---------------------------------------------------------------------------------------------------------
+#define LQ_R8(r, o) "=r"(r[o]), "=r"(r[o + 1]), "=r"(r[o + 2]), "=r"(r[o + 3]), "=r"(r[o + 4]), "=r"(r[o + 5]), "=r"(r[o + 6]), "=r"(r[o + 7])
+#define LQ_I8(r, o) "r"(r[o]), "r"(r[o + 1]), "r"(r[o + 2]), "r"(r[o + 3]), "r"(r[o + 4]), "r"(r[o + 5]), "r"(r[o + 6]), "r"(r[o + 7])
+
+// columns of this warp's 32 lanes; the wait is part of the statement, so no use can move before it
+__device__ __forceinline__ void tmem_load32(uint32_t (&r)[32], uint32_t addr) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,"
+      "%24,%25,%26,%27,%28,%29,%30,%31}, [%32];\n\ttcgen05.wait::ld.sync.aligned;"
+      : LQ_R8(r, 0), LQ_R8(r, 8), LQ_R8(r, 16), LQ_R8(r, 24)
+      : "r"(addr)
+      : "memory");
+}
+__device__ __forceinline__ void tmem_load64(uint32_t (&r)[64], uint32_t addr) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x64.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,"
+      "%24,%25,%26,%27,%28,%29,%30,%31,%32,%33,%34,%35,%36,%37,%38,%39,%40,%41,%42,%43,%44,%45,%46,%47,%48,%49,%50,%51,%52,%53,%54,%55,"
+      "%56,%57,%58,%59,%60,%61,%62,%63}, [%64];\n\ttcgen05.wait::ld.sync.aligned;"
+      : LQ_R8(r, 0), LQ_R8(r, 8), LQ_R8(r, 16), LQ_R8(r, 24), LQ_R8(r, 32), LQ_R8(r, 40), LQ_R8(r, 48), LQ_R8(r, 56)
+      : "r"(addr)
+      : "memory");
+}
+__device__ __forceinline__ void tmem_store32(uint32_t addr, const uint32_t (&r)[32]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%32], {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,"
+      "%22,%23,%24,%25,%26,%27,%28,%29,%30,%31};" ::LQ_I8(r, 0), LQ_I8(r, 8), LQ_I8(r, 16), LQ_I8(r, 24), "r"(addr)
+      : "memory");
+}
+__device__ __forceinline__ void tmem_store8(uint32_t addr, const uint32_t (&r)[8]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%8], {%0,%1,%2,%3,%4,%5,%6,%7};" ::LQ_I8(r, 0), "r"(addr) : "memory");
+}
+__device__ __forceinline__ void tmem_wait_store() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ void fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ void fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
+
+// D[128 x N] (+)= A B, A from TMEM, B from shared memory, fp16 in, fp32 accumulate
+__device__ __forceinline__ void mma_ts(uint32_t d, uint32_t a, uint64_t b_desc, uint32_t idesc, bool accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d),
+      "r"(a), "l"(b_desc), "r"(idesc), "r"(accumulate ? 1u : 0u)
+      : "memory");
+}
+__device__ __forceinline__ void mma_commit(uint64_t* bar) {
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+// fp16 inputs, fp32 accumulators, M = 128; K tile: N = 64 tokens, dims contiguous; V tile: N = 128 dims, dims contiguous (N-major)
+constexpr uint32_t kIdescS = (1u << 4) | ((64u / 8) << 17) | ((128u / 16) << 24);
+constexpr uint32_t kIdescO = (1u << 4) | (1u << 16) | ((128u / 8) << 17) | ((128u / 16) << 24);
+// Shared-memory matrix descriptor, 128-byte swizzle.  Stride offset 1024: the next eight rows of 128 bytes; lbo: the next
+// 64 dims of an N-major tile.
+__device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo) {
+  return static_cast<uint64_t>((addr & 0x3FFFF) >> 4) | (static_cast<uint64_t>(lbo >> 4) << 16) | (static_cast<uint64_t>(1024 >> 4) << 32) |
+         (1ull << 46) | (2ull << 61);
+}
+
+struct Shared {
+  uint64_t k_full[2], k_empty[2], v_full[2], v_empty[2], s_done[2], p_ready[2], o_done[2];
+  // Per 16 tokens: 2^Ek, Ev and 2^-Ev.  Four tiles deep: a K stage is free again when its products are done, which can be before
+  // a slow thread has read the factors; tile j + 4 comes after the products of j + 2, and those come after that read.
+  float k_factor[4][4], v_exp[4][4], v_inv[4][4];
+  uint32_t tmem;
+};
+
+// Polls with a limit; a wait that runs out is recorded in the device status word.  The result is the same for the whole warp.
+__device__ __forceinline__ bool wait_bar(uint64_t* bar, uint32_t parity) {
+  bool done = false;
+  for (uint32_t i = 0; i < kWaitLimit && !done; ++i) done = mbar_try_wait(bar, parity);
+  if (__all_sync(0xFFFFFFFFu, done)) return true;
+  atomicOr(&g_int4_device_status, 1);
+  return false;
+}
+
+__device__ __forceinline__ float pow2_of(int e) { return __uint_as_float(static_cast<uint32_t>(e + 127) << 23); }
+__device__ __forceinline__ uint32_t pack_half2(float lo, float hi) {
+  const __half2 h = __floats2half2_rn(lo, hi);
+  return *reinterpret_cast<const uint32_t*>(&h);
+}
+
+// ---- unpacking -------------------------------------------------------------------------------------------------------
+// One 32-bit word (8 nibbles) -> four fp16 pairs in the order (0,4) (1,5) (2,6) (3,7), exact.  The dims of K, Q and V are
+// all kept in this order; the output is put right when it is stored.  (x & M) ^ K lays a nibble with its top bit
+// flipped (n + 8) under the fp16 pattern of 1024: at bit 0 it counts ones, at bit 4 sixteens.
+__device__ __forceinline__ void unpack8(uint32_t x, __half2 (&n)[4]) {
+  const uint32_t y = x >> 8;
+  const uint32_t b0 = (x & 0x000F000Fu) ^ 0x64086408u, b1 = (x & 0x00F000F0u) ^ 0x64806480u;
+  const uint32_t b2 = (y & 0x000F000Fu) ^ 0x64086408u, b3 = (y & 0x00F000F0u) ^ 0x64806480u;
+  const __half2 off = __float2half2_rn(-1032.0f), sixteenth = __float2half2_rn(0.0625f), off16 = __float2half2_rn(-72.0f);
+  n[0] = __hadd2(*reinterpret_cast<const __half2*>(&b0), off);
+  n[1] = __hfma2(*reinterpret_cast<const __half2*>(&b1), sixteenth, off16);
+  n[2] = __hadd2(*reinterpret_cast<const __half2*>(&b2), off);
+  n[3] = __hfma2(*reinterpret_cast<const __half2*>(&b3), sixteenth, off16);
+}
+
+// What a lane of the unpacking warps holds of a tile: 16 bytes (32 dims) of two tokens, K and V, and their scales
+struct RawTile {
+  uint4 k[2], v[2];
+  float ks[2], vs[2];
+};
+
+// The exponent that brings the largest of a warp's scales to [2^11, 2^12): n * scale then stays below 2^15
+__device__ __forceinline__ int scale_exponent(float a, float b) {
+  const uint32_t m = __reduce_max_sync(0xFFFFFFFFu, max(__float_as_uint(a), __float_as_uint(b)));  // scales are positive or zero
+  const int field = static_cast<int>((m >> 23) & 0xFFu);
+  return field == 0 ? 0 : min(max(field - 127 - 11, -110), 110);
+}
+
+// 32 dims of one token -> shared memory: 64 bytes of the hi part and of the lo part
+__device__ __forceinline__ void store_chunk(uint8_t* part_hi, int token, int chunk, const uint4& raw, float scale, int e) {
+  const float s = scale * pow2_of(-e);
+  const __half2 hi = __float2half2_rn(__uint_as_float(__float_as_uint(s) & 0xFFFF0000u));
+  const __half2 lo = __float2half2_rn(s - __low2float(hi));
+  const uint32_t words[4] = {raw.x, raw.y, raw.z, raw.w};
+  uint8_t* row = part_hi + (chunk >> 1) * (kPart / 2) + token * 128;
+#pragma unroll
+  for (int w = 0; w < 4; ++w) {
+    __half2 n[4];
+    unpack8(words[w], n);
+    uint32_t h[4], l[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const __half2 a = __hmul2(n[i], hi), b = __hmul2(n[i], lo);
+      h[i] = *reinterpret_cast<const uint32_t*>(&a);
+      l[i] = *reinterpret_cast<const uint32_t*>(&b);
+    }
+    uint8_t* dst = row + ((((chunk & 1) * 4 + w) ^ (token & 7)) << 4);
+    *reinterpret_cast<uint4*>(dst) = make_uint4(h[0], h[1], h[2], h[3]);
+    *reinterpret_cast<uint4*>(dst + kPart) = make_uint4(l[0], l[1], l[2], l[3]);
+  }
+}
+
+__device__ __forceinline__ void unpack_tiles(const Params& p, Shared& sh, uint8_t* smem, int b, int kvh, int ntiles) {
+  const lq_int4_cache& c = p.a.cache;
+  const int warp = (threadIdx.x >> 5) & 3, lane = threadIdx.x & 31;
+  // lanes 0..7 hold eight tokens of chunk 0, lanes 8..15 the same tokens of chunk 1, ...: 512 contiguous bytes per load, and
+  // the eight lanes of a shared-memory store phase hit eight different swizzle positions
+  const int chunk = lane >> 3, row = 16 * warp + (lane & 7);
+  const int groups_log2 = 7 - p.gs_log2, grp = (chunk * 32) >> p.gs_log2;
+  const uint8_t* kp = c.k_packed + b * c.kp_stride[0] + kvh * c.kp_stride[1] + chunk * 16;
+  const uint8_t* vp = c.v_packed + b * c.vp_stride[0] + kvh * c.vp_stride[1] + chunk * 16;
+  const float* ks = c.k_scale + b * c.ks_stride[0] + kvh * c.ks_stride[1] + grp;
+  const float* vs = c.v_scale + b * c.vs_stride[0] + kvh * c.vs_stride[1] + grp;
+  auto fetch = [&](int tile, RawTile& r) {
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int64_t tok = static_cast<int64_t>(tile) * kTok + row + 8 * i;
+      const bool ok = tok < p.kv_len;
+      r.k[i] = ok ? __ldg(reinterpret_cast<const uint4*>(kp + tok * 64)) : make_uint4(0, 0, 0, 0);
+      r.v[i] = ok ? __ldg(reinterpret_cast<const uint4*>(vp + tok * 64)) : make_uint4(0, 0, 0, 0);
+      r.ks[i] = ok ? __ldg(ks + (tok << groups_log2)) : 0.0f;
+      r.vs[i] = ok ? __ldg(vs + (tok << groups_log2)) : 0.0f;
+    }
+  };
+  RawTile cur, nxt;
+  fetch(0, cur);
+  for (int j = 0; j < ntiles; ++j) {
+    if (j + 1 < ntiles) fetch(j + 1, nxt);
+    const int st = j & 1;
+    const uint32_t parity = ((j >> 1) & 1) ^ 1;  // the first use of a stage finds it empty
+    const int ek = scale_exponent(cur.ks[0], cur.ks[1]), ev = scale_exponent(cur.vs[0], cur.vs[1]);
+    if (!wait_bar(&sh.k_empty[st], parity)) return;
+    if (lane == 0) {
+      sh.k_factor[j & 3][warp] = pow2_of(ek);
+      sh.v_exp[j & 3][warp] = static_cast<float>(ev);
+      sh.v_inv[j & 3][warp] = pow2_of(-ev);
+    }
+#pragma unroll
+    for (int i = 0; i < 2; ++i) store_chunk(smem + st * kStageBytes, row + 8 * i, chunk, cur.k[i], cur.ks[i], ek);
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&sh.k_full[st]);
+    if (!wait_bar(&sh.v_empty[st], parity)) return;
+#pragma unroll
+    for (int i = 0; i < 2; ++i) store_chunk(smem + (2 + st) * kStageBytes, row + 8 * i, chunk, cur.v[i], cur.vs[i], ev);
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&sh.v_full[st]);
+    cur = nxt;
+  }
+}
+
+// ---- products --------------------------------------------------------------------------------------------------------
+__device__ __forceinline__ void issue_products(Shared& sh, uint8_t* smem, int groups, int ntiles) {
+  const bool leader = (threadIdx.x & 31) == 0;
+  const uint32_t tmem = sh.tmem;
+  const uint64_t k_desc = smem_desc(smem_u32(smem), 16), v_desc = smem_desc(smem_u32(smem) + 2 * kStageBytes, kPart / 2);
+  // S = Q Khi + Q Klo; 16 dims per product: 32 bytes inside a half of 64 dims
+  auto issue_s = [&](int g, int j) {
+    const uint32_t tm = tmem + g * kColsPerGroup;
+    const uint64_t d = k_desc + (j & 1) * (kStageBytes >> 4);
+#pragma unroll
+    for (int hl = 0; hl < 2; ++hl)
+#pragma unroll
+      for (int k = 0; k < 8; ++k)
+        mma_ts(tm + kColS, tm + kColQ + 8 * k, d + ((hl * kPart + (k >> 2) * (kPart / 2) + (k & 3) * 32) >> 4), kIdescS, hl + k > 0);
+    mma_commit(&sh.s_done[g]);
+  };
+  // O += Phi Vhi + Plo Vhi + Phi Vlo; 16 tokens per product: 2048 bytes
+  auto issue_o = [&](int g, int j) {
+    const uint32_t tm = tmem + g * kColsPerGroup;
+    const uint64_t d = v_desc + (j & 1) * (kStageBytes >> 4);
+#pragma unroll
+    for (int t = 0; t < 3; ++t)
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        mma_ts(tm + kColO, tm + kColS + (t == 1 ? 32 : 0) + 8 * k, d + (((t == 2 ? kPart : 0) + k * 2048) >> 4), kIdescO, j + t + k > 0);
+    mma_commit(&sh.o_done[g]);
+  };
+  if (!wait_bar(&sh.k_full[0], 0)) return;
+  fence_after();
+  if (leader) {
+    for (int g = 0; g < groups; ++g) issue_s(g, 0);
+    mma_commit(&sh.k_empty[0]);
+  }
+  for (int j = 0; j < ntiles; ++j) {
+    const bool more = j + 1 < ntiles;
+    for (int g = 0; g < groups; ++g) {
+      if (g == 0 && !wait_bar(&sh.v_full[j & 1], (j >> 1) & 1)) return;
+      if (g == 0 && more && !wait_bar(&sh.k_full[(j + 1) & 1], ((j + 1) >> 1) & 1)) return;
+      if (!wait_bar(&sh.p_ready[g], j & 1)) return;
+      fence_after();
+      if (leader) {
+        issue_o(g, j);
+        if (g == groups - 1) mma_commit(&sh.v_empty[j & 1]);
+        if (more) {
+          issue_s(g, j + 1);
+          if (g == groups - 1) mma_commit(&sh.k_empty[(j + 1) & 1]);
+        }
+      }
+      __syncwarp();
+    }
+  }
+}
+
+// ---- softmax ---------------------------------------------------------------------------------------------------------
+// 128 dims of a query row in the caller's 16-bit type, two per word
+__device__ __forceinline__ void load_query_row(const lq_int4_prefill_args& a, int64_t base, bool vec, uint32_t (&raw)[64]) {
+  if (vec) {
+    const uint4* src = reinterpret_cast<const uint4*>(static_cast<const uint16_t*>(a.q) + base);
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      const uint4 v = __ldg(src + i);
+      raw[4 * i] = v.x; raw[4 * i + 1] = v.y; raw[4 * i + 2] = v.z; raw[4 * i + 3] = v.w;
+    }
+  } else {
+    const uint16_t* src = static_cast<const uint16_t*>(a.q) + base;
+#pragma unroll
+    for (int i = 0; i < 64; ++i) raw[i] = src[2 * i * a.q_stride[3]] | (static_cast<uint32_t>(src[(2 * i + 1) * a.q_stride[3]]) << 16);
+  }
+}
+__device__ __forceinline__ float2 unpack16x2(uint32_t w, bool bf16) {
+  if (bf16) return make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xFFFF0000u));
+  return __half22float2(*reinterpret_cast<const __half2*>(&w));
+}
+__device__ __forceinline__ float max3(float a, float b, float c) { return fmaxf(fmaxf(a, b), c); }
+
+// Query row -> fp16 in TMEM, its largest value brought to [2^14, 2^15); returns the factor of a product of this row,
+// 2^Eq log2(e) / sqrt(128)
+__device__ __forceinline__ float load_query(const lq_int4_prefill_args& a, int64_t base, bool live, uint32_t tm_q) {
+  uint32_t raw[64];
+  const bool bf16 = a.dtype == LQ_BF16;
+  if (live) {
+    load_query_row(a, base, a.q_stride[3] == 1 && ((reinterpret_cast<uintptr_t>(a.q) + 2 * base) & 15) == 0, raw);
+  } else {
+#pragma unroll
+    for (int i = 0; i < 64; ++i) raw[i] = 0u;
+  }
+  float amax = 0.0f;
+#pragma unroll
+  for (int i = 0; i < 64; ++i) {
+    const float2 v = unpack16x2(raw[i], bf16);
+    amax = max3(amax, fabsf(v.x), fabsf(v.y));
+  }
+  int field = static_cast<int>(__float_as_uint(amax) >> 23);
+  field = field == 0 ? 141 : min(max(field, 15), 254);  // a row of zeros keeps the factor 1
+  const float to_half = __uint_as_float(static_cast<uint32_t>(268 - field) << 23);
+#pragma unroll
+  for (int half = 0; half < 2; ++half) {
+    uint32_t q[32];
+#pragma unroll
+    for (int w = 0; w < 8; ++w) {  // word of eight dims: pairs (0,4) (1,5) (2,6) (3,7)
+      float d[8];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float2 v = unpack16x2(raw[32 * half + 4 * w + i], bf16);
+        d[2 * i] = v.x * to_half;
+        d[2 * i + 1] = v.y * to_half;
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) q[4 * w + i] = pack_half2(d[i], d[i + 4]);
+    }
+    tmem_store32(tm_q + 32 * half, q);
+  }
+  tmem_wait_store();
+  return __uint_as_float(static_cast<uint32_t>(field - 14) << 23) * (1.4426950408889634f * 0.08838834764831845f);
+}
+
+__device__ __forceinline__ void store_output(const lq_int4_prefill_args& a, int64_t ob, uint32_t tm_o, float inv, bool live) {
+  const bool vec = a.out_stride[3] == 1 && ((reinterpret_cast<uintptr_t>(a.out) + 2 * ob) & 15) == 0;
+#pragma unroll 1
+  for (int q = 0; q < 4; ++q) {
+    uint32_t o[32];
+    tmem_load32(o, tm_o + 32 * q);
+    if (!live) continue;
+#pragma unroll
+    for (int w = 0; w < 4; ++w) {
+      float d[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) d[(i >> 1) + 4 * (i & 1)] = __uint_as_float(o[8 * w + i]) * inv;
+      const int dim = 32 * q + 8 * w;
+      if (vec) {
+        uint32_t v[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          if (a.dtype == LQ_BF16) {
+            const __nv_bfloat162 r = __floats2bfloat162_rn(d[2 * i], d[2 * i + 1]);
+            v[i] = *reinterpret_cast<const uint32_t*>(&r);
+          } else {
+            v[i] = pack_half2(d[2 * i], d[2 * i + 1]);
+          }
+        }
+        *reinterpret_cast<uint4*>(static_cast<uint16_t*>(a.out) + ob + dim) = make_uint4(v[0], v[1], v[2], v[3]);
+      } else {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) store_from_float(a.out, ob + (dim + i) * a.out_stride[3], a.dtype, d[i]);
+      }
+    }
+  }
+}
+
+// One row of scores, a tile at a time: S -> P in place, running maximum and sum.
+__device__ __forceinline__ void softmax_rows(const Params& p, Shared& sh, int b, int kvh, int pos0, int ntiles, float cq) {
+  const lq_int4_prefill_args& a = p.a;
+  const int group = threadIdx.x >> 7, warp = (threadIdx.x >> 5) & 3, lane = threadIdx.x & 31;
+  const int row = warp * 32 + lane;  // = TMEM lane
+  const int pos = pos0 + ((group * kGroupRows + row) >> p.ratio_log2);
+  const int limit = a.first_len + min(pos, a.q_len - 1);  // tokens this row sees
+  // the tokens that every row of the warp sees
+  const int warp_limit = a.first_len + min(pos0 + ((group * kGroupRows + warp * 32) >> p.ratio_log2), a.q_len - 1);
+  const uint32_t tm = sh.tmem + group * kColsPerGroup + (static_cast<uint32_t>(warp * 32) << 16);
+  float m_run = 0.0f, l_run = 0.0f;
+  for (int j = 0; j < ntiles; ++j) {
+    const int tok0 = j * kTok, f = j & 3;
+    if (!wait_bar(&sh.s_done[group], j & 1)) return;
+    fence_after();
+    uint32_t s[64];
+    tmem_load64(s, tm + kColS);
+    if (tok0 + kTok > warp_limit) {
+#pragma unroll
+      for (int i = 0; i < 64; ++i)
+        if (tok0 + i >= limit) s[i] = 0xFF800000u;  // -inf
+    }
+    float cw[4], ev[4], mt[4];
+#pragma unroll
+    for (int w = 0; w < 4; ++w) {
+      cw[w] = fmaxf(cq * sh.k_factor[f][w], 1.17549435e-38f);  // never 0: -inf * 0 would be NaN
+      ev[w] = sh.v_exp[f][w];
+      const auto at = [&](int i) { return __uint_as_float(s[16 * w + i]); };
+      const float m0 = max3(at(0), at(1), at(2)), m1 = max3(at(3), at(4), at(5)), m2 = max3(at(6), at(7), at(8));
+      const float m3 = max3(at(9), at(10), at(11)), m4 = max3(at(12), at(13), at(14));
+      mt[w] = fmaf(max3(max3(m0, m1, m2), max3(m3, m4, at(15)), m2), cw[w], ev[w]);
+    }
+    const float m_tile = fmaxf(fmaxf(mt[0], mt[1]), fmaxf(mt[2], mt[3]));
+    if (j == 0) {
+      m_run = m_tile;  // every row sees token 0
+    } else if (__any_sync(0xFFFFFFFFu, m_tile > m_run + kSlack)) {
+      // rare: the running sums of this warp's rows move to a larger maximum.  The products into O have to be done.
+      if (!wait_bar(&sh.o_done[group], (j - 1) & 1)) return;
+      fence_after();
+      const float m_new = fmaxf(m_run, m_tile), alpha = exp2f(m_run - m_new);
+      m_run = m_new;
+      l_run *= alpha;
+#pragma unroll 1
+      for (int q = 0; q < 4; ++q) {
+        uint32_t o[32];
+        tmem_load32(o, tm + kColO + 32 * q);
+#pragma unroll
+        for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+        tmem_store32(tm + kColO + 32 * q, o);
+      }
+    }
+#pragma unroll
+    for (int w = 0; w < 4; ++w) {
+      const float off = ev[w] - m_run;
+      float2 sum = make_float2(0.0f, 0.0f);
+      uint32_t hi[8], lo[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const float2 x = __ffma2_rn(make_float2(__uint_as_float(s[16 * w + 2 * i]), __uint_as_float(s[16 * w + 2 * i + 1])), make_float2(cw[w], cw[w]),
+                                    make_float2(off, off));
+        const float2 pr = make_float2(mma::fast_exp2(x.x), mma::fast_exp2(x.y));
+        sum = __fadd2_rn(sum, pr);
+        // leading 11 bits by truncation (exact in fp16), the rest rounded to fp16
+        const float2 top = make_float2(__uint_as_float(__float_as_uint(pr.x) & 0xFFFFE000u), __uint_as_float(__float_as_uint(pr.y) & 0xFFFFE000u));
+        const float2 rest = __ffma2_rn(top, make_float2(-1.0f, -1.0f), pr);
+        hi[i] = pack_half2(top.x, top.y);
+        lo[i] = pack_half2(rest.x, rest.y);
+      }
+      tmem_store8(tm + kColS + 8 * w, hi);
+      tmem_store8(tm + kColS + 32 + 8 * w, lo);
+      l_run = fmaf(sum.x + sum.y, sh.v_inv[f][w], l_run);
+    }
+    tmem_wait_store();
+    fence_before();
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&sh.p_ready[group]);
+  }
+  if (!wait_bar(&sh.o_done[group], (ntiles - 1) & 1)) return;
+  fence_after();
+  const int head = (kvh << p.ratio_log2) + (row & ((1 << p.ratio_log2) - 1));
+  const int64_t ob = b * a.out_stride[0] + head * a.out_stride[1] + static_cast<int64_t>(pos) * a.out_stride[2];
+  store_output(a, ob, tm + kColO, 1.0f / l_run, pos < a.q_len);
+}
+
+// Heaviest row blocks first: a block's work grows with its last position, and the tail of the grid is then made of short ones.
+__global__ void __launch_bounds__(kThreads, 1) int4_prefill_kernel(const Params p) {
+  extern __shared__ uint8_t smem_raw[];
+  __shared__ Shared sh;
+  const lq_int4_prefill_args& a = p.a;
+  const int bh = a.cache.batch * a.cache.kv_heads;
+  const int qb = p.nqb - 1 - static_cast<int>(blockIdx.x) / bh, rest = static_cast<int>(blockIdx.x) % bh;
+  const int b = rest / a.cache.kv_heads, kvh = rest % a.cache.kv_heads;
+  const int pos_per_cta = kCtaRows >> p.ratio_log2;
+  const int pos0 = qb * pos_per_cta;
+  const int groups = pos0 + (pos_per_cta >> 1) < a.q_len ? 2 : 1;  // softmax groups with a position of their own
+  const int ntiles = (a.first_len + min(pos0 + pos_per_cta - 1, a.q_len - 1) + kTok - 1) / kTok;
+  uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
+  const int warp = threadIdx.x >> 5;
+  if (warp == 12) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(&sh.tmem)) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+  }
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(&sh.k_full[i], 4);
+      mbar_init(&sh.v_full[i], 4);
+      mbar_init(&sh.k_empty[i], 1);
+      mbar_init(&sh.v_empty[i], 1);
+      mbar_init(&sh.s_done[i], 1);
+      mbar_init(&sh.p_ready[i], 4);
+      mbar_init(&sh.o_done[i], 1);
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  fence_before();
+  __syncthreads();
+  fence_after();
+  if (warp >= 8) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 88;");
+    if (warp < 12) {
+      asm volatile("barrier.cta.arrive 1, %0;" ::"n"(kWorkers) : "memory");
+      unpack_tiles(p, sh, smem, b, kvh, ntiles);
+    } else if (warp == 12) {
+      asm volatile("barrier.cta.sync 1, %0;" ::"n"(kWorkers) : "memory");  // Q is in TMEM
+      fence_after();
+      issue_products(sh, smem, groups, ntiles);
+    }
+  } else {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 168;");
+    float cq = 0.0f;
+    if ((warp >> 2) < groups) {  // the unpacking warps start on the first tiles while the query rows travel
+      const int row = threadIdx.x & 127, pos = pos0 + (static_cast<int>(threadIdx.x) >> p.ratio_log2);
+      const int head = (kvh << p.ratio_log2) + (row & ((1 << p.ratio_log2) - 1));
+      const int64_t base = b * a.q_stride[0] + head * a.q_stride[1] + static_cast<int64_t>(pos) * a.q_stride[2];
+      cq = load_query(a, base, pos < a.q_len, sh.tmem + (warp >> 2) * kColsPerGroup + (static_cast<uint32_t>((warp & 3) * 32) << 16) + kColQ);
+      fence_before();
+    }
+    asm volatile("barrier.cta.arrive 1, %0;" ::"n"(kWorkers) : "memory");
+    if ((warp >> 2) < groups) softmax_rows(p, sh, b, kvh, pos0, ntiles, cq);
+  }
+  fence_before();
+  __syncthreads();
+  if (warp == 12) {
+    fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(sh.tmem));
+  }
+}
+
+}  // namespace prefill
+}  // namespace lq

@@ -387,3 +387,29 @@ def test_prefill_matches_reference_kernel_fixture(golden_dir, name):
     out = m._prefill_attention(t(g["q"], torch.float32), cache, hq // hkv, gs)
     assert_out_close(out, g["out"])
     assert_out_close(m._prefill_attention(t(g["q"], torch.bfloat16), cache, hq // hkv, gs), g["out"])
+
+
+@pytest.mark.parametrize("ratio,tq,first,k_size,v_size", [
+    (4, 32, 1, 1.0, 1.0), (4, 33, 32, 1.0, 1.0), (4, 64, 1, 1.0, 1.0), (4, 65, 64, 1.0, 1.0), (8, 17, 1000, 1.0, 1.0), (1, 257, 3, 1.0, 1.0),
+    (4, 70, 130, 3e-5, 1e5), (4, 70, 130, 40.0, 1e-7), (2, 130, 1, 1e-20, 1e20), (4, 40, 200, "mixed", "mixed"), (4, 40, 200, 0.0, 0.0)])
+def test_prefill_tensor_core_edges(ratio, tq, first, k_size, v_size):
+    """16-bit queries: rows and tokens around the tile edges (32 / 64 positions, 64 tokens), and magnitudes that the powers of two
+    taken out of K, V and Q have to carry; "mixed" changes the magnitude from token to token."""
+    m = ia()
+    b, hkv, gs = 2, 2, 32
+    total = first + tq - 1
+    k, v = make_kv(51 + tq, b, hkv, total)
+    sizes = np.where(np.arange(total) % 7 == 3, 30.0, np.where(np.arange(total) % 5 == 1, 1e-3, 1.0))[:, None]
+    k, v = (bf16r(x * (sizes if size == "mixed" else size)) for x, size in ((k, k_size), (v, v_size)))
+    q = bf16r(np.random.default_rng(tq).standard_normal((b, hkv * ratio, tq, 128)) * 0.5)
+    cache = fill_cache(m, k, v, gs, capacity=(total + 15) // 16 * 16)
+    ref = oracle.int4_prefill_attention(q, *cache_np(cache), first, gs)
+    for dtype in (torch.bfloat16, torch.float16):
+        if dtype == torch.float16 and v_size == 1e20:
+            continue  # beyond the output type
+        out = m._prefill_attention(t(q, dtype), cache, ratio, gs, first_len=first)
+        if dtype == torch.float16 and v_size in (1e-7, 1e5):  # subnormal outputs / outputs past 65504
+            continue
+        assert_out_close(out, ref)
+    from layer_quant_b200 import _lib
+    assert _lib.device_status() == 0
