@@ -7,7 +7,7 @@
 //   12        issues the tcgen05.mma of both groups: O += P V of a tile, then S of the group's next tile into the columns
 //             that P has just been read from (the tensor pipe takes one thread's products in order)
 // Registers: launched with 128 a thread; the softmax groups raise theirs to 168, the other two groups go down to 88.
-// TMEM (512 columns, 256 per group): O 128, Q 64 (fp16, A operand), S 64; P replaces S (A operand).
+// TMEM (all 512 columns, so addresses start at 0; 256 per group): O 128, Q 64 (fp16, A operand), S 64; P replaces S (A operand).
 //
 // Precision.  A dequantised value n * scale (n in [-8, 7]) is held as two fp16 numbers: the leading 8 bits of the scale
 // times n, exact in fp16, and the rest of the scale times n, rounded to fp16: 2^-20 relative in all.  P is split
@@ -80,16 +80,21 @@ __device__ __forceinline__ void tmem_wait_store() { asm volatile("tcgen05.wait::
 __device__ __forceinline__ void fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
-// D[128 x N] (+)= A B, A from TMEM, B from shared memory, fp16 in, fp32 accumulate
-__device__ __forceinline__ void mma_ts(uint32_t d, uint32_t a, uint64_t b_desc, uint32_t idesc, bool accumulate) {
+// D[128 x N] (+)= A B, A from TMEM, B from shared memory, fp16 in, fp32 accumulate.  Called by a whole warp and predicated to
+// its leader: in a divergent branch every operand would go through vector registers (74 cycles per product, longer than it runs).
+__device__ __forceinline__ void mma_ts(uint32_t leader, uint32_t d, uint32_t a, uint64_t b_desc, uint32_t idesc, bool accumulate) {
   asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d),
-      "r"(a), "l"(b_desc), "r"(idesc), "r"(accumulate ? 1u : 0u)
+      "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d),
+      "r"(a), "l"(b_desc), "r"(idesc), "r"(accumulate ? 1u : 0u), "r"(leader)
       : "memory");
 }
-__device__ __forceinline__ void mma_commit(uint64_t* bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
+__device__ __forceinline__ void mma_commit(uint32_t leader, uint64_t* bar) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %1, 0;\n\t"
+      "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(smem_u32(bar)),
+      "r"(leader)
+      : "memory");
 }
 // fp16 inputs, fp32 accumulators, M = 128; K tile: N = 64 tokens, dims contiguous; V tile: N = 128 dims, dims contiguous (N-major)
 constexpr uint32_t kIdescS = (1u << 4) | ((64u / 8) << 17) | ((128u / 16) << 24);
@@ -102,9 +107,11 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo) {
 }
 
 struct Shared {
-  uint64_t k_full[2], k_empty[2], v_full[2], v_empty[2], s_done[2], p_ready[2], o_done[2];
-  // Per 16 tokens: 2^Ek, Ev and 2^-Ev.  Four tiles deep: a K stage is free again when its products are done, which can be before
-  // a slow thread has read the factors; tile j + 4 comes after the products of j + 2, and those come after that read.
+  // Few barriers: the thread that issues products runs only a few of them ahead of the tensor pipe, so every wait and commit of
+  // its loop costs tensor time.  Unit j of the unpacking warps is V of tile j and K of tile j + 1, what the products of
+  // iteration j read; s_done of a tile also says that all products before it are done, O of the tile before among them.
+  uint64_t k_first, full[2], empty[2], s_done[2], p_ready[2];
+  // Per 16 tokens: 2^Ek, Ev and 2^-Ev of the tile, four tiles deep (they are written a unit ahead of V)
   float k_factor[4][4], v_exp[4][4], v_inv[4][4];
   uint32_t tmem;
 };
@@ -138,12 +145,6 @@ __device__ __forceinline__ void unpack8(uint32_t x, __half2 (&n)[4]) {
   n[2] = __hadd2(*reinterpret_cast<const __half2*>(&b2), off);
   n[3] = __hfma2(*reinterpret_cast<const __half2*>(&b3), sixteenth, off16);
 }
-
-// What a lane of the unpacking warps holds of a tile: 16 bytes (32 dims) of two tokens, K and V, and their scales
-struct RawTile {
-  uint4 k[2], v[2];
-  float ks[2], vs[2];
-};
 
 // The exponent that brings the largest of a warp's scales to [2^11, 2^12): n * scale then stays below 2^15
 __device__ __forceinline__ int scale_exponent(float a, float b) {
@@ -187,95 +188,122 @@ __device__ __forceinline__ void unpack_tiles(const Params& p, Shared& sh, uint8_
   const uint8_t* vp = c.v_packed + b * c.vp_stride[0] + kvh * c.vp_stride[1] + chunk * 16;
   const float* ks = c.k_scale + b * c.ks_stride[0] + kvh * c.ks_stride[1] + grp;
   const float* vs = c.v_scale + b * c.vs_stride[0] + kvh * c.vs_stride[1] + grp;
-  auto fetch = [&](int tile, RawTile& r) {
+  // 16 bytes (32 dims) of this lane's two tokens of a tile, and their scales
+  auto fetch = [&](const uint8_t* codes, int tile, uint4 (&raw)[2]) {
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
       const int64_t tok = static_cast<int64_t>(tile) * kTok + row + 8 * i;
-      const bool ok = tok < p.kv_len;
-      r.k[i] = ok ? __ldg(reinterpret_cast<const uint4*>(kp + tok * 64)) : make_uint4(0, 0, 0, 0);
-      r.v[i] = ok ? __ldg(reinterpret_cast<const uint4*>(vp + tok * 64)) : make_uint4(0, 0, 0, 0);
-      r.ks[i] = ok ? __ldg(ks + (tok << groups_log2)) : 0.0f;
-      r.vs[i] = ok ? __ldg(vs + (tok << groups_log2)) : 0.0f;
+      raw[i] = tok < p.kv_len ? __ldg(reinterpret_cast<const uint4*>(codes + tok * 64)) : make_uint4(0, 0, 0, 0);
     }
   };
-  RawTile cur, nxt;
-  fetch(0, cur);
-  for (int j = 0; j < ntiles; ++j) {
-    if (j + 1 < ntiles) fetch(j + 1, nxt);
-    const int st = j & 1;
-    const uint32_t parity = ((j >> 1) & 1) ^ 1;  // the first use of a stage finds it empty
-    const int ek = scale_exponent(cur.ks[0], cur.ks[1]), ev = scale_exponent(cur.vs[0], cur.vs[1]);
-    if (!wait_bar(&sh.k_empty[st], parity)) return;
-    if (lane == 0) {
-      sh.k_factor[j & 3][warp] = pow2_of(ek);
-      sh.v_exp[j & 3][warp] = static_cast<float>(ev);
-      sh.v_inv[j & 3][warp] = pow2_of(-ev);
+  auto fetch_scales = [&](const float* scales, int tile, float (&sc)[2]) {
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int64_t tok = static_cast<int64_t>(tile) * kTok + row + 8 * i;
+      sc[i] = tok < p.kv_len ? __ldg(scales + (tok << groups_log2)) : 0.0f;
     }
+  };
+  auto publish = [&](int tile, int ek, int ev) {
+    if (lane == 0) {
+      sh.k_factor[tile & 3][warp] = pow2_of(ek);
+      sh.v_exp[tile & 3][warp] = static_cast<float>(ev);
+      sh.v_inv[tile & 3][warp] = pow2_of(-ev);
+    }
+  };
+  auto store = [&](int stage, const uint4 (&raw)[2], const float (&sc)[2], int e) {
 #pragma unroll
-    for (int i = 0; i < 2; ++i) store_chunk(smem + st * kStageBytes, row + 8 * i, chunk, cur.k[i], cur.ks[i], ek);
+    for (int i = 0; i < 2; ++i) store_chunk(smem + stage * kStageBytes, row + 8 * i, chunk, raw[i], sc[i], e);
+  };
+  auto arrive = [&](uint64_t* bar) {
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     __syncwarp();
-    if (lane == 0) mbar_arrive(&sh.k_full[st]);
-    if (!wait_bar(&sh.v_empty[st], parity)) return;
+    if (lane == 0) mbar_arrive(bar);
+  };
+  uint4 k[2], v[2], k_next[2], v_next[2];
+  float ks_cur[2], vs_cur[2], vs_ahead[2], ks_next[2], vs_next[2];  // scales of k and v above; of V one tile further
+  fetch(kp, 0, k);
+  fetch_scales(ks, 0, ks_cur);
+  fetch_scales(vs, 0, vs_cur);
+  fetch(vp, 0, v);
+  fetch(kp, 1, k_next);
+  fetch_scales(ks, 1, ks_next);
+  fetch_scales(vs, 1, vs_ahead);
+  int ev = scale_exponent(vs_cur[0], vs_cur[1]);
+  {
+    const int ek = scale_exponent(ks_cur[0], ks_cur[1]);
+    publish(0, ek, ev);
+    store(0, k, ks_cur, ek);
+    arrive(&sh.k_first);
+  }
+  for (int j = 0; j < ntiles; ++j) {
 #pragma unroll
-    for (int i = 0; i < 2; ++i) store_chunk(smem + (2 + st) * kStageBytes, row + 8 * i, chunk, cur.v[i], cur.vs[i], ev);
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    __syncwarp();
-    if (lane == 0) mbar_arrive(&sh.v_full[st]);
-    cur = nxt;
+    for (int i = 0; i < 2; ++i) {
+      k[i] = k_next[i];
+      ks_cur[i] = ks_next[i];
+    }
+    fetch(kp, j + 2, k_next);  // past the last tile: zeros, not loaded
+    fetch_scales(ks, j + 2, ks_next);
+    fetch(vp, j + 1, v_next);
+    fetch_scales(vs, j + 2, vs_next);
+    const int ek = scale_exponent(ks_cur[0], ks_cur[1]), ev_ahead = scale_exponent(vs_ahead[0], vs_ahead[1]);
+    // iteration j - 2 is done (its last products are S of tile j - 1); unit 0 finds its stages empty, unit 1 waits for S of tile 0
+    if (!wait_bar(&sh.empty[j & 1], ((j >> 1) ^ j ^ 1) & 1)) return;
+    publish(j + 1, ek, ev_ahead);
+    store(2 + (j & 1), v, vs_cur, ev);
+    if (j + 1 < ntiles) store((j + 1) & 1, k, ks_cur, ek);
+    arrive(&sh.full[j & 1]);
+    ev = ev_ahead;
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      v[i] = v_next[i];
+      vs_cur[i] = vs_ahead[i];
+      vs_ahead[i] = vs_next[i];
+    }
   }
 }
 
 // ---- products --------------------------------------------------------------------------------------------------------
 __device__ __forceinline__ void issue_products(Shared& sh, uint8_t* smem, int groups, int ntiles) {
-  const bool leader = (threadIdx.x & 31) == 0;
-  const uint32_t tmem = sh.tmem;
+  const uint32_t leader = (threadIdx.x & 31) == 0;
   const uint64_t k_desc = smem_desc(smem_u32(smem), 16), v_desc = smem_desc(smem_u32(smem) + 2 * kStageBytes, kPart / 2);
   // S = Q Khi + Q Klo; 16 dims per product: 32 bytes inside a half of 64 dims
   auto issue_s = [&](int g, int j) {
-    const uint32_t tm = tmem + g * kColsPerGroup;
+    const uint32_t tm = g * kColsPerGroup;
     const uint64_t d = k_desc + (j & 1) * (kStageBytes >> 4);
 #pragma unroll
     for (int hl = 0; hl < 2; ++hl)
 #pragma unroll
       for (int k = 0; k < 8; ++k)
-        mma_ts(tm + kColS, tm + kColQ + 8 * k, d + ((hl * kPart + (k >> 2) * (kPart / 2) + (k & 3) * 32) >> 4), kIdescS, hl + k > 0);
-    mma_commit(&sh.s_done[g]);
+        mma_ts(leader, tm + kColS, tm + kColQ + 8 * k, d + ((hl * kPart + (k >> 2) * (kPart / 2) + (k & 3) * 32) >> 4), kIdescS, hl + k > 0);
   };
   // O += Phi Vhi + Plo Vhi + Phi Vlo; 16 tokens per product: 2048 bytes
   auto issue_o = [&](int g, int j) {
-    const uint32_t tm = tmem + g * kColsPerGroup;
+    const uint32_t tm = g * kColsPerGroup;
     const uint64_t d = v_desc + (j & 1) * (kStageBytes >> 4);
 #pragma unroll
     for (int t = 0; t < 3; ++t)
 #pragma unroll
       for (int k = 0; k < 4; ++k)
-        mma_ts(tm + kColO, tm + kColS + (t == 1 ? 32 : 0) + 8 * k, d + (((t == 2 ? kPart : 0) + k * 2048) >> 4), kIdescO, j + t + k > 0);
-    mma_commit(&sh.o_done[g]);
+        mma_ts(leader, tm + kColO, tm + kColS + (t == 1 ? 32 : 0) + 8 * k, d + (((t == 2 ? kPart : 0) + k * 2048) >> 4), kIdescO, j + t + k > 0);
   };
-  if (!wait_bar(&sh.k_full[0], 0)) return;
+  if (!wait_bar(&sh.k_first, 0)) return;
   fence_after();
-  if (leader) {
-    for (int g = 0; g < groups; ++g) issue_s(g, 0);
-    mma_commit(&sh.k_empty[0]);
+  for (int g = 0; g < groups; ++g) {
+    issue_s(g, 0);
+    mma_commit(leader, &sh.s_done[g]);
   }
+  mma_commit(leader, &sh.empty[1]);
   for (int j = 0; j < ntiles; ++j) {
     const bool more = j + 1 < ntiles;
+    if (!wait_bar(&sh.full[j & 1], (j >> 1) & 1)) return;
     for (int g = 0; g < groups; ++g) {
-      if (g == 0 && !wait_bar(&sh.v_full[j & 1], (j >> 1) & 1)) return;
-      if (g == 0 && more && !wait_bar(&sh.k_full[(j + 1) & 1], ((j + 1) >> 1) & 1)) return;
       if (!wait_bar(&sh.p_ready[g], j & 1)) return;
       fence_after();
-      if (leader) {
-        issue_o(g, j);
-        if (g == groups - 1) mma_commit(&sh.v_empty[j & 1]);
-        if (more) {
-          issue_s(g, j + 1);
-          if (g == groups - 1) mma_commit(&sh.k_empty[(j + 1) & 1]);
-        }
-      }
-      __syncwarp();
+      issue_o(g, j);
+      if (more) issue_s(g, j + 1);
+      mma_commit(leader, &sh.s_done[g]);
     }
+    mma_commit(leader, &sh.empty[j & 1]);
   }
 }
 
@@ -384,7 +412,7 @@ __device__ __forceinline__ void softmax_rows(const Params& p, Shared& sh, int b,
   const int limit = a.first_len + min(pos, a.q_len - 1);  // tokens this row sees
   // the tokens that every row of the warp sees
   const int warp_limit = a.first_len + min(pos0 + ((group * kGroupRows + warp * 32) >> p.ratio_log2), a.q_len - 1);
-  const uint32_t tm = sh.tmem + group * kColsPerGroup + (static_cast<uint32_t>(warp * 32) << 16);
+  const uint32_t tm = group * kColsPerGroup + (static_cast<uint32_t>(warp * 32) << 16);
   float m_run = 0.0f, l_run = 0.0f;
   for (int j = 0; j < ntiles; ++j) {
     const int tok0 = j * kTok, f = j & 3;
@@ -411,9 +439,7 @@ __device__ __forceinline__ void softmax_rows(const Params& p, Shared& sh, int b,
     if (j == 0) {
       m_run = m_tile;  // every row sees token 0
     } else if (__any_sync(0xFFFFFFFFu, m_tile > m_run + kSlack)) {
-      // rare: the running sums of this warp's rows move to a larger maximum.  The products into O have to be done.
-      if (!wait_bar(&sh.o_done[group], (j - 1) & 1)) return;
-      fence_after();
+      // rare: the running sums of this warp's rows move to a larger maximum (the products into O of the tile before are done)
       const float m_new = fmaxf(m_run, m_tile), alpha = exp2f(m_run - m_new);
       m_run = m_new;
       l_run *= alpha;
@@ -452,7 +478,7 @@ __device__ __forceinline__ void softmax_rows(const Params& p, Shared& sh, int b,
     __syncwarp();
     if (lane == 0) mbar_arrive(&sh.p_ready[group]);
   }
-  if (!wait_bar(&sh.o_done[group], (ntiles - 1) & 1)) return;
+  if (!wait_bar(&sh.s_done[group], ntiles & 1)) return;
   fence_after();
   const int head = (kvh << p.ratio_log2) + (row & ((1 << p.ratio_log2) - 1));
   const int64_t ob = b * a.out_stride[0] + head * a.out_stride[1] + static_cast<int64_t>(pos) * a.out_stride[2];
@@ -478,14 +504,12 @@ __global__ void __launch_bounds__(kThreads, 1) int4_prefill_kernel(const Params 
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
   if (threadIdx.x == 0) {
+    mbar_init(&sh.k_first, 4);
     for (int i = 0; i < 2; ++i) {
-      mbar_init(&sh.k_full[i], 4);
-      mbar_init(&sh.v_full[i], 4);
-      mbar_init(&sh.k_empty[i], 1);
-      mbar_init(&sh.v_empty[i], 1);
+      mbar_init(&sh.full[i], 4);
+      mbar_init(&sh.empty[i], 1);
       mbar_init(&sh.s_done[i], 1);
       mbar_init(&sh.p_ready[i], 4);
-      mbar_init(&sh.o_done[i], 1);
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -509,7 +533,7 @@ __global__ void __launch_bounds__(kThreads, 1) int4_prefill_kernel(const Params 
       const int row = threadIdx.x & 127, pos = pos0 + (static_cast<int>(threadIdx.x) >> p.ratio_log2);
       const int head = (kvh << p.ratio_log2) + (row & ((1 << p.ratio_log2) - 1));
       const int64_t base = b * a.q_stride[0] + head * a.q_stride[1] + static_cast<int64_t>(pos) * a.q_stride[2];
-      cq = load_query(a, base, pos < a.q_len, sh.tmem + (warp >> 2) * kColsPerGroup + (static_cast<uint32_t>((warp & 3) * 32) << 16) + kColQ);
+      cq = load_query(a, base, pos < a.q_len, (warp >> 2) * kColsPerGroup + (static_cast<uint32_t>((warp & 3) * 32) << 16) + kColQ);
       fence_before();
     }
     asm volatile("barrier.cta.arrive 1, %0;" ::"n"(kWorkers) : "memory");
