@@ -80,21 +80,24 @@ __device__ __forceinline__ void tmem_wait_store() { asm volatile("tcgen05.wait::
 __device__ __forceinline__ void fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
-// D[128 x N] (+)= A B, A from TMEM, B from shared memory, fp16 in, fp32 accumulate.  Called by a whole warp and predicated to
-// its leader: in a divergent branch every operand would go through vector registers (74 cycles per product, longer than it runs).
-__device__ __forceinline__ void mma_ts(uint32_t leader, uint32_t d, uint32_t a, uint64_t b_desc, uint32_t idesc, bool accumulate) {
+// One thread of a converged warp.  The compiler knows that the branch on it is taken by one thread and keeps the operands of the
+// products in uniform registers: 16 cycles of issue per product, where a branch on the lane index costs 54 to 64, longer
+// than a product of 64 columns runs (32).
+__device__ __forceinline__ bool elect_one() {
+  uint32_t r;
+  asm volatile("{\n\t.reg .pred q;\n\t.reg .b32 x;\n\telect.sync x|q, 0xFFFFFFFF;\n\tselp.u32 %0, 1, 0, q;\n\t}" : "=r"(r));
+  return r != 0;
+}
+// D[128 x N] (+)= A B, A from TMEM, B from shared memory, fp16 in, fp32 accumulate
+__device__ __forceinline__ void mma_ts(uint32_t d, uint32_t a, uint64_t b_desc, uint32_t idesc, bool accumulate) {
   asm volatile(
-      "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t"
-      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d),
-      "r"(a), "l"(b_desc), "r"(idesc), "r"(accumulate ? 1u : 0u), "r"(leader)
+      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d),
+      "r"(a), "l"(b_desc), "r"(idesc), "r"(accumulate ? 1u : 0u)
       : "memory");
 }
-__device__ __forceinline__ void mma_commit(uint32_t leader, uint64_t* bar) {
-  asm volatile(
-      "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %1, 0;\n\t"
-      "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(smem_u32(bar)),
-      "r"(leader)
-      : "memory");
+__device__ __forceinline__ void mma_commit(uint64_t* bar) {
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 // fp16 inputs, fp32 accumulators, M = 128; K tile: N = 64 tokens, dims contiguous; V tile: N = 128 dims, dims contiguous (N-major)
 constexpr uint32_t kIdescS = (1u << 4) | ((64u / 8) << 17) | ((128u / 16) << 24);
@@ -108,7 +111,7 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo) {
 
 struct Shared {
   // Few barriers: the thread that issues products runs only a few of them ahead of the tensor pipe, so every wait and commit of
-  // its loop costs tensor time.  Unit j of the unpacking warps is V of tile j and K of tile j + 1, what the products of
+  // its loop can cost tensor time.  Unit j of the unpacking warps is V of tile j and K of tile j + 1, what the products of
   // iteration j read; s_done of a tile also says that all products before it are done, O of the tile before among them.
   uint64_t k_first, full[2], empty[2], s_done[2], p_ready[2];
   // Per 16 tokens: 2^Ek, Ev and 2^-Ev of the tile, four tiles deep (they are written a unit ahead of V)
@@ -264,7 +267,6 @@ __device__ __forceinline__ void unpack_tiles(const Params& p, Shared& sh, uint8_
 
 // ---- products --------------------------------------------------------------------------------------------------------
 __device__ __forceinline__ void issue_products(Shared& sh, uint8_t* smem, int groups, int ntiles) {
-  const uint32_t leader = (threadIdx.x & 31) == 0;
   const uint64_t k_desc = smem_desc(smem_u32(smem), 16), v_desc = smem_desc(smem_u32(smem) + 2 * kStageBytes, kPart / 2);
   // S = Q Khi + Q Klo; 16 dims per product: 32 bytes inside a half of 64 dims
   auto issue_s = [&](int g, int j) {
@@ -274,7 +276,7 @@ __device__ __forceinline__ void issue_products(Shared& sh, uint8_t* smem, int gr
     for (int hl = 0; hl < 2; ++hl)
 #pragma unroll
       for (int k = 0; k < 8; ++k)
-        mma_ts(leader, tm + kColS, tm + kColQ + 8 * k, d + ((hl * kPart + (k >> 2) * (kPart / 2) + (k & 3) * 32) >> 4), kIdescS, hl + k > 0);
+        mma_ts(tm + kColS, tm + kColQ + 8 * k, d + ((hl * kPart + (k >> 2) * (kPart / 2) + (k & 3) * 32) >> 4), kIdescS, hl + k > 0);
   };
   // O += Phi Vhi + Plo Vhi + Phi Vlo; 16 tokens per product: 2048 bytes
   auto issue_o = [&](int g, int j) {
@@ -284,26 +286,32 @@ __device__ __forceinline__ void issue_products(Shared& sh, uint8_t* smem, int gr
     for (int t = 0; t < 3; ++t)
 #pragma unroll
       for (int k = 0; k < 4; ++k)
-        mma_ts(leader, tm + kColO, tm + kColS + (t == 1 ? 32 : 0) + 8 * k, d + (((t == 2 ? kPart : 0) + k * 2048) >> 4), kIdescO, j + t + k > 0);
+        mma_ts(tm + kColO, tm + kColS + (t == 1 ? 32 : 0) + 8 * k, d + (((t == 2 ? kPart : 0) + k * 2048) >> 4), kIdescO, j + t + k > 0);
   };
   if (!wait_bar(&sh.k_first, 0)) return;
   fence_after();
-  for (int g = 0; g < groups; ++g) {
-    issue_s(g, 0);
-    mma_commit(leader, &sh.s_done[g]);
+  if (elect_one()) {
+    for (int g = 0; g < groups; ++g) {
+      issue_s(g, 0);
+      mma_commit(&sh.s_done[g]);
+    }
+    mma_commit(&sh.empty[1]);
   }
-  mma_commit(leader, &sh.empty[1]);
+  __syncwarp();
   for (int j = 0; j < ntiles; ++j) {
     const bool more = j + 1 < ntiles;
     if (!wait_bar(&sh.full[j & 1], (j >> 1) & 1)) return;
     for (int g = 0; g < groups; ++g) {
       if (!wait_bar(&sh.p_ready[g], j & 1)) return;
       fence_after();
-      issue_o(g, j);
-      if (more) issue_s(g, j + 1);
-      mma_commit(leader, &sh.s_done[g]);
+      if (elect_one()) {
+        issue_o(g, j);
+        if (more) issue_s(g, j + 1);
+        mma_commit(&sh.s_done[g]);
+        if (g == groups - 1) mma_commit(&sh.empty[j & 1]);
+      }
+      __syncwarp();
     }
-    mma_commit(leader, &sh.empty[j & 1]);
   }
 }
 
