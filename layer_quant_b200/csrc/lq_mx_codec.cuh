@@ -43,6 +43,7 @@ struct MxRoundCtx {
   uint32_t wrap32;       // PHILOX_REF: counters are taken modulo 2^32 with a zero high word
   uint32_t step, layer;  // PHILOX_LAYERED
   const uint32_t* words; // SUPPLIED / SUPPLIED_FIXED: 16 words of this block
+  const PhiloxStream* stream = nullptr;  // the layered modes: where the caller carries the generator along, used instead of the counter
 };
 
 // 1.0f if a > b else 0.0f, as one FSET.
@@ -71,7 +72,8 @@ constexpr float kByteMagic = 49152.0f;  // 1.5 * 2^15: ulp 2^-8, mantissa bits 8
 //    FMA, q = floor(t) - 49152, i.e. stochastic rounding with an 8-bit uniform draw r8; q (two's
 //    complement) is byte 1 of t's bit pattern.  No clamp is needed: |h| / scale never exceeds
 //    M + 2^-9 (the few-ulp overshoot of the rounded log2 is orders of magnitude smaller).
-template <int BITS, int MODE>
+// PACKED_NIBBLES: codes[0..1] are the 16 nibbles as the packed MX4 layout stores them.
+template <int BITS, int MODE, bool PACKED_NIBBLES = false>
 __device__ __forceinline__ void mx_encode_block(const float (&h)[16], const unsigned int* __restrict__ cut_table,
                                                 const MxRoundCtx& ctx, const PhiloxKeys& keys, uint32_t (&codes)[4],
                                                 uint32_t& exp_byte, uint32_t& micro_bits) {
@@ -105,14 +107,16 @@ __device__ __forceinline__ void mx_encode_block(const float (&h)[16], const unsi
 #pragma unroll
     for (int qd = 0; qd < 4; ++qd) {
       const uint64_t c = ctx.counter + qd;
-      const Philox4 r = philox4x32_10(static_cast<uint32_t>(c), static_cast<uint32_t>(c >> 32), ctx.step, ctx.layer, keys);
+      const Philox4 r = ctx.stream ? ctx.stream->block(qd, keys)
+                                   : philox4x32_10(static_cast<uint32_t>(c), static_cast<uint32_t>(c >> 32), ctx.step, ctx.layer, keys);
       rnd[4 * qd] = r.w0; rnd[4 * qd + 1] = r.w1; rnd[4 * qd + 2] = r.w2; rnd[4 * qd + 3] = r.w3;
     }
   }
   uint32_t pw[4] = {0u, 0u, 0u, 0u};  // PHILOX_LAYERED: 16 random bytes, value i = byte i & 3 of word i >> 2
   if (MODE == LQ_ROUND_PHILOX_LAYERED) {
-    const Philox4 r = philox4x32_10(static_cast<uint32_t>(ctx.counter), static_cast<uint32_t>(ctx.counter >> 32), ctx.step,
-                                    ctx.layer, keys);
+    const Philox4 r = ctx.stream ? ctx.stream->block(0, keys)
+                                 : philox4x32_10(static_cast<uint32_t>(ctx.counter), static_cast<uint32_t>(ctx.counter >> 32), ctx.step,
+                                                 ctx.layer, keys);
     pw[0] = r.w0; pw[1] = r.w1; pw[2] = r.w2; pw[3] = r.w3;
   }
 
@@ -166,7 +170,15 @@ __device__ __forceinline__ void mx_encode_block(const float (&h)[16], const unsi
     }
   }
 #pragma unroll
-  for (int w = 0; w < 4; ++w) codes[w] = gather_byte1(tb[4 * w], tb[4 * w + 1], tb[4 * w + 2], tb[4 * w + 3]);
+  for (int w = 0; w < 4; ++w) {
+    if (!PACKED_NIBBLES) {
+      codes[w] = gather_byte1(tb[4 * w], tb[4 * w + 1], tb[4 * w + 2], tb[4 * w + 3]);
+    } else if (w < 2) {  // even values to the low nibbles, odd ones to the high
+      const uint32_t ev = gather_byte1(tb[8 * w], tb[8 * w + 2], tb[8 * w + 4], tb[8 * w + 6]);
+      const uint32_t od = gather_byte1(tb[8 * w + 1], tb[8 * w + 3], tb[8 * w + 5], tb[8 * w + 7]);
+      codes[w] = (ev & 0x0F0F0F0Fu) | ((od << 4) & 0xF0F0F0F0u);
+    }
+  }
   micro_bits = __float_as_uint(macc + 8388608.0f) & 0xFFu;
 }
 
@@ -175,21 +187,111 @@ __device__ __forceinline__ void mx_encode_block(const float (&h)[16], const unsi
 // Association as in the reference kernel (mamba_state_8b_kernel.py:158, dB = B * dt, then state * dA + dB * x):
 // dB rounded, t = dB * x rounded, then fma(h, dA, t), which is what a compiler that contracts the reference's
 // expression produces; the read-out keeps four partial sums over i mod 4, added as (y0 + y1) + (y2 + y3).
-__device__ __forceinline__ float mx_update_readout16(float (&hv)[16], const float (&Bv)[16], const float (&Cv)[16], float dA,
+// h is given as q * s with s a power of two: fma(h, dA, t) = fma(q, s dA, t), for s dA is exact.  sd: s dA of the pairs,
+// ONE: of the whole block (sd[0]).
+template <bool ONE>
+__device__ __forceinline__ float mx_update_readout16(float (&hv)[16], const float (&Bv)[16], const float (&Cv)[16], const float (&sd)[8],
                                                      float dt, float x) {
-  const float2 dA2 = make_float2(dA, dA), dt2 = make_float2(dt, dt), x2 = make_float2(x, x);
+  const float2 dt2 = make_float2(dt, dt), x2 = make_float2(x, x);
   float2 ya = make_float2(0.0f, 0.0f), yb = make_float2(0.0f, 0.0f);
 #pragma unroll
   for (int i = 0; i < 16; i += 4) {
+    const float s0 = sd[ONE ? 0 : i / 2], s1 = sd[ONE ? 0 : i / 2 + 1];
     const float2 t0 = __fmul2_rn(__fmul2_rn(make_float2(Bv[i], Bv[i + 1]), dt2), x2);
     const float2 t1 = __fmul2_rn(__fmul2_rn(make_float2(Bv[i + 2], Bv[i + 3]), dt2), x2);
-    const float2 h0 = __ffma2_rn(make_float2(hv[i], hv[i + 1]), dA2, t0);
-    const float2 h1 = __ffma2_rn(make_float2(hv[i + 2], hv[i + 3]), dA2, t1);
+    float2 h0, h1;
+    if (ONE) {
+      h0 = __ffma2_rn(make_float2(hv[i], hv[i + 1]), make_float2(s0, s0), t0);
+      h1 = __ffma2_rn(make_float2(hv[i + 2], hv[i + 3]), make_float2(s1, s1), t1);
+    } else {  // scalar: a packed operand would need each pair's factor twice
+      h0 = make_float2(fmaf(hv[i], s0, t0.x), fmaf(hv[i + 1], s0, t0.y));
+      h1 = make_float2(fmaf(hv[i + 2], s1, t1.x), fmaf(hv[i + 3], s1, t1.y));
+    }
     hv[i] = h0.x; hv[i + 1] = h0.y; hv[i + 2] = h1.x; hv[i + 3] = h1.y;
     ya = __ffma2_rn(h0, make_float2(Cv[i], Cv[i + 1]), ya);
     yb = __ffma2_rn(h1, make_float2(Cv[i + 2], Cv[i + 3]), yb);
   }
   return (ya.x + ya.y) + (yb.x + yb.y);
+}
+
+// What a stored block and dA = exp(A dt) give the update: q[i] and sd with h dA = q[i] sd of the pair, both exact.
+// Byte codes: q the code, sd = 2^(e - 127 + micro) dA.  The factor 1 or 2 of four pairs comes from a 16-entry table in shared memory
+// (two 128-bit loads in place of a mask, a multiply and a multiply per pair).  Packed nibbles: the micro-exponent doubles
+// the code instead, in bytes of unsigned integers (q + 16 or 2 q + 16), so one factor serves the block; `table` holds
+// a byte mask per pair, entry = micro byte.
+// Every stored exponent in [1, e_max + 1], dA within 2^20 (the caller sets e_max to 0 otherwise): nothing overflows on the way.
+// Other exponents, which no quantiser emits, take the plain form: q the value itself, sd = dA.
+struct MxPairFactors {
+  float4 f[16];
+  __device__ __forceinline__ void fill(int i) {
+    if (i < 16) f[i] = make_float4(i & 1 ? 2.0f : 1.0f, i & 2 ? 2.0f : 1.0f, i & 4 ? 2.0f : 1.0f, i & 8 ? 2.0f : 1.0f);
+  }
+};
+struct MxPairMasks {
+  uint2 m[256];
+  __device__ __forceinline__ void fill(int i) {
+    const auto spread = [](uint32_t n) {
+      return (n & 1 ? 0xFFu : 0u) | (n & 2 ? 0xFF00u : 0u) | (n & 4 ? 0xFF0000u : 0u) | (n & 8 ? 0xFF000000u : 0u);
+    };
+    m[i] = make_uint2(spread(i & 15), spread(i >> 4));
+  }
+};
+
+__device__ __forceinline__ void mx_decode_block(const uint32_t (&codes)[4], uint32_t e, uint32_t micro_bits, float (&h)[16]);
+__device__ __forceinline__ void mx4_nibbles_to_bytes(uint32_t lo, uint32_t hi, uint32_t (&codes)[4]);
+
+__device__ __forceinline__ void mx_decode_scaled(const uint4& raw, uint32_t e, uint32_t micro_bits, float dA, uint32_t e_max, const MxPairFactors& table,
+                                                 float (&q)[16], float (&sd)[8]) {
+  const uint32_t codes[4] = {raw.x, raw.y, raw.z, raw.w};
+  if (__all_sync(0xFFFFFFFFu, e - 1u <= e_max)) {
+    const float4 f0 = table.f[micro_bits & 15u], f1 = table.f[micro_bits >> 4];
+    const float base = __uint_as_float(e << 23) * dA;
+    sd[0] = f0.x * base; sd[1] = f0.y * base; sd[2] = f0.z * base; sd[3] = f0.w * base;
+    sd[4] = f1.x * base; sd[5] = f1.y * base; sd[6] = f1.z * base; sd[7] = f1.w * base;
+#pragma unroll
+    for (int w = 0; w < 4; ++w) {
+      const uint32_t biased = codes[w] ^ 0x80808080u;  // q + 128 as unsigned bytes
+#pragma unroll
+      for (int k = 0; k < 4; k += 2) {
+        const float2 r = __fadd2_rn(make_float2(__uint_as_float(__byte_perm(biased, 0x47000000u, 0x7604 | (k << 4))),
+                                                __uint_as_float(__byte_perm(biased, 0x47000000u, 0x7604 | ((k + 1) << 4)))),
+                                    make_float2(-32896.0f, -32896.0f));
+        q[4 * w + k] = r.x;
+        q[4 * w + k + 1] = r.y;
+      }
+    }
+  } else {
+    mx_decode_block(codes, e, micro_bits, q);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) sd[j] = dA;
+  }
+}
+
+__device__ __forceinline__ void mx_decode_scaled(const uint4& raw, uint32_t e, uint32_t micro_bits, float dA, uint32_t e_max, const MxPairMasks& table,
+                                                 float (&q)[16], float (&sd)[8]) {
+  if (__all_sync(0xFFFFFFFFu, e - 1u <= e_max)) {
+    sd[0] = __uint_as_float(e << 23) * dA;
+    const uint2 mask = table.m[micro_bits];
+#pragma unroll
+    for (int w = 0; w < 2; ++w) {
+      const uint32_t x = w ? raw.y : raw.x, m = w ? mask.y : mask.x;
+      const uint32_t ev = (x & 0x0F0F0F0Fu) ^ 0x08080808u, od = ((x >> 4) & 0x0F0F0F0Fu) ^ 0x08080808u;  // q + 8; byte k = pair k
+      const uint32_t ev2 = ev + ((m & ev) | (~m & 0x08080808u)), od2 = od + ((m & od) | (~m & 0x08080808u));
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const float2 r = __fadd2_rn(make_float2(__uint_as_float(__byte_perm(ev2, 0x47000000u, 0x7604 | (k << 4))),
+                                                __uint_as_float(__byte_perm(od2, 0x47000000u, 0x7604 | (k << 4)))),
+                                    make_float2(-32784.0f, -32784.0f));
+        q[8 * w + 2 * k] = r.x;
+        q[8 * w + 2 * k + 1] = r.y;
+      }
+    }
+  } else {
+    uint32_t codes[4];
+    mx4_nibbles_to_bytes(raw.x, raw.y, codes);
+    mx_decode_block(codes, e, micro_bits, q);
+    sd[0] = dA;
+  }
 }
 
 // int8 lanes of `codes` times 2^(e - 127 + micro of the pair) -> fp32 (reference :132).

@@ -13,6 +13,7 @@
 // and decode + update + read-out + exponent + rounding + random bits need more than that.
 #include <algorithm>
 #include <cstdlib>
+#include <type_traits>
 
 #include "lq_mx_codec.cuh"
 #include "lq_ssm_operands.cuh"
@@ -60,12 +61,11 @@ struct MxBlockIO {
     return r;
   }
 
+  // codes: the words as stored (packed nibbles: codes[0..1])
   __device__ __forceinline__ static void store_ptr(uint8_t* q, uint8_t* e, uint8_t* m, const uint32_t (&codes)[4], uint32_t ev,
                                                    uint32_t mic) {
     if (kNibbles) {
-      uint32_t lo, hi;
-      mx4_bytes_to_nibbles(codes, lo, hi);
-      *reinterpret_cast<uint2*>(q) = make_uint2(lo, hi);
+      *reinterpret_cast<uint2*>(q) = make_uint2(codes[0], codes[1]);
     } else {
       *reinterpret_cast<uint4*>(q) = make_uint4(codes[0], codes[1], codes[2], codes[3]);
     }
@@ -264,11 +264,13 @@ __global__ void __launch_bounds__(kUpdateThreads, 4) mx_state_update_kernel(cons
         mx_decode_block(codes, cur.e, cur.mic, hv);
         const float xv = sxh[p];
         if (hoisted) {
-          y = mx_update_readout16(hv, Bv, Cv, dA_h, dt_h, xv);  // h' = h exp(A dt) + (B dt) x
+          const float one[8] = {dA_h};
+          y = mx_update_readout16<true>(hv, Bv, Cv, one, dt_h, xv);  // h' = h exp(A dt) + (B dt) x
         } else {
           const float dt = d.dt_uniform ? dt_h : row_dt(h, p);
           if (d.a_scalar) {
-            y = mx_update_readout16(hv, Bv, Cv, expf(load_as_float(a.A, h * a.A_stride[0], a.A_dtype) * dt), dt, xv);
+            const float one[8] = {expf(load_as_float(a.A, h * a.A_stride[0], a.A_dtype) * dt)};
+            y = mx_update_readout16<true>(hv, Bv, Cv, one, dt, xv);
           } else {
 #pragma unroll
             for (int i = 0; i < 16; ++i) {
@@ -386,13 +388,15 @@ __global__ void __launch_bounds__(kFastThreads, kFastCtasPerSm) mx_state_update_
   uint8_t* qptr = static_cast<uint8_t*>(s.q_state) + (R0 + r_first) * q_row + blk * IO::kQBytes;
   uint8_t* eptr = s.shared_exp + (R0 + r_first) * e_row + blk;
   uint8_t* mptr = s.micro_exp + (R0 + r_first) * m_row + blk * IO::kMicroBytes;
-  // linear index of the block's first value, kept pre-shifted to the Philox counter in the layered modes (block index /
-  // quad index), so that the loop carries the counter itself
+  // linear index of the block's first value; in the layered modes the Philox counter (block index / quad index)
   constexpr int kCtrShift = MODE == LQ_ROUND_PHILOX_LAYERED ? 4 : (MODE == LQ_ROUND_PHILOX_LAYERED4 ? 2 : 0);
   uint64_t lin = ((R0 + r_first) * dstate + n0) >> kCtrShift;
   uint32_t row = r_first;
   const uint32_t dq = rows_per_pass * q_row, de = rows_per_pass * e_row, dm = rows_per_pass * m_row,
                  dl = (rows_per_pass * dstate) >> kCtrShift;
+  using Table = std::conditional_t<IO::kNibbles, MxPairMasks, MxPairFactors>;
+  __shared__ Table table;
+  for (int i = threadIdx.x; i < (IO::kNibbles ? 256 : 16); i += kFastThreads) table.fill(i);
   // everything above is arithmetic on the arguments; from here on memory the predecessor may have written is read
   asm volatile("griddepcontrol.wait;" ::: "memory");
   // the first row's block travels while the operands below are staged
@@ -422,6 +426,11 @@ __global__ void __launch_bounds__(kFastThreads, kFastCtasPerSm) mx_state_update_
   load_bc16(a.B, a.B_stride, a.B_dtype, b_cur, g_cur, n0, Bv);
   load_bc16(a.C, a.C_stride, a.C_dtype, b_cur, g_cur, n0, Cv);
   const MxRoundBase rb = make_round_base(a.rounding, static_cast<uint64_t>(s.batch) * H * P * dstate);
+  // layered modes: the counters of the whole state fit 32 bits (fast_update_applies), so the stream carries them
+  constexpr bool kStream = MODE == LQ_ROUND_PHILOX_LAYERED || MODE == LQ_ROUND_PHILOX_LAYERED4;
+  PhiloxStream stream;
+  if (kStream) stream.init(static_cast<uint32_t>(lin), 0u, rb.step, rb.layer, d.keys);
+  const uint64_t stream_step = static_cast<uint64_t>(kPhiloxM0) * dl;
 
   __syncthreads();
 
@@ -430,6 +439,7 @@ __global__ void __launch_bounds__(kFastThreads, kFastCtasPerSm) mx_state_update_
   while (u < n_units) {
     // units of one head
     const float dt_h = sdt[head_i], dA_h = sdA[head_i];
+    const uint32_t e_max = dA_h <= 1048576.0f ? 228u : 0u;
     const int u_head_end = min(n_units, u + units_per_head - unit_in_head);
 #pragma unroll 1
     for (; u < u_head_end; ++u) {
@@ -439,16 +449,14 @@ __global__ void __launch_bounds__(kFastThreads, kFastCtasPerSm) mx_state_update_
       MxRaw nxt = cur;
       if (u + 1 < n_units) nxt = IO::load_ptr(qn, en, mn);
 
-      uint32_t codes[4];
-      IO::codes_of(cur, codes);
-      float hv[16];
-      mx_decode_block(codes, cur.e, cur.mic, hv);
-      float y = mx_update_readout16(hv, Bv, Cv, dA_h, dt_h, sx[row]);  // h' = h exp(A dt) + (B dt) x
+      float hv[16], sd[8];
+      mx_decode_scaled(cur.q, cur.e, cur.mic, dA_h, e_max, table, hv, sd);
+      float y = mx_update_readout16<IO::kNibbles>(hv, Bv, Cv, sd, dt_h, sx[row]);  // h' = h exp(A dt) + (B dt) x
 
-      MxRoundCtx ctx = round_ctx_at<MODE>(rb, lin << kCtrShift);
-      if (kCtrShift) ctx.counter = lin;
-      uint32_t e_new, mic_new;
-      mx_encode_block<BITS, MODE>(hv, cut, ctx, d.keys, codes, e_new, mic_new);
+      MxRoundCtx ctx = round_ctx_at<MODE>(rb, lin);
+      if (kStream) ctx.stream = &stream;
+      uint32_t codes[4], e_new, mic_new;
+      mx_encode_block<BITS, MODE, IO::kNibbles>(hv, cut, ctx, d.keys, codes, e_new, mic_new);
       IO::store_ptr(qptr, eptr, mptr, codes, e_new, mic_new);
 
       if (NBLK_T == 8) {
@@ -459,7 +467,7 @@ __global__ void __launch_bounds__(kFastThreads, kFastCtasPerSm) mx_state_update_
       }
       cur = nxt;
       qptr = qn; eptr = en; mptr = mn;
-      lin += dl;
+      if (kStream) stream.pa += stream_step; else lin += dl;
       row += rows_per_pass;
     }
     // the next unit, if any, starts another head; B / C change only with the (batch, group)
@@ -616,8 +624,12 @@ static bool fast_update_applies(const lq_mx_update_args& a, const MxUpdateDerive
                      s.micro_stride[1] == m_row * s.dim && s.micro_stride[0] == m_row * s.dim * s.heads;
   // fewer than 2^31 units keep the kernel's index arithmetic in 32 bits and its multiply-high divisions exact
   const uint64_t units = static_cast<uint64_t>(s.batch) * s.heads * (s.dim / rows_per_pass);
+  // Philox counters of the layered modes stay in 32 bits
+  const int counter_log2 = a.rounding.mode == LQ_ROUND_PHILOX_LAYERED4 ? 2 : 4;
+  const uint64_t counters = a.rounding.mode == LQ_ROUND_PHILOX_LAYERED || a.rounding.mode == LQ_ROUND_PHILOX_LAYERED4
+                                ? (static_cast<uint64_t>(s.batch) * s.heads * s.dim * s.dstate) >> counter_log2 : 0;
   return dense && d.dt_uniform && d.a_scalar && a.h_out == nullptr && (1 << d.lpr_log2) == d.nblk &&
-         s.dim % rows_per_pass == 0 && units < (1ull << 31);
+         s.dim % rows_per_pass == 0 && units < (1ull << 31) && counters <= (1ull << 32);
 }
 
 template <int BITS, int LAYOUT>
