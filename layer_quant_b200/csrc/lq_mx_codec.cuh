@@ -29,6 +29,8 @@ template <int BITS>
 struct MxFormat {
   static constexpr float kMax = BITS == 8 ? 63.0f : 7.0f;
   static constexpr int kShift = BITS == 8 ? 6 : 3;  // floor(log2(2 * kMax))
+  static constexpr uint32_t kCutFirst = BITS == 8 ? 0x7C0000u : 0x600000u;  // smallest and largest entry of the table that matter
+  static constexpr uint32_t kCutLast = kCutFirst + 0x40u;
 };
 
 // 2^(e - 127 + micro) for stored bytes e in [0, 255], micro in {0, 1} (reference: tl.exp2 at :132).
@@ -45,6 +47,12 @@ struct MxRoundCtx {
   const uint32_t* words; // SUPPLIED / SUPPLIED_FIXED: 16 words of this block
   const PhiloxStream* stream = nullptr;  // the layered modes: where the caller carries the generator along, used instead of the counter
 };
+
+__device__ __forceinline__ float max3(float a, float b, float c) {  // one three-input instruction (sm_100)
+  float r;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
 
 // 1.0f if a > b else 0.0f, as one FSET.
 __device__ __forceinline__ float set_gt(float a, float b) {
@@ -74,19 +82,25 @@ constexpr float kByteMagic = 49152.0f;  // 1.5 * 2^15: ulp 2^-8, mantissa bits 8
 //    M + 2^-9 (the few-ulp overshoot of the rounded log2 is orders of magnitude smaller).
 // PACKED_NIBBLES: codes[0..1] are the 16 nibbles as the packed MX4 layout stores them.
 template <int BITS, int MODE, bool PACKED_NIBBLES = false>
-__device__ __forceinline__ void mx_encode_block(const float (&h)[16], const unsigned int* __restrict__ cut_table,
-                                                const MxRoundCtx& ctx, const PhiloxKeys& keys, uint32_t (&codes)[4],
+__device__ __forceinline__ void mx_encode_block(const float (&h)[16], const MxRoundCtx& ctx, const PhiloxKeys& keys, uint32_t (&codes)[4],
                                                 uint32_t& exp_byte, uint32_t& micro_bits) {
   constexpr float M = MxFormat<BITS>::kMax;
   constexpr bool kFixed = (MODE == LQ_ROUND_PHILOX_LAYERED || MODE == LQ_ROUND_SUPPLIED_FIXED);
   float pa[8];
 #pragma unroll
   for (int j = 0; j < 8; ++j) pa[j] = fmaxf(fabsf(h[2 * j]), fabsf(h[2 * j + 1]));
-  const float amax = fmaxf(fmaxf(fmaxf(pa[0], pa[1]), fmaxf(pa[2], pa[3])), fmaxf(fmaxf(pa[4], pa[5]), fmaxf(pa[6], pa[7])));
-  // biased = clamp(ceil(log2(max(amax / 2M, 1e-30))) + 127, 1, 254): always in [28, 252]
+  const float amax = max3(max3(pa[0], pa[1], pa[2]), max3(pa[3], pa[4], pa[5]), fmaxf(pa[6], pa[7]));
+  // biased = clamp(ceil(log2(max(amax / 2M, 1e-30))) + 127, 1, 254): always in [28, 252].  The mantissa at which it steps up depends
+  // on the exponent (the rounded logarithm), but always lies in [kCutFirst, kCutLast] (below field 34 it makes no
+  // difference): only a maximum in that sliver, one in 200,000, has to look it up.
   const uint32_t abits = __float_as_uint(amax);
-  const uint32_t field = abits >> 23;
-  int biased = static_cast<int>(field) - MxFormat<BITS>::kShift + ((abits & 0x7FFFFFu) > __ldg(cut_table + field) ? 1 : 0);
+  uint32_t up = (abits + (0x7FFFFFu - MxFormat<BITS>::kCutFirst)) >> 23;
+  if (up != (abits + (0x7FFFFFu - MxFormat<BITS>::kCutLast)) >> 23) {
+    uint32_t cut;  // volatile: a branch, not a load that every block waits for
+    asm volatile("ld.global.nc.u32 %0, [%1];" : "=r"(cut) : "l"(mx_exp_cut_table<BITS>() + (abits >> 23)));
+    up = (abits >> 23) + ((abits & 0x7FFFFFu) > cut ? 1u : 0u);
+  }
+  int biased = static_cast<int>(up) - MxFormat<BITS>::kShift;
   biased = biased < 28 ? 28 : biased;
   exp_byte = static_cast<uint32_t>(biased);
   // amax == 0 makes the reference use base 1.0; every mantissa is 0 with either base.
@@ -185,20 +199,20 @@ __device__ __forceinline__ void mx_encode_block(const float (&h)[16], const unsi
 // h' = h * dA + (B * dt) * x on 16 values and the block's share of <h', C>, with packed fp32x2 instructions
 // (sm_100: two IEEE fp32 results per instruction, same rounding per component as the scalar forms).
 // Association as in the reference kernel (mamba_state_8b_kernel.py:158, dB = B * dt, then state * dA + dB * x):
-// dB rounded, t = dB * x rounded, then fma(h, dA, t), which is what a compiler that contracts the reference's
+// dB rounded (by the caller), t = dB * x rounded, then fma(h, dA, t), which is what a compiler that contracts the reference's
 // expression produces; the read-out keeps four partial sums over i mod 4, added as (y0 + y1) + (y2 + y3).
 // h is given as q * s with s a power of two: fma(h, dA, t) = fma(q, s dA, t), for s dA is exact.  sd: s dA of the pairs,
 // ONE: of the whole block (sd[0]).
 template <bool ONE>
-__device__ __forceinline__ float mx_update_readout16(float (&hv)[16], const float (&Bv)[16], const float (&Cv)[16], const float (&sd)[8],
-                                                     float dt, float x) {
-  const float2 dt2 = make_float2(dt, dt), x2 = make_float2(x, x);
+__device__ __forceinline__ float mx_update_readout16(float (&hv)[16], const float (&dB)[16], const float (&Cv)[16], const float (&sd)[8],
+                                                     float x) {
+  const float2 x2 = make_float2(x, x);
   float2 ya = make_float2(0.0f, 0.0f), yb = make_float2(0.0f, 0.0f);
 #pragma unroll
   for (int i = 0; i < 16; i += 4) {
     const float s0 = sd[ONE ? 0 : i / 2], s1 = sd[ONE ? 0 : i / 2 + 1];
-    const float2 t0 = __fmul2_rn(__fmul2_rn(make_float2(Bv[i], Bv[i + 1]), dt2), x2);
-    const float2 t1 = __fmul2_rn(__fmul2_rn(make_float2(Bv[i + 2], Bv[i + 3]), dt2), x2);
+    const float2 t0 = __fmul2_rn(make_float2(dB[i], dB[i + 1]), x2);
+    const float2 t1 = __fmul2_rn(make_float2(dB[i + 2], dB[i + 3]), x2);
     float2 h0, h1;
     if (ONE) {
       h0 = __ffma2_rn(make_float2(hv[i], hv[i + 1]), make_float2(s0, s0), t0);

@@ -163,13 +163,14 @@ struct MxUpdateDerived {
   int32_t lpr_log2;    // lanes per row = 1 << lpr_log2 >= nblk
   int32_t dt_uniform;  // dt and dt_bias do not depend on the row (dim) index
   int32_t a_scalar;    // A depends on the head only
+  int32_t vec;         // x, out, B, C in 16 bits, aligned for vectors; D per head, no z; dim a multiple of 4
   int32_t heads_per_cta;  // consecutive heads of one B/C group handled by one CTA
   PhiloxKeys keys;        // round keys of rounding.seed
   uint64_t units_total;   // fast path: batch * heads * dim / rows per pass (< 2^31)
   // fast path: the slab of a CTA without a division.  units_per_cta / units_rem: CTA c owns units_per_cta units, the
   // first units_rem CTAs one more.  FastDiv: floor(n / d) for n < 2^31 as (mulhi(n, magic) + n) >> shift.
   uint32_t units_per_cta, units_rem;
-  struct FastDiv { uint32_t magic, shift; } div_units_per_head, div_heads, div_dim, div_heads_per_group;
+  struct FastDiv { uint32_t magic, shift; } div_steps_per_head, div_heads, div_dim, div_heads_per_group, div_groups;
 };
 
 __device__ __forceinline__ uint32_t fast_div(uint32_t n, const MxUpdateDerived::FastDiv& f) { return (__umulhi(n, f.magic) + n) >> f.shift; }
@@ -198,7 +199,6 @@ __global__ void __launch_bounds__(kUpdateThreads, 4) mx_state_update_kernel(cons
   const bool blk_ok = blk < d.nblk;
   const int n0 = blk * 16;
   const int grp = h0 / (H / a.ngroups);  // the same for every head of the CTA
-  const unsigned int* cut = mx_exp_cut_table<BITS>();
 
   auto row_dt = [&](int h, int p) {
     float dt = load_as_float(a.dt, b * a.dt_stride[0] + h * a.dt_stride[1] + p * a.dt_stride[2], a.dt_dtype);
@@ -234,6 +234,9 @@ __global__ void __launch_bounds__(kUpdateThreads, 4) mx_state_update_kernel(cons
     const int h = h0 + hh;
     const float dt_h = d.dt_uniform ? sdt[hh] : 0.0f;
     const float dA_h = sdA[hh];
+    float dBv[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) dBv[i] = __fmul_rn(Bv[i], dt_h);
     const uint64_t lin_head = (static_cast<uint64_t>(b) * H + h) * P * static_cast<uint64_t>(N) + n0;
     const int64_t qbase = b * s.q_stride[0] + h * s.q_stride[1];
     const int64_t ebase = b * s.exp_stride[0] + h * s.exp_stride[1];
@@ -265,12 +268,15 @@ __global__ void __launch_bounds__(kUpdateThreads, 4) mx_state_update_kernel(cons
         const float xv = sxh[p];
         if (hoisted) {
           const float one[8] = {dA_h};
-          y = mx_update_readout16<true>(hv, Bv, Cv, one, dt_h, xv);  // h' = h exp(A dt) + (B dt) x
+          y = mx_update_readout16<true>(hv, dBv, Cv, one, xv);  // h' = h exp(A dt) + (B dt) x
         } else {
           const float dt = d.dt_uniform ? dt_h : row_dt(h, p);
           if (d.a_scalar) {
             const float one[8] = {expf(load_as_float(a.A, h * a.A_stride[0], a.A_dtype) * dt)};
-            y = mx_update_readout16<true>(hv, Bv, Cv, one, dt, xv);
+            float dBr[16];
+#pragma unroll
+            for (int i = 0; i < 16; ++i) dBr[i] = __fmul_rn(Bv[i], dt);
+            y = mx_update_readout16<true>(hv, dBr, Cv, one, xv);
           } else {
 #pragma unroll
             for (int i = 0; i < 16; ++i) {
@@ -296,7 +302,7 @@ __global__ void __launch_bounds__(kUpdateThreads, 4) mx_state_update_kernel(cons
         }
         const MxRoundCtx ctx = round_ctx_at<MODE>(rb, lin);
         uint32_t e_new, mic_new;
-        mx_encode_block<BITS, MODE>(hv, cut, ctx, d.keys, codes, e_new, mic_new);
+        mx_encode_block<BITS, MODE>(hv, ctx, d.keys, codes, e_new, mic_new);
         IO::store(s, qbase + p * s.q_stride[2], ebase + p * s.exp_stride[2], mbase + p * s.micro_stride[2], blk, codes, e_new,
                   mic_new);
       }
@@ -318,59 +324,132 @@ __global__ void __launch_bounds__(kUpdateThreads, 4) mx_state_update_kernel(cons
 }
 
 // Fast path of the fused update: the shape every Mamba2 decode step has.  Requirements (checked
-// on the host): dense state tensors, dt / dt_bias / A per head only, dstate / 16 a power of two,
-// dim a multiple of the rows one CTA pass covers, no h_out, fewer than 2^31 units.
+// on the host): dense 16-byte aligned state tensors, dt / dt_bias / A per head only, dstate / 16 a power of two,
+// dim a multiple of the rows two warps cover, no h_out, fewer than 2^30 units.
 //
-// Work is cut into units of `rows_per_pass` consecutive rows (one pass of the CTA's two warps).
+// A step is 32 consecutive blocks: one per lane, `32 / (dstate / 16)` rows.  A unit is two steps.
 // Units are numbered in memory order and dealt out contiguously, U / G to each of the G CTAs and one
-// more to the first U mod G: a contiguous
-// slab of the state, balanced to within one unit whatever the batch, and the grid is one wave of
-// resident CTAs whenever the slab's x / y staging fits in shared memory.  Every lane is always
-// active, the three state pointers move by a constant per pass (also across head boundaries), and
-// B / C are reloaded only when the slab crosses into another (batch, B/C group).
+// more to the first U mod G: a contiguous slab of the state, balanced to within one unit whatever the batch, the first half of
+// its steps for warp 0 and the second for warp 1.  The grid is one wave of resident CTAs whenever the slab's x / y
+// staging fits in shared memory.
+//
+// The state comes through a ring of two stages of four steps per warp (cp.async: a warp synchronises with itself only), so that a
+// step has no global address arithmetic, no copies of prefetched registers, and its loads are one to two stages old.
+// B and C of the slab's (batch, group)s wait in shared memory as [quarter][block] float4; dB = B dt of the
+// current head and C of the current group are kept in registers.
 // NBLK_T = dstate / 16 when known at compile time (8 for Nemotron-H: all lane and address arithmetic
-// folds to constants and the read-out reduction unrolls), 0 = taken from the arguments.
+// folds to constants), 0 = taken from the arguments.
+constexpr int kRingSteps = 4, kRingStages = 2;
+constexpr int kPartialStride = 36;  // floats of a step's read-out partials: 32 and a shift of one 16-byte bank column
+template <int BITS, int LAYOUT>
+struct MxRing {
+  using IO = MxBlockIO<BITS, LAYOUT>;
+  static constexpr uint32_t kQ = 32 * IO::kQBytes, kM = 32 * IO::kMicroBytes, kE = 32;  // bytes of a step
+  static constexpr uint32_t kEChunks = kRingSteps * kE / 16;
+  static constexpr uint32_t kOffE = kRingSteps * kQ, kOffM = kOffE + kRingSteps * kE;
+  static constexpr uint32_t kStage = kOffM + kRingSteps * kM;
+  static constexpr uint32_t kBytes = (kFastThreads / 32) * kRingStages * kStage;
+
+  // Chunk c of a tensor's part of a stage goes through lane c mod 32 (e: the first kEChunks lanes, m: the next ones, so that packed e and m are
+  // one instruction); chunks of steps from `left` on do not exist.  src: q / e or m at the warp's first step, plus 16 bytes per lane.
+  struct Source {
+    const uint8_t *q, *em, *m;  // em: e, or packed m on the next lanes; m: unpacked micro-exponents
+    uint32_t dst_q, dst_em;
+    __device__ __forceinline__ Source(uint32_t ring, const uint8_t* q0, const uint8_t* e0, const uint8_t* m0, uint32_t lane) {
+      q = q0 + lane * 16;
+      em = lane < kEChunks ? e0 + lane * 16 : m0 + (lane - kEChunks) * 16;
+      m = m0 + lane * 16;
+      dst_q = ring + lane * 16;
+      dst_em = ring + (lane < kEChunks ? kOffE + lane * 16 : kOffM + (lane - kEChunks) * 16);
+    }
+  };
+  __device__ __forceinline__ static void cp16(uint32_t dst, const uint8_t* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+  }
+  __device__ __forceinline__ static void issue(Source& s, uint32_t stage, uint32_t lane, int left, int advance = kRingSteps) {
+    const uint32_t off = stage * kStage;
+#pragma unroll
+    for (uint32_t c = 0; c < kRingSteps * kQ / 16; c += 32)
+      if (static_cast<int>(((c + lane) * 16) / kQ) < left) cp16(s.dst_q + off + c * 16, s.q + c * 16);
+    if (lane < (LAYOUT == LQ_MX_LAYOUT_PACKED ? 2 * kEChunks : kEChunks) && static_cast<int>((lane & (kEChunks - 1)) >> 1) < left) cp16(s.dst_em + off, s.em);
+    if (LAYOUT != LQ_MX_LAYOUT_PACKED) {
+#pragma unroll
+      for (uint32_t c = 0; c < kRingSteps * kM / 16; c += 32)
+        if (static_cast<int>(((c + lane) * 16) / kM) < left) cp16(s.dst_q + off + kOffM + c * 16, s.m + c * 16);
+      s.m += advance * kM;
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    s.q += advance * kQ;
+    s.em += advance * kE;
+  }
+  // this lane's block of step k
+  __device__ __forceinline__ static MxRaw read(const uint8_t* stage, uint32_t k, uint32_t lane) {
+    MxRaw r;
+    const uint8_t* q = stage + k * kQ + lane * IO::kQBytes;
+    if (IO::kNibbles) {
+      const uint2 v = *reinterpret_cast<const uint2*>(q);
+      r.q = make_uint4(v.x, v.y, 0u, 0u);
+    } else {
+      r.q = *reinterpret_cast<const uint4*>(q);
+    }
+    r.e = stage[kOffE + k * kE + lane];
+    if (LAYOUT == LQ_MX_LAYOUT_PACKED) {
+      r.mic = stage[kOffM + k * kM + lane];
+    } else {
+      const uint2 mm = *reinterpret_cast<const uint2*>(stage + kOffM + k * kM + lane * 8);
+      r.mic = (((mm.x & 0x01010101u) * 0x10204080u) >> 28) | ((((mm.y & 0x01010101u) * 0x10204080u) >> 28) << 4);
+    }
+    return r;
+  }
+};
+
 template <int BITS, int LAYOUT, int MODE, int NBLK_T>
 __global__ void __launch_bounds__(kFastThreads, kFastCtasPerSm) mx_state_update_fast_kernel(const lq_mx_update_args a, const MxUpdateDerived d) {
   using IO = MxBlockIO<BITS, LAYOUT>;
-  extern __shared__ float smem_xy[];
+  using Ring = MxRing<BITS, LAYOUT>;
+  // MX8: a first stage of one step lets every warp start before the other stages queue up in memory (batch 8: 11.0 -> 10.7 us),
+  // and a block is read where it is used (batch 250: 192 -> 190 us, six copies less per step).  MX4 moves half the bytes and is
+  // better off the other way (batch 64: 53.3 -> 51.7 us).
+  constexpr int kFirstSteps = BITS == 8 ? 1 : kRingSteps;
+  constexpr bool kAhead = BITS == 4;
+  extern __shared__ __align__(16) uint8_t smem_fast[];
   const lq_mx_state& s = a.state;
   const int H = s.heads, P = s.dim;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int nblk = NBLK_T ? NBLK_T : d.nblk;
   const int lpr_log2 = NBLK_T == 8 ? 3 : d.lpr_log2;
   const int dstate = NBLK_T ? NBLK_T * 16 : s.dstate;
   const int blk = lane & (nblk - 1);
-  const int rsub = lane >> lpr_log2;
-  const int rows_per_warp = 32 >> lpr_log2;
-  const int rows_per_pass = rows_per_warp * (kFastThreads / 32);
-  const int units_per_head = P / rows_per_pass;
+  const int rows_per_step = 32 >> lpr_log2;
+  const int rows_per_unit = rows_per_step * (kFastThreads / 32);
+  const uint32_t steps_per_head = static_cast<uint32_t>(P / rows_per_step);
   const int heads_per_group = H / a.ngroups;
-  const int n0 = blk * 16;
-  const unsigned int* cut = mx_exp_cut_table<BITS>();
 
   // this CTA's slab: units [u0, u1), rows [R0, R1) of the [batch * heads * dim] row space; the first units_rem CTAs
   // take one unit more than the others
   const uint32_t u0 = blockIdx.x * d.units_per_cta + min(blockIdx.x, d.units_rem);
-  const int n_units = static_cast<int>(d.units_per_cta + (blockIdx.x < d.units_rem ? 1u : 0u));
-  const uint32_t u1 = u0 + n_units;
+  const uint32_t n_units = d.units_per_cta + (blockIdx.x < d.units_rem ? 1u : 0u);
   // let the next kernel in the stream be scheduled behind this one (no effect without the launch attribute)
   asm volatile("griddepcontrol.launch_dependents;");
   if (n_units == 0) return;
-  const uint64_t R0 = static_cast<uint64_t>(u0) * rows_per_pass;
-  const int n_rows = n_units * rows_per_pass;
-  const uint32_t bh_first = fast_div(u0, d.div_units_per_head);  // first (batch * heads + head) index touched
-  const int n_heads = static_cast<int>(fast_div(u1 - 1, d.div_units_per_head) - bh_first) + 1;
-  float* sx = smem_xy;        // x of the slab's rows
+  const uint64_t R0 = static_cast<uint64_t>(u0) * rows_per_unit;
+  const int n_rows = static_cast<int>(n_units) * rows_per_unit;
+  const uint32_t step_first = 2 * u0, step_end = step_first + 2 * n_units;
+  const uint32_t bh_first = fast_div(step_first, d.div_steps_per_head);  // first (batch * heads + head) index touched
+  const uint32_t bh_last = fast_div(step_end - 1, d.div_steps_per_head);
+  const uint32_t bg_first = fast_div(bh_first, d.div_heads_per_group);   // the same for (batch * groups + group)
+  const int n_heads = static_cast<int>(bh_last - bh_first) + 1;
+  const int n_bg = static_cast<int>(fast_div(bh_last, d.div_heads_per_group) - bg_first) + 1;
+  float* const bc = reinterpret_cast<float*>(smem_fast + Ring::kBytes);  // per (batch, group): B, then C
+  float* const sx = bc + n_bg * 2 * dstate;  // x of the slab's rows
   // read-out of the slab's rows: one partial sum per 16-value block when a row spans eight lanes (added up when
   // the slab's y is written, in the order a butterfly over the eight lanes would add them), else the row's sum
-  float* sy = sx + n_rows;
-  float* sdt = sy + n_rows * (NBLK_T == 8 ? 8 : 1);   // per touched head
-  float* sdA = sdt + n_heads;
+  float* const sy = sx + n_rows;
+  float* const sdt = sy + (NBLK_T == 8 ? static_cast<int>(n_units) * 2 * kPartialStride : n_rows);   // per touched head
+  float* const sdA = sdt + n_heads;
 
   // (batch, head, row) of the slab's first row, once per CTA
-  const int unit_in_head0 = static_cast<int>(u0 - bh_first * static_cast<uint32_t>(units_per_head));
-  const int p_first = unit_in_head0 * rows_per_pass;
+  const int p_first = static_cast<int>(step_first - bh_first * steps_per_head) * rows_per_step;
   const int b_first = static_cast<int>(fast_div(bh_first, d.div_heads));
   const int h_first = static_cast<int>(bh_first - static_cast<uint32_t>(b_first) * static_cast<uint32_t>(H));
   auto row_coords = [&](int i, int& b, int& h, int& p) {
@@ -382,116 +461,233 @@ __global__ void __launch_bounds__(kFastThreads, kFastCtasPerSm) mx_state_update_
     b = b_first + static_cast<int>(bq);
     h = static_cast<int>(hh - bq * static_cast<uint32_t>(H));
   };
-  const uint32_t q_row = nblk * IO::kQBytes, m_row = nblk * IO::kMicroBytes, e_row = nblk;
-  const uint32_t r_first = warp * rows_per_warp + rsub;
-  // this lane's block of its first row; every pass moves all three pointers by a constant
-  uint8_t* qptr = static_cast<uint8_t*>(s.q_state) + (R0 + r_first) * q_row + blk * IO::kQBytes;
-  uint8_t* eptr = s.shared_exp + (R0 + r_first) * e_row + blk;
-  uint8_t* mptr = s.micro_exp + (R0 + r_first) * m_row + blk * IO::kMicroBytes;
+  // this warp's steps [0, n_units) start at block `block0` of the state
+  const uint32_t my_step0 = step_first + warp * n_units;
+  const int n_mine = static_cast<int>(n_units);
+  const uint64_t block0 = static_cast<uint64_t>(my_step0) * 32;
+  uint8_t* qptr = static_cast<uint8_t*>(s.q_state) + (block0 + lane) * IO::kQBytes;
+  uint8_t* eptr = s.shared_exp + block0 + lane;
+  uint8_t* mptr = s.micro_exp + (block0 + lane) * IO::kMicroBytes;
   // linear index of the block's first value; in the layered modes the Philox counter (block index / quad index)
   constexpr int kCtrShift = MODE == LQ_ROUND_PHILOX_LAYERED ? 4 : (MODE == LQ_ROUND_PHILOX_LAYERED4 ? 2 : 0);
-  uint64_t lin = ((R0 + r_first) * dstate + n0) >> kCtrShift;
-  uint32_t row = r_first;
-  const uint32_t dq = rows_per_pass * q_row, de = rows_per_pass * e_row, dm = rows_per_pass * m_row,
-                 dl = (rows_per_pass * dstate) >> kCtrShift;
+  constexpr uint32_t dl = 512 >> kCtrShift;
+  uint64_t lin = ((block0 + lane) * 16) >> kCtrShift;
   using Table = std::conditional_t<IO::kNibbles, MxPairMasks, MxPairFactors>;
   __shared__ Table table;
   for (int i = threadIdx.x; i < (IO::kNibbles ? 256 : 16); i += kFastThreads) table.fill(i);
+  uint8_t* const ring = smem_fast + warp * (kRingStages * Ring::kStage);
+  typename Ring::Source source(static_cast<uint32_t>(__cvta_generic_to_shared(ring)), static_cast<const uint8_t*>(s.q_state) + block0 * IO::kQBytes,
+                               s.shared_exp + block0, s.micro_exp + block0 * IO::kMicroBytes, lane);
   // everything above is arithmetic on the arguments; from here on memory the predecessor may have written is read
   asm volatile("griddepcontrol.wait;" ::: "memory");
-  // the first row's block travels while the operands below are staged
-  MxRaw cur = IO::load_ptr(qptr, eptr, mptr);
+  // the first stages travel while the operands below are staged
+  Ring::issue(source, 0, lane, min(n_mine, kFirstSteps), kFirstSteps);
 
-  for (int i = threadIdx.x; i < n_rows; i += kFastThreads) {
-    int b, h, p;
-    row_coords(i, b, h, p);
-    sx[i] = load_as_float(a.x, b * a.x_stride[0] + h * a.x_stride[1] + p * a.x_stride[2], a.x_dtype);
-  }
-  for (int i = threadIdx.x; i < n_heads; i += kFastThreads) {
+  // B / C of (batch, group) bgi, block kb; `which` 0: B, 1: C
+  const int n_bc = n_bg * nblk * 2;
+  auto bc_source = [&](int i, const void*& base, const int64_t*& st, int& dtype, int& b, int& g, int& kb) {
+    const int bgi = i >> (lpr_log2 + 1);
+    kb = (i >> 1) & (nblk - 1);
+    const uint32_t bg = bg_first + bgi;
+    b = static_cast<int>(fast_div(bg, d.div_groups));
+    g = static_cast<int>(bg) - b * a.ngroups;
+    base = i & 1 ? a.C : a.B;
+    st = i & 1 ? a.C_stride : a.B_stride;
+    dtype = i & 1 ? a.C_dtype : a.B_dtype;
+  };
+  auto store_bc = [&](int i, const float (&v)[16]) {
+    const int kb = (i >> 1) & (nblk - 1);
+    float4* dst = reinterpret_cast<float4*>(bc + ((i >> (lpr_log2 + 1)) * 2 + (i & 1)) * dstate) + kb;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) dst[k * nblk] = make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
+  };
+  auto stage_bc = [&](int i) {
+    const void* base; const int64_t* st; int dtype, b, g, kb;
+    bc_source(i, base, st, dtype, b, g, kb);
+    float v[16];
+    const int64_t (&strides)[3] = *reinterpret_cast<const int64_t (*)[3]>(st);
+    load_bc16(base, strides, dtype, b, g, kb * 16, v);
+    store_bc(i, v);
+  };
+  auto head_operands = [&](int i, float& dt, float& bias, float& A) {
     const unsigned hh = static_cast<unsigned>(h_first + i);
-    const int h = static_cast<int>(hh % static_cast<unsigned>(H)), b = b_first + static_cast<int>(hh / static_cast<unsigned>(H));
-    float dt = load_as_float(a.dt, b * a.dt_stride[0] + h * a.dt_stride[1], a.dt_dtype);
-    if (a.dt_bias) dt += load_as_float(a.dt_bias, h * a.dt_bias_stride[0], a.dt_bias_dtype);
+    const unsigned bq = fast_div(hh, d.div_heads);
+    const int h = static_cast<int>(hh - bq * static_cast<unsigned>(H)), b = b_first + static_cast<int>(bq);
+    dt = load_as_float(a.dt, b * a.dt_stride[0] + h * a.dt_stride[1], a.dt_dtype);
+    bias = a.dt_bias ? load_as_float(a.dt_bias, h * a.dt_bias_stride[0], a.dt_bias_dtype) : 0.0f;
+    A = load_as_float(a.A, h * a.A_stride[0], a.A_dtype);
+  };
+  auto stage_head = [&](int i, float dt, float bias, float A) {
+    if (a.dt_bias) dt += bias;
     if (a.dt_softplus) dt = softplus_ref(dt);
     sdt[i] = dt;
-    sdA[i] = expf(load_as_float(a.A, h * a.A_stride[0], a.A_dtype) * dt);
+    sdA[i] = expf(A * dt);
+  };
+  const int tid = threadIdx.x;
+  if (NBLK_T == 8 && d.vec) {
+    // 16-bit operands in vectors.  The first round of every kind is requested before any of it is used: one latency, not three
+    auto x_vec = [&](int i) {
+      int b, h, p;
+      row_coords(4 * i, b, h, p);
+      return *reinterpret_cast<const uint2*>(static_cast<const uint16_t*>(a.x) + b * a.x_stride[0] + h * a.x_stride[1] + p);
+    };
+    auto to_float4 = [&](uint2 w) {
+      if (a.x_dtype == LQ_BF16)
+        return make_float4(__uint_as_float(w.x << 16), __uint_as_float(w.x & 0xFFFF0000u), __uint_as_float(w.y << 16), __uint_as_float(w.y & 0xFFFF0000u));
+      const float2 lo = __half22float2(*reinterpret_cast<const __half2*>(&w.x)), hi = __half22float2(*reinterpret_cast<const __half2*>(&w.y));
+      return make_float4(lo.x, lo.y, hi.x, hi.y);
+    };
+    uint2 x0 = make_uint2(0u, 0u);
+    float dt = 0.0f, bias = 0.0f, A = 0.0f;
+    if (tid < n_heads) head_operands(tid, dt, bias, A);
+    if (4 * tid < n_rows) x0 = x_vec(tid);
+    if (tid < n_bc) stage_bc(tid);
+    if (4 * tid < n_rows) reinterpret_cast<float4*>(sx)[tid] = to_float4(x0);
+    if (tid < n_heads) stage_head(tid, dt, bias, A);
+    for (int i = tid + kFastThreads; 4 * i < n_rows; i += kFastThreads) reinterpret_cast<float4*>(sx)[i] = to_float4(x_vec(i));
+  } else {
+    if (tid < n_bc) stage_bc(tid);
+    for (int i = tid; i < n_rows; i += kFastThreads) {
+      int b, h, p;
+      row_coords(i, b, h, p);
+      sx[i] = load_as_float(a.x, b * a.x_stride[0] + h * a.x_stride[1] + p * a.x_stride[2], a.x_dtype);
+    }
+    if (tid < n_heads) {
+      float dt, bias, A;
+      head_operands(tid, dt, bias, A);
+      stage_head(tid, dt, bias, A);
+    }
   }
-  // position of the first unit: head index inside the slab, unit inside the head, head inside its group
-  int head_i = 0;
-  int unit_in_head = unit_in_head0;
-  int b_cur = b_first;
-  int g_cur = static_cast<int>(fast_div(static_cast<uint32_t>(h_first), d.div_heads_per_group));  // B / C group of the current head ...
-  int h_in_group = h_first - g_cur * heads_per_group;    // ... and the head's place in it: advanced without divisions
-  float Bv[16], Cv[16];
-  load_bc16(a.B, a.B_stride, a.B_dtype, b_cur, g_cur, n0, Bv);
-  load_bc16(a.C, a.C_stride, a.C_dtype, b_cur, g_cur, n0, Cv);
+  for (int i = tid + kFastThreads; i < n_bc; i += kFastThreads) stage_bc(i);
+  for (int i = tid + kFastThreads; i < n_heads; i += kFastThreads) {
+    float dt, bias, A;
+    head_operands(i, dt, bias, A);
+    stage_head(i, dt, bias, A);
+  }
   const MxRoundBase rb = make_round_base(a.rounding, static_cast<uint64_t>(s.batch) * H * P * dstate);
   // layered modes: the counters of the whole state fit 32 bits (fast_update_applies), so the stream carries them
   constexpr bool kStream = MODE == LQ_ROUND_PHILOX_LAYERED || MODE == LQ_ROUND_PHILOX_LAYERED4;
   PhiloxStream stream;
   if (kStream) stream.init(static_cast<uint32_t>(lin), 0u, rb.step, rb.layer, d.keys);
-  const uint64_t stream_step = static_cast<uint64_t>(kPhiloxM0) * dl;
 
+  for (int i = 1; i < kRingStages; ++i) Ring::issue(source, i, lane, n_mine - kFirstSteps - (i - 1) * kRingSteps);
   __syncthreads();
 
-  int u = 0;
-#pragma unroll 1
-  while (u < n_units) {
-    // units of one head
-    const float dt_h = sdt[head_i], dA_h = sdA[head_i];
-    const uint32_t e_max = dA_h <= 1048576.0f ? 228u : 0u;
-    const int u_head_end = min(n_units, u + units_per_head - unit_in_head);
-#pragma unroll 1
-    for (; u < u_head_end; ++u) {
-      uint8_t* const qn = qptr + dq;
-      uint8_t* const en = eptr + de;
-      uint8_t* const mn = mptr + dm;
-      MxRaw nxt = cur;
-      if (u + 1 < n_units) nxt = IO::load_ptr(qn, en, mn);
+  // current head of this warp: its operands, and the steps left in it
+  const uint32_t bh_mine = fast_div(my_step0, d.div_steps_per_head);
+  uint32_t left = steps_per_head - (my_step0 - bh_mine * steps_per_head);
+  const float* head = sdt + (bh_mine - bh_first);
+  const uint32_t bg_mine = fast_div(bh_mine, d.div_heads_per_group);
+  int h_in_group = static_cast<int>(bh_mine - bg_mine * static_cast<uint32_t>(heads_per_group));
+  const float4* bcp = reinterpret_cast<const float4*>(bc + (bg_mine - bg_first) * 2 * dstate) + blk;
+  float dB[16], Cv[16], dA;
+  uint32_t e_max;
+  auto read16 = [&](const float4* src, float (&v)[16]) {
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const float4 f = src[k * nblk];
+      v[4 * k] = f.x; v[4 * k + 1] = f.y; v[4 * k + 2] = f.z; v[4 * k + 3] = f.w;
+    }
+  };
+  auto load_head = [&]() {
+    const float dt = head[0];
+    dA = head[n_heads];
+    e_max = dA <= 1048576.0f ? 228u : 0u;
+    read16(bcp, dB);
+#pragma unroll
+    for (int i = 0; i < 16; ++i) dB[i] = __fmul_rn(dB[i], dt);
+  };
+  load_head();
+  read16(bcp + dstate / 4, Cv);
 
+  auto next_head = [&]() {  // B / C change only with the (batch, group)
+    left = steps_per_head;
+    ++head;
+    if (++h_in_group == heads_per_group) {
+      h_in_group = 0;
+      bcp += dstate / 2;
+      read16(bcp + dstate / 4, Cv);
+    }
+    load_head();
+  };
+
+  const float* xp = sx + warp * n_mine * rows_per_step + (lane >> lpr_log2);
+  float* yp = NBLK_T == 8 ? sy + warp * n_mine * kPartialStride + lane : sy + warp * n_mine * rows_per_step + (lane >> lpr_log2);
+  uint32_t stage = 0;
+#pragma unroll 1
+  for (int todo = n_mine, len = kFirstSteps; todo > 0; todo -= len, len = kRingSteps) {  // steps to do from this stage on, steps in it
+    asm volatile("cp.async.wait_group %0;" ::"n"(kRingStages - 1) : "memory");
+    __syncwarp();
+    const uint8_t* const buf = ring + stage * Ring::kStage;
+    MxRaw cur = {make_uint4(0u, 0u, 0u, 0u), 0u, 0u};
+    if (kAhead) cur = Ring::read(buf, 0, lane);
+#pragma unroll 1
+    for (int k = 0; k < kRingSteps; ++k) {
+      if (k >= min(len, todo)) break;
+      const MxRaw now = kAhead ? cur : Ring::read(buf, k, lane);
+      if (kAhead && k + 1 < kRingSteps) cur = Ring::read(buf, k + 1, lane);  // a step that does not exist: stale bytes, not used
+      if (left == 0) next_head();
+      --left;
       float hv[16], sd[8];
-      mx_decode_scaled(cur.q, cur.e, cur.mic, dA_h, e_max, table, hv, sd);
-      float y = mx_update_readout16<IO::kNibbles>(hv, Bv, Cv, sd, dt_h, sx[row]);  // h' = h exp(A dt) + (B dt) x
-
+      mx_decode_scaled(now.q, now.e, now.mic, dA, e_max, table, hv, sd);
+      float y = mx_update_readout16<IO::kNibbles>(hv, dB, Cv, sd, xp[k * rows_per_step]);  // h' = h exp(A dt) + (B dt) x
       MxRoundCtx ctx = round_ctx_at<MODE>(rb, lin);
       if (kStream) ctx.stream = &stream;
       uint32_t codes[4], e_new, mic_new;
-      mx_encode_block<BITS, MODE, IO::kNibbles>(hv, cut, ctx, d.keys, codes, e_new, mic_new);
-      IO::store_ptr(qptr, eptr, mptr, codes, e_new, mic_new);
-
+      mx_encode_block<BITS, MODE, IO::kNibbles>(hv, ctx, d.keys, codes, e_new, mic_new);
+      IO::store_ptr(qptr + k * Ring::kQ, eptr + k * Ring::kE, mptr + k * Ring::kM, codes, e_new, mic_new);
       if (NBLK_T == 8) {
-        sy[row * 8 + blk] = y;
+        yp[k * kPartialStride] = y;
       } else {
         for (int o = nblk >> 1; o > 0; o >>= 1) y += __shfl_xor_sync(0xFFFFFFFFu, y, o);
-        if (blk == 0) sy[row] = y;
+        if (blk == 0) yp[k * rows_per_step] = y;
       }
-      cur = nxt;
-      qptr = qn; eptr = en; mptr = mn;
-      if (kStream) stream.pa += stream_step; else lin += dl;
-      row += rows_per_pass;
+      if (kStream) stream.pa += static_cast<uint64_t>(kPhiloxM0) * dl; else lin += dl;
     }
-    // the next unit, if any, starts another head; B / C change only with the (batch, group)
-    unit_in_head = 0;
-    ++head_i;
-    if (u < n_units && ++h_in_group == heads_per_group) {
-      h_in_group = 0;
-      if (++g_cur == a.ngroups) {
-        g_cur = 0;
-        ++b_cur;
-      }
-      load_bc16(a.B, a.B_stride, a.B_dtype, b_cur, g_cur, n0, Bv);
-      load_bc16(a.C, a.C_stride, a.C_dtype, b_cur, g_cur, n0, Cv);
-    }
+    __syncwarp();  // the stage has been read
+    Ring::issue(source, stage, lane, todo - len - (kRingStages - 1) * kRingSteps);
+    qptr += len * Ring::kQ; eptr += len * Ring::kE; mptr += len * Ring::kM;
+    xp += len * rows_per_step;
+    yp += len * (NBLK_T == 8 ? kPartialStride : rows_per_step);
+    stage ^= 1u;
   }
   __syncthreads();
   // y = <h', C> + D x (* z), stored for the whole slab at once
-  for (int i = threadIdx.x; i < n_rows; i += kFastThreads) {
+  const auto row_sum = [](const float4& p0, const float4& p1) {  // in the butterfly's order
+    return ((p0.x + p1.x) + (p0.z + p1.z)) + ((p0.y + p1.y) + (p0.w + p1.w));
+  };
+  if (NBLK_T == 8 && d.vec) {  // a thread takes the four rows of a step
+    for (int i = tid; 4 * i < n_rows; i += kFastThreads) {
+      int b, h, p;
+      row_coords(4 * i, b, h, p);
+      const float4* part = reinterpret_cast<const float4*>(sy + i * kPartialStride);
+      float y[4];
+#pragma unroll
+      for (int r = 0; r < 4; ++r) y[r] = row_sum(part[2 * r], part[2 * r + 1]);
+      if (a.D) {
+        const float D = load_as_float(a.D, h * a.D_stride[0], a.D_dtype);
+        const float4 x = reinterpret_cast<const float4*>(sx)[i];
+        y[0] += x.x * D; y[1] += x.y * D; y[2] += x.z * D; y[3] += x.w * D;
+      }
+      uint2 w;
+      if (a.out_dtype == LQ_BF16) {
+        const __nv_bfloat162 lo = __floats2bfloat162_rn(y[0], y[1]), hi = __floats2bfloat162_rn(y[2], y[3]);
+        w = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+      } else {
+        const __half2 lo = __floats2half2_rn(y[0], y[1]), hi = __floats2half2_rn(y[2], y[3]);
+        w = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+      }
+      *reinterpret_cast<uint2*>(static_cast<uint16_t*>(a.out) + b * a.out_stride[0] + h * a.out_stride[1] + p) = w;
+    }
+    return;
+  }
+  for (int i = tid; i < n_rows; i += kFastThreads) {
     int b, h, p;
     row_coords(i, b, h, p);
     float y;
     if (NBLK_T == 8) {
-      const float4 p0 = *reinterpret_cast<const float4*>(sy + i * 8), p1 = *reinterpret_cast<const float4*>(sy + i * 8 + 4);
-      y = ((p0.x + p1.x) + (p0.z + p1.z)) + ((p0.y + p1.y) + (p0.w + p1.w));  // the butterfly's order
+      const float4* part = reinterpret_cast<const float4*>(sy + (i >> 2) * kPartialStride + (i & 3) * 8);
+      y = row_sum(part[0], part[1]);
     } else {
       y = sy[i];
     }
@@ -507,7 +703,6 @@ __global__ void mx_quantize_kernel(const lq_mx_state s, const void* __restrict__
                                    const lq_rounding rnd, const PhiloxKeys keys, int64_t total_blocks) {
   using IO = MxBlockIO<BITS, LAYOUT>;
   const int nblk = s.dstate / 16;
-  const unsigned int* cut = mx_exp_cut_table<BITS>();
   const MxRoundBase rb = make_round_base(rnd, static_cast<uint64_t>(s.batch) * s.heads * s.dim * s.dstate);
   for (int64_t t = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; t < total_blocks;
        t += static_cast<int64_t>(gridDim.x) * blockDim.x) {
@@ -523,7 +718,7 @@ __global__ void mx_quantize_kernel(const lq_mx_state s, const void* __restrict__
     const uint64_t lin = static_cast<uint64_t>(row) * s.dstate + blk * 16;
     const MxRoundCtx ctx = round_ctx_at<MODE>(rb, lin);
     uint32_t codes[4], e, mic;
-    mx_encode_block<BITS, MODE>(hv, cut, ctx, keys, codes, e, mic);
+    mx_encode_block<BITS, MODE>(hv, ctx, keys, codes, e, mic);
     IO::store(s, b * s.q_stride[0] + h * s.q_stride[1] + p * s.q_stride[2],
               b * s.exp_stride[0] + h * s.exp_stride[1] + p * s.exp_stride[2],
               b * s.micro_stride[0] + h * s.micro_stride[1] + p * s.micro_stride[2], blk, codes, e, mic);
@@ -622,31 +817,46 @@ static bool fast_update_applies(const lq_mx_update_args& a, const MxUpdateDerive
                      s.exp_stride[2] == d.nblk && s.exp_stride[1] == static_cast<int64_t>(d.nblk) * s.dim &&
                      s.exp_stride[0] == static_cast<int64_t>(d.nblk) * s.dim * s.heads && s.micro_stride[2] == m_row &&
                      s.micro_stride[1] == m_row * s.dim && s.micro_stride[0] == m_row * s.dim * s.heads;
-  // fewer than 2^31 units keep the kernel's index arithmetic in 32 bits and its multiply-high divisions exact
+  // the ring's 16-byte copies (q_state is aligned in any case)
+  const bool aligned = reinterpret_cast<uintptr_t>(s.q_state) % 16 == 0 && reinterpret_cast<uintptr_t>(s.shared_exp) % 16 == 0 &&
+                       reinterpret_cast<uintptr_t>(s.micro_exp) % 16 == 0;
+  // fewer than 2^30 units (2^31 steps) keep the kernel's index arithmetic in 32 bits and its multiply-high divisions exact
   const uint64_t units = static_cast<uint64_t>(s.batch) * s.heads * (s.dim / rows_per_pass);
   // Philox counters of the layered modes stay in 32 bits
   const int counter_log2 = a.rounding.mode == LQ_ROUND_PHILOX_LAYERED4 ? 2 : 4;
   const uint64_t counters = a.rounding.mode == LQ_ROUND_PHILOX_LAYERED || a.rounding.mode == LQ_ROUND_PHILOX_LAYERED4
                                 ? (static_cast<uint64_t>(s.batch) * s.heads * s.dim * s.dstate) >> counter_log2 : 0;
   return dense && d.dt_uniform && d.a_scalar && a.h_out == nullptr && (1 << d.lpr_log2) == d.nblk &&
-         s.dim % rows_per_pass == 0 && units < (1ull << 31) && counters <= (1ull << 32);
+         s.dim % rows_per_pass == 0 && aligned && units < (1ull << 30) && counters <= (1ull << 32);
 }
 
 template <int BITS, int LAYOUT>
 static void launch_update_mode(const lq_mx_update_args& a, const MxUpdateDerived& d, cudaStream_t st) {
+  using IO = MxBlockIO<BITS, LAYOUT>;
   if (fast_update_applies<BITS, LAYOUT>(a, d)) {
-    // One wave of resident CTAs (8 per SM) when a CTA's slab stays within kMaxUnitsPerCta units
-    // (its x / y staging in shared memory: 36 bytes per row, 18 KB per CTA at most); more waves of equally sized
-    // slabs otherwise.
-    uint64_t kMaxUnitsPerCta = 64;
-    if (const char* env = getenv("LQ_MX_MAX_UNITS")) kMaxUnitsPerCta = std::min(80, std::max(1, atoi(env)));  // tuning aid; 80 units stay under 48 KB
+    // One wave of resident CTAs when a CTA's slab stays within max_units units (its x / y staging: 40 bytes per row, as much as
+    // lets kFastCtasPerSm CTAs share an SM's 228 KB); more waves of equally sized slabs otherwise.
     const int rows_per_pass = (32 >> d.lpr_log2) * (kFastThreads / 32);
+    const size_t row_bytes = sizeof(float) * (d.nblk == 8 ? 1 + kPartialStride / 4 : 2);
+    const auto smem_of = [&](uint64_t units) {
+      const uint64_t heads = units / (a.state.dim / rows_per_pass) + 2, groups = heads / (a.state.heads / a.ngroups) + 2;
+      return MxRing<BITS, LAYOUT>::kBytes + row_bytes * units * rows_per_pass + sizeof(float) * (2 * heads + 2 * a.state.dstate * groups);
+    };
+    const size_t budget = 228 * 1024 / kFastCtasPerSm - 1024 - (IO::kNibbles ? sizeof(MxPairMasks) : sizeof(MxPairFactors));
+    uint64_t max_units = 64;
+    if (const char* env = getenv("LQ_MX_MAX_UNITS")) max_units = std::min(80, std::max(1, atoi(env)));  // tuning aid
+    while (max_units > 1 && smem_of(max_units) > budget) --max_units;
     MxUpdateDerived dd = d;
+    const auto vec16 = [](const void* p, int dtype, const int64_t* st, int mult) {  // 16-bit, innermost contiguous, `mult` elements aligned
+      return dtype != LQ_F32 && st[2] == 1 && st[0] % mult == 0 && st[1] % mult == 0 && reinterpret_cast<uintptr_t>(p) % (2 * mult) == 0;
+    };
+    dd.vec = vec16(a.x, a.x_dtype, a.x_stride, 4) && vec16(a.out, a.out_dtype, a.out_stride, 4) && vec16(a.B, a.B_dtype, a.B_stride, 8) &&
+             vec16(a.C, a.C_dtype, a.C_stride, 8) && a.state.dim % 4 == 0 && !a.z && (!a.D || a.D_stride[1] == 0);
     dd.units_total = static_cast<uint64_t>(a.state.batch) * a.state.heads * (a.state.dim / rows_per_pass);
     const uint64_t wave = static_cast<uint64_t>(kFastCtasPerSm) * sm_count();
     uint64_t ctas = std::min<uint64_t>(dd.units_total, wave);
-    if (dd.units_total > ctas * kMaxUnitsPerCta) {
-      ctas = (dd.units_total + kMaxUnitsPerCta - 1) / kMaxUnitsPerCta;
+    if (dd.units_total > ctas * max_units) {
+      ctas = (dd.units_total + max_units - 1) / max_units;
       ctas = (ctas + wave - 1) / wave * wave;
     }
     dd.units_per_cta = static_cast<uint32_t>(dd.units_total / ctas);
@@ -658,14 +868,13 @@ static void launch_update_mode(const lq_mx_update_args& a, const MxUpdateDerived
       f.magic = static_cast<uint32_t>(((1ull << (32 + f.shift)) + dv - 1) / dv - (1ull << 32));
       return f;
     };
-    dd.div_units_per_head = fast_div_of(static_cast<uint32_t>(a.state.dim / rows_per_pass));
+    dd.div_steps_per_head = fast_div_of(static_cast<uint32_t>(2 * (a.state.dim / rows_per_pass)));
+    dd.div_groups = fast_div_of(static_cast<uint32_t>(a.ngroups));
     dd.div_heads = fast_div_of(static_cast<uint32_t>(a.state.heads));
     dd.div_dim = fast_div_of(static_cast<uint32_t>(a.state.dim));
     dd.div_heads_per_group = fast_div_of(static_cast<uint32_t>(a.state.heads / a.ngroups));
-    const uint64_t max_units = (dd.units_total + ctas - 1) / ctas;
-    const uint64_t max_heads = max_units / (a.state.dim / rows_per_pass) + 2;
     const dim3 grid(static_cast<unsigned>(ctas)), block(kFastThreads);
-    const size_t smem = sizeof(float) * ((d.nblk == 8 ? 9 : 2) * max_units * rows_per_pass + 2 * max_heads);
+    const size_t smem = smem_of((dd.units_total + ctas - 1) / ctas);
     const MxUpdateDerived& d = dd;
     // Programmatic dependent launch: the kernel may be scheduled while its predecessor in the stream is still
     // running (its CTAs take the slots the predecessor's CTAs leave); it touches no global memory before its
