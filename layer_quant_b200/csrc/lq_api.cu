@@ -1,4 +1,6 @@
 // Library-level entry points: ABI version, last-error text, device properties.
+#include <cstdlib>
+
 #include "lq_common.cuh"
 
 namespace lq {
@@ -18,6 +20,14 @@ int sm_count() {
     cached[dev] = n;
   }
   return cached[dev];
+}
+
+bool use_pdl() {
+  static const bool on = [] {
+    const char* env = getenv("LQ_MX_PDL");
+    return env == nullptr || atoi(env) != 0;
+  }();
+  return on;
 }
 
 int int4_read_device_status(int32_t* status);  // lq_int4_kv.cu

@@ -42,6 +42,40 @@ inline int dtype_bytes(int dt) { return dt == LQ_F32 ? 4 : 2; }
 
 int sm_count();  // multiprocessors of the current device (cached per device; lq_api.cu)
 
+// floor(n / d) for n < 2^31 without a division: (mulhi(n, magic) + n) >> shift
+struct FastDiv {
+  uint32_t magic, shift;
+};
+inline FastDiv fast_div_of(uint32_t d) {
+  FastDiv f;
+  f.shift = 0;
+  while ((1ull << f.shift) < d) ++f.shift;  // ceil(log2 d)
+  f.magic = static_cast<uint32_t>(((1ull << (32 + f.shift)) + d - 1) / d - (1ull << 32));
+  return f;
+}
+__device__ __forceinline__ uint32_t fast_div(uint32_t n, const FastDiv& f) { return (__umulhi(n, f.magic) + n) >> f.shift; }
+
+// Programmatic dependent launch: the kernel may be scheduled while its predecessor in the stream is still running (its CTAs take
+// the slots the predecessor's CTAs leave); it touches no memory before its griddepcontrol.wait, which returns once the
+// predecessor has completed and its writes are visible.  LQ_MX_PDL=0 switches it off.
+bool use_pdl();  // lq_api.cu
+template <class... Params, class... Args>
+inline cudaError_t launch_dependent(void (*kernel)(Params...), dim3 grid, unsigned block, size_t smem, cudaStream_t stream, const Args&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = use_pdl() ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+__device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // ---- device helpers --------------------------------------------------------------------------
 __device__ __forceinline__ float load_as_float(const void* p, int64_t i, int dt) {
   if (dt == LQ_BF16) return __bfloat162float(static_cast<const __nv_bfloat16*>(p)[i]);

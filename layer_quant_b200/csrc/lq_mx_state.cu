@@ -168,12 +168,10 @@ struct MxUpdateDerived {
   PhiloxKeys keys;        // round keys of rounding.seed
   uint64_t units_total;   // fast path: batch * heads * dim / rows per pass (< 2^31)
   // fast path: the slab of a CTA without a division.  units_per_cta / units_rem: CTA c owns units_per_cta units, the
-  // first units_rem CTAs one more.  FastDiv: floor(n / d) for n < 2^31 as (mulhi(n, magic) + n) >> shift.
+  // first units_rem CTAs one more
   uint32_t units_per_cta, units_rem;
-  struct FastDiv { uint32_t magic, shift; } div_steps_per_head, div_heads, div_dim, div_heads_per_group, div_groups;
+  FastDiv div_steps_per_head, div_heads, div_dim, div_heads_per_group, div_groups;
 };
-
-__device__ __forceinline__ uint32_t fast_div(uint32_t n, const MxUpdateDerived::FastDiv& f) { return (__umulhi(n, f.magic) + n) >> f.shift; }
 
 // One CTA = `hpc` consecutive heads of one (batch, B/C group): B and C are fetched once and stay in
 // registers for hpc * dim rows.  gridDim.x = batch * (heads / hpc).
@@ -430,7 +428,7 @@ __global__ void __launch_bounds__(kFastThreads, kFastCtasPerSm) mx_state_update_
   const uint32_t u0 = blockIdx.x * d.units_per_cta + min(blockIdx.x, d.units_rem);
   const uint32_t n_units = d.units_per_cta + (blockIdx.x < d.units_rem ? 1u : 0u);
   // let the next kernel in the stream be scheduled behind this one (no effect without the launch attribute)
-  asm volatile("griddepcontrol.launch_dependents;");
+  pdl_launch_dependents();
   if (n_units == 0) return;
   const uint64_t R0 = static_cast<uint64_t>(u0) * rows_per_unit;
   const int n_rows = static_cast<int>(n_units) * rows_per_unit;
@@ -478,8 +476,16 @@ __global__ void __launch_bounds__(kFastThreads, kFastCtasPerSm) mx_state_update_
   uint8_t* const ring = smem_fast + warp * (kRingStages * Ring::kStage);
   typename Ring::Source source(static_cast<uint32_t>(__cvta_generic_to_shared(ring)), static_cast<const uint8_t*>(s.q_state) + block0 * IO::kQBytes,
                                s.shared_exp + block0, s.micro_exp + block0 * IO::kMicroBytes, lane);
+  // what the first stages will read, asked for in L2 while the predecessor still runs (a prefetch reads nothing): 10.6 -> 10.1 us at
+  // batch 8
+  if (lane == 0) {
+    const uint32_t ahead = min(n_units, static_cast<uint32_t>(kRingSteps));
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(static_cast<const uint8_t*>(s.q_state) + block0 * IO::kQBytes), "r"(ahead * Ring::kQ) : "memory");
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(s.shared_exp + block0), "r"(ahead * Ring::kE) : "memory");
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(s.micro_exp + block0 * IO::kMicroBytes), "r"(ahead * Ring::kM) : "memory");
+  }
   // everything above is arithmetic on the arguments; from here on memory the predecessor may have written is read
-  asm volatile("griddepcontrol.wait;" ::: "memory");
+  pdl_wait();
   // the first stages travel while the operands below are staged
   Ring::issue(source, 0, lane, min(n_mine, kFirstSteps), kFirstSteps);
 
@@ -725,6 +731,45 @@ __global__ void mx_quantize_kernel(const lq_mx_state s, const void* __restrict__
   }
 }
 
+// Dense state and source: block t of one is block t of the other, 32 or 64 bytes in and one block out per thread, nothing divided.
+// Bound by the bytes: 8 x 128 x 64 x 128 values from bf16, 26 MB: 11.2 -> 5 us.
+template <int BITS, int LAYOUT, int MODE, int SRC>
+__global__ void __launch_bounds__(128) mx_quantize_dense_kernel(const lq_mx_state s, const void* src, const lq_rounding rnd, const PhiloxKeys keys,
+                                                                int64_t total_blocks, uint64_t numel) {
+  using IO = MxBlockIO<BITS, LAYOUT>;
+  pdl_launch_dependents();
+  const int64_t t = blockIdx.x * 128ll + threadIdx.x;
+  pdl_wait();
+  if (t >= total_blocks) return;
+  float hv[16];
+  if (SRC == LQ_F32) {
+    const float4* p = static_cast<const float4*>(src) + t * 4;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float4 f = p[i];
+      hv[4 * i] = f.x; hv[4 * i + 1] = f.y; hv[4 * i + 2] = f.z; hv[4 * i + 3] = f.w;
+    }
+  } else {
+    const uint4* p = static_cast<const uint4*>(src) + t * 2;
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const uint4 q = p[i];
+      const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float2 f = SRC == LQ_BF16 ? make_float2(__uint_as_float(w[j] << 16), __uint_as_float(w[j] & 0xFFFF0000u))
+                                        : __half22float2(*reinterpret_cast<const __half2*>(&w[j]));
+        hv[8 * i + 2 * j] = f.x;
+        hv[8 * i + 2 * j + 1] = f.y;
+      }
+    }
+  }
+  const MxRoundCtx ctx = round_ctx_at<MODE>(make_round_base(rnd, numel), static_cast<uint64_t>(t) * 16);
+  uint32_t codes[4], e, mic;
+  mx_encode_block<BITS, MODE, IO::kNibbles>(hv, ctx, keys, codes, e, mic);
+  IO::store_ptr(static_cast<uint8_t*>(s.q_state) + t * IO::kQBytes, s.shared_exp + t, s.micro_exp + t * IO::kMicroBytes, codes, e, mic);
+}
+
 template <int BITS, int LAYOUT>
 __global__ void mx_dequantize_kernel(const lq_mx_state s, float* __restrict__ dst, int64_t dst_row_stride, int64_t total_blocks) {
   using IO = MxBlockIO<BITS, LAYOUT>;
@@ -861,42 +906,18 @@ static void launch_update_mode(const lq_mx_update_args& a, const MxUpdateDerived
     }
     dd.units_per_cta = static_cast<uint32_t>(dd.units_total / ctas);
     dd.units_rem = static_cast<uint32_t>(dd.units_total % ctas);
-    auto fast_div_of = [](uint32_t dv) {
-      MxUpdateDerived::FastDiv f;
-      f.shift = 0;
-      while ((1ull << f.shift) < dv) ++f.shift;  // ceil(log2 dv)
-      f.magic = static_cast<uint32_t>(((1ull << (32 + f.shift)) + dv - 1) / dv - (1ull << 32));
-      return f;
-    };
     dd.div_steps_per_head = fast_div_of(static_cast<uint32_t>(2 * (a.state.dim / rows_per_pass)));
     dd.div_groups = fast_div_of(static_cast<uint32_t>(a.ngroups));
     dd.div_heads = fast_div_of(static_cast<uint32_t>(a.state.heads));
     dd.div_dim = fast_div_of(static_cast<uint32_t>(a.state.dim));
     dd.div_heads_per_group = fast_div_of(static_cast<uint32_t>(a.state.heads / a.ngroups));
-    const dim3 grid(static_cast<unsigned>(ctas)), block(kFastThreads);
+    const unsigned grid = static_cast<unsigned>(ctas);
     const size_t smem = smem_of((dd.units_total + ctas - 1) / ctas);
     const MxUpdateDerived& d = dd;
-    // Programmatic dependent launch: the kernel may be scheduled while its predecessor in the stream is still
-    // running (its CTAs take the slots the predecessor's CTAs leave); it touches no global memory before its
-    // griddepcontrol.wait, which returns once the predecessor has completed and its writes are visible.
-    static const bool pdl = [] {
-      const char* env = getenv("LQ_MX_PDL");
-      return env == nullptr || atoi(env) != 0;
-    }();
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = block;
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = pdl ? 1 : 0;
 #define LQ_FAST_LAUNCH(MODE_)                                                                         \
   do {                                                                                               \
-    if (d.nblk == 8) cudaLaunchKernelEx(&cfg, mx_state_update_fast_kernel<BITS, LAYOUT, MODE_, 8>, a, d); \
-    else cudaLaunchKernelEx(&cfg, mx_state_update_fast_kernel<BITS, LAYOUT, MODE_, 0>, a, d);         \
+    if (d.nblk == 8) launch_dependent(mx_state_update_fast_kernel<BITS, LAYOUT, MODE_, 8>, grid, kFastThreads, smem, st, a, d); \
+    else launch_dependent(mx_state_update_fast_kernel<BITS, LAYOUT, MODE_, 0>, grid, kFastThreads, smem, st, a, d); \
   } while (0)
     switch (a.rounding.mode) {
       case LQ_ROUND_HALF_UP: LQ_FAST_LAUNCH(LQ_ROUND_HALF_UP); break;
@@ -929,6 +950,20 @@ static void launch_quantize_mode(const lq_mx_state& s, const void* src, int dt, 
   const int block = 128;
   const int grid = static_cast<int>(std::min<int64_t>((total + block - 1) / block, 1 << 20));
   const PhiloxKeys keys = make_philox_keys(r.seed);
+  using IO = MxBlockIO<BITS, LAYOUT>;
+  const int64_t nblk = s.dstate / 16, rows_b = static_cast<int64_t>(s.heads) * s.dim;
+  const bool dense = stride == s.dstate && s.q_stride[2] == nblk * IO::kQBytes && s.exp_stride[2] == nblk && s.micro_stride[2] == nblk * IO::kMicroBytes &&
+                     (s.heads == 1 || (s.q_stride[1] == s.dim * s.q_stride[2] && s.exp_stride[1] == s.dim * nblk && s.micro_stride[1] == s.dim * s.micro_stride[2])) &&
+                     (s.batch == 1 || (s.q_stride[0] == rows_b * s.q_stride[2] && s.exp_stride[0] == rows_b * nblk && s.micro_stride[0] == rows_b * s.micro_stride[2]));
+  // the rounding of the one-off quantiser; the other modes (tests, tools) stay on the general kernel
+  if (r.mode == LQ_ROUND_HALF_EVEN && dense && reinterpret_cast<uintptr_t>(src) % 16 == 0 && total < (1ll << 37)) {
+    const unsigned g = static_cast<unsigned>((total + 127) / 128);
+    const uint64_t numel = static_cast<uint64_t>(total) * 16;
+    if (dt == LQ_BF16) launch_dependent(mx_quantize_dense_kernel<BITS, LAYOUT, LQ_ROUND_HALF_EVEN, LQ_BF16>, g, 128, 0, st, s, src, r, keys, total, numel);
+    else if (dt == LQ_F16) launch_dependent(mx_quantize_dense_kernel<BITS, LAYOUT, LQ_ROUND_HALF_EVEN, LQ_F16>, g, 128, 0, st, s, src, r, keys, total, numel);
+    else launch_dependent(mx_quantize_dense_kernel<BITS, LAYOUT, LQ_ROUND_HALF_EVEN, LQ_F32>, g, 128, 0, st, s, src, r, keys, total, numel);
+    return;
+  }
   switch (r.mode) {
     case LQ_ROUND_HALF_UP: mx_quantize_kernel<BITS, LAYOUT, LQ_ROUND_HALF_UP><<<grid, block, 0, st>>>(s, src, dt, stride, r, keys, total); break;
     case LQ_ROUND_HALF_EVEN: mx_quantize_kernel<BITS, LAYOUT, LQ_ROUND_HALF_EVEN><<<grid, block, 0, st>>>(s, src, dt, stride, r, keys, total); break;
