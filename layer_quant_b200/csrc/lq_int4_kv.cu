@@ -165,61 +165,88 @@ __global__ void int4_append_kernel(const AppendParams p, int64_t total_chunks, i
   }
 }
 
-// The usual case: 16-bit K and V with contiguous, 16-byte aligned rows, group size 32, 64 or 128, head dim 128.  A thread takes 16 bytes of
-// a row (eight values) and makes one 32-bit word; a warp takes two consecutive tokens of a head, so its stores are
-// 128 contiguous bytes.  gridDim.y = 2: K, V.
-// It is the divisions that bound a kernel like this.  code = rint(x / scale) with IEEE division; here x times the reciprocal (error
-// below 2^-20 at |x / scale| <= 7, the reciprocal's 2^-23 included) decides unless it lies within 1e-5 of a rounding edge, where the
-// division decides (NaN and infinity end up there as well).  8 x 1024 tokens: 38 -> 9 us.
+// x / d, with inv the rounded reciprocal of d: an approximate quotient and one correction from its exact remainder (Markstein,
+// "Computation of elementary functions on the IBM RISC System/6000 processor", 1990).  For x of a 16-bit type this is the
+// correctly rounded quotient wherever the codec can tell (every pair of values is tried in the tests); finite x and d only.
+__device__ __forceinline__ float quotient16(float x, float d, float inv) {
+  const float q = x * inv;
+  return fmaf(fmaf(-q, d, x), inv, q);
+}
+__device__ __forceinline__ float max_nan(float a, float b) {
+  float r;
+  asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+  return r;
+}
+
+// The usual case: 16-bit K and V with contiguous, 16-byte aligned rows, group size 32, 64 or 128, head dim 128.  A thread takes 16 bytes
+// (eight values, one 32-bit word of codes) of two rows, of K and of V; a warp's stores are 128 contiguous bytes (two
+// consecutive tokens of a head).  Divisions are what such a kernel spends its time on, so they are multiplications here
+// (quotient16), codes are gathered with one shift-and-add each, and the index arithmetic serves four chunks.
+// 8 x 1024 tokens: 38 -> 14 us.
+constexpr int kAppendRows = 32;  // rows per CTA
 template <int DT>
-__global__ void __launch_bounds__(256) int4_append_vec_kernel(const AppendParams p, const FastDiv div_tokens, const FastDiv div_heads, uint32_t total,
+__global__ void __launch_bounds__(256) int4_append_vec_kernel(const AppendParams p, const FastDiv div_tokens, const FastDiv div_heads, uint32_t rows,
                                                               int lanes_per_group_log2) {
   pdl_launch_dependents();
-  const uint32_t i = blockIdx.x * 256 + threadIdx.x;
-  const bool v_side = blockIdx.y != 0;
-  const uint32_t row = min(i, total - 1) >> 4, chunk = threadIdx.x & 15;
-  const uint32_t bh = fast_div(row, div_tokens), tok = row - bh * static_cast<uint32_t>(p.q_len);
-  const uint32_t b = fast_div(bh, div_heads), h = bh - b * static_cast<uint32_t>(p.c.kv_heads);
-  const int64_t* ss = v_side ? p.vs : p.ks;
-  const int64_t* ps = v_side ? p.c.vp_stride : p.c.kp_stride;
-  const int64_t* sst = v_side ? p.c.vs_stride : p.c.ks_stride;
-  const uint16_t* src = static_cast<const uint16_t*>(v_side ? p.v : p.k) + b * ss[0] + h * ss[1] + tok * ss[2] + chunk * 8;
-  uint8_t* const packed = (v_side ? p.c.v_packed : p.c.k_packed) + b * ps[0] + h * ps[1] + chunk * 4;
-  float* const scales = (v_side ? p.c.v_scale : p.c.k_scale) + b * sst[0] + h * sst[1];
+  const uint32_t chunk = threadIdx.x & 15, row0 = blockIdx.x * kAppendRows + (threadIdx.x >> 4);
+  uint32_t b[2], h[2], tok[2];
+#pragma unroll
+  for (int j = 0; j < 2; ++j) {
+    const uint32_t row = min(row0 + 16 * j, rows - 1);
+    const uint32_t bh = fast_div(row, div_tokens);
+    tok[j] = row - bh * static_cast<uint32_t>(p.q_len);
+    b[j] = fast_div(bh, div_heads);
+    h[j] = bh - b[j] * static_cast<uint32_t>(p.c.kv_heads);
+  }
   pdl_wait();
-  const uint4 raw = *reinterpret_cast<const uint4*>(src);
-  const int64_t pos = p.positions[tok];
-  const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
-  float x[8];
-  float amax = 0.0f;
+  uint4 raw[2][2];
+  int64_t pos[2];
 #pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    const float2 f = DT == LQ_BF16 ? make_float2(__uint_as_float(w[k] << 16), __uint_as_float(w[k] & 0xFFFF0000u))
-                                   : __half22float2(*reinterpret_cast<const __half2*>(&w[k]));
-    x[2 * k] = f.x;
-    x[2 * k + 1] = f.y;
-    amax = fmaxf(amax, fmaxf(fabsf(f.x), fabsf(f.y)));
+  for (int j = 0; j < 2; ++j) {
+    raw[j][0] = *reinterpret_cast<const uint4*>(static_cast<const uint16_t*>(p.k) + b[j] * p.ks[0] + h[j] * p.ks[1] + tok[j] * p.ks[2] + chunk * 8);
+    raw[j][1] = *reinterpret_cast<const uint4*>(static_cast<const uint16_t*>(p.v) + b[j] * p.vs[0] + h[j] * p.vs[1] + tok[j] * p.vs[2] + chunk * 8);
+    pos[j] = p.positions[tok[j]];
   }
-  for (int o = (1 << lanes_per_group_log2) >> 1; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, o));
-  const float scale = int4_scale(amax);
-  const float inv = __frcp_rn(scale);
-  uint32_t word = 0;
-  bool edge = false;
 #pragma unroll
-  for (int k = 0; k < 8; ++k) {
-    const float t = x[k] * inv;
-    const float m = t + 12582912.0f;  // 1.5 * 2^23: the nearest integer is in the low bits
-    edge |= !(fabsf(t - (m - 12582912.0f)) < 0.49999f);
-    word |= (__float_as_uint(m) & 15u) << (4 * k);
-  }
-  if (edge) {
-    word = 0;
+  for (int j = 0; j < 2; ++j)
 #pragma unroll
-    for (int k = 0; k < 8; ++k) word |= int4_code(x[k], scale) << (4 * k);
-  }
-  if (i >= total) return;
-  *reinterpret_cast<uint32_t*>(packed + pos * ps[2]) = word;
-  if ((chunk & ((1u << lanes_per_group_log2) - 1)) == 0) scales[pos * sst[2] + (chunk >> lanes_per_group_log2) * sst[3]] = scale;
+    for (int side = 0; side < 2; ++side) {
+      const uint32_t w[4] = {raw[j][side].x, raw[j][side].y, raw[j][side].z, raw[j][side].w};
+      float x[8];
+      float amax = 0.0f;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const float2 f = DT == LQ_BF16 ? make_float2(__uint_as_float(w[k] << 16), __uint_as_float(w[k] & 0xFFFF0000u))
+                                       : __half22float2(*reinterpret_cast<const __half2*>(&w[k]));
+        x[2 * k] = f.x;
+        x[2 * k + 1] = f.y;
+        amax = max_nan(amax, max_nan(fabsf(f.x), fabsf(f.y)));
+      }
+      for (int o = (1 << lanes_per_group_log2) >> 1; o > 0; o >>= 1) amax = max_nan(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, o));
+      float scale = fmaxf(quotient16(amax, 7.0f, 1.0f / 7.0f), 1.0e-8f);
+      uint32_t word = 0;
+      if (__all_sync(0xFFFFFFFFu, amax < INFINITY)) {
+        const float inv = __frcp_rn(scale);
+        constexpr uint32_t kMagicBits = 0x4B400008u;  // 1.5 * 2^23 + 8: the low bits of q + it are the nearest integer + 8, in [1, 15]
+#pragma unroll
+        for (int k = 7; k >= 0; --k) word = (word << 4) + (__float_as_uint(quotient16(x[k], scale, inv) + __uint_as_float(kMagicBits)) - (kMagicBits & ~15u));
+        word ^= 0x88888888u;
+      } else {  // infinities or NaNs in some group of the warp
+        amax = 0.0f;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) amax = fmaxf(amax, fabsf(x[k]));
+        for (int o = (1 << lanes_per_group_log2) >> 1; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, o));
+        scale = int4_scale(amax);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) word |= int4_code(x[k], scale) << (4 * k);
+      }
+      if (row0 + 16 * j >= rows) continue;
+      const int64_t* ps = side ? p.c.vp_stride : p.c.kp_stride;
+      const int64_t* sst = side ? p.c.vs_stride : p.c.ks_stride;
+      *reinterpret_cast<uint32_t*>((side ? p.c.v_packed : p.c.k_packed) + b[j] * ps[0] + h[j] * ps[1] + pos[j] * ps[2] + chunk * 4) = word;
+      if ((chunk & ((1u << lanes_per_group_log2) - 1)) == 0)
+        (side ? p.c.v_scale : p.c.k_scale)[b[j] * sst[0] + h[j] * sst[1] + pos[j] * sst[2] + (chunk >> lanes_per_group_log2) * sst[3]] = scale;
+    }
 }
 
 // Any even group size: one thread per group.
@@ -813,10 +840,10 @@ LQ_EXPORT int lq_int4_kv_append(const lq_int4_cache* cache, const void* k, const
     return s[3] == 1 && s[0] % 4 == 0 && s[1] % 4 == 0 && s[2] % 4 == 0 && reinterpret_cast<uintptr_t>(ptr) % 4 == 0;
   };
   if (dtype != LQ_F32 && D == 128 && (gs == 32 || gs == 64 || gs == 128) && rows16(k, k_stride) && rows16(v, v_stride) &&
-      words(cache->k_packed, cache->kp_stride) && words(cache->v_packed, cache->vp_stride) && rows / 2 * 16 < (1ll << 31)) {
-    const uint32_t total = static_cast<uint32_t>(rows / 2 * 16);
+      words(cache->k_packed, cache->kp_stride) && words(cache->v_packed, cache->vp_stride) && rows / 2 < (1ll << 31) - kAppendRows) {
+    const uint32_t total = static_cast<uint32_t>(rows / 2);
     const FastDiv div_tokens = fast_div_of(static_cast<uint32_t>(q_len)), div_heads = fast_div_of(static_cast<uint32_t>(cache->kv_heads));
-    const dim3 grid((total + 255) / 256, 2);
+    const unsigned grid = (total + kAppendRows - 1) / kAppendRows;
     LQ_CHECK_CUDA(dtype == LQ_BF16 ? launch_dependent(int4_append_vec_kernel<LQ_BF16>, grid, 256, 0, st, p, div_tokens, div_heads, total, lg)
                                    : launch_dependent(int4_append_vec_kernel<LQ_F16>, grid, 256, 0, st, p, div_tokens, div_heads, total, lg));
     return LQ_OK;

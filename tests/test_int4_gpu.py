@@ -413,3 +413,57 @@ def test_prefill_tensor_core_edges(ratio, tq, first, k_size, v_size):
         assert_out_close(out, ref)
     from layer_quant_b200 import _lib
     assert _lib.device_status() == 0
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_append_divisions_exhaustively(dtype):
+    """The 16-bit append forms its quotients without a division: against IEEE division (numpy, and the fp32 kernel) for every
+    mantissa of the group's largest value, every mantissa below it and the exponents at which a code can differ from 0."""
+    m = ia()
+    bits, exps = (7, 5) if dtype == torch.bfloat16 else (10, 5)
+    n = 1 << bits
+    mant = 1.0 + np.arange(n) / n
+    step = 1 if dtype == torch.bfloat16 else 3  # a third of the fp16 maxima (the scale depends on nothing else)
+    cols = 126  # values beside the maximum and its negative in a row of one group
+    vals = (mant[None, :] * 2.0 ** -np.arange(exps)[:, None]).reshape(-1)
+    pad = -len(vals) % cols
+    vals = np.concatenate([vals, np.zeros(pad)]).reshape(-1, cols)
+    amax = mant[::step]
+    for at in range(0, len(amax), 64):
+        a = amax[at:at + 64]
+        x = np.empty((len(a), len(vals), 128), np.float32)
+        x[:, :, 0] = a[:, None] * 2
+        x[:, :, 1] = -a[:, None] * 2
+        x[:, :, 2:] = np.minimum(vals[None], a[:, None, None] * 2)
+        k = torch.from_numpy(x).to(dtype).reshape(1, 1, -1, 128)
+        assert torch.equal(k.float().reshape(x.shape), torch.from_numpy(x))
+        rows = k.shape[2]
+        got, ref = (m._allocate_layer_cache(1, 1, rows, 128, 1, dev()) for _ in range(2))
+        pos = torch.arange(rows, device=dev())
+        m._pack_kv_into_cache(got, k.to(dev()), -k.to(dev()), pos, 128)
+        m._pack_kv_into_cache(ref, k.float().to(dev()), -k.float().to(dev()), pos, 128)
+        for name in ("k_packed", "v_packed", "k_scale", "v_scale"):
+            assert torch.equal(getattr(got, name), getattr(ref, name)), name
+    q, s = oracle.int4_encode(x.reshape(1, 1, -1, 128), 128)
+    assert np.array_equal(got.k_packed.cpu().numpy(), oracle.int4_pack_nibbles(q)) and np.array_equal(got.k_scale.cpu().numpy(), s)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_append_vector_path_extremes(dtype):
+    """Infinities, NaNs, zero groups and groups at the scale's floor: as the general kernel packs them, group by group."""
+    m = ia()
+    g = torch.Generator().manual_seed(4)
+    k = torch.randn(2, 2, 19, 128, generator=g)
+    k[0, 0, 0, 5] = float("inf"); k[0, 1, 1, 70] = float("nan"); k[1, 0, 2, :32] = 0.0; k[1, 1, 3, 32:64] = float("nan")
+    k[1, 1, 4, :64] *= 1e-7; k[1, 1, 5] *= 1e-9; k[0, 0, 6, 3] = -float("inf"); k[0, 0, 6, 4] = float("nan")
+    k = k.to(dtype)
+    pos = torch.randperm(40, generator=g)[:19].to(dev())
+    for gs in (32, 64, 128):
+        got, ref = (m._allocate_layer_cache(2, 2, 64, 128, 128 // gs, dev()) for _ in range(2))
+        for c in (got, ref):
+            for x in (c.k_packed, c.v_packed, c.k_scale, c.v_scale):
+                x.zero_()
+        m._pack_kv_into_cache(got, k.to(dev()), k.flip(0).to(dev()), pos, gs)
+        m._pack_kv_into_cache(ref, k.float().to(dev()), k.float().flip(0).to(dev()), pos, gs)
+        for name in ("k_packed", "v_packed", "k_scale", "v_scale"):
+            assert torch.equal(getattr(got, name).view(torch.uint8), getattr(ref, name).view(torch.uint8)), (gs, name)
