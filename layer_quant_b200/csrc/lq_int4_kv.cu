@@ -685,6 +685,7 @@ __global__ void __launch_bounds__(kDecodeThreads, 1) int4_decode_kernel(const De
 }  // namespace lq
 
 #include "lq_int4_mma.cuh"
+#include "lq_int4_decode.cuh"
 #include "lq_int4_prefill.cuh"
 
 namespace lq {
@@ -764,19 +765,21 @@ static int launch_decode(const DecodeParams& p, cudaStream_t st) {
 
 template <int R, int GS>
 static int launch_decode_mma(const DecodeParams& p, cudaStream_t st) {
-  using L = mma::TileLayout<GS>;
-  const size_t smem = mma::kStagesM * L::kStage + L::kNewBytes;
-  const dim3 grid(p.splits, p.a.cache.kv_heads, p.a.cache.batch), block(mma::kThreadsM);
-#define LQ_MMA_LAUNCH(MASK_, SPLIT_)                                                                                \
+  constexpr size_t smem = mma::WarpStage<GS>::kSmem;
+  const dim3 grid(p.splits, p.a.cache.kv_heads, p.a.cache.batch);
+#define LQ_MMA_LAUNCH(MASK_, QM_)                                                                                   \
   do {                                                                                                              \
-    LQ_SET_SMEM_ONCE((mma::int4_decode_mma_kernel<R, GS, MASK_, SPLIT_>), smem);                                    \
-    mma::int4_decode_mma_kernel<R, GS, MASK_, SPLIT_><<<grid, block, smem, st>>>(p);                                \
+    LQ_SET_SMEM_ONCE((mma::int4_decode_warp_kernel<R, GS, MASK_, QM_>), smem);                                      \
+    if (dependent) LQ_CHECK_CUDA(launch_dependent(mma::int4_decode_warp_kernel<R, GS, MASK_, QM_>, grid, mma::kThreadsM, smem, st, p)); \
+    else mma::int4_decode_warp_kernel<R, GS, MASK_, QM_><<<grid, mma::kThreadsM, smem, st>>>(p);                    \
   } while (0)
-  const bool qsplit = p.a.dtype != LQ_BF16;
+  // A dependent launch is placed while its predecessor still runs.  Where every SM gets one CTA at most that hides launch and set-up; a
+  // larger grid would be dealt unevenly around the predecessor's last CTAs.
+  const bool dependent = static_cast<int64_t>(grid.x) * grid.y * grid.z <= sm_count();
   if (p.a.mask) {
-    if (qsplit) LQ_MMA_LAUNCH(true, true); else LQ_MMA_LAUNCH(true, false);
+    if (p.a.dtype == LQ_BF16) LQ_MMA_LAUNCH(true, mma::kQBf16); else if (p.a.dtype == LQ_F16) LQ_MMA_LAUNCH(true, mma::kQF16); else LQ_MMA_LAUNCH(true, mma::kQF32);
   } else {
-    if (qsplit) LQ_MMA_LAUNCH(false, true); else LQ_MMA_LAUNCH(false, false);
+    if (p.a.dtype == LQ_BF16) LQ_MMA_LAUNCH(false, mma::kQBf16); else if (p.a.dtype == LQ_F16) LQ_MMA_LAUNCH(false, mma::kQF16); else LQ_MMA_LAUNCH(false, mma::kQF32);
   }
 #undef LQ_MMA_LAUNCH
   LQ_CHECK_CUDA(cudaGetLastError());
