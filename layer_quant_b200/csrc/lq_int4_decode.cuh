@@ -403,24 +403,31 @@ __global__ void __launch_bounds__(kThreadsM, (R <= 4 && QM != kQF32) ? 3 : 2) in
   // ---- main loop -------------------------------------------------------------------------------------------
   // The biases of a stage's tokens (rows g and g + 8 of its two steps) are fetched a stage ahead: a mask read where it is used
   // would put a global load into every step.
-  float bias[2][2] = {{0.0f, 0.0f}, {0.0f, 0.0f}}, bias_next[2][2];
-  auto fetch_bias = [&](int first, float (&v)[2][2]) {
+  uint2 raw_next[2][2];
+  auto fetch_mask = [&](int first) {
 #pragma unroll
     for (int st = 0; st < 2; ++st)
 #pragma unroll
       for (int r = 0; r < 2; ++r) {
         const int n = first + 16 * st + 8 * r + g;
-        v[st][r] = n < tok_end ? mask_bias(a, b, n) : 0.0f;
+        if (n < min(tok_end, a.mask_k_len)) raw_next[st][r] = mask_load(a, b, n);
       }
   };
-  if (HAS_MASK) fetch_bias(tok, bias);
+  if (HAS_MASK) fetch_mask(tok);
   uint32_t cur = 0;
 #pragma unroll 1
   while (tok < tok_end) {
     cp_async_wait<kStagesD - 2>();
     __syncwarp();  // the stage has landed for the whole warp, and the whole warp is done with the one before
     issue();
-    if (HAS_MASK) fetch_bias(tok + kStageTok, bias_next);
+    float bias[2][2] = {{0.0f, 0.0f}, {0.0f, 0.0f}};
+    if (HAS_MASK) {
+#pragma unroll
+      for (int st = 0; st < 2; ++st)
+#pragma unroll
+        for (int r = 0; r < 2; ++r) bias[st][r] = tok + 16 * st + 8 * r + g < a.mask_k_len ? mask_value(a, raw_next[st][r]) : -INFINITY;
+      fetch_mask(tok + kStageTok);
+    }
     const uint8_t* const stage = smem + warp * L::kWarp + cur;
     const uint32_t sb = ring + cur;
     if (tok_end - tok >= kStageTok) {
@@ -434,13 +441,6 @@ __global__ void __launch_bounds__(kThreadsM, (R <= 4 && QM != kQF32) ? 3 : 2) in
         const float bs[2] = {st ? bias[1][0] : bias[0][0], st ? bias[1][1] : bias[0][1]};
         step16(std::false_type{}, sb + L::kKc + st * 1024, sb + L::kVc + st * 1024, stage + L::kKs + st * (16 * G * 4),
                stage + L::kVs + st * (16 * G * 4), tok_end - tok - 16 * st, bs);
-      }
-    }
-    if (HAS_MASK) {
-#pragma unroll
-      for (int st = 0; st < 2; ++st) {
-        bias[st][0] = bias_next[st][0];
-        bias[st][1] = bias_next[st][1];
       }
     }
     tok += kStageTok;

@@ -93,19 +93,26 @@ __device__ __forceinline__ uint32_t int4_code(float x, float scale) {
   return static_cast<uint32_t>(q) & 15u;
 }
 
-// Bias of token n in sequence b: the mask in the caller's own type, read where it is used (a 2-D tokenizer mask costs no
-// conversion pass); tokens past the mask are masked out.
-__device__ __forceinline__ float mask_bias(const lq_int4_decode_args& a, int b, int n) {
-  if (n >= a.mask_k_len) return -INFINITY;
+// The mask in the caller's own type (a 2-D tokenizer mask costs no conversion pass), in two parts, so that an element can be
+// requested long before it is used: its bits as loaded, and the bias of a token that they mean.
+__device__ __forceinline__ uint2 mask_load(const lq_int4_decode_args& a, int b, int n) {
   const int64_t i = b * a.mask_stride_b + n * a.mask_stride_k;
-  switch (a.mask_kind) {
-    case LQ_MASK_ADD_F32: return static_cast<const float*>(a.mask)[i];
-    case LQ_MASK_ADD_BF16: return load_as_float(a.mask, i, LQ_BF16);
-    case LQ_MASK_ADD_F16: return load_as_float(a.mask, i, LQ_F16);
-    case LQ_MASK_KEEP_U8: return static_cast<const uint8_t*>(a.mask)[i] ? 0.0f : -INFINITY;
-    case LQ_MASK_KEEP_I32: return static_cast<const int32_t*>(a.mask)[i] ? 0.0f : -INFINITY;
-    default: return static_cast<const long long*>(a.mask)[i] ? 0.0f : -INFINITY;
-  }
+  uint2 raw = make_uint2(0u, 0u);
+  if (a.mask_kind == LQ_MASK_KEEP_I64) raw = static_cast<const uint2*>(a.mask)[i];
+  else if (a.mask_kind == LQ_MASK_ADD_F32 || a.mask_kind == LQ_MASK_KEEP_I32) raw.x = static_cast<const uint32_t*>(a.mask)[i];
+  else if (a.mask_kind == LQ_MASK_KEEP_U8) raw.x = static_cast<const uint8_t*>(a.mask)[i];
+  else raw.x = static_cast<const uint16_t*>(a.mask)[i];
+  return raw;
+}
+__device__ __forceinline__ float mask_value(const lq_int4_decode_args& a, uint2 raw) {
+  if (a.mask_kind >= LQ_MASK_KEEP_U8) return (raw.x | raw.y) ? 0.0f : -INFINITY;
+  if (a.mask_kind == LQ_MASK_ADD_F32) return __uint_as_float(raw.x);
+  if (a.mask_kind == LQ_MASK_ADD_BF16) return __uint_as_float(raw.x << 16);
+  return __half2float(__ushort_as_half(static_cast<unsigned short>(raw.x)));
+}
+// Bias of token n in sequence b; tokens past the mask are masked out
+__device__ __forceinline__ float mask_bias(const lq_int4_decode_args& a, int b, int n) {
+  return n < a.mask_k_len ? mask_value(a, mask_load(a, b, n)) : -INFINITY;
 }
 
 struct AppendParams {
