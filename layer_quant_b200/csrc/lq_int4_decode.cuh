@@ -68,9 +68,6 @@ __global__ void __launch_bounds__(kThreadsM, (R <= 4 && QM != kQF32) ? 3 : 2) in
   const bool is_lo = DUP && t >= 2;
   const uint32_t lo_mul = is_lo ? 65536u : 0u, lo_mask = is_lo ? 0xFFFF0000u : 0u;
   uint8_t* const newtile = smem + L::kSmem - N::kNewBytes;
-  pdl_launch_dependents();
-  pdl_wait();
-
   const RunLengths rl = run_lengths(p);
   const bool do_new = a.k_new != nullptr && split == p.splits - 1;
   if (threadIdx.x == 0) s_is_last = 0;
