@@ -716,14 +716,15 @@ static size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 constexpr size_t kMaxTickets = 65536;
 constexpr size_t kTicketBytes = kMaxTickets * sizeof(int32_t);
 
-// Split count from a cost model fitted to measurements on B200 (times in units of one 64-token tile
-// on one SM, about 0.38 us): an SM works through its CTAs' tiles at the same rate whether one or three
-// CTAs are resident, every CTA adds about five tiles' worth of set-up and merge, a lone CTA per SM
-// cannot hide its set-up behind a neighbour, and every split adds a little merge traffic.
+// Split count from a cost model in microseconds, fitted to 360 measurements on B200 (batch 1 to 200, 33 to 131072 tokens, 1 to 64
+// splits; 6 % rms, the choice within 1 % of the best on average).  An SM holds three CTAs; a 64-token tile of one, two or
+// three at a time takes 0.35, 0.57 and 0.77 us; a further wave of CTAs pays its set-up again, more CTAs per SM start
+// later, and more than one split pays the merge.
 static int pick_splits(int batch, int kv_heads, int ctx_len) {
   const int ntiles = std::max(1, (ctx_len + kTile - 1) / kTile);
   const int sms = sm_count();
   const int64_t base = static_cast<int64_t>(batch) * kv_heads;
+  constexpr double kTileUs[4] = {0.0, 0.352, 0.571, 0.766};
   int best = 1;
   double best_cost = 1.0e300;
   const int max_splits = std::min(ntiles, 128);
@@ -731,8 +732,11 @@ static int pick_splits(int batch, int kv_heads, int ctx_len) {
     const int tps = (ntiles + s - 1) / s;
     if ((ntiles + tps - 1) / tps != s) continue;  // would leave empty splits
     const int64_t per_sm = (base * s + sms - 1) / sms;  // CTAs on the busiest SM
-    const double cost = static_cast<double>(per_sm) * (tps + 5.3) + (per_sm == 1 ? 10.5 : 0.0) + 0.05 * s;
-    if (cost < best_cost * 0.999) {  // ties go to fewer splits
+    const int64_t waves = (per_sm + 2) / 3;
+    const double cost = 3.5 + (s > 1 ? 3.2 + 0.016 * s : 0.0) + tps * ((per_sm / 3) * kTileUs[3] + kTileUs[per_sm % 3]) + 4.0 * (waves - 1) +
+                        1.1 * std::min<int64_t>(per_sm, 3);
+    // ties go to fewer splits; in launches of 200 us and more HBM evens out what the deal to the SMs leaves uneven
+    if (cost < best_cost * (best_cost > 200.0 ? 0.98 : 0.999)) {
       best_cost = cost;
       best = s;
     }
