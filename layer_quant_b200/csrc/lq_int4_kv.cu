@@ -299,7 +299,7 @@ struct DecodeParams {
   int32_t* counters;       // [B * Hkv] tickets (workspace)
   float* part_ml;          // [B * Hq * splits * 2]
   float* part_acc;         // [B * Hq * splits * 128]
-  // causal prefill over the quantised cache (tensor-pipe kernel with QB > 0 only)
+  // causal prefill over the quantised cache only
   int32_t q_len = 1;       // query positions per sequence
   int32_t nqb = 1;         // query blocks per sequence = ceil(q_len / QB)
   int32_t first_len = 0;   // tokens the first query position sees (its own included)
@@ -964,13 +964,8 @@ static int launch_prefill_mma(const DecodeParams& p, cudaStream_t st) {
   constexpr int QB = 8 / R;  // query positions per CTA: R * QB = 8 head columns
   const size_t smem = mma::kStagesM * L::kStage + L::kNewBytes;
   const dim3 grid(static_cast<unsigned>(p.a.cache.batch) * p.nqb, p.a.cache.kv_heads, 1), block(mma::kThreadsM);
-#define LQ_PREFILL_LAUNCH(SPLIT_)                                                                                   \
-  do {                                                                                                              \
-    LQ_SET_SMEM_ONCE((mma::int4_decode_mma_kernel<R, GS, false, SPLIT_, QB>), smem);                                \
-    mma::int4_decode_mma_kernel<R, GS, false, SPLIT_, QB><<<grid, block, smem, st>>>(p);                            \
-  } while (0)
-  if (p.a.dtype != LQ_BF16) LQ_PREFILL_LAUNCH(true); else LQ_PREFILL_LAUNCH(false);
-#undef LQ_PREFILL_LAUNCH
+  LQ_SET_SMEM_ONCE((mma::int4_prefill_mma_kernel<R, GS, QB>), smem);
+  mma::int4_prefill_mma_kernel<R, GS, QB><<<grid, block, smem, st>>>(p);
   LQ_CHECK_CUDA(cudaGetLastError());
   return LQ_OK;
 }
@@ -980,9 +975,7 @@ static int launch_prefill_gs(const DecodeParams& p, cudaStream_t st) {
   switch (p.a.cache.group_size) {
     case 32: return launch_prefill_mma<R, 32>(p, st);
     case 64: return launch_prefill_mma<R, 64>(p, st);
-    case 128: return launch_prefill_mma<R, 128>(p, st);
-    default:
-      return fail(LQ_ERR_UNSUPPORTED, "lq_int4_prefill_attn: group_size=%d (supported: 32, 64, 128)", p.a.cache.group_size);
+    default: return launch_prefill_mma<R, 128>(p, st);
   }
 }
 
@@ -1032,8 +1025,9 @@ LQ_EXPORT int lq_int4_prefill_attn(const lq_int4_prefill_args* args, void* cuda_
   const int ratio = a.q_heads / c.kv_heads;
   if (ratio != 1 && ratio != 2 && ratio != 4 && ratio != 8)
     return fail(LQ_ERR_UNSUPPORTED, "lq_int4_prefill_attn: %d query heads per kv head (supported: 1, 2, 4, 8)", ratio);
-  if (a.dtype != LQ_F32 && (c.group_size == 32 || c.group_size == 64 || c.group_size == 128))
-    return launch_prefill_tc(a, ratio, static_cast<cudaStream_t>(cuda_stream));
+  if (c.group_size != 32 && c.group_size != 64 && c.group_size != 128)
+    return fail(LQ_ERR_UNSUPPORTED, "lq_int4_prefill_attn: group_size=%d (supported: 32, 64, 128)", c.group_size);
+  if (a.dtype != LQ_F32) return launch_prefill_tc(a, ratio, static_cast<cudaStream_t>(cuda_stream));
   DecodeParams p;
   p.a = lq_int4_decode_args{};
   p.a.cache = c;

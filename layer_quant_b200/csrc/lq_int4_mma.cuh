@@ -1,24 +1,22 @@
-// q_len = 1 GQA decode attention over the packed INT4 KV cache on the tensor pipe.
+// Attention over the packed INT4 KV cache on mma.sync: what the decode kernel (lq_int4_decode.cuh) and the fp32-query
+// prefill kernel below share, and that kernel.
 //
-// Per kv head the step is a small GEMM pair, S = Q K^T ([R x 128] . [128 x T]) and O = P V
-// ([R x T] . [T x 128]) with R = query heads per kv head (4 for Nemotron-H).  On CUDA cores that is
+// Per kv head a decode step is a small GEMM pair with R = query heads per kv head (4 for Nemotron-H).  On CUDA cores that is
 // 4 FMAs per loaded nibble plus the unpack -- about four times the instruction issue a B200 SM can
-// spend per byte at HBM speed.  Here the multiply-accumulates go to mma.sync (m16n8k16, bf16 inputs,
-// fp32 accumulation): signed nibbles are exact in bf16 and q is bf16 already, so products are exact,
+// spend per byte at HBM speed.  Here the multiply-accumulates go to mma.sync (m16n8k16, 16-bit inputs,
+// fp32 accumulation): signed nibbles are exact in a 16-bit type, so products are exact,
 // and what is left for the CUDA cores is unpacking (about one instruction per nibble pair), the
 // scales and the softmax.
 //
 // Layout of one 16-token step of a warp:
-//   S:  M = heads (rows 0..R-1 of the 16), N = 8 tokens, K = 16 head dims.  A 16-byte chunk of a K
-//       row (32 nibbles) is one quantisation group at group size 32, so every k-step lies inside one
-//       group and each chunk gets its own accumulator; scales are applied to the accumulators in
-//       fp32.  K nibbles reach the B fragment through ldmatrix (8 token rows x 16 bytes); the k
-//       order inside a chunk is permuted, the same permutation is baked into the Q fragments.
-//   O:  M = heads, N = 8 head dims, K = 16 tokens.  A = P * v_scale of the chunk, split into
-//       bf16 hi (rows 0..7) + lo (rows 8..15) so that P keeps 16 bits of mantissa; the two halves
-//       of the fp32 accumulator are added at the end.  V nibbles reach the B fragment through
+//   S^T = K Q^T:  M = 16 tokens, N = 8 head columns, K = 16 head dims.  A 16-byte chunk of a K row (32 nibbles) lies inside one
+//       quantisation group, so each chunk gets its own accumulator; scales are applied to the accumulators in
+//       fp32.  The unpacked codes are the A operand; the k order inside a chunk is what ldmatrix delivers, the same
+//       permutation is baked into the Q fragments.
+//   O^T = V^T (P v_scale)^T:  M = 16 head dims, N = 8 head columns, K = 16 tokens.  P * v_scale of the chunk's group is split into
+//       bf16 hi + lo so that P keeps 16 bits of mantissa.  V nibbles reach the A fragment through
 //       ldmatrix.trans, which hands each thread the same 4 dims of two consecutive tokens.
-// Tiles of 64 tokens are staged with 16-byte cp.async copies into a 4-stage ring; the 16-byte
+// Codes are staged by 16-byte cp.async copies; the 16-byte
 // chunks of a row are XOR-swizzled by (row >> 1) & 3 so that ldmatrix reads without bank conflicts.
 #pragma once
 
@@ -145,60 +143,36 @@ struct TileLayout {
 };
 
 
-// One CTA (4 warps) per (split, kv head, batch); warp w owns tokens [16 w, 16 w + 16) of every
-// 64-token tile.  DecodeParams, int4_scale and int4_code come from lq_int4_kv.cu.
-// QSPLIT: the query is not bf16 (fp16 / fp32 callers): it enters the tensor pipe as bf16 hi (rows 0..7)
-// + bf16 lo (rows 8..15, otherwise idle), 16 bits of mantissa in all.
-// QB: 0 = decode (one query token per sequence).  QB >= 1 = causal prefill over the quantised cache: every
-// WARP of the CTA serves QB consecutive query positions of one (batch, kv head) -- 4 QB positions per CTA --
-// each (query, head) pair being one head column with its own causal limit (R * QB <= 8 columns); a warp
+// Causal attention of fp32 queries over the quantised cache (16-bit queries: lq_int4_prefill.cuh).  Every
+// warp of the CTA serves QB consecutive query positions of one (batch, kv head) -- 4 QB positions per CTA --
+// each (query, head) pair being one head column with its own causal limit (R * QB = 8 columns); a warp
 // walks all 64 tokens of every staged tile its positions may see, so a tile is fetched once for 4 QB
-// positions and nothing is merged between warps.  One split, no mask, no fused append.
-template <int R, int GS, bool HAS_MASK, bool QSPLIT, int QB = 0>
-__global__ void __launch_bounds__(kThreadsM, (R * (QB > 0 ? QB : 1) <= 4 && !QSPLIT) ? 3 : 2)
-    int4_decode_mma_kernel(const DecodeParams p) {
-  constexpr bool PREFILL = QB > 0;
-  constexpr int RV = R * (PREFILL ? QB : 1);  // head columns in use
-  static_assert(RV <= 8 && !(PREFILL && HAS_MASK), "at most eight head columns; prefill takes no mask");
+// positions and nothing is merged between warps.  The query enters the tensor pipe as bf16 hi + lo, 16 bits of mantissa.
+// DecodeParams comes from lq_int4_kv.cu.
+template <int R, int GS, int QB>
+__global__ void __launch_bounds__(kThreadsM, 2) int4_prefill_mma_kernel(const DecodeParams p) {
+  constexpr int RV = R * QB;  // head columns in use
+  static_assert(RV == 8, "eight head columns");
   using L = TileLayout<GS>;
   constexpr int G = L::kG;
   extern __shared__ __align__(128) uint8_t smem[];
-  __shared__ int s_is_last;
-  __shared__ float s_m[kWarpsM][8], s_l[kWarpsM][8];
+  __shared__ float s_l[kWarpsM][8];
 
   const lq_int4_decode_args& a = p.a;
   const lq_int4_cache& c = a.cache;
-  const int split = PREFILL ? 0 : blockIdx.x, kvh = blockIdx.y;
-  const int b = PREFILL ? static_cast<int>(blockIdx.x) / p.nqb : blockIdx.z;
-  const int cta_q_first = PREFILL ? (static_cast<int>(blockIdx.x) - b * p.nqb) * (QB * kWarpsM) : 0;  // first position of the CTA
+  const int kvh = blockIdx.y;
+  const int b = static_cast<int>(blockIdx.x) / p.nqb;
+  const int cta_q_first = (static_cast<int>(blockIdx.x) - b * p.nqb) * (QB * kWarpsM);  // first position of the CTA
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int g = lane >> 2, t = lane & 3;  // mma fragment coordinates: row / column group
-  const int q_first = PREFILL ? cta_q_first + warp * QB : 0;  // first query position of this warp
-  // Head columns.  Both products put the heads on the n side (8 columns).  Up to four query heads per kv
-  // head: columns 4..7 repeat columns 0..3, so that the O^T product can take the bf16 hi part of
-  // P * v_scale from columns 0..3 and the lo part from columns 4..7 of ONE n-tile.  Eight heads: columns
-  // are heads, hi and lo parts go to two n-tiles.  In the Q^T fragments (B operand) column n = g; in the
-  // accumulators a lane owns columns 2t and 2t + 1.
-  constexpr bool DUP = RV <= 4;
-  constexpr int NT = DUP ? 1 : 2;
-  const int hrow = DUP ? (g & 3) : g;
-  const bool is_lo = DUP && t >= 2;
-  const uint32_t lo_mul = is_lo ? 65536u : 0u, lo_mask = is_lo ? 0xFFFF0000u : 0u;
-  const bool fused_new = !PREFILL && a.k_new != nullptr;
-  uint8_t* newtile = smem + kStagesM * L::kStage;
+  const int q_first = cta_q_first + warp * QB;  // first query position of this warp
+  // Both products put the (position, head) pairs on the n side (8 columns); hi and lo parts of P * v_scale go to two n-tiles.
+  // In the Q^T fragments (B operand) column n = g; in the accumulators a lane owns columns 2t and 2t + 1.
+  constexpr int NT = 2;
+  const int hrow = g;
 
-  RunLengths rl = run_lengths(p);
-  if (PREFILL) {  // the CTA reads up to its last query's own position
-    rl.seq_len = p.first_len + min(cta_q_first + QB * kWarpsM - 1, p.q_len - 1);
-    rl.ctx_len = rl.seq_len;
-    rl.tiles_per_split = (rl.ctx_len + kTileTok - 1) / kTileTok;
-  }
-  const int ntiles = (rl.ctx_len + kTileTok - 1) / kTileTok;
-  const int tile_begin = split * rl.tiles_per_split;
-  const int tile_end = min(ntiles, tile_begin + rl.tiles_per_split);
-  const int my_tiles = max(0, tile_end - tile_begin);
-  const bool do_new = fused_new && split == p.splits - 1;
-  if (threadIdx.x == 0) s_is_last = 0;
+  const int ctx_len = p.first_len + min(cta_q_first + QB * kWarpsM - 1, p.q_len - 1);  // the CTA reads up to its last query's own position
+  const int my_tiles = (ctx_len + kTileTok - 1) / kTileTok;
 
   const int64_t kp_base = b * c.kp_stride[0] + kvh * c.kp_stride[1];
   const int64_t vp_base = b * c.vp_stride[0] + kvh * c.vp_stride[1];
@@ -220,20 +194,20 @@ __global__ void __launch_bounds__(kThreadsM, (R * (QB > 0 ? QB : 1) <= 4 && !QSP
   const uint32_t smem_base = s2u(smem);
   // Tiles are issued in order, so a full tile costs five copies from running pointers; the last, partial tile of the
   // context takes the general form with per-row byte counts (rows past the end are zero-filled).
-  const uint8_t* k_src = k_rows + static_cast<int64_t>(tile_begin) * (kTileTok * 64) + code_src_off;
-  const uint8_t* v_src = v_rows + static_cast<int64_t>(tile_begin) * (kTileTok * 64) + code_src_off;
-  const uint8_t* s_src = scale_rows + static_cast<int64_t>(tile_begin) * (kTileTok * G * 4) + scale_off;
+  const uint8_t* k_src = k_rows + code_src_off;
+  const uint8_t* v_src = v_rows + code_src_off;
+  const uint8_t* s_src = scale_rows + scale_off;
   auto issue_tile = [&](int it) {
     const uint32_t stage = smem_base + (it % kStagesM) * L::kStage;
-    const int tok0 = (tile_begin + it) * kTileTok;
-    if (tok0 + kTileTok <= rl.ctx_len) {
+    const int tok0 = it * kTileTok;
+    if (tok0 + kTileTok <= ctx_len) {
       cp_async16_full(stage + L::kKc + code_dst_off, k_src);
       cp_async16_full(stage + L::kKc + code_dst_off + 2048, k_src + 2048);
       cp_async16_full(stage + L::kVc + code_dst_off, v_src);
       cp_async16_full(stage + L::kVc + code_dst_off + 2048, v_src + 2048);
       if (has_scale_chunk) cp_async16_full(stage + (scale_which ? L::kVs : L::kKs) + scale_off, s_src);
     } else {
-      const int rows = rl.ctx_len - tok0;
+      const int rows = ctx_len - tok0;
       const uint32_t ok0 = static_cast<int>(r0) < rows ? 16u : 0u, ok1 = static_cast<int>(r0) + 32 < rows ? 16u : 0u;
       const int64_t back = -static_cast<int64_t>(code_src_off);  // rows past the end copy nothing, from the tile's first byte
       cp_async16(stage + L::kKc + code_dst_off, k_src + (ok0 ? 0 : back), ok0);
@@ -251,23 +225,10 @@ __global__ void __launch_bounds__(kThreadsM, (R * (QB > 0 ? QB : 1) <= 4 && !QSP
     s_src += kTileTok * G * 4;
   };
 
-  // start the ring now: the first tiles travel while the new row is quantised and the Q fragments are built
+  // start the ring now: the first tiles travel while the Q fragments are built
   for (int it = 0; it < kStagesM - 1; ++it) {
     if (it < my_tiles) issue_tile(it);
     cp_async_commit();
-  }
-
-  // the new row's values are fetched now and quantised after the Q fragments, so that the two sets of
-  // loads are in flight together
-  float xnew[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-  if (do_new && warp < 2) {
-    const void* src = warp == 0 ? a.k_new : a.v_new;
-    const int64_t* ss = warp == 0 ? a.k_new_stride : a.v_new_stride;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) xnew[i] = load_as_float(src, b * ss[0] + kvh * ss[1] + (lane * 4 + i) * ss[2], a.dtype);
-  }
-  if (do_new) {
-    for (int i = threadIdx.x; i < L::kNewBytes / 16; i += kThreadsM) reinterpret_cast<uint4*>(newtile)[i] = make_uint4(0, 0, 0, 0);
   }
 
   // ---- Q fragments (A operand of S), in the k order the K unpack produces ------------------------------
@@ -275,100 +236,52 @@ __global__ void __launch_bounds__(kThreadsM, (R * (QB > 0 ? QB : 1) <= 4 && !QSP
   // The K side feeds 136 + n to the tensor pipe and starts each chunk's accumulator at -136 * sum(q over
   // the chunk) instead (two mma per accumulator, so no long cancellation); qoff[i] is that start value
   // for head g, the sum taken over the bf16 values the fragments actually hold.
-  uint32_t qa[4][2][2];
-  uint32_t ql[QSPLIT ? 4 : 1][2][2];  // lo halves (QSPLIT only)
-  float qoff[4], qoff_lo[QSPLIT ? 4 : 1];
+  uint32_t qa[4][2][2], ql[4][2][2];  // hi and lo halves
+  float qoff[4];
   auto bf_lo = [](uint32_t v) { return __uint_as_float(v << 16); };
   auto bf_hi = [](uint32_t v) { return __uint_as_float(v & 0xFFFF0000u); };
-  // this lane's query row; a bf16 query whose head dims are contiguous and 16-byte aligned arrives as one 128-bit load per
-  // chunk (the lane's eight dims 32 i + 8 t .. + 7), anything else as scalar loads
-  const bool q_row_valid = hrow < RV && (!PREFILL || q_first + hrow / R < p.q_len);
-  const int64_t q_row_base = b * a.q_stride[0] + (kvh * R + hrow % R) * a.q_stride[1] +
-                             (PREFILL ? (q_first + hrow / R) * p.q_stride_t : 0);
-  const bool q_vec = !QSPLIT && a.dtype == LQ_BF16 && a.q_stride[2] == 1 &&
-                     ((reinterpret_cast<uintptr_t>(a.q) | (static_cast<uint64_t>(a.q_stride[0]) * 2) |
-                       (static_cast<uint64_t>(a.q_stride[1]) * 2) | (PREFILL ? static_cast<uint64_t>(p.q_stride_t) * 2 : 0)) & 15) == 0;
+  const bool q_row_valid = q_first + hrow / R < p.q_len;
+  const int64_t q_row_base = b * a.q_stride[0] + (kvh * R + hrow % R) * a.q_stride[1] + (q_first + hrow / R) * p.q_stride_t;
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     float qs = 0.0f, qs_lo = 0.0f;
-    uint4 qw = make_uint4(0u, 0u, 0u, 0u);  // dims 8t .. 8t+7 of chunk i as bf16 pairs (vector path)
-    if (q_vec && q_row_valid)
-      qw = __ldg(reinterpret_cast<const uint4*>(static_cast<const uint16_t*>(a.q) + q_row_base + 32 * i + 8 * t));
 #pragma unroll
     for (int s = 0; s < 2; ++s) {
       const int d0 = 32 * i + 8 * t + 2 * s;
-      uint32_t pa, pb;
       float q0 = 0.f, q1 = 0.f, q2 = 0.f, q3 = 0.f;
-      if (q_vec) {  // (dim d0, d0 + 4) and (d0 + 1, d0 + 5) out of the eight loaded values
-        const uint32_t wl = s == 0 ? qw.x : qw.y, wh = s == 0 ? qw.z : qw.w;
-        pa = __byte_perm(wl, wh, 0x5410);
-        pb = __byte_perm(wl, wh, 0x7632);
-      } else {
-        if (q_row_valid) {
-          q0 = load_as_float(a.q, q_row_base + (d0 + 0) * a.q_stride[2], a.dtype);
-          q1 = load_as_float(a.q, q_row_base + (d0 + 4) * a.q_stride[2], a.dtype);
-          q2 = load_as_float(a.q, q_row_base + (d0 + 1) * a.q_stride[2], a.dtype);
-          q3 = load_as_float(a.q, q_row_base + (d0 + 5) * a.q_stride[2], a.dtype);
-        }
-        pa = pack_bf16x2(q0, q1);
-        pb = pack_bf16x2(q2, q3);
+      if (q_row_valid) {
+        q0 = load_as_float(a.q, q_row_base + (d0 + 0) * a.q_stride[2], a.dtype);
+        q1 = load_as_float(a.q, q_row_base + (d0 + 4) * a.q_stride[2], a.dtype);
+        q2 = load_as_float(a.q, q_row_base + (d0 + 1) * a.q_stride[2], a.dtype);
+        q3 = load_as_float(a.q, q_row_base + (d0 + 5) * a.q_stride[2], a.dtype);
       }
-      qa[i][s][0] = pa;  // a0: row g, k = 2t, 2t+1
-      qa[i][s][1] = pb;  // a2: row g, k = 2t+8, 2t+9
+      const uint32_t pa = pack_bf16x2(q0, q1), pb = pack_bf16x2(q2, q3);
+      qa[i][s][0] = pa;  // k = 2t, 2t+1
+      qa[i][s][1] = pb;  // k = 2t+8, 2t+9
       qs += (bf_lo(pa) + bf_hi(pa)) + (bf_lo(pb) + bf_hi(pb));  // of the values the fragments hold
-      if (QSPLIT) {
-        const uint32_t la = pack_bf16x2(q0 - bf_lo(pa), q1 - bf_hi(pa)), lb = pack_bf16x2(q2 - bf_lo(pb), q3 - bf_hi(pb));
-        ql[i][s][0] = la;  // a1: row g + 8
-        ql[i][s][1] = lb;  // a3
-        qs_lo += (bf_lo(la) + bf_hi(la)) + (bf_lo(lb) + bf_hi(lb));
-      }
+      const uint32_t la = pack_bf16x2(q0 - bf_lo(pa), q1 - bf_hi(pa)), lb = pack_bf16x2(q2 - bf_lo(pb), q3 - bf_hi(pb));
+      ql[i][s][0] = la;
+      ql[i][s][1] = lb;
+      qs_lo += (bf_lo(la) + bf_hi(la)) + (bf_lo(lb) + bf_hi(lb));
     }
     qs += __shfl_xor_sync(0xFFFFFFFFu, qs, 1);  // the chunk's 32 dims live in the four lanes of row g
     qs += __shfl_xor_sync(0xFFFFFFFFu, qs, 2);
-    qoff[i] = -136.0f * qs;
-    if (QSPLIT) {
-      qs_lo += __shfl_xor_sync(0xFFFFFFFFu, qs_lo, 1);
-      qs_lo += __shfl_xor_sync(0xFFFFFFFFu, qs_lo, 2);
-      qoff_lo[i] = -136.0f * qs_lo;
-    }
+    qs_lo += __shfl_xor_sync(0xFFFFFFFFu, qs_lo, 1);
+    qs_lo += __shfl_xor_sync(0xFFFFFFFFu, qs_lo, 2);
+    qoff[i] = -136.0f * qs - 136.0f * qs_lo;
   }
   // accumulator start values of this lane's two columns (the sums live in the lanes of row g = column)
   float qstart[4][2];
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    const float v = QSPLIT ? qoff[i] + qoff_lo[QSPLIT ? i : 0] : qoff[i];
+    const float v = qoff[i];
     qstart[i][0] = __shfl_sync(0xFFFFFFFFu, v, 8 * t);      // lane (g = 2t, t = 0)
     qstart[i][1] = __shfl_sync(0xFFFFFFFFu, v, 8 * t + 4);  // lane (g = 2t + 1, t = 0)
   }
-  // ---- fused append: quantise the new K / V row, write it to the cache and into a 16-row tile -------
-  __syncthreads();  // the tile of the new row is zeroed
-  if (do_new && warp < 2) {
-    float amax = 0.0f;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) amax = fmaxf(amax, fabsf(xnew[i]));
-#pragma unroll
-    for (int o = GS / 8; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, o));
-    const float scale = int4_scale(amax);
-    uint32_t half = 0;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) half |= int4_code(xnew[i], scale) << (4 * i);
-    const int pos = rl.seq_len - 1;
-    uint8_t* gcodes = (warp == 0 ? c.k_packed + kp_base + static_cast<int64_t>(pos) * c.kp_stride[2]
-                                 : c.v_packed + vp_base + static_cast<int64_t>(pos) * c.vp_stride[2]);
-    reinterpret_cast<uint16_t*>(gcodes)[lane] = static_cast<uint16_t>(half);
-    reinterpret_cast<uint16_t*>(newtile + (warp == 0 ? L::kNewKc : L::kNewVc))[lane] = static_cast<uint16_t>(half);  // row 0: no swizzle
-    if ((lane * 4) % GS == 0) {
-      float* gsc = (warp == 0 ? c.k_scale + ks_base + static_cast<int64_t>(pos) * c.ks_stride[2]
-                              : c.v_scale + vs_base + static_cast<int64_t>(pos) * c.vs_stride[2]);
-      gsc[lane * 4 / GS] = scale;
-      reinterpret_cast<float*>(newtile + (warp == 0 ? L::kNewKs : L::kNewVs))[lane * 4 / GS] = scale;
-    }
-  }
-
   const float scale_sm = 1.4426950408889634f / sqrtf(static_cast<float>(kD));
 
   // O^T accumulators: m-tile (chunk i, half sp) has row g = dim 32 i + 4 g + 2 sp and row g + 8 = that
-  // dim + 1; columns 2t, 2t+1 are heads (DUP: head c & 3, hi part for c < 4, lo part for c >= 4).
+  // dim + 1; columns 2t, 2t+1 are (position, head) pairs, hi part in one n-tile, lo part in the other.
   float oacc[4][2][NT][4];
 #pragma unroll
   for (int i = 0; i < 4; ++i)
@@ -378,18 +291,15 @@ __global__ void __launch_bounds__(kThreadsM, (R * (QB > 0 ? QB : 1) <= 4 && !QSP
       for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
         for (int e = 0; e < 4; ++e) oacc[i][sp][nt][e] = 0.0f;
-  const int col_head0 = DUP ? ((2 * t) & 3) : 2 * t;  // head column of accumulator column 2t (column 2t+1: the next one)
-  // prefill: the tokens a column may see, [0, its query's position]
-  int col_limit[2] = {0x7FFFFFFF, 0x7FFFFFFF};
-  int warp_limit = 0x7FFFFFFF;  // tokens this warp's positions may see at all (0: the warp has no position)
-  if (PREFILL) {
+  const int col_head0 = 2 * t;  // head column of accumulator column 2t (column 2t+1: the next one)
+  // the tokens a column may see, [0, its query's position], and those this warp's positions may see at all (0: it has none)
+  int col_limit[2];
 #pragma unroll
-    for (int cc = 0; cc < 2; ++cc) col_limit[cc] = p.first_len + min(q_first + (col_head0 + cc) / R, p.q_len - 1);
-    warp_limit = q_first < p.q_len ? p.first_len + min(q_first + QB - 1, p.q_len - 1) : 0;
-  }
+  for (int cc = 0; cc < 2; ++cc) col_limit[cc] = p.first_len + min(q_first + (col_head0 + cc) / R, p.q_len - 1);
+  const int warp_limit = q_first < p.q_len ? p.first_len + min(q_first + QB - 1, p.q_len - 1) : 0;
   float m_run[2] = {kNegBigM, kNegBigM}, l_run[2] = {0.0f, 0.0f};  // this lane's two columns (l: this lane's share)
 
-  // Per-thread offsets inside a tile for this warp's 16 rows (row0 = 16 * warp; 0 for the new-row tile):
+  // Per-thread offsets inside 16 rows of a tile:
   // ldmatrix row addresses for K (two 8-token halves) and V (two chunk pairs), and the scale rows of
   // the two tokens this thread owns in the S^T fragments (rows g and g + 8).
   auto make_offsets = [&](int row0, uint32_t (&koff)[2], uint32_t (&voff)[2], uint32_t (&soff)[2]) {
@@ -402,7 +312,7 @@ __global__ void __launch_bounds__(kThreadsM, (R * (QB > 0 ? QB : 1) <= 4 && !QSP
     for (int r = 0; r < 2; ++r) soff[r] = (row0 + g + 8 * r) * G * 4;
   };
   uint32_t koff[2], voff[2], soff[2];
-  make_offsets(PREFILL ? 0 : 16 * warp, koff, voff, soff);
+  make_offsets(0, koff, voff, soff);
 
   // One 16-token step of this warp.  kc / vc / ksc / vsc: shared-memory addresses of the tile's parts.
   // FULL: all 16 rows hold tokens (no validity selects); otherwise the first `valid` rows do, and the
@@ -422,14 +332,12 @@ __global__ void __launch_bounds__(kThreadsM, (R * (QB > 0 ? QB : 1) <= 4 && !QSP
         const uint32_t w0 = kr0[i], w1 = kr1[i];
         mma_bf16_from(sacc[i], nib_pair_biased(w0), nib_pair_biased(w1), nib_pair_biased(w0 >> 4), nib_pair_biased(w1 >> 4),
                       qa[i][0][0], qa[i][0][1], qstart[i][0], qstart[i][1], qstart[i][0], qstart[i][1]);
-        if (QSPLIT)
           mma_bf16(sacc[i], nib_pair_biased(w0), nib_pair_biased(w1), nib_pair_biased(w0 >> 4), nib_pair_biased(w1 >> 4),
-                   ql[QSPLIT ? i : 0][0][0], ql[QSPLIT ? i : 0][0][1]);
+                   ql[i][0][0], ql[i][0][1]);
         mma_bf16(sacc[i], nib_pair_biased(w0 >> 8), nib_pair_biased(w1 >> 8), nib_pair_biased(w0 >> 12), nib_pair_biased(w1 >> 12),
                  qa[i][1][0], qa[i][1][1]);
-        if (QSPLIT)
           mma_bf16(sacc[i], nib_pair_biased(w0 >> 8), nib_pair_biased(w1 >> 8), nib_pair_biased(w0 >> 12),
-                   nib_pair_biased(w1 >> 12), ql[QSPLIT ? i : 0][1][0], ql[QSPLIT ? i : 0][1][1]);
+                   nib_pair_biased(w1 >> 12), ql[i][1][0], ql[i][1][1]);
       }
     }
     // scores of tokens g (r = 0) and g + 8 (r = 1) for this lane's two columns
@@ -439,11 +347,6 @@ __global__ void __launch_bounds__(kThreadsM, (R * (QB > 0 ? QB : 1) <= 4 && !QSP
       float sc[G];
       load_scales(ksc + so[r], sc);
       const int rr = g + 8 * r;
-      float bias = 0.0f;
-      if (HAS_MASK) {
-        const int n = tok_first + rr;
-        bias = (FULL || rr < valid) ? mask_bias(a, b, n) : -INFINITY;
-      }
       // both columns of the token at once: packed fp32x2 FMA / MUL (sm_100), same rounding per component
       float2 sum2 = make_float2(0.0f, 0.0f);
 #pragma unroll
@@ -456,8 +359,7 @@ __global__ void __launch_bounds__(kThreadsM, (R * (QB > 0 ? QB : 1) <= 4 && !QSP
 #pragma unroll
       for (int cc = 0; cc < 2; ++cc) {
         float sum = sums[cc];
-        if (HAS_MASK) sum += bias;
-        sv[r][cc] = ((FULL || rr < valid) && (!PREFILL || tok_first + rr < col_limit[cc])) ? sum : -INFINITY;
+        sv[r][cc] = ((FULL || rr < valid) && tok_first + rr < col_limit[cc]) ? sum : -INFINITY;
       }
     }
     // online softmax per column; the running max of a column is shared by the eight lanes that hold it.
@@ -498,9 +400,7 @@ __global__ void __launch_bounds__(kThreadsM, (R * (QB > 0 ? QB : 1) <= 4 && !QSP
       }
     // B operand of O^T: (P * v_scale)^T per scale group, k = the tokens 2t, 2t+1 (+8), n = column g.  What
     // this lane has is the other way round (token g / g + 8, columns 2t, 2t+1), so each packed pair goes
-    // through movmatrix.  A lane of columns 0..3 keeps the bf16 rounding of the product, a lane of
-    // columns 4..7 the bf16 rounding of what that left over (one formula: the part taken off is masked
-    // to zero on the hi lanes).
+    // through movmatrix: the bf16 rounding of the product, and the bf16 rounding of what that left over.
     uint32_t pb[G][2][NT];
 #pragma unroll
     for (int r = 0; r < 2; ++r) {
@@ -510,14 +410,9 @@ __global__ void __launch_bounds__(kThreadsM, (R * (QB > 0 ? QB : 1) <= 4 && !QSP
       for (int q = 0; q < G; ++q) {
         const float2 pp = __fmul2_rn(make_float2(pv[r][0], pv[r][1]), make_float2(vs[q], vs[q]));
         const uint32_t hi = pack_bf16x2(pp.x, pp.y);
-        if (DUP) {
-          const float2 lo = __ffma2_rn(make_float2(__uint_as_float(hi * lo_mul), __uint_as_float(hi & lo_mask)), make_float2(-1.0f, -1.0f), pp);
-          pb[q][r][0] = movmatrix_trans(pack_bf16x2(lo.x, lo.y));
-        } else {
-          const float2 lo = __ffma2_rn(make_float2(__uint_as_float(hi << 16), __uint_as_float(hi & 0xFFFF0000u)), make_float2(-1.0f, -1.0f), pp);
-          pb[q][r][0] = movmatrix_trans(hi);
-          pb[q][r][NT - 1] = movmatrix_trans(pack_bf16x2(lo.x, lo.y));
-        }
+        const float2 lo = __ffma2_rn(make_float2(__uint_as_float(hi << 16), __uint_as_float(hi & 0xFFFF0000u)), make_float2(-1.0f, -1.0f), pp);
+        pb[q][r][0] = movmatrix_trans(hi);
+        pb[q][r][1] = movmatrix_trans(pack_bf16x2(lo.x, lo.y));
       }
     }
     // O^T += V^T (P * v_scale)^T, chunk by chunk: the unpacked codes are the A operand
@@ -548,160 +443,55 @@ __global__ void __launch_bounds__(kThreadsM, (R * (QB > 0 ? QB : 1) <= 4 && !QSP
     if (it + kStagesM - 1 < my_tiles) issue_tile(it + kStagesM - 1);
     cp_async_commit();
     const uint8_t* stage = smem + (it % kStagesM) * L::kStage;
-    const int tok0 = (tile_begin + it) * kTileTok;
-    const int rows = min(kTileTok, rl.ctx_len - tok0);
+    const int tok0 = it * kTileTok;
+    const int rows = min(kTileTok, ctx_len - tok0);
     const uint32_t sb = s2u(stage);
-    if (PREFILL) {
 #pragma unroll 1
-      for (int blk = 0; blk < kTileTok / 16; ++blk) {  // the warp's own positions over the whole tile
-        const int r16 = 16 * blk;
-        if (r16 >= rows || tok0 + r16 >= warp_limit) break;
-        const uint32_t cb = blk * (16 * 64);
-        const int sbo = blk * (16 * G * 4);
-        if (rows - r16 >= 16)
-          step16(std::true_type{}, sb + L::kKc + cb, sb + L::kVc + cb, stage + L::kKs + sbo, stage + L::kVs + sbo, koff, voff, soff,
-                 16, tok0 + r16);
-        else
-          step16(std::false_type{}, sb + L::kKc + cb, sb + L::kVc + cb, stage + L::kKs + sbo, stage + L::kVs + sbo, koff, voff,
-                 soff, rows - r16, tok0 + r16);
-      }
-      continue;
+    for (int blk = 0; blk < kTileTok / 16; ++blk) {  // the warp's own positions over the whole tile
+      const int r16 = 16 * blk;
+      if (r16 >= rows || tok0 + r16 >= warp_limit) break;
+      const uint32_t cb = blk * (16 * 64);
+      const int sbo = blk * (16 * G * 4);
+      if (rows - r16 >= 16)
+        step16(std::true_type{}, sb + L::kKc + cb, sb + L::kVc + cb, stage + L::kKs + sbo, stage + L::kVs + sbo, koff, voff, soff,
+               16, tok0 + r16);
+      else
+        step16(std::false_type{}, sb + L::kKc + cb, sb + L::kVc + cb, stage + L::kKs + sbo, stage + L::kVs + sbo, koff, voff,
+               soff, rows - r16, tok0 + r16);
     }
-    const int row0 = 16 * warp;
-    if (rows - row0 >= 16)
-      step16(std::true_type{}, sb + L::kKc, sb + L::kVc, stage + L::kKs, stage + L::kVs, koff, voff, soff, 16, tok0 + row0);
-    else if (row0 < rows)
-      step16(std::false_type{}, sb + L::kKc, sb + L::kVc, stage + L::kKs, stage + L::kVs, koff, voff, soff, rows - row0,
-             tok0 + row0);
   }
   cp_async_wait<0>();
   __syncthreads();
-  if (do_new && warp == 0) {
-    uint32_t ko0[2], vo0[2], so0[2];
-    make_offsets(0, ko0, vo0, so0);
-    const uint32_t nb = s2u(newtile);
-    step16(std::false_type{}, nb + L::kNewKc, nb + L::kNewVc, newtile + L::kNewKs, newtile + L::kNewVs, ko0, vo0, so0, 1,
-           rl.seq_len - 1);
-  }
 
-  // ---- merge the warps -------------------------------------------------------------------------------------
+  // ---- outputs: every warp holds complete results for its own positions -------------------------------------
 #pragma unroll
   for (int o = 4; o < 32; o <<= 1) {  // a column's denominator: over the eight lanes (token rows) that share it
     l_run[0] += __shfl_xor_sync(0xFFFFFFFFu, l_run[0], o);
     l_run[1] += __shfl_xor_sync(0xFFFFFFFFu, l_run[1], o);
   }
-  float* s_acc = reinterpret_cast<float*>(smem);  // [warps][R][128], reuses the ring
+  float* s_acc = reinterpret_cast<float*>(smem);  // [warps][RV][128], reuses the ring
 #pragma unroll
   for (int i = 0; i < 4; ++i)
 #pragma unroll
     for (int sp = 0; sp < 2; ++sp)
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        float v;
-        if (DUP) {
-          v = oacc[i][sp][0][e];
-          v += __shfl_xor_sync(0xFFFFFFFFu, v, 2);  // hi columns (t < 2) + lo columns (t >= 2) of the same heads
-        } else {
-          v = oacc[i][sp][0][e] + oacc[i][sp][NT - 1][e];
-        }
-        const int head = col_head0 + (e & 1);
-        const int dim = 32 * i + 4 * g + 2 * sp + (e >> 1);
-        if ((!DUP || t < 2) && head < RV) s_acc[(warp * RV + head) * kD + dim] = v;
-      }
-  if (g == 0 && (!DUP || t < 2)) {
-#pragma unroll
-    for (int cc = 0; cc < 2; ++cc)
-      if (col_head0 + cc < RV) {
-        s_m[warp][col_head0 + cc] = m_run[cc];
-        s_l[warp][col_head0 + cc] = l_run[cc];
-      }
+      for (int e = 0; e < 4; ++e)
+        s_acc[(warp * RV + col_head0 + (e & 1)) * kD + 32 * i + 4 * g + 2 * sp + (e >> 1)] = oacc[i][sp][0][e] + oacc[i][sp][1][e];
+  if (g == 0) {
+    s_l[warp][col_head0] = l_run[0];
+    s_l[warp][col_head0 + 1] = l_run[1];
   }
   __syncthreads();
-  const int hq0 = kvh * R;
   for (int o = threadIdx.x; o < RV * kD; o += kThreadsM) {
     const int r = o / kD, d = o - r * kD;
-    float M = kNegBigM;
-#pragma unroll
-    for (int w = 0; w < kWarpsM; ++w) M = fmaxf(M, s_m[w][r]);
-    float Lsum = 0.0f, O = 0.0f;
 #pragma unroll
     for (int w = 0; w < kWarpsM; ++w) {
-      const float fct = exp2f(s_m[w][r] - M);
-      Lsum = fmaf(s_l[w][r], fct, Lsum);
-      O = fmaf(s_acc[(w * RV + r) * kD + d], fct, O);
-    }
-    if (PREFILL) {
-      // every warp holds complete results for its own positions: nothing to merge
-#pragma unroll
-      for (int w = 0; w < kWarpsM; ++w) {
-        const int qi = cta_q_first + w * QB + r / R;
-        if (qi < p.q_len)
-          store_from_float(a.out, b * a.out_stride[0] + (hq0 + r % R) * a.out_stride[1] + qi * p.out_stride_t + d * a.out_stride[2],
-                           a.dtype, s_acc[(w * RV + r) * kD + d] / s_l[w][r]);
-      }
-    } else if (p.splits == 1) {
-      store_from_float(a.out, b * a.out_stride[0] + (hq0 + r) * a.out_stride[1] + d * a.out_stride[2], a.dtype, O / Lsum);
-    } else {
-      const int64_t slot = (static_cast<int64_t>(b) * a.q_heads + hq0 + r) * p.splits + split;
-      p.part_acc[slot * kD + d] = O;
-      if (d == 0) {
-        p.part_ml[slot * 2] = M;
-        p.part_ml[slot * 2 + 1] = Lsum;
-      }
+      const int qi = cta_q_first + w * QB + r / R;
+      if (qi < p.q_len)
+        store_from_float(a.out, b * a.out_stride[0] + (kvh * R + r % R) * a.out_stride[1] + qi * p.out_stride_t + d * a.out_stride[2],
+                         a.dtype, s_acc[(w * RV + r) * kD + d] / s_l[w][r]);
     }
   }
-  if (PREFILL || p.splits == 1) return;
-
-  // Ticket: the CTA that completes the set merges the splits.  No CTA waits for another.
-  __threadfence();
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    const int ticket = atomicAdd(&p.counters[b * c.kv_heads + kvh], 1);
-    s_is_last = (ticket == p.splits - 1) ? 1 : 0;
-  }
-  __syncthreads();
-  if (!s_is_last) return;
-  __threadfence();
-  // (1) one warp per head: the maximum over the splits, each split's factor (to shared memory) and the
-  // denominator; (2) one thread per output: the weighted sum, its loads independent of one another.
-  float* s_f = reinterpret_cast<float*>(smem);  // [R][kMaxSplitsM], reuses the ring
-  float* s_den = s_f + R * kMaxSplitsM;         // [R]
-  for (int r = warp; r < R; r += kWarpsM) {
-    const float* ml = p.part_ml + (static_cast<int64_t>(b) * a.q_heads + hq0 + r) * p.splits * 2;
-    float M = kNegBigM;
-    for (int s = lane; s < p.splits; s += 32) M = fmaxf(M, __ldcg(ml + 2 * s));
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) M = fmaxf(M, __shfl_xor_sync(0xFFFFFFFFu, M, o));
-    float den = 0.0f;
-    for (int s = lane; s < p.splits; s += 32) {
-      const float fct = exp2f(__ldcg(ml + 2 * s) - M);
-      s_f[r * kMaxSplitsM + s] = fct;
-      den = fmaf(__ldcg(ml + 2 * s + 1), fct, den);
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) den += __shfl_xor_sync(0xFFFFFFFFu, den, o);
-    if (lane == 0) s_den[r] = den;
-  }
-  __syncthreads();
-  // four outputs per thread: the splits' partial results arrive as independent 128-bit loads, eight in flight per thread
-  for (int o = threadIdx.x; o < R * (kD / 4); o += kThreadsM) {
-    const int r = o / (kD / 4), d = (o - r * (kD / 4)) * 4;
-    const float4* acc = reinterpret_cast<const float4*>(p.part_acc + (static_cast<int64_t>(b) * a.q_heads + hq0 + r) * p.splits * kD + d);
-    float4 O = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-#pragma unroll 8
-    for (int s = 0; s < p.splits; ++s) {
-      const float4 v = __ldcg(acc + static_cast<int64_t>(s) * (kD / 4));
-      const float f = s_f[r * kMaxSplitsM + s];
-      O.x = fmaf(v.x, f, O.x); O.y = fmaf(v.y, f, O.y); O.z = fmaf(v.z, f, O.z); O.w = fmaf(v.w, f, O.w);
-    }
-    const float den = s_den[r];
-    const int64_t ob = b * a.out_stride[0] + (hq0 + r) * a.out_stride[1] + d * a.out_stride[2];
-    store_from_float(a.out, ob, a.dtype, O.x / den);
-    store_from_float(a.out, ob + a.out_stride[2], a.dtype, O.y / den);
-    store_from_float(a.out, ob + 2 * a.out_stride[2], a.dtype, O.z / den);
-    store_from_float(a.out, ob + 3 * a.out_stride[2], a.dtype, O.w / den);
-  }
-  if (threadIdx.x == 0) p.counters[b * c.kv_heads + kvh] = 0;  // ready for the next launch
 }
 
 }  // namespace mma
