@@ -1,7 +1,8 @@
 // Packed signed-INT4 KV cache: append (quantise + pack) and q_len = 1 GQA decode attention with a
 // split over the context (flash-decoding).  sm_100a.
 //
-// Decode kernel: one CTA per (split, kv head, batch).  A producer warp streams 64-token tiles of
+// Group sizes 32 / 64 / 128 take the tensor-pipe kernel of lq_int4_decode.cuh.  The CUDA-core decode kernel below
+// serves group size 16: one CTA per (split, kv head, batch).  A producer warp streams 64-token tiles of
 // the packed K / V codes and their fp32 group scales from HBM into a 4-stage shared-memory ring
 // with bulk asynchronous copies (cp.async.bulk, completion on an mbarrier; rows of one (batch,
 // kv head) are contiguous, so a tile is four plain 1-D copies).  Eight consumer warps read the

@@ -1,16 +1,15 @@
 // Mamba2 selective-state update on an MX8 / MX4-held recurrent state, fused in one pass, plus the
 // stand-alone MX codec kernels.  sm_100a.
 //
-// Work decomposition of the fused kernel: one CTA per (batch, head); inside it one lane owns one
-// 16-value block of a row (so block maximum, pair maxima, exponent and micro-exponent bits never
-// leave the thread), dstate/16 neighbouring lanes own one row, and the <h', C> read-out is a
-// shuffle reduction over those lanes.  B and C of the head's group stay in registers for all
-// `dim` rows.  Each lane moves 16 B of mantissas per row with one 128-bit load and one 128-bit
-// store; the next row's loads are issued before the current row is computed.
+// In every update kernel one lane owns one 16-value block of a row, so block maximum, pair maxima, exponent
+// and micro-exponent bits never leave the thread, and dstate/16 neighbouring lanes own one row.
+// mx_state_update_fast_kernel (dense states, every Mamba2 decode step) deals the rows in contiguous slabs to one
+// wave of two-warp CTAs; mx_state_update_kernel takes any strides, per-row dt and ragged shapes, one CTA per
+// (batch, head).
 //
-// The kernel is bound by instruction issue, not by HBM, on B200: at 18 bytes per block read and
-// written the memory system could deliver one value every ~12 issue slots per SM sub-partition,
-// and decode + update + read-out + exponent + rounding + random bits need more than that.
+// Both are bound by instruction issue and latency, not by HBM: at 18 bytes per block read and written the memory
+// system could deliver one value every ~12 issue slots per SM sub-partition, and decode + update + read-out +
+// exponent + rounding + random bits need more than that.
 #include <algorithm>
 #include <cstdlib>
 #include <type_traits>
