@@ -142,3 +142,45 @@ def test_dense_update_against_reference_mx_fixtures(golden_dir, name):
     assert_out_close(y, g["y0"])
     if "h0" in g:
         np.testing.assert_allclose(state.cpu().numpy(), g["h0"], rtol=3e-6, atol=1e-7)
+
+
+@pytest.mark.parametrize("state_dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("shape", [(1, 1, 4, 128, 1), (1, 3, 4, 128, 1), (3, 5, 12, 128, 5), (2, 7, 20, 128, 7), (9, 32, 64, 128, 8)])
+def test_rows_kernel_edges(state_dtype, shape):
+    """One step of four rows, an odd number of steps, runs across heads, groups and sequences."""
+    test_dense_update_matches_oracle(state_dtype, shape)
+
+
+def test_both_sides_of_the_batch_rule():
+    """A batch just large enough for the ring kernel equals its two halves, which the rows kernel takes: the update is the
+    same fp32 expression (a 16-bit state may differ by one rounding, 2**-8 relative), y a sum of 128 terms in another order."""
+    b, h, p, n, g = 464, 128, 64, 128, 8
+    gen = torch.Generator(device=dev()).manual_seed(1)
+    rnd = lambda *s: torch.randn(*s, generator=gen, device=dev()).to(torch.bfloat16)
+    state, x, dt, B, C = rnd(b, h, p, n), rnd(b, h, p), rnd(b, h), rnd(b, g, n), rnd(b, g, n)
+    A = -torch.ones(h, device=dev())
+    halves = state.clone()
+    run = lambda s, r: ds().selective_state_update(s, x[r], dt[r][..., None].expand(-1, h, p), A[:, None, None].expand(h, p, n), B[r], C[r],
+                                                   dt_softplus=True)
+    y = run(state, slice(0, b))
+    yh = torch.cat([run(halves[:232], slice(0, 232)), run(halves[232:], slice(232, b))])
+    assert ((state.float() - halves.float()).abs() <= 2.0 ** -7 * halves.float().abs() + 1e-7).all()
+    assert_out_close(y, yh.float().cpu().numpy())
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("b,c,act,bias", [(1, 2, "silu", True), (3, 254, None, True), (5, 1284, "silu", False), (2, 10240, "silu", True)])
+def test_conv1d_two_channels_per_thread(dtype, b, c, act, bias):
+    m = ds()
+    rng = np.random.default_rng(c)
+    cur, weight = bf16r(rng.standard_normal((b, c, 4))), bf16r(rng.standard_normal((c, 4)) * 0.5)
+    cur, weight = (t(v, dtype).float().cpu().numpy() for v in (cur, weight))
+    bv = t(bf16r(rng.standard_normal(c)), dtype) if bias else None
+    conv_state = t(cur, dtype)
+    for _ in range(2):
+        x = t(bf16r(rng.standard_normal((b, c + 6))), dtype)[:, :c]  # rows are not contiguous
+        win, want = oracle.causal_conv1d_update(cur, x.float().cpu().numpy(), weight, None if bv is None else bv.float().cpu().numpy(), silu=act is not None)
+        out = m.causal_conv1d_update(x, conv_state, t(weight, dtype), bv, act)
+        np.testing.assert_array_equal(conv_state.float().cpu().numpy(), win)
+        assert_out_close(out, want)
+        cur = win

@@ -467,3 +467,23 @@ def test_append_vector_path_extremes(dtype):
         m._pack_kv_into_cache(ref, k.float().to(dev()), k.float().flip(0).to(dev()), pos, gs)
         for name in ("k_packed", "v_packed", "k_scale", "v_scale"):
             assert torch.equal(getattr(got, name).view(torch.uint8), getattr(ref, name).view(torch.uint8)), (gs, name)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("tlen", [16, 31, 32, 33, 95, 96, 97, 383, 384, 385, 511, 513])
+def test_decode_ring_edges(tlen, dtype):
+    """A warp takes a quarter of its CTA's tokens in stages of 32, three of them in flight; masked tokens at both ends of every stage."""
+    m = ia()
+    b, hq, hkv, gs = 2, 8, 2, 32
+    k, v = make_kv(tlen, b, hkv, tlen)
+    q = t(bf16r(np.random.default_rng(tlen + 1).standard_normal((b, hq, 1, 128))), dtype)
+    cache = fill_cache(m, k, v, gs)
+    keep = torch.ones(b, tlen, dtype=torch.bool, device=dev())
+    keep[1, 31::32] = False
+    keep[1, 32::32] = False
+    bias = torch.where(keep, 0.0, -1e9).cpu().numpy()
+    qf = q.float().cpu().numpy()[:, :, 0]
+    for splits in (1, 2):
+        assert_out_close(m._decode_attention(q, cache, tlen, 4, gs, splits=splits), oracle.int4_decode_attention(qf, *cache_np(cache), tlen, gs))
+        assert_out_close(m._decode_attention(q, cache, tlen, 4, gs, attention_mask=keep, splits=splits),
+                         oracle.int4_decode_attention(qf, *cache_np(cache), tlen, gs, bias))

@@ -415,3 +415,53 @@ def test_graph_mode_step_counters_match_host_steps(shared):
         assert torch.equal(a, bb)
     for a, bb in zip(want_c, got_c):
         assert torch.equal(a.q_state, bb.q_state) and torch.equal(a.shared_exp, bb.shared_exp) and torch.equal(a.micro_exp, bb.micro_exp)
+
+
+@pytest.mark.parametrize("bits,layout", [(8, "packed"), (8, "reference"), (4, "packed"), (4, "reference")])
+@pytest.mark.parametrize("shape,x_dtype", [
+    ((1, 1, 8, 128, 1), torch.bfloat16),      # one unit: one CTA, one step per warp
+    ((2, 3, 24, 128, 3), torch.float32),      # scalar staging of x, B and C; slabs of one unit
+    ((1, 4, 64, 16, 2), torch.float16),       # one block per row
+    ((3, 5, 20, 256, 5), torch.bfloat16),     # a row takes half a warp, rows per head not a power of two
+    ((10, 128, 64, 128, 8), torch.bfloat16),  # slabs of eight and nine units: ring stages partly filled
+    ((80, 128, 64, 128, 8), torch.bfloat16),  # more units than one wave of CTAs stages
+])
+def test_slab_kernel_edges_equal_general_kernel(bits, layout, shape, x_dtype):
+    """Partly filled ring stages, slabs across heads, groups and sequences, both ways of staging x and y, and block exponents for
+    which the decoder takes its plain form (values about 2**114 and 2**-130): the fp32 dump sends the second run to the general kernel."""
+    m = mk()
+    b, h, p, n, g = shape
+    gen = torch.Generator(device=dev()).manual_seed(b * p + n)
+    rnd = lambda *s: torch.randn(*s, generator=gen, device=dev())
+    state = rnd(b, h, p, n)
+    state[:, :, 0] *= 2.0 ** 114
+    state[:, :, 1] *= 2.0 ** -130
+    x, B, C = (v.to(x_dtype) for v in (rnd(b, h, p), rnd(b, g, n), rnd(b, g, n)))
+    dt = rnd(b, h).to(x_dtype)[..., None].expand(b, h, p)
+    A = -torch.exp(rnd(h))[:, None, None].expand(h, p, n)
+    D = torch.ones(h, device=dev())[:, None].expand(h, p)
+    res = []
+    for extra in ({}, dict(h_out=torch.empty((b, h, p, n), dtype=torch.float32, device=dev()))):
+        cache = m.allocate_state_kernel_cache(state, 16, bits, layout=layout)
+        y = m.mx_state_selective_update(cache, x, dt, A, B, C, D=D, dt_softplus=True, stochastic=True, seed=5, **extra)
+        res.append((y, cache.q_state, cache.shared_exp, cache.micro_exp))
+    for got, want in zip(*res):
+        assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("bits,layout", [(8, "packed"), (8, "reference"), (4, "packed"), (4, "reference")])
+@pytest.mark.parametrize("rows", [1, 15, 16, 31, 33])  # a CTA takes 256 blocks of 16 values
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+def test_dense_quantiser_equals_strided(bits, layout, rows, dtype):
+    from layer_quant_b200 import _lib
+    m = mk()
+    gen = torch.Generator(device=dev()).manual_seed(rows)
+    wide = (torch.randn(1, 1, rows, 256, generator=gen, device=dev()) * 100).to(dtype)
+    strided = wide[..., :128]
+    caches = []
+    for src in (strided.contiguous(), strided):
+        cache = m._empty_cache((1, 1, rows, 128), bits, layout, dev())
+        m._quantize_into(cache, src, _lib.Rounding(mode=_lib.LQ_ROUND_HALF_EVEN))
+        caches.append(cache)
+    a, c = caches
+    assert torch.equal(a.q_state, c.q_state) and torch.equal(a.shared_exp, c.shared_exp) and torch.equal(a.micro_exp, c.micro_exp)
