@@ -991,10 +991,15 @@ static int launch_prefill_tc(const lq_int4_prefill_args& a, int ratio, cudaStrea
   const int pos_per_cta = prefill::kCtaRows / ratio;
   p.nqb = (a.q_len + pos_per_cta - 1) / pos_per_cta;
   p.kv_len = a.first_len + a.q_len - 1;
-  const int64_t grid = static_cast<int64_t>(p.nqb) * a.cache.batch * a.cache.kv_heads;
-  LQ_CHECK_ARG(grid <= 0x7FFFFFFFLL, "lq_int4_prefill_attn: batch * kv heads * query blocks too large for one launch");
+  const int64_t blocks = static_cast<int64_t>(p.nqb) * a.cache.batch * a.cache.kv_heads;
+  LQ_CHECK_ARG(blocks <= 0x3FFFFFFFLL, "lq_int4_prefill_attn: batch * kv heads * query blocks too large for one launch");
+  // Blocks that fill no more than half of the last round are dealt as halves, one softmax group each: a tile of one group takes
+  // less time than a tile of two, and the other SMs would have nothing to do.
+  const int sms = sm_count(), rest = static_cast<int>(blocks % sms);
+  p.whole = static_cast<int>(blocks) - (2 * rest <= sms ? rest : 0);
+  p.entries = p.whole + 2 * (static_cast<int>(blocks) - p.whole);
   LQ_SET_SMEM_ONCE(prefill::int4_prefill_kernel, prefill::kSmemBytes);
-  prefill::int4_prefill_kernel<<<static_cast<unsigned>(grid), prefill::kThreads, prefill::kSmemBytes, st>>>(p);
+  prefill::int4_prefill_kernel<<<static_cast<unsigned>(std::min(p.entries, sms)), prefill::kThreads, prefill::kSmemBytes, st>>>(p);
   LQ_CHECK_CUDA(cudaGetLastError());
   return LQ_OK;
 }

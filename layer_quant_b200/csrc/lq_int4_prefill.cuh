@@ -30,7 +30,6 @@ constexpr int kTok = 64;                      // tokens per tile
 constexpr int kGroupRows = 128;               // rows of a softmax group
 constexpr int kCtaRows = 2 * kGroupRows;
 constexpr int kThreads = 512;                 // four warp groups; warps 13 .. 15 only fill the last one
-constexpr int kWorkers = 416;
 constexpr int kPart = kTok * 128 * 2;         // 16 KB: fp16 [64 tokens][128 dims], as two 128-byte-swizzled halves of 64 dims
 constexpr int kStageBytes = 2 * kPart;        // hi and lo part
 constexpr int kSmemBytes = 4 * kStageBytes + 1024;  // K stages 0, 1, V stages 0, 1; alignment of the swizzle atoms
@@ -43,7 +42,35 @@ struct Params {
   int32_t gs_log2;      // group size
   int32_t nqb;          // row blocks per (batch, kv head)
   int32_t kv_len;       // rows of the cache that hold tokens: first_len + q_len - 1
+  int32_t whole;        // entries of the work list that are whole row blocks; the rest are halves of one softmax group each
+  int32_t entries;
 };
+
+// An entry of the work list.  Heaviest row blocks first: a block's work grows with its last position.
+struct Block {
+  int b, kvh, pos0, groups, ntiles;
+};
+__device__ __forceinline__ Block block_at(const Params& p, int i) {
+  const int bh = p.a.cache.batch * p.a.cache.kv_heads;
+  int rows = kCtaRows >> p.ratio_log2, first = 0;
+  if (i >= p.whole) {
+    rows >>= 1;
+    first = (i - p.whole) & 1 ? rows : 0;
+    i = p.whole + ((i - p.whole) >> 1);
+  }
+  const int qb = p.nqb - 1 - i / bh, rest = i % bh;
+  Block k;
+  k.b = rest / p.a.cache.kv_heads;
+  k.kvh = rest % p.a.cache.kv_heads;
+  k.pos0 = qb * (kCtaRows >> p.ratio_log2) + first;
+  k.groups = rows == (kCtaRows >> p.ratio_log2) && k.pos0 + (rows >> 1) < p.a.q_len ? 2 : 1;  // softmax groups with a position of their own
+  k.ntiles = (p.a.first_len + min(k.pos0 + rows - 1, p.a.q_len - 1) + kTok - 1) / kTok;
+  return k;
+}
+// Round r of this CTA: the list is dealt forwards and backwards in turn, so that long and short blocks even out
+__device__ __forceinline__ int entry_of(int r) {
+  return r * static_cast<int>(gridDim.x) + static_cast<int>(r & 1 ? gridDim.x - 1 - blockIdx.x : blockIdx.x);
+}
 
 // ---- tcgen05 ---------------------------------------------------------------------------------------------------------
 #define LQ_R8(r, o) "=r"(r[o]), "=r"(r[o + 1]), "=r"(r[o + 2]), "=r"(r[o + 3]), "=r"(r[o + 4]), "=r"(r[o + 5]), "=r"(r[o + 6]), "=r"(r[o + 7])
@@ -113,7 +140,8 @@ struct Shared {
   // Few barriers: the thread that issues products runs only a few of them ahead of the tensor pipe, so every wait and commit of
   // its loop can cost tensor time.  Unit j of the unpacking warps is V of tile j and K of tile j + 1, what the products of
   // iteration j read; s_done of a tile also says that all products before it are done, O of the tile before among them.
-  uint64_t k_first, full[2], empty[2], s_done[2], p_ready[2];
+  // The tiles of a CTA's blocks are counted through, and K of the next block's first tile is part of the last unit of a block.
+  uint64_t k_first, full[2], empty[2], s_done[2], p_ready[2], q_ready[2];
   // Per 16 tokens: 2^Ek, Ev and 2^-Ev of the tile, four tiles deep (they are written a unit ahead of V)
   float k_factor[4][4], v_exp[4][4], v_inv[4][4];
   uint32_t tmem;
@@ -180,31 +208,49 @@ __device__ __forceinline__ void store_chunk(uint8_t* part_hi, int token, int chu
   }
 }
 
-__device__ __forceinline__ void unpack_tiles(const Params& p, Shared& sh, uint8_t* smem, int b, int kvh, int ntiles) {
+__device__ __forceinline__ void unpack_tiles(const Params& p, Shared& sh, uint8_t* smem) {
   const lq_int4_cache& c = p.a.cache;
   const int warp = (threadIdx.x >> 5) & 3, lane = threadIdx.x & 31;
   // lanes 0..7 hold eight tokens of chunk 0, lanes 8..15 the same tokens of chunk 1, ...: 512 contiguous bytes per load, and
   // the eight lanes of a shared-memory store phase hit eight different swizzle positions
   const int chunk = lane >> 3, row = 16 * warp + (lane & 7);
   const int groups_log2 = 7 - p.gs_log2, grp = (chunk * 32) >> p.gs_log2;
-  const uint8_t* kp = c.k_packed + b * c.kp_stride[0] + kvh * c.kp_stride[1] + chunk * 16;
-  const uint8_t* vp = c.v_packed + b * c.vp_stride[0] + kvh * c.vp_stride[1] + chunk * 16;
-  const float* ks = c.k_scale + b * c.ks_stride[0] + kvh * c.ks_stride[1] + grp;
-  const float* vs = c.v_scale + b * c.vs_stride[0] + kvh * c.vs_stride[1] + grp;
-  // 16 bytes (32 dims) of this lane's two tokens of a tile, and their scales
-  auto fetch = [&](const uint8_t* codes, int tile, uint4 (&raw)[2]) {
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      const int64_t tok = static_cast<int64_t>(tile) * kTok + row + 8 * i;
-      raw[i] = tok < p.kv_len ? __ldg(reinterpret_cast<const uint4*>(codes + tok * 64)) : make_uint4(0, 0, 0, 0);
+  // where the loads stand: a tile of a block; behind the last block no token is in range
+  constexpr int kNoToken = 0x7FFF0000;
+  int round = 0, tok = 0, tok_end = 0;
+  const uint8_t *kp = nullptr, *vp = nullptr;
+  const float *ks = nullptr, *vs = nullptr;
+  auto open_block = [&]() {
+    tok = row;
+    if (entry_of(round) >= p.entries) {
+      tok += kNoToken;
+      tok_end = 0x7FFFFFFF;
+      return;
+    }
+    const Block k = block_at(p, entry_of(round));
+    tok_end = k.ntiles * kTok;
+    kp = c.k_packed + k.b * c.kp_stride[0] + k.kvh * c.kp_stride[1] + chunk * 16;
+    vp = c.v_packed + k.b * c.vp_stride[0] + k.kvh * c.vp_stride[1] + chunk * 16;
+    ks = c.k_scale + k.b * c.ks_stride[0] + k.kvh * c.ks_stride[1] + grp;
+    vs = c.v_scale + k.b * c.vs_stride[0] + k.kvh * c.vs_stride[1] + grp;
+  };
+  auto advance = [&]() {
+    if (tok >= kNoToken) return;
+    tok += kTok;
+    if (tok >= tok_end) {
+      ++round;
+      open_block();
     }
   };
-  auto fetch_scales = [&](const float* scales, int tile, float (&sc)[2]) {
+  // 16 bytes (32 dims) of this lane's two tokens of a tile, and their scales
+  auto fetch = [&](const uint8_t* codes, int token, uint4 (&raw)[2]) {
 #pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      const int64_t tok = static_cast<int64_t>(tile) * kTok + row + 8 * i;
-      sc[i] = tok < p.kv_len ? __ldg(scales + (tok << groups_log2)) : 0.0f;
-    }
+    for (int i = 0; i < 2; ++i)
+      raw[i] = token + 8 * i < p.kv_len ? __ldg(reinterpret_cast<const uint4*>(codes + static_cast<int64_t>(token + 8 * i) * 64)) : make_uint4(0, 0, 0, 0);
+  };
+  auto fetch_scales = [&](const float* scales, int token, float (&sc)[2]) {
+#pragma unroll
+    for (int i = 0; i < 2; ++i) sc[i] = token + 8 * i < p.kv_len ? __ldg(scales + (static_cast<int64_t>(token + 8 * i) << groups_log2)) : 0.0f;
   };
   auto publish = [&](int tile, int ek, int ev) {
     if (lane == 0) {
@@ -224,13 +270,15 @@ __device__ __forceinline__ void unpack_tiles(const Params& p, Shared& sh, uint8_
   };
   uint4 k[2], v[2], k_next[2], v_next[2];
   float ks_cur[2], vs_cur[2], vs_ahead[2], ks_next[2], vs_next[2];  // scales of k and v above; of V one tile further
-  fetch(kp, 0, k);
-  fetch_scales(ks, 0, ks_cur);
-  fetch_scales(vs, 0, vs_cur);
-  fetch(vp, 0, v);
-  fetch(kp, 1, k_next);
-  fetch_scales(ks, 1, ks_next);
-  fetch_scales(vs, 1, vs_ahead);
+  open_block();
+  fetch(kp, tok, k);
+  fetch_scales(ks, tok, ks_cur);
+  fetch_scales(vs, tok, vs_cur);
+  fetch(vp, tok, v);
+  advance();
+  fetch(kp, tok, k_next);
+  fetch_scales(ks, tok, ks_next);
+  fetch_scales(vs, tok, vs_ahead);
   int ev = scale_exponent(vs_cur[0], vs_cur[1]);
   {
     const int ek = scale_exponent(ks_cur[0], ks_cur[1]);
@@ -238,22 +286,25 @@ __device__ __forceinline__ void unpack_tiles(const Params& p, Shared& sh, uint8_
     store(0, k, ks_cur, ek);
     arrive(&sh.k_first);
   }
-  for (int j = 0; j < ntiles; ++j) {
+  int total = 0;  // tiles of all blocks of this CTA
+  for (int r = 0; entry_of(r) < p.entries; ++r) total += block_at(p, entry_of(r)).ntiles;
+  for (int j = 0; j < total; ++j) {
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
       k[i] = k_next[i];
       ks_cur[i] = ks_next[i];
     }
-    fetch(kp, j + 2, k_next);  // past the last tile: zeros, not loaded
-    fetch_scales(ks, j + 2, ks_next);
-    fetch(vp, j + 1, v_next);
-    fetch_scales(vs, j + 2, vs_next);
+    fetch(vp, tok, v_next);
+    advance();
+    fetch(kp, tok, k_next);
+    fetch_scales(ks, tok, ks_next);
+    fetch_scales(vs, tok, vs_next);
     const int ek = scale_exponent(ks_cur[0], ks_cur[1]), ev_ahead = scale_exponent(vs_ahead[0], vs_ahead[1]);
     // iteration j - 2 is done (its last products are S of tile j - 1); unit 0 finds its stages empty, unit 1 waits for S of tile 0
     if (!wait_bar(&sh.empty[j & 1], ((j >> 1) ^ j ^ 1) & 1)) return;
     publish(j + 1, ek, ev_ahead);
     store(2 + (j & 1), v, vs_cur, ev);
-    if (j + 1 < ntiles) store((j + 1) & 1, k, ks_cur, ek);
+    if (j + 1 < total) store((j + 1) & 1, k, ks_cur, ek);
     arrive(&sh.full[j & 1]);
     ev = ev_ahead;
 #pragma unroll
@@ -266,7 +317,7 @@ __device__ __forceinline__ void unpack_tiles(const Params& p, Shared& sh, uint8_
 }
 
 // ---- products --------------------------------------------------------------------------------------------------------
-__device__ __forceinline__ void issue_products(Shared& sh, uint8_t* smem, int groups, int ntiles) {
+__device__ __forceinline__ void issue_products(const Params& p, Shared& sh, uint8_t* smem) {
   const uint64_t k_desc = smem_desc(smem_u32(smem), 16), v_desc = smem_desc(smem_u32(smem) + 2 * kStageBytes, kPart / 2);
   // S = Q Khi + Q Klo; 16 dims per product: 32 bytes inside a half of 64 dims
   auto issue_s = [&](int g, int j) {
@@ -279,39 +330,56 @@ __device__ __forceinline__ void issue_products(Shared& sh, uint8_t* smem, int gr
         mma_ts(tm + kColS, tm + kColQ + 8 * k, d + ((hl * kPart + (k >> 2) * (kPart / 2) + (k & 3) * 32) >> 4), kIdescS, hl + k > 0);
   };
   // O += Phi Vhi + Plo Vhi + Phi Vlo; 16 tokens per product: 2048 bytes
-  auto issue_o = [&](int g, int j) {
+  auto issue_o = [&](int g, int j, bool first) {
     const uint32_t tm = g * kColsPerGroup;
     const uint64_t d = v_desc + (j & 1) * (kStageBytes >> 4);
 #pragma unroll
     for (int t = 0; t < 3; ++t)
 #pragma unroll
       for (int k = 0; k < 4; ++k)
-        mma_ts(tm + kColO, tm + kColS + (t == 1 ? 32 : 0) + 8 * k, d + (((t == 2 ? kPart : 0) + k * 2048) >> 4), kIdescO, j + t + k > 0);
+        mma_ts(tm + kColO, tm + kColS + (t == 1 ? 32 : 0) + 8 * k, d + (((t == 2 ? kPart : 0) + k * 2048) >> 4), kIdescO, !first || t + k > 0);
   };
-  if (!wait_bar(&sh.k_first, 0)) return;
-  fence_after();
-  if (elect_one()) {
+  uint32_t p_parity = 0, q_parity = 0;  // bit g
+  // S of a block's first tile, once the groups have put their query rows into TMEM
+  auto open_block = [&](int groups, int tile) {
     for (int g = 0; g < groups; ++g) {
-      issue_s(g, 0);
-      mma_commit(&sh.s_done[g]);
-    }
-    mma_commit(&sh.empty[1]);
-  }
-  __syncwarp();
-  for (int j = 0; j < ntiles; ++j) {
-    const bool more = j + 1 < ntiles;
-    if (!wait_bar(&sh.full[j & 1], (j >> 1) & 1)) return;
-    for (int g = 0; g < groups; ++g) {
-      if (!wait_bar(&sh.p_ready[g], j & 1)) return;
+      if (!wait_bar(&sh.q_ready[g], (q_parity >> g) & 1)) return false;
+      q_parity ^= 1u << g;
       fence_after();
       if (elect_one()) {
-        issue_o(g, j);
-        if (more) issue_s(g, j + 1);
+        issue_s(g, tile);
         mma_commit(&sh.s_done[g]);
-        if (g == groups - 1) mma_commit(&sh.empty[j & 1]);
+        if (g == groups - 1) mma_commit(&sh.empty[(tile - 1) & 1]);
       }
       __syncwarp();
     }
+    return true;
+  };
+  if (!wait_bar(&sh.k_first, 0)) return;
+  Block k = block_at(p, entry_of(0));
+  if (!open_block(k.groups, 0)) return;
+  int tile = 0;
+  for (int r = 0;;) {
+    for (int j = 0; j < k.ntiles; ++j, ++tile) {
+      const bool more = j + 1 < k.ntiles;
+      if (!wait_bar(&sh.full[tile & 1], (tile >> 1) & 1)) return;
+      for (int g = 0; g < k.groups; ++g) {
+        if (!wait_bar(&sh.p_ready[g], (p_parity >> g) & 1)) return;
+        p_parity ^= 1u << g;
+        fence_after();
+        if (elect_one()) {
+          issue_o(g, tile, j == 0);
+          if (more) issue_s(g, tile + 1);
+          mma_commit(&sh.s_done[g]);
+          if (more && g == k.groups - 1) mma_commit(&sh.empty[tile & 1]);
+        }
+        __syncwarp();
+      }
+    }
+    ++r;
+    if (entry_of(r) >= p.entries) return;
+    k = block_at(p, entry_of(r));
+    if (!open_block(k.groups, tile)) return;
   }
 }
 
@@ -411,8 +479,9 @@ __device__ __forceinline__ void store_output(const lq_int4_prefill_args& a, int6
   }
 }
 
-// One row of scores, a tile at a time: S -> P in place, running maximum and sum.
-__device__ __forceinline__ void softmax_rows(const Params& p, Shared& sh, int b, int kvh, int pos0, int ntiles, float cq) {
+// One row of scores of one block, a tile at a time: S -> P in place, running maximum and sum.  tile: the block's first, counted over
+// all blocks; parity: of the next wait for products of this group; l_run: the sum.  False after a wait that ran out.
+__device__ __forceinline__ bool softmax_rows(const Params& p, Shared& sh, int pos0, int ntiles, int tile, uint32_t& parity, float cq, float& l_run) {
   const lq_int4_prefill_args& a = p.a;
   const int group = threadIdx.x >> 7, warp = (threadIdx.x >> 5) & 3, lane = threadIdx.x & 31;
   const int row = warp * 32 + lane;  // = TMEM lane
@@ -421,10 +490,12 @@ __device__ __forceinline__ void softmax_rows(const Params& p, Shared& sh, int b,
   // the tokens that every row of the warp sees
   const int warp_limit = a.first_len + min(pos0 + ((group * kGroupRows + warp * 32) >> p.ratio_log2), a.q_len - 1);
   const uint32_t tm = group * kColsPerGroup + (static_cast<uint32_t>(warp * 32) << 16);
-  float m_run = 0.0f, l_run = 0.0f;
+  float m_run = 0.0f;
+  l_run = 0.0f;
   for (int j = 0; j < ntiles; ++j) {
-    const int tok0 = j * kTok, f = j & 3;
-    if (!wait_bar(&sh.s_done[group], j & 1)) return;
+    const int tok0 = j * kTok, f = (tile + j) & 3;
+    if (!wait_bar(&sh.s_done[group], parity)) return false;
+    parity ^= 1;
     fence_after();
     uint32_t s[64];
     tmem_load64(s, tm + kColS);
@@ -486,25 +557,61 @@ __device__ __forceinline__ void softmax_rows(const Params& p, Shared& sh, int b,
     __syncwarp();
     if (lane == 0) mbar_arrive(&sh.p_ready[group]);
   }
-  if (!wait_bar(&sh.s_done[group], ntiles & 1)) return;
-  fence_after();
-  const int head = (kvh << p.ratio_log2) + (row & ((1 << p.ratio_log2) - 1));
-  const int64_t ob = b * a.out_stride[0] + head * a.out_stride[1] + static_cast<int64_t>(pos) * a.out_stride[2];
-  store_output(a, ob, tm + kColO, 1.0f / l_run, pos < a.q_len);
+  return true;
 }
 
-// Heaviest row blocks first: a block's work grows with its last position, and the tail of the grid is then made of short ones.
-__global__ void __launch_bounds__(kThreads, 1) int4_prefill_kernel(const Params p) {
+__device__ __forceinline__ void softmax_blocks(const Params& p, Shared& sh) {
+  const lq_int4_prefill_args& a = p.a;
+  const int group = threadIdx.x >> 7, warp = (threadIdx.x >> 5) & 3, lane = threadIdx.x & 31;
+  const int row = threadIdx.x & 127, in_block = static_cast<int>(threadIdx.x) >> p.ratio_log2;
+  const uint32_t tm = group * kColsPerGroup + (static_cast<uint32_t>(warp * 32) << 16);
+  const auto head_of = [&](const Block& k) { return (k.kvh << p.ratio_log2) + (row & ((1 << p.ratio_log2) - 1)); };
+  // the group's query rows of its first block from round r on, none of whose S has been asked for yet
+  const auto load_next = [&](int r, float& cq) {
+    for (; entry_of(r) < p.entries; ++r) {
+      const Block k = block_at(p, entry_of(r));
+      if (group >= k.groups) continue;
+      const int pos = k.pos0 + in_block;
+      const int64_t base = k.b * a.q_stride[0] + head_of(k) * a.q_stride[1] + static_cast<int64_t>(pos) * a.q_stride[2];
+      cq = load_query(a, base, pos < a.q_len, tm + kColQ);
+      fence_before();
+      __syncwarp();
+      return true;
+    }
+    return false;
+  };
+  uint32_t parity = 0;
+  int tile = 0;
+  float cq = 0.0f, l_run;
+  if (load_next(0, cq) && lane == 0) mbar_arrive(&sh.q_ready[group]);
+#pragma unroll 1
+  for (int r = 0; entry_of(r) < p.entries; ++r) {
+    const Block k = block_at(p, entry_of(r));
+    if (group < k.groups) {
+      if (!softmax_rows(p, sh, k.pos0, k.ntiles, tile, parity, cq, l_run)) return;
+      const bool more = load_next(r + 1, cq);  // all S of this block are done; its last products run meanwhile
+      // the wait stands before the arrival that lets the next S be asked for: s_done is never two phases ahead of a warp
+      if (!wait_bar(&sh.s_done[group], parity)) return;
+      parity ^= 1;
+      fence_after();
+      if (more && lane == 0) mbar_arrive(&sh.q_ready[group]);
+      const int pos = k.pos0 + in_block;
+      const int64_t ob = k.b * a.out_stride[0] + head_of(k) * a.out_stride[1] + static_cast<int64_t>(pos) * a.out_stride[2];
+      store_output(a, ob, tm + kColO, 1.0f / l_run, pos < a.q_len);
+    }
+    tile += k.ntiles;
+  }
+}
+
+// One CTA per SM works through a list of row blocks, and a block's start overlaps the end of the one before: its first tiles are
+// unpacked, its query rows loaded and its first scores made while the last products run and the output is stored.  A tile
+// takes 2.05 us (five products at 91 % of the measured dense rate); as one CTA per block, start and end added 8 to 9 us to every
+// block.  8 x 1024 tokens: 185 -> 160 us; 2 x 2000 behind 6001: 884 -> 855; 16 x 256: 53 -> 43; 1 x 128 behind 4000 (halves): 135 -> 110.
+// Dropped: two score buffers of 32 tokens per group, which would let the tensor pipe run ahead of the softmax (a product of 32 columns
+// takes as long as one of 64: 2.31 us a tile), and starting the products of a tile's first half while its second is made (2.1 us).
+__global__ void __launch_bounds__(kThreads, 1) int4_prefill_kernel(const __grid_constant__ Params p) {
   extern __shared__ uint8_t smem_raw[];
   __shared__ Shared sh;
-  const lq_int4_prefill_args& a = p.a;
-  const int bh = a.cache.batch * a.cache.kv_heads;
-  const int qb = p.nqb - 1 - static_cast<int>(blockIdx.x) / bh, rest = static_cast<int>(blockIdx.x) % bh;
-  const int b = rest / a.cache.kv_heads, kvh = rest % a.cache.kv_heads;
-  const int pos_per_cta = kCtaRows >> p.ratio_log2;
-  const int pos0 = qb * pos_per_cta;
-  const int groups = pos0 + (pos_per_cta >> 1) < a.q_len ? 2 : 1;  // softmax groups with a position of their own
-  const int ntiles = (a.first_len + min(pos0 + pos_per_cta - 1, a.q_len - 1) + kTok - 1) / kTok;
   uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
   const int warp = threadIdx.x >> 5;
   if (warp == 12) {
@@ -518,6 +625,7 @@ __global__ void __launch_bounds__(kThreads, 1) int4_prefill_kernel(const Params 
       mbar_init(&sh.empty[i], 1);
       mbar_init(&sh.s_done[i], 1);
       mbar_init(&sh.p_ready[i], 4);
+      mbar_init(&sh.q_ready[i], 4);
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -526,26 +634,11 @@ __global__ void __launch_bounds__(kThreads, 1) int4_prefill_kernel(const Params 
   fence_after();
   if (warp >= 8) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 88;");
-    if (warp < 12) {
-      asm volatile("barrier.cta.arrive 1, %0;" ::"n"(kWorkers) : "memory");
-      unpack_tiles(p, sh, smem, b, kvh, ntiles);
-    } else if (warp == 12) {
-      asm volatile("barrier.cta.sync 1, %0;" ::"n"(kWorkers) : "memory");  // Q is in TMEM
-      fence_after();
-      issue_products(sh, smem, groups, ntiles);
-    }
+    if (warp < 12) unpack_tiles(p, sh, smem);
+    else if (warp == 12) issue_products(p, sh, smem);
   } else {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 168;");
-    float cq = 0.0f;
-    if ((warp >> 2) < groups) {  // the unpacking warps start on the first tiles while the query rows travel
-      const int row = threadIdx.x & 127, pos = pos0 + (static_cast<int>(threadIdx.x) >> p.ratio_log2);
-      const int head = (kvh << p.ratio_log2) + (row & ((1 << p.ratio_log2) - 1));
-      const int64_t base = b * a.q_stride[0] + head * a.q_stride[1] + static_cast<int64_t>(pos) * a.q_stride[2];
-      cq = load_query(a, base, pos < a.q_len, (warp >> 2) * kColsPerGroup + (static_cast<uint32_t>((warp & 3) * 32) << 16) + kColQ);
-      fence_before();
-    }
-    asm volatile("barrier.cta.arrive 1, %0;" ::"n"(kWorkers) : "memory");
-    if ((warp >> 2) < groups) softmax_rows(p, sh, b, kvh, pos0, ntiles, cq);
+    softmax_blocks(p, sh);
   }
   fence_before();
   __syncthreads();

@@ -487,3 +487,23 @@ def test_decode_ring_edges(tlen, dtype):
         assert_out_close(m._decode_attention(q, cache, tlen, 4, gs, splits=splits), oracle.int4_decode_attention(qf, *cache_np(cache), tlen, gs))
         assert_out_close(m._decode_attention(q, cache, tlen, 4, gs, attention_mask=keep, splits=splits),
                          oracle.int4_decode_attention(qf, *cache_np(cache), tlen, gs, bias))
+
+
+@pytest.mark.parametrize("batch,tq,first", [(74, 40, 1), (38, 130, 100), (31, 300, 1), (75, 33, 65)])
+def test_prefill_work_list_equals_single_sequences(batch, tq, first):
+    """Blocks dealt over several rounds, as wholes and as halves, with one or two softmax groups: a row's arithmetic does not depend on
+    the deal, so each sequence must equal, bit for bit, a launch of its own (whose few blocks are halves of one round)."""
+    m = ia()
+    gen = torch.Generator(device=dev()).manual_seed(batch)
+    cap = 512
+    cache = m._allocate_layer_cache(batch, 2, cap, 128, 4, dev())
+    k, v = (torch.randn(batch, 2, first + tq - 1, 128, generator=gen, device=dev()).to(torch.bfloat16) for _ in range(2))
+    m._pack_kv_into_cache(cache, k, v, torch.arange(first + tq - 1, device=dev()), 32)
+    q = torch.randn(batch, 8, tq, 128, generator=gen, device=dev()).to(torch.bfloat16)
+    out = m._prefill_attention(q, cache, 4, 32, first_len=first)
+    for b in range(0, batch, 3):
+        one = m._allocate_layer_cache(1, 2, cap, 128, 4, dev())
+        m._pack_kv_into_cache(one, k[b:b + 1], v[b:b + 1], torch.arange(first + tq - 1, device=dev()), 32)
+        assert torch.equal(out[b:b + 1], m._prefill_attention(q[b:b + 1], one, 4, 32, first_len=first))
+    from layer_quant_b200 import _lib
+    assert _lib.device_status() == 0
