@@ -11,8 +11,9 @@
 //
 // Precision.  A dequantised value n * scale (n in [-8, 7]) is held as two fp16 numbers: the leading 8 bits of the scale
 // times n, exact in fp16, and the rest of the scale times n, rounded to fp16: 2^-20 relative in all.  P is split
-// the same way (2^-22).  Q is exact in fp16 for 16-bit queries.  S = Q Khi + Q Klo, O = Phi Vhi + Plo Vhi + Phi Vlo: five
-// products per tile pair, all in fp32 accumulators.  (The mma.sync kernel keeps 16 bits of P * v_scale.)
+// the same way: 2^-22 of a weight or 2^-35 of the row's largest, whichever is more.  (The mma.sync kernel keeps 2^-17 of every
+// weight.  The absolute part adds up to less than that over 2^17 tokens.)  Q is exact in fp16 for 16-bit queries.
+// S = Q Khi + Q Klo, O = Phi Vhi + Plo Vhi + Phi Vlo: five products per tile pair, all in fp32 accumulators.
 // Range.  Powers of two are taken out of every row of Q and of the K and V scales of every 16 tokens, so the
 // fp16 operands sit at the top of their range; the exponents come back for free, in the factor and the offset of the
 // exp2 argument.  With p' = 2^(s + Ev - m) the V exponent Ev is part of the running maximum m.
@@ -34,7 +35,11 @@ constexpr int kPart = kTok * 128 * 2;         // 16 KB: fp16 [64 tokens][128 dim
 constexpr int kStageBytes = 2 * kPart;        // hi and lo part
 constexpr int kSmemBytes = 4 * kStageBytes + 1024;  // K stages 0, 1, V stages 0, 1; alignment of the swizzle atoms
 constexpr uint32_t kColO = 0, kColQ = 128, kColS = 192, kColsPerGroup = 256;
-constexpr float kSlack = 8.0f;                // the running maximum is raised when a score exceeds it by more (log2 units)
+// The running maximum is raised when a score exceeds it by more than kSlack (log2 units), and weights are held times 2^kLift: what
+// fp16 cannot hold is the absolute 2^-24, so the top of its range has to be used.  2^(kSlack + kLift) must stay below 65504.  A wider slack
+// raises the maximum less often and leaves less lift: with 8 and 0 weights below 2^-25 of the largest were lost altogether, at 969 us
+// against 977 for 2 x 2000 tokens behind 6001.
+constexpr float kSlack = 4.0f, kLift = 11.0f;
 
 struct Params {
   lq_int4_prefill_args a;
@@ -533,7 +538,7 @@ __device__ __forceinline__ bool softmax_rows(const Params& p, Shared& sh, int po
     }
 #pragma unroll
     for (int w = 0; w < 4; ++w) {
-      const float off = ev[w] - m_run;
+      const float off = ev[w] - m_run + kLift;
       float2 sum = make_float2(0.0f, 0.0f);
       uint32_t hi[8], lo[8];
 #pragma unroll
@@ -542,7 +547,7 @@ __device__ __forceinline__ bool softmax_rows(const Params& p, Shared& sh, int po
                                     make_float2(off, off));
         const float2 pr = make_float2(mma::fast_exp2(x.x), mma::fast_exp2(x.y));
         sum = __fadd2_rn(sum, pr);
-        // leading 11 bits by truncation (exact in fp16), the rest rounded to fp16
+        // leading 11 bits by truncation (exact in fp16 from 2^-14 on), the rest rounded to fp16
         const float2 top = make_float2(__uint_as_float(__float_as_uint(pr.x) & 0xFFFFE000u), __uint_as_float(__float_as_uint(pr.y) & 0xFFFFE000u));
         const float2 rest = __ffma2_rn(top, make_float2(-1.0f, -1.0f), pr);
         hi[i] = pack_half2(top.x, top.y);

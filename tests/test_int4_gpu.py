@@ -507,3 +507,22 @@ def test_prefill_work_list_equals_single_sequences(batch, tq, first):
         assert torch.equal(out[b:b + 1], m._prefill_attention(q[b:b + 1], one, 4, 32, first_len=first))
     from layer_quant_b200 import _lib
     assert _lib.device_status() == 0
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("delta", [9.3, 16.45, 20.4, 22.7, 24.4, 26.3])
+def test_prefill_keeps_small_weights(delta, dtype):
+    """One token outweighs each of 8191 others by 2**delta and its V is zero, so the output is the others' weights alone.  A weight is
+    held to 2**-35 of the largest one (fp16 hi + lo under an offset of 2**11), or 2**-20 of itself if that is more; the rest is the
+    output's own rounding.  All weights are equal, so their errors add up."""
+    m = ia()
+    tlen, gs = 8192, 32
+    k, v = np.zeros((1, 1, tlen, 128), np.float32), np.ones((1, 1, tlen, 128), np.float32)
+    k[0, 0, 0] = delta * np.log(2.0) / np.sqrt(128.0)  # a query of ones scores it delta in units of a factor of two
+    v[0, 0, 0] = 0.0
+    cache = fill_cache(m, k, v, gs, dtype=torch.float32)
+    q = np.ones((1, 4, 2, 128), np.float32)
+    ref = oracle.int4_prefill_attention(q, *cache_np(cache), tlen - 1, gs)
+    got = m._prefill_attention(t(q, dtype), cache, 4, gs, first_len=tlen - 1).float().cpu().numpy()
+    out_rounding = 2.0 ** -9 if dtype == torch.bfloat16 else 2.0 ** -12
+    assert np.abs(got / ref - 1.0).max() <= 2 * out_rounding + 2.0 ** (delta - 35) + 2.0 ** -18
