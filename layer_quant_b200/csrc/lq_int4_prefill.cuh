@@ -17,6 +17,11 @@
 // Range.  Powers of two are taken out of every row of Q and of the K and V scales of every 16 tokens, so the
 // fp16 operands sit at the top of their range; the exponents come back for free, in the factor and the offset of the
 // exp2 argument.  With p' = 2^(s + Ev - m) the V exponent Ev is part of the running maximum m.
+// Sixteen tokens whose scales lie more than 2^kSpread apart or are not all finite ("wide") get an exponent each, applied in a pass
+// of its own over the tile's scores: a very large K or V changes nothing for the rows before it.  An infinite or NaN scale is
+// stored as zero; the rows that attend to it get a NaN score (K) or NaN in the 32 dims (V).
+// What remains relative to the largest: inside a token the group scales below 2^-15 of its largest lose bits, and a weight times
+// V counts with the row's largest (first item), whichever group that is in.
 //
 // What bounds it: the five products take 5/2 of the tensor time of a bf16 attention.  Per 256 x 64 tile that is 2620 cycles;
 // shared memory moves 230 KB meanwhile (1800 cycles), which is why Q is an operand in TMEM, and the exp2 take 1024.
@@ -35,6 +40,7 @@ constexpr int kPart = kTok * 128 * 2;         // 16 KB: fp16 [64 tokens][128 dim
 constexpr int kStageBytes = 2 * kPart;        // hi and lo part
 constexpr int kSmemBytes = 4 * kStageBytes + 1024;  // K stages 0, 1, V stages 0, 1; alignment of the swizzle atoms
 constexpr uint32_t kColO = 0, kColQ = 128, kColS = 192, kColsPerGroup = 256;
+constexpr int kSpread = 8;                    // binades that the scales of 16 tokens may span under one exponent
 // The running maximum is raised when a score exceeds it by more than kSlack (log2 units), and weights are held times 2^kLift: what
 // fp16 cannot hold is the absolute 2^-24, so the top of its range has to be used.  2^(kSlack + kLift) must stay below 65504.  A wider slack
 // raises the maximum less often and leaves less lift: with 8 and 0 weights below 2^-25 of the largest were lost altogether, at 969 us
@@ -82,6 +88,14 @@ __device__ __forceinline__ int entry_of(int r) {
 #define LQ_I8(r, o) "r"(r[o]), "r"(r[o + 1]), "r"(r[o + 2]), "r"(r[o + 3]), "r"(r[o + 4]), "r"(r[o + 5]), "r"(r[o + 6]), "r"(r[o + 7])
 
 // columns of this warp's 32 lanes; the wait is part of the statement, so no use can move before it
+__device__ __forceinline__ void tmem_load16(uint32_t (&r)[16], uint32_t addr) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n\t"
+      "tcgen05.wait::ld.sync.aligned;"
+      : LQ_R8(r, 0), LQ_R8(r, 8)
+      : "r"(addr)
+      : "memory");
+}
 __device__ __forceinline__ void tmem_load32(uint32_t (&r)[32], uint32_t addr) {
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,"
@@ -103,6 +117,11 @@ __device__ __forceinline__ void tmem_store32(uint32_t addr, const uint32_t (&r)[
   asm volatile(
       "tcgen05.st.sync.aligned.32x32b.x32.b32 [%32], {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,"
       "%22,%23,%24,%25,%26,%27,%28,%29,%30,%31};" ::LQ_I8(r, 0), LQ_I8(r, 8), LQ_I8(r, 16), LQ_I8(r, 24), "r"(addr)
+      : "memory");
+}
+__device__ __forceinline__ void tmem_store16(uint32_t addr, const uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%16], {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15};" ::LQ_I8(r, 0), LQ_I8(r, 8), "r"(addr)
       : "memory");
 }
 __device__ __forceinline__ void tmem_store8(uint32_t addr, const uint32_t (&r)[8]) {
@@ -148,7 +167,12 @@ struct Shared {
   // The tiles of a CTA's blocks are counted through, and K of the next block's first tile is part of the last unit of a block.
   uint64_t k_first, full[2], empty[2], s_done[2], p_ready[2], q_ready[2];
   // Per 16 tokens: 2^Ek, Ev and 2^-Ev of the tile, four tiles deep (they are written a unit ahead of V)
-  float k_factor[4][4], v_exp[4][4], v_inv[4][4];
+  float k_factor[5][4], v_exp[5][4], v_inv[5][4];  // slot 4: 1, 0, 0
+  // A byte per 16 tokens: they are wide.  Then the same per token (k_factor NaN: the scale is not finite), and the 32-dim chunks of V
+  // whose scale is not finite, a bit each
+  uint32_t wide[4];
+  float k_factor_tok[4][kTok], v_exp_tok[4][kTok], v_inv_tok[4][kTok];
+  uint8_t v_bad_tok[4][kTok];
   uint32_t tmem;
 };
 
@@ -182,11 +206,39 @@ __device__ __forceinline__ void unpack8(uint32_t x, __half2 (&n)[4]) {
   n[3] = __hfma2(*reinterpret_cast<const __half2*>(&b3), sixteenth, off16);
 }
 
-// The exponent that brings the largest of a warp's scales to [2^11, 2^12): n * scale then stays below 2^15
-__device__ __forceinline__ int scale_exponent(float a, float b) {
-  const uint32_t m = __reduce_max_sync(0xFFFFFFFFu, max(__float_as_uint(a), __float_as_uint(b)));  // scales are positive or zero
-  const int field = static_cast<int>((m >> 23) & 0xFFu);
-  return field == 0 ? 0 : min(max(field - 127 - 11, -110), 110);
+// The exponent that brings a scale (its bits) to [2^11, 2^12): n * scale then stays below 2^15
+__device__ __forceinline__ int exponent_of(uint32_t bits) {
+  const int field = static_cast<int>(bits >> 23);
+  return field == 0 ? 0 : max(field - 127 - 11, -110);
+}
+// The scales of a warp's 16 tokens, two tokens of one chunk per lane (the chunks eight lanes apart): one exponent, that of the largest, or
+// where they are wide one per token.  bad: a ballot of the scales that are not finite, per token of the lane; these become 0.
+struct Exponents {
+  int e[2];
+  uint32_t bad[2];
+  bool wide;
+};
+__device__ __forceinline__ Exponents exponents_of(float (&sc)[2]) {
+  Exponents r;
+  const uint32_t b[2] = {__float_as_uint(sc[0]), __float_as_uint(sc[1])};  // scales are positive or zero
+  const uint32_t hi = __reduce_max_sync(0xFFFFFFFFu, max(b[0], b[1]));
+  r.e[0] = r.e[1] = exponent_of(hi);
+  r.bad[0] = r.bad[1] = 0u;
+  const uint32_t least = min(b[0] - 1, b[1] - 1);  // 0 (a row without a token) does not count
+  r.wide = __any_sync(0xFFFFFFFFu, hi >= 0x7F800000u || (hi >> 23) > (least >> 23) + kSpread);
+  if (r.wide) {
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const bool finite = (b[i] & 0x7FFFFFFFu) < 0x7F800000u;
+      r.bad[i] = __ballot_sync(0xFFFFFFFFu, !finite);
+      if (!finite) sc[i] = 0.0f;
+      uint32_t m = finite ? b[i] & 0x7FFFFFFFu : 0u;
+      m = max(m, __shfl_xor_sync(0xFFFFFFFFu, m, 8));
+      m = max(m, __shfl_xor_sync(0xFFFFFFFFu, m, 16));
+      r.e[i] = exponent_of(m);
+    }
+  }
+  return r;
 }
 
 // 32 dims of one token -> shared memory: 64 bytes of the hi part and of the lo part
@@ -257,16 +309,30 @@ __device__ __forceinline__ void unpack_tiles(const Params& p, Shared& sh, uint8_
 #pragma unroll
     for (int i = 0; i < 2; ++i) sc[i] = token + 8 * i < p.kv_len ? __ldg(scales + (static_cast<int64_t>(token + 8 * i) << groups_log2)) : 0.0f;
   };
-  auto publish = [&](int tile, int ek, int ev) {
+  auto publish = [&](int tile, const Exponents& ek, const Exponents& ev) {
+    const int f = tile & 3;
+    const bool wide = ek.wide || ev.wide;
     if (lane == 0) {
-      sh.k_factor[tile & 3][warp] = pow2_of(ek);
-      sh.v_exp[tile & 3][warp] = static_cast<float>(ev);
-      sh.v_inv[tile & 3][warp] = pow2_of(-ev);
+      sh.k_factor[f][warp] = pow2_of(ek.e[0]);
+      sh.v_exp[f][warp] = static_cast<float>(ev.e[0]);
+      sh.v_inv[f][warp] = pow2_of(-ev.e[0]);
+      reinterpret_cast<uint8_t*>(&sh.wide[f])[warp] = wide;
+    }
+    if (wide && chunk == 0) {
+      constexpr uint32_t kChunks = 0x01010101u;  // a token's bits of a ballot
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const uint32_t v_bad = (ev.bad[i] >> lane) & kChunks;
+        sh.k_factor_tok[f][row + 8 * i] = (ek.bad[i] >> lane) & kChunks ? __uint_as_float(0x7FC00000u) : pow2_of(ek.e[i]);
+        sh.v_exp_tok[f][row + 8 * i] = static_cast<float>(ev.e[i]);
+        sh.v_inv_tok[f][row + 8 * i] = pow2_of(-ev.e[i]);
+        sh.v_bad_tok[f][row + 8 * i] = static_cast<uint8_t>((v_bad | v_bad >> 7 | v_bad >> 14 | v_bad >> 21) & 15u);
+      }
     }
   };
-  auto store = [&](int stage, const uint4 (&raw)[2], const float (&sc)[2], int e) {
+  auto store = [&](int stage, const uint4 (&raw)[2], const float (&sc)[2], const int (&e)[2]) {
 #pragma unroll
-    for (int i = 0; i < 2; ++i) store_chunk(smem + stage * kStageBytes, row + 8 * i, chunk, raw[i], sc[i], e);
+    for (int i = 0; i < 2; ++i) store_chunk(smem + stage * kStageBytes, row + 8 * i, chunk, raw[i], sc[i], e[i]);
   };
   auto arrive = [&](uint64_t* bar) {
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -284,11 +350,13 @@ __device__ __forceinline__ void unpack_tiles(const Params& p, Shared& sh, uint8_
   fetch(kp, tok, k_next);
   fetch_scales(ks, tok, ks_next);
   fetch_scales(vs, tok, vs_ahead);
-  int ev = scale_exponent(vs_cur[0], vs_cur[1]);
+  int ev[2];
   {
-    const int ek = scale_exponent(ks_cur[0], ks_cur[1]);
-    publish(0, ek, ev);
-    store(0, k, ks_cur, ek);
+    const Exponents ek = exponents_of(ks_cur), ev_first = exponents_of(vs_cur);
+    ev[0] = ev_first.e[0];
+    ev[1] = ev_first.e[1];
+    publish(0, ek, ev_first);
+    store(0, k, ks_cur, ek.e);
     arrive(&sh.k_first);
   }
   int total = 0;  // tiles of all blocks of this CTA
@@ -304,16 +372,16 @@ __device__ __forceinline__ void unpack_tiles(const Params& p, Shared& sh, uint8_
     fetch(kp, tok, k_next);
     fetch_scales(ks, tok, ks_next);
     fetch_scales(vs, tok, vs_next);
-    const int ek = scale_exponent(ks_cur[0], ks_cur[1]), ev_ahead = scale_exponent(vs_ahead[0], vs_ahead[1]);
+    const Exponents ek = exponents_of(ks_cur), ev_ahead = exponents_of(vs_ahead);
     // iteration j - 2 is done (its last products are S of tile j - 1); unit 0 finds its stages empty, unit 1 waits for S of tile 0
     if (!wait_bar(&sh.empty[j & 1], ((j >> 1) ^ j ^ 1) & 1)) return;
     publish(j + 1, ek, ev_ahead);
     store(2 + (j & 1), v, vs_cur, ev);
-    if (j + 1 < total) store((j + 1) & 1, k, ks_cur, ek);
+    if (j + 1 < total) store((j + 1) & 1, k, ks_cur, ek.e);
     arrive(&sh.full[j & 1]);
-    ev = ev_ahead;
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
+      ev[i] = ev_ahead.e[i];
       v[i] = v_next[i];
       vs_cur[i] = vs_ahead[i];
       vs_ahead[i] = vs_next[i];
@@ -451,13 +519,15 @@ __device__ __forceinline__ float load_query(const lq_int4_prefill_args& a, int64
   return __uint_as_float(static_cast<uint32_t>(field - 14) << 23) * (1.4426950408889634f * 0.08838834764831845f);
 }
 
-__device__ __forceinline__ void store_output(const lq_int4_prefill_args& a, int64_t ob, uint32_t tm_o, float inv, bool live) {
+// bad: a bit per 32 dims that are NaN
+__device__ __forceinline__ void store_output(const lq_int4_prefill_args& a, int64_t ob, uint32_t tm_o, float inv_row, uint32_t bad, bool live) {
   const bool vec = a.out_stride[3] == 1 && ((reinterpret_cast<uintptr_t>(a.out) + 2 * ob) & 15) == 0;
 #pragma unroll 1
   for (int q = 0; q < 4; ++q) {
     uint32_t o[32];
     tmem_load32(o, tm_o + 32 * q);
     if (!live) continue;
+    const float inv = (bad >> q) & 1 ? __uint_as_float(0x7FC00000u) : inv_row;
 #pragma unroll
     for (int w = 0; w < 4; ++w) {
       float d[8];
@@ -485,8 +555,10 @@ __device__ __forceinline__ void store_output(const lq_int4_prefill_args& a, int6
 }
 
 // One row of scores of one block, a tile at a time: S -> P in place, running maximum and sum.  tile: the block's first, counted over
-// all blocks; parity: of the next wait for products of this group; l_run: the sum.  False after a wait that ran out.
-__device__ __forceinline__ bool softmax_rows(const Params& p, Shared& sh, int pos0, int ntiles, int tile, uint32_t& parity, float cq, float& l_run) {
+// all blocks; parity: of the next wait for products of this group; l_run: the sum; bad: the 32-dim chunks for which the row has
+// attended to a V that is not finite.  False after a wait that ran out.
+__device__ __forceinline__ bool softmax_rows(const Params& p, Shared& sh, int pos0, int ntiles, int tile, uint32_t& parity, float cq, float& l_run,
+                                             uint32_t& bad) {
   const lq_int4_prefill_args& a = p.a;
   const int group = threadIdx.x >> 7, warp = (threadIdx.x >> 5) & 3, lane = threadIdx.x & 31;
   const int row = warp * 32 + lane;  // = TMEM lane
@@ -497,23 +569,46 @@ __device__ __forceinline__ bool softmax_rows(const Params& p, Shared& sh, int po
   const uint32_t tm = group * kColsPerGroup + (static_cast<uint32_t>(warp * 32) << 16);
   float m_run = 0.0f;
   l_run = 0.0f;
+  bad = 0u;
   for (int j = 0; j < ntiles; ++j) {
     const int tok0 = j * kTok, f = (tile + j) & 3;
     if (!wait_bar(&sh.s_done[group], parity)) return false;
     parity ^= 1;
     fence_after();
+    const uint32_t wide = sh.wide[f];
     uint32_t s[64];
     tmem_load64(s, tm + kColS);
-    if (tok0 + kTok > warp_limit) {
+    // Rare cases share the branches that are there anyway: with branches of their own 1 x 128 behind 4000 took 115 us instead of 109.
+    if (tok0 + kTok > warp_limit || wide != 0u) {
+      if (wide != 0u) {  // the finished score of every token in place of the raw one
+#pragma unroll 1
+        for (int w = 0; w < 4; ++w) {
+          const bool own = (wide >> (8 * w)) & 1u;
+          const float* const kf = own ? &sh.k_factor_tok[f][16 * w] : &sh.k_factor[f][w];
+          const float* const ve = own ? &sh.v_exp_tok[f][16 * w] : &sh.v_exp[f][w];
+          uint32_t raw[16];
+          tmem_load16(raw, tm + kColS + 16 * w);
+#pragma unroll
+          for (int i = 0; i < 16; ++i) {
+            raw[i] = __float_as_uint(fmaf(__uint_as_float(raw[i]), cq * kf[own ? i : 0], ve[own ? i : 0]));
+            if (own && tok0 + 16 * w + i < limit) bad |= sh.v_bad_tok[f][16 * w + i];
+          }
+          tmem_store16(tm + kColS + 16 * w, raw);
+        }
+        tmem_wait_store();
+        tmem_load64(s, tm + kColS);
+      }
 #pragma unroll
       for (int i = 0; i < 64; ++i)
         if (tok0 + i >= limit) s[i] = 0xFF800000u;  // -inf
     }
+    const int slot = wide != 0u ? 4 : f;  // 4: scores are finished, the sum is taken further down
+    const float cq_tile = wide != 0u ? 1.0f : cq;
     float cw[4], ev[4], mt[4];
 #pragma unroll
     for (int w = 0; w < 4; ++w) {
-      cw[w] = fmaxf(cq * sh.k_factor[f][w], 1.17549435e-38f);  // never 0: -inf * 0 would be NaN
-      ev[w] = sh.v_exp[f][w];
+      cw[w] = fmaxf(cq_tile * sh.k_factor[slot][w], 1.17549435e-38f);  // never 0: -inf * 0 would be NaN
+      ev[w] = sh.v_exp[slot][w];
       const auto at = [&](int i) { return __uint_as_float(s[16 * w + i]); };
       const float m0 = max3(at(0), at(1), at(2)), m1 = max3(at(3), at(4), at(5)), m2 = max3(at(6), at(7), at(8));
       const float m3 = max3(at(9), at(10), at(11)), m4 = max3(at(12), at(13), at(14));
@@ -522,23 +617,38 @@ __device__ __forceinline__ bool softmax_rows(const Params& p, Shared& sh, int po
     const float m_tile = fmaxf(fmaxf(mt[0], mt[1]), fmaxf(mt[2], mt[3]));
     if (j == 0) {
       m_run = m_tile;  // every row sees token 0
-    } else if (__any_sync(0xFFFFFFFFu, m_tile > m_run + kSlack)) {
-      // rare: the running sums of this warp's rows move to a larger maximum (the products into O of the tile before are done)
-      const float m_new = fmaxf(m_run, m_tile), alpha = exp2f(m_run - m_new);
-      m_run = m_new;
-      l_run *= alpha;
+    }
+    if (__any_sync(0xFFFFFFFFu, m_tile > m_run + kSlack || wide != 0u)) {
+      if (j > 0) {
+        // rare: the running sums of this warp's rows move to a larger maximum (the products into O of the tile before are done)
+        const float m_new = fmaxf(m_run, m_tile), alpha = exp2f(m_run - m_new);
+        m_run = m_new;
+        l_run *= alpha;
 #pragma unroll 1
-      for (int q = 0; q < 4; ++q) {
-        uint32_t o[32];
-        tmem_load32(o, tm + kColO + 32 * q);
+        for (int q = 0; q < 4; ++q) {
+          uint32_t o[32];
+          tmem_load32(o, tm + kColO + 32 * q);
 #pragma unroll
-        for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
-        tmem_store32(tm + kColO + 32 * q, o);
+          for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+          tmem_store32(tm + kColO + 32 * q, o);
+        }
+      }
+      if (wide != 0u) {  // the sum of the very weights that are stored below
+#pragma unroll 1
+        for (int w = 0; w < 4; ++w) {
+          const bool own = (wide >> (8 * w)) & 1u;
+          const float* const vi = own ? &sh.v_inv_tok[f][16 * w] : &sh.v_inv[f][w];
+          uint32_t x[16];
+          tmem_load16(x, tm + kColS + 16 * w);
+#pragma unroll
+          for (int i = 0; i < 16; ++i)
+            if (tok0 + 16 * w + i < limit) l_run = fmaf(mma::fast_exp2(__uint_as_float(x[i]) + (kLift - m_run)), vi[own ? i : 0], l_run);
+        }
       }
     }
 #pragma unroll
     for (int w = 0; w < 4; ++w) {
-      const float off = ev[w] - m_run + kLift;
+      const float off = ev[w] + (kLift - m_run);
       float2 sum = make_float2(0.0f, 0.0f);
       uint32_t hi[8], lo[8];
 #pragma unroll
@@ -555,7 +665,7 @@ __device__ __forceinline__ bool softmax_rows(const Params& p, Shared& sh, int po
       }
       tmem_store8(tm + kColS + 8 * w, hi);
       tmem_store8(tm + kColS + 32 + 8 * w, lo);
-      l_run = fmaf(sum.x + sum.y, sh.v_inv[f][w], l_run);
+      l_run = fmaf(sum.x + sum.y, sh.v_inv[slot][w], l_run);
     }
     tmem_wait_store();
     fence_before();
@@ -588,12 +698,13 @@ __device__ __forceinline__ void softmax_blocks(const Params& p, Shared& sh) {
   uint32_t parity = 0;
   int tile = 0;
   float cq = 0.0f, l_run;
+  uint32_t bad;
   if (load_next(0, cq) && lane == 0) mbar_arrive(&sh.q_ready[group]);
 #pragma unroll 1
   for (int r = 0; entry_of(r) < p.entries; ++r) {
     const Block k = block_at(p, entry_of(r));
     if (group < k.groups) {
-      if (!softmax_rows(p, sh, k.pos0, k.ntiles, tile, parity, cq, l_run)) return;
+      if (!softmax_rows(p, sh, k.pos0, k.ntiles, tile, parity, cq, l_run, bad)) return;
       const bool more = load_next(r + 1, cq);  // all S of this block are done; its last products run meanwhile
       // the wait stands before the arrival that lets the next S be asked for: s_done is never two phases ahead of a warp
       if (!wait_bar(&sh.s_done[group], parity)) return;
@@ -602,7 +713,7 @@ __device__ __forceinline__ void softmax_blocks(const Params& p, Shared& sh) {
       if (more && lane == 0) mbar_arrive(&sh.q_ready[group]);
       const int pos = k.pos0 + in_block;
       const int64_t ob = k.b * a.out_stride[0] + head_of(k) * a.out_stride[1] + static_cast<int64_t>(pos) * a.out_stride[2];
-      store_output(a, ob, tm + kColO, 1.0f / l_run, pos < a.q_len);
+      store_output(a, ob, tm + kColO, 1.0f / l_run, bad, pos < a.q_len);
     }
     tile += k.ntiles;
   }
@@ -622,6 +733,10 @@ __global__ void __launch_bounds__(kThreads, 1) int4_prefill_kernel(const __grid_
   if (warp == 12) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(&sh.tmem)) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+  }
+  if (threadIdx.x < 4) {
+    sh.k_factor[4][threadIdx.x] = 1.0f;
+    sh.v_exp[4][threadIdx.x] = sh.v_inv[4][threadIdx.x] = 0.0f;
   }
   if (threadIdx.x == 0) {
     mbar_init(&sh.k_first, 4);

@@ -526,3 +526,32 @@ def test_prefill_keeps_small_weights(delta, dtype):
     got = m._prefill_attention(t(q, dtype), cache, 4, gs, first_len=tlen - 1).float().cpu().numpy()
     out_rounding = 2.0 ** -9 if dtype == torch.bfloat16 else 2.0 ** -12
     assert np.abs(got / ref - 1.0).max() <= 2 * out_rounding + 2.0 ** (delta - 35) + 2.0 ** -18
+
+
+@pytest.mark.parametrize("gs", [32, 64, 128])
+@pytest.mark.parametrize("which", ["k", "v"])
+@pytest.mark.parametrize("size", [1e3, 3e4, 1e6, 1e14, 1e36, np.inf])
+def test_prefill_rows_do_not_depend_on_later_tokens(size, which, gs):
+    """A very large or infinite key or value: rows before it equal the oracle, as if it were not there; rows that attend to it equal the
+    oracle within what is largest in them, and where the oracle has no number they have none either."""
+    m = ia()
+    tq, at = 150, (10, 77)  # the first inside a tile's first 16 tokens, the second in the second tile
+    k, v = make_kv(61, 1, 2, tq)
+    q = bf16r(np.random.default_rng(62).standard_normal((1, 8, tq, 128)) * 0.5)
+    for head, token in enumerate(at):
+        (k if which == "k" else v)[0, head, token, 40:44] = size
+    cache = fill_cache(m, k, v, gs, dtype=torch.float32)
+    with np.errstate(all="ignore"):
+        ref = oracle.int4_prefill_attention(q, *cache_np(cache), 1, gs)
+    out = m._prefill_attention(t(q, torch.bfloat16), cache, 4, gs)
+    for head in range(8):
+        token = at[head // 4]
+        if which == "v" and not np.isfinite(size):
+            ref[0, head, :token] = oracle.int4_prefill_attention(q[:, head:head + 1, :token], *(x[:, head // 4:head // 4 + 1] for x in cache_np(cache)), 1, gs)[0, 0]
+        assert np.isfinite(ref[0, head, :token]).all()
+        for row in range(tq):
+            want, got = ref[0, head, row], out[0, head, row]
+            finite = np.isfinite(want)
+            assert not torch.isfinite(got[torch.from_numpy(~finite)]).any()
+            if finite.any():
+                assert_out_close(got[torch.from_numpy(finite)], want[finite])
