@@ -46,6 +46,10 @@ constexpr int kSpread = 8;                    // binades that the scales of 16 t
 // raises the maximum less often and leaves less lift: with 8 and 0 weights below 2^-25 of the largest were lost altogether, at 969 us
 // against 977 for 2 x 2000 tokens behind 6001.
 constexpr float kSlack = 4.0f, kLift = 11.0f;
+// A score and the maximum part in one FMA, so the rounding of the maximum is in the difference; beyond scores of 2^24 that would
+// overflow P.  Queries below kLargeQ and K scales below kLargeK (values below 8 kLargeK) keep scores below 2^21.3; larger ones are rounded
+// before the difference is taken, in the pass that wide tiles take.
+constexpr float kLargeQ = 512.0f, kLargeK = 32.0f;
 
 struct Params {
   lq_int4_prefill_args a;
@@ -168,8 +172,8 @@ struct Shared {
   uint64_t k_first, full[2], empty[2], s_done[2], p_ready[2], q_ready[2];
   // Per 16 tokens: 2^Ek, Ev and 2^-Ev of the tile, four tiles deep (they are written a unit ahead of V)
   float k_factor[5][4], v_exp[5][4], v_inv[5][4];  // slot 4: 1, 0, 0
-  // A byte per 16 tokens: they are wide.  Then the same per token (k_factor NaN: the scale is not finite), and the 32-dim chunks of V
-  // whose scale is not finite, a bit each
+  // A byte per 16 tokens, bit 0: they are wide, bit 1: large K scales.  Then for wide ones the same per token (k_factor NaN: the
+  // scale is not finite), and the 32-dim chunks of V whose scale is not finite, a bit each
   uint32_t wide[4];
   float k_factor_tok[4][kTok], v_exp_tok[4][kTok], v_inv_tok[4][kTok];
   uint8_t v_bad_tok[4][kTok];
@@ -212,11 +216,11 @@ __device__ __forceinline__ int exponent_of(uint32_t bits) {
   return field == 0 ? 0 : max(field - 127 - 11, -110);
 }
 // The scales of a warp's 16 tokens, two tokens of one chunk per lane (the chunks eight lanes apart): one exponent, that of the largest, or
-// where they are wide one per token.  bad: a ballot of the scales that are not finite, per token of the lane; these become 0.
+// where they are wide one per token.  large: of K (kLargeK).  bad: a ballot of the scales that are not finite, per token of the lane; these become 0.
 struct Exponents {
   int e[2];
   uint32_t bad[2];
-  bool wide;
+  bool wide, large;
 };
 __device__ __forceinline__ Exponents exponents_of(float (&sc)[2]) {
   Exponents r;
@@ -224,6 +228,7 @@ __device__ __forceinline__ Exponents exponents_of(float (&sc)[2]) {
   const uint32_t hi = __reduce_max_sync(0xFFFFFFFFu, max(b[0], b[1]));
   r.e[0] = r.e[1] = exponent_of(hi);
   r.bad[0] = r.bad[1] = 0u;
+  r.large = hi >= __float_as_uint(kLargeK);
   const uint32_t least = min(b[0] - 1, b[1] - 1);  // 0 (a row without a token) does not count
   r.wide = __any_sync(0xFFFFFFFFu, hi >= 0x7F800000u || (hi >> 23) > (least >> 23) + kSpread);
   if (r.wide) {
@@ -316,7 +321,7 @@ __device__ __forceinline__ void unpack_tiles(const Params& p, Shared& sh, uint8_
       sh.k_factor[f][warp] = pow2_of(ek.e[0]);
       sh.v_exp[f][warp] = static_cast<float>(ev.e[0]);
       sh.v_inv[f][warp] = pow2_of(-ev.e[0]);
-      reinterpret_cast<uint8_t*>(&sh.wide[f])[warp] = wide;
+      reinterpret_cast<uint8_t*>(&sh.wide[f])[warp] = (wide ? 1 : 0) | (ek.large ? 2 : 0);
     }
     if (wide && chunk == 0) {
       constexpr uint32_t kChunks = 0x01010101u;  // a token's bits of a ballot
@@ -479,8 +484,8 @@ __device__ __forceinline__ float2 unpack16x2(uint32_t w, bool bf16) {
 __device__ __forceinline__ float max3(float a, float b, float c) { return fmaxf(fmaxf(a, b), c); }
 
 // Query row -> fp16 in TMEM, its largest value brought to [2^14, 2^15); returns the factor of a product of this row,
-// 2^Eq log2(e) / sqrt(128)
-__device__ __forceinline__ float load_query(const lq_int4_prefill_args& a, int64_t base, bool live, uint32_t tm_q) {
+// 2^Eq log2(e) / sqrt(128).  large: of any row of the warp, as bits of Shared::wide
+__device__ __forceinline__ float load_query(const lq_int4_prefill_args& a, int64_t base, bool live, uint32_t tm_q, uint32_t& large) {
   uint32_t raw[64];
   const bool bf16 = a.dtype == LQ_BF16;
   if (live) {
@@ -495,6 +500,7 @@ __device__ __forceinline__ float load_query(const lq_int4_prefill_args& a, int64
     const float2 v = unpack16x2(raw[i], bf16);
     amax = max3(amax, fabsf(v.x), fabsf(v.y));
   }
+  large = __any_sync(0xFFFFFFFFu, amax >= kLargeQ) ? 0x02020202u : 0u;
   int field = static_cast<int>(__float_as_uint(amax) >> 23);
   field = field == 0 ? 141 : min(max(field, 15), 254);  // a row of zeros keeps the factor 1
   const float to_half = __uint_as_float(static_cast<uint32_t>(268 - field) << 23);
@@ -557,8 +563,8 @@ __device__ __forceinline__ void store_output(const lq_int4_prefill_args& a, int6
 // One row of scores of one block, a tile at a time: S -> P in place, running maximum and sum.  tile: the block's first, counted over
 // all blocks; parity: of the next wait for products of this group; l_run: the sum; bad: the 32-dim chunks for which the row has
 // attended to a V that is not finite.  False after a wait that ran out.
-__device__ __forceinline__ bool softmax_rows(const Params& p, Shared& sh, int pos0, int ntiles, int tile, uint32_t& parity, float cq, float& l_run,
-                                             uint32_t& bad) {
+__device__ __forceinline__ bool softmax_rows(const Params& p, Shared& sh, int pos0, int ntiles, int tile, uint32_t& parity, float cq, uint32_t large_q,
+                                             float& l_run, uint32_t& bad) {
   const lq_int4_prefill_args& a = p.a;
   const int group = threadIdx.x >> 7, warp = (threadIdx.x >> 5) & 3, lane = threadIdx.x & 31;
   const int row = warp * 32 + lane;  // = TMEM lane
@@ -575,7 +581,7 @@ __device__ __forceinline__ bool softmax_rows(const Params& p, Shared& sh, int po
     if (!wait_bar(&sh.s_done[group], parity)) return false;
     parity ^= 1;
     fence_after();
-    const uint32_t wide = sh.wide[f];
+    const uint32_t wide = sh.wide[f] | large_q;
     uint32_t s[64];
     tmem_load64(s, tm + kColS);
     // Rare cases share the branches that are there anyway: with branches of their own 1 x 128 behind 4000 took 115 us instead of 109.
@@ -681,14 +687,16 @@ __device__ __forceinline__ void softmax_blocks(const Params& p, Shared& sh) {
   const int row = threadIdx.x & 127, in_block = static_cast<int>(threadIdx.x) >> p.ratio_log2;
   const uint32_t tm = group * kColsPerGroup + (static_cast<uint32_t>(warp * 32) << 16);
   const auto head_of = [&](const Block& k) { return (k.kvh << p.ratio_log2) + (row & ((1 << p.ratio_log2) - 1)); };
+  float cq = 0.0f, l_run;
+  uint32_t large_q = 0u, bad;
   // the group's query rows of its first block from round r on, none of whose S has been asked for yet
-  const auto load_next = [&](int r, float& cq) {
+  const auto load_next = [&](int r) {
     for (; entry_of(r) < p.entries; ++r) {
       const Block k = block_at(p, entry_of(r));
       if (group >= k.groups) continue;
       const int pos = k.pos0 + in_block;
       const int64_t base = k.b * a.q_stride[0] + head_of(k) * a.q_stride[1] + static_cast<int64_t>(pos) * a.q_stride[2];
-      cq = load_query(a, base, pos < a.q_len, tm + kColQ);
+      cq = load_query(a, base, pos < a.q_len, tm + kColQ, large_q);
       fence_before();
       __syncwarp();
       return true;
@@ -697,15 +705,13 @@ __device__ __forceinline__ void softmax_blocks(const Params& p, Shared& sh) {
   };
   uint32_t parity = 0;
   int tile = 0;
-  float cq = 0.0f, l_run;
-  uint32_t bad;
-  if (load_next(0, cq) && lane == 0) mbar_arrive(&sh.q_ready[group]);
+  if (load_next(0) && lane == 0) mbar_arrive(&sh.q_ready[group]);
 #pragma unroll 1
   for (int r = 0; entry_of(r) < p.entries; ++r) {
     const Block k = block_at(p, entry_of(r));
     if (group < k.groups) {
-      if (!softmax_rows(p, sh, k.pos0, k.ntiles, tile, parity, cq, l_run, bad)) return;
-      const bool more = load_next(r + 1, cq);  // all S of this block are done; its last products run meanwhile
+      if (!softmax_rows(p, sh, k.pos0, k.ntiles, tile, parity, cq, large_q, l_run, bad)) return;
+      const bool more = load_next(r + 1);  // all S of this block are done; its last products run meanwhile
       // the wait stands before the arrival that lets the next S be asked for: s_done is never two phases ahead of a warp
       if (!wait_bar(&sh.s_done[group], parity)) return;
       parity ^= 1;

@@ -555,3 +555,16 @@ def test_prefill_rows_do_not_depend_on_later_tokens(size, which, gs):
             assert not torch.isfinite(got[torch.from_numpy(~finite)]).any()
             if finite.any():
                 assert_out_close(got[torch.from_numpy(finite)], want[finite])
+
+
+@pytest.mark.parametrize("size", [3e5, 1e7, 1e9, 1e30])
+def test_prefill_huge_scores(size):
+    """Keys so large that a score's last bit is worth more than the softmax has range: each row is one token's V, as in fp64."""
+    m = ia()
+    tq, gs = 70, 32
+    k, v = make_kv(71, 1, 2, tq)
+    k = bf16r(k * size)
+    q = bf16r(np.random.default_rng(72).standard_normal((1, 8, tq, 128)))
+    cache = fill_cache(m, k, v, gs, dtype=torch.float32)
+    ref = oracle.int4_prefill_attention(q, *cache_np(cache), 1, gs)
+    assert_out_close(m._prefill_attention(t(q, torch.bfloat16), cache, 4, gs), ref)
