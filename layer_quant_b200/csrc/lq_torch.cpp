@@ -9,11 +9,14 @@
 // or type, a status other than LQ_OK from the library).  The Python caller then takes its general path, which
 // makes the same launch through ctypes or raises the error that belongs to it, so error behaviour has one home.
 #include <ATen/ATen.h>
+#include <c10/cuda/CUDAException.h>
 #include <c10/cuda/CUDAStream.h>
+#include <cuda_runtime_api.h>
 #include <dlfcn.h>
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
+#include <algorithm>
 #include <map>
 #include <utility>
 
@@ -317,20 +320,43 @@ bool cache_struct(Call& c, PyObject* cache, int64_t group, lq_int4_cache& s) {
          tvs->scalar_type() == at::kFloat && group > 0 && tks->size(3) * group == s.head_dim;
 }
 
-// Scratch of the split merge: one zeroed buffer per (device, stream), grown on demand, at most kMaxWorkspaces of them.
-// The kernels leave the ticket counters at zero.  A buffer is allocated on the stream that uses it, so one that
-// is dropped here (or replaced by a larger one) is handed out again by the allocator in stream order only.
+// Scratch of the split merge, per (device, stream), zeroed once: the kernels leave the ticket counters at zero.
+//
+// Calls that run now share one buffer, grown on demand.  It is allocated on the stream that uses it, so one that is replaced by a larger
+// one or dropped (the longest unused of more than kMaxWorkspaces) is handed out again by the allocator in stream order only.
+// A call that is being recorded must not use it: a graph holds the bare address, and a replay knows nothing of that order.  Each capture
+// gets a buffer of its own from the graph's memory pool, where the address stays the graph's, and whose zeroing is recorded ahead of
+// its first use.
+struct Workspace {
+  at::Tensor now, recorded;
+  unsigned long long capture = 0;  // the capture that `recorded` belongs to, 0: none
+  uint64_t last_use = 0;
+};
 constexpr size_t kMaxWorkspaces = 64;
-std::map<std::pair<int, void*>, at::Tensor> workspaces;
+std::map<std::pair<int, void*>, Workspace>& workspaces() {
+  static auto& all = *new std::map<std::pair<int, void*>, Workspace>;  // never destroyed: the allocator may be gone at exit
+  return all;
+}
 
-const at::Tensor& workspace(int device, void* stream, size_t nbytes) {
+at::Tensor workspace(int device, void* stream, size_t nbytes) {
+  static uint64_t uses = 0;
+  auto& all = workspaces();
   const auto key = std::make_pair(device, stream);
-  auto it = workspaces.find(key);
-  if (it != workspaces.end() && static_cast<size_t>(it->second.numel()) >= nbytes) return it->second;
-  if (it == workspaces.end() && workspaces.size() >= kMaxWorkspaces) workspaces.erase(workspaces.begin());
-  at::Tensor ws = at::zeros({static_cast<int64_t>(std::max<size_t>(nbytes, 1 << 20))},
-                            at::TensorOptions().dtype(at::kByte).device(at::kCUDA, static_cast<c10::DeviceIndex>(device)));
-  return workspaces[key] = std::move(ws);
+  if (all.size() >= kMaxWorkspaces && all.find(key) == all.end())
+    all.erase(std::min_element(all.begin(), all.end(), [](const auto& a, const auto& b) { return a.second.last_use < b.second.last_use; }));
+  Workspace& w = all[key];
+  w.last_use = ++uses;
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  unsigned long long id = 0;
+  C10_CUDA_CHECK(cudaStreamGetCaptureInfo(static_cast<cudaStream_t>(stream), &status, &id));
+  if (status == cudaStreamCaptureStatusNone) id = 0;
+  if (w.capture != id) w.recorded.reset();
+  w.capture = id;
+  at::Tensor& ws = id != 0 ? w.recorded : w.now;
+  if (!ws.defined() || static_cast<size_t>(ws.numel()) < nbytes)
+    ws = at::zeros({static_cast<int64_t>(std::max<size_t>(nbytes, 1 << 20))},
+                   at::TensorOptions().dtype(at::kByte).device(at::kCUDA, static_cast<c10::DeviceIndex>(device)));
+  return ws;
 }
 
 // workspace_for(device, nbytes): the same buffer for prepared launches
@@ -417,7 +443,7 @@ PyObject* decode_attn(PyObject*, PyObject* const* a, Py_ssize_t n) {
   d.splits = static_cast<int32_t>(std::min<int64_t>(splits, INT32_MAX));
   void* stream = c.stream();
   if (splits > 1) {
-    const at::Tensor& ws = workspace(c.device, stream, L.int4_decode_workspace_bytes(batch, heads, d.cache.kv_heads, dim, d.splits));
+    const at::Tensor ws = workspace(c.device, stream, L.int4_decode_workspace_bytes(batch, heads, d.cache.kv_heads, dim, d.splits));
     d.workspace = ws.data_ptr();
     d.workspace_bytes = ws.numel();
   }

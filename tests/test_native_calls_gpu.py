@@ -88,3 +88,49 @@ def test_errors_come_from_the_general_path():
         ia._decode_attention(q, kv, 4, 4, 32, attention_mask=torch.zeros(1, 1, 4, device=d))
     with pytest.raises(ValueError, match="do not match state"):
         dense_state.selective_state_update(torch.zeros(1, 2, 16, 128, device=d), x[:, :, :8], x, A, B, B)
+
+
+def test_recorded_decode_owns_its_scratch():
+    """A recorded decode call whose splits need scratch replays correctly whatever eager calls do to the scratch of its stream: grow it, or
+    push it out with calls on more streams than are kept; the memory they gave back is filled with ones (tickets that start there never
+    come to their end, and the output is not written)."""
+    from layer_quant_b200 import int4_8b_attention as m
+    g = torch.Generator(device=dev()).manual_seed(9)
+    tlen, gs, splits = 250, 32, 4
+    small, large = (_cache(m, b, 2, tlen, gs, g) for b in (2, 64))
+    q = torch.randn(2, 8, 1, 128, generator=g, device=dev()).to(torch.bfloat16)
+    q_large = torch.randn(64, 8, 1, 128, generator=g, device=dev()).to(torch.bfloat16)
+    want = m._decode_attention(q, small, tlen, 4, gs, splits=splits)
+    want_large = m._decode_attention(q_large, large, tlen, 4, gs, splits=splits)
+    stream = torch.cuda.Stream()
+    stream.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(stream):
+        m._decode_attention(q, small, tlen, 4, gs, splits=splits)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        first = m._decode_attention(q, small, tlen, 4, gs, splits=splits)
+        second = m._decode_attention(q_large, large, tlen, 4, gs, splits=splits)  # larger: the capture's scratch grows, too
+        third = m._decode_attention(q, small, tlen, 4, gs, splits=splits)
+
+    def check():
+        for out in (first, second, third):
+            out.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(first, want) and torch.equal(third, want) and torch.equal(second, want_large)
+
+    check()
+    with torch.cuda.stream(stream):
+        assert torch.equal(m._decode_attention(q_large, large, tlen, 4, gs, splits=splits), want_large)
+        held = [torch.full((1 << 20,), 1, dtype=torch.uint8, device=dev()) for _ in range(64)]
+    check()
+    streams = {s.cuda_stream: s for p in (0, -1, -2, -3) for s in (torch.cuda.Stream(priority=p) for _ in range(32))}
+    assert len(streams) > 64
+    for s in streams.values():
+        s.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(s):
+            assert torch.equal(m._decode_attention(q, small, tlen, 4, gs, splits=splits), want)
+    with torch.cuda.stream(stream):
+        held += [torch.full((1 << 20,), 1, dtype=torch.uint8, device=dev()) for _ in range(64)]
+    check()
+    assert held
