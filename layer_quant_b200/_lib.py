@@ -220,6 +220,17 @@ def stream_ptr(device: torch.device) -> int:
     return torch.cuda.current_stream(device).cuda_stream
 
 
+def launch(device: torch.device, fn, *args) -> None:
+    """``fn(*args, stream)`` on torch's current stream of ``device``; a status other than LQ_OK raises.  A kernel goes to the
+    device that is current, so the operands' device is made that for the length of the call."""
+    if torch.cuda.current_device() == device.index:
+        rc = fn(*args, stream_ptr(device))
+    else:
+        with torch.cuda.device(device):
+            rc = fn(*args, stream_ptr(device))
+    check(rc)
+
+
 def set_ptr_strides(struct, name: str, t: torch.Tensor | None, nstride: int, with_dtype: bool = True) -> None:
     """Fill ``name``, ``name_stride`` (last ``nstride`` dims) and ``name_dtype`` of a ctypes struct."""
     if t is None:

@@ -67,7 +67,7 @@ def selective_state_update(state, x, dt, A, B, C, D=None, z=None, dt_bias=None, 
                        ("D", D, 2), ("z", z, 3), ("out", out, 3)):
         _lib.set_ptr_strides(a, name, t, n)
     a.ngroups, a.dt_softplus = B.shape[1], int(bool(dt_softplus))
-    _lib.check(_lib.lib().lq_dense_state_update(ct.byref(a), _lib.stream_ptr(dev)))
+    _lib.launch(dev, _lib.lib().lq_dense_state_update, ct.byref(a))
     return out.squeeze(1) if squeeze else out
 
 
@@ -106,5 +106,5 @@ def causal_conv1d_update(x, conv_state, weight, bias=None, activation=None, *, o
     for name, t, n in (("x", x, 2), ("weight", weight, 2), ("bias", bias, 1), ("out", out, 2)):
         _lib.set_ptr_strides(a, name, t, n)
     a.batch, a.channels, a.width, a.silu = batch, channels, width, int(activation is not None)
-    _lib.check(_lib.lib().lq_causal_conv1d_update(ct.byref(a), _lib.stream_ptr(dev)))
+    _lib.launch(dev, _lib.lib().lq_causal_conv1d_update, ct.byref(a))
     return out.unsqueeze(2) if unsqueeze else out

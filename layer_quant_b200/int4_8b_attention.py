@@ -166,8 +166,8 @@ def _pack_kv_into_cache(cache: Int4KVLayerCache, key_states: torch.Tensor, value
         raise ValueError(f"positions has {positions.numel()} entries for q_len={q_len}")
     ks = (ct.c_int64 * 4)(*key_states.stride())
     vs = (ct.c_int64 * 4)(*value_states.stride())
-    _lib.check(_lib.lib().lq_int4_kv_append(ct.byref(c), key_states.data_ptr(), ks, value_states.data_ptr(), vs,
-                                           _lib.dtype_code(key_states), positions.data_ptr(), q_len, _lib.stream_ptr(dev)))
+    _lib.launch(dev, _lib.lib().lq_int4_kv_append, ct.byref(c), key_states.data_ptr(), ks, value_states.data_ptr(), vs,
+                _lib.dtype_code(key_states), positions.data_ptr(), q_len)
     cache.length = max(cache.length, known_len if known_len is not None else int(positions.max().item()) + 1)
 
 
@@ -242,7 +242,7 @@ def _decode_args(query_states, cache, seq_len, group_size, mask, k_new=None, v_n
 
 def _launch_decode(query_states, cache, seq_len, group_size, mask, k_new=None, v_new=None, splits=0, out=None):
     a, out, _keep = _decode_args(query_states, cache, seq_len, group_size, mask, k_new, v_new, splits, out)
-    _lib.check(_lib.lib().lq_int4_decode_attn(ct.byref(a), _lib.stream_ptr(out.device)))
+    _lib.launch(out.device, _lib.lib().lq_int4_decode_attn, ct.byref(a))
     return out
 
 
@@ -278,7 +278,7 @@ class Int4DecodePlan:
 
 def advance_seq_len(seq_len_counter: torch.Tensor, inc: int = 1) -> None:
     """``*seq_len_counter += inc`` on the current stream (a one-thread kernel; records into CUDA graphs)."""
-    _lib.check(_lib.lib().lq_counter_add(seq_len_counter.data_ptr(), int(inc), _lib.stream_ptr(seq_len_counter.device)))
+    _lib.launch(seq_len_counter.device, _lib.lib().lq_counter_add, seq_len_counter.data_ptr(), int(inc))
 
 
 def _decode_attention(query_states: torch.Tensor, cache: Int4KVLayerCache, seq_len: int, num_key_value_groups: int,
@@ -346,7 +346,7 @@ def _prefill_attention(query_states: torch.Tensor, cache: Int4KVLayerCache, num_
         a.q_stride[i], a.out_stride[i] = query_states.stride(i), out.stride(i)
     a.dtype = _lib.dtype_code(query_states)
     a.q_heads, a.q_len, a.first_len = n_heads, q_len, first_len
-    _lib.check(_lib.lib().lq_int4_prefill_attn(ct.byref(a), _lib.stream_ptr(dev)))
+    _lib.launch(dev, _lib.lib().lq_int4_prefill_attn, ct.byref(a))
     return out
 
 
@@ -388,7 +388,7 @@ def _graph_decode_step(query_states, key_states, value_states, cache, group_size
         return out
     a, out, keep = _decode_args(query_states, cache, capacity, group_size, None, key_states, value_states,
                                 seq_len_counter=cache.length_counter)
-    _lib.check(_lib.lib().lq_int4_decode_attn(ct.byref(a), _lib.stream_ptr(out.device)))
+    _lib.launch(out.device, _lib.lib().lq_int4_decode_attn, ct.byref(a))
     return out
 
 

@@ -94,7 +94,7 @@ class MambaStateKernelCache:
         out = _empty_cache(self.state_shape, self.format_bits, layout, self.q_state.device)
         out.step, out.layer = self.step, self.layer
         src, dst = _state_struct(self), _state_struct(out)
-        _lib.check(_lib.lib().lq_mx_convert_layout(ct.byref(src), ct.byref(dst), _lib.stream_ptr(self.q_state.device)))
+        _lib.launch(self.q_state.device, _lib.lib().lq_mx_convert_layout, ct.byref(src), ct.byref(dst))
         return out
 
     def dequantize(self) -> torch.Tensor:
@@ -102,7 +102,7 @@ class MambaStateKernelCache:
         b, h, p, n = self.state_shape
         out = torch.empty((b, h, p, n), dtype=torch.float32, device=self.q_state.device)
         st = _state_struct(self)
-        _lib.check(_lib.lib().lq_mx_dequantize(ct.byref(st), out.data_ptr(), n, _lib.stream_ptr(out.device)))
+        _lib.launch(out.device, _lib.lib().lq_mx_dequantize, ct.byref(st), out.data_ptr(), n)
         return out
 
 
@@ -151,8 +151,7 @@ def _quantize_into(cache: MambaStateKernelCache, src: torch.Tensor, rounding: _l
     if src2.stride(-1) != 1:
         src2 = src2.contiguous()
     st = _state_struct(cache)
-    _lib.check(_lib.lib().lq_mx_quantize(ct.byref(st), src2.data_ptr(), _lib.dtype_code(src2), src2.stride(0),
-                                         ct.byref(rounding), _lib.stream_ptr(src.device)))
+    _lib.launch(src.device, _lib.lib().lq_mx_quantize, ct.byref(st), src2.data_ptr(), _lib.dtype_code(src2), src2.stride(0), ct.byref(rounding))
 
 
 def _quantize_initial_state_mx(
@@ -314,7 +313,7 @@ def advance_step_counter(step_counter: torch.Tensor, inc: int = 1) -> None:
     """``step_counter += inc`` on the current stream with the library's own one-thread kernel
     (capturable in a CUDA graph together with the update launches that read the counter)."""
     dev = _lib.require_cuda(step_counter)
-    _lib.check(_lib.lib().lq_counter_add(step_counter.data_ptr(), int(inc), _lib.stream_ptr(dev)))
+    _lib.launch(dev, _lib.lib().lq_counter_add, step_counter.data_ptr(), int(inc))
 
 
 def mx_state_selective_update(

@@ -285,3 +285,37 @@ def test_prepare_graph_decode_counters_on_the_host():
     assert len({c.step_counter.data_ptr() for c in cs}) == 3 and all(c.advances_counter for c in cs)
     assert mk.graph_decode_steps(model) == {7: 3, 2: 3, 11: 3}
     mk.prepare_graph_decode(SimpleNamespace())  # a model without registered caches: nothing to do
+
+
+@pytest.mark.parametrize("current", [0, 1])
+@pytest.mark.parametrize("status", [0, -1])
+def test_launch_makes_the_operands_device_current(monkeypatch, current, status):
+    """A kernel goes to the current device: a call on tensors of device 1 runs with device 1 current and leaves the old one behind, an
+    error status included."""
+    from layer_quant_b200 import _lib
+    state = {"device": current, "seen": []}
+
+    class Device:
+        def __init__(self, device):
+            self.index = device.index
+
+        def __enter__(self):
+            self.before, state["device"] = state["device"], self.index
+
+        def __exit__(self, *exc):
+            state["device"] = self.before
+
+    def entry_point(a, stream):
+        state["seen"].append((a, stream, state["device"]))
+        return status
+
+    monkeypatch.setattr(torch.cuda, "current_device", lambda: state["device"])
+    monkeypatch.setattr(torch.cuda, "device", Device)
+    monkeypatch.setattr(_lib, "stream_ptr", lambda device: 100 + device.index)
+    if status:
+        monkeypatch.setattr(_lib, "check", lambda rc: (_ for _ in ()).throw(ValueError(rc)))
+        with pytest.raises(ValueError):
+            _lib.launch(torch.device("cuda", 1), entry_point, "a")
+    else:
+        _lib.launch(torch.device("cuda", 1), entry_point, "a")
+    assert state["seen"] == [("a", 101, 1)] and state["device"] == current
