@@ -406,7 +406,7 @@ bool decode_mask(Call& c, PyObject* o, int64_t batch, int64_t seq_len, lq_int4_d
   return true;
 }
 
-// decode_attn(q [B,Hq,1,D], cache, seq_len, query heads per kv head (0: not checked), group_size, mask, k_new, v_new, splits, counter)
+// decode_attn(q [B,Hq,1,D], cache, seq_len, query heads per kv head (-1: not checked), group_size, mask, k_new, v_new, splits, counter)
 PyObject* decode_attn(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   int64_t seq_len, ratio, group, splits;
@@ -420,7 +420,7 @@ PyObject* decode_attn(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const int64_t batch = q->size(0), heads = q->size(1), dim = q->size(3);
   d.dtype = c.dtype(*q);
   if (!c.ok || q->size(2) != 1 || batch != d.cache.batch || dim != d.cache.head_dim || seq_len < 1 || seq_len > d.cache.capacity ||
-      (ratio > 0 && heads != ratio * d.cache.kv_heads))
+      (ratio != -1 && heads != ratio * d.cache.kv_heads))
     return none();
   d.q = q->data_ptr();
   d.q_stride[0] = q->stride(0);

@@ -285,7 +285,7 @@ def _decode_attention(query_states: torch.Tensor, cache: Int4KVLayerCache, seq_l
                       group_size: int, attention_mask: torch.Tensor | None = None, *, splits: int = 0) -> torch.Tensor:
     """softmax(q K^T / sqrt(D) [+ mask]) V over cache rows [0, seq_len) for one query token.
     query_states [B, Hq, 1, D] -> [B, Hq, D] in the query's dtype."""
-    out = _lib.native().decode_attn(query_states, cache, seq_len, num_key_value_groups, group_size, attention_mask, None, None,
+    out = _lib.native().decode_attn(query_states, cache, seq_len, max(num_key_value_groups, 0), group_size, attention_mask, None, None,
                                     splits, None)
     if out is not None:
         return out
@@ -303,7 +303,7 @@ def _append_decode_attention(query_states, key_states, value_states, cache, seq_
     """Decode step in one launch: quantise the new K/V row [B, Hkv, 1, D] into cache row
     ``seq_len - 1`` and attend over rows [0, seq_len).  Equals ``_pack_kv_into_cache`` followed by
     ``_decode_attention``."""
-    out = _lib.native().decode_attn(query_states, cache, seq_len, 0, group_size, attention_mask, key_states, value_states, splits, None)
+    out = _lib.native().decode_attn(query_states, cache, seq_len, -1, group_size, attention_mask, key_states, value_states, splits, None)
     if out is not None:
         cache.length = max(cache.length, seq_len)
         return out
@@ -383,7 +383,7 @@ def _graph_decode_step(query_states, key_states, value_states, cache, group_size
         raise NotImplementedError("recorded decode steps take no attention_mask: a mask's length changes every step")
     advance_seq_len(cache.length_counter)  # the new token's position + 1
     capacity = cache.k_packed.shape[2]
-    out = _lib.native().decode_attn(query_states, cache, capacity, 0, group_size, None, key_states, value_states, 0, cache.length_counter)
+    out = _lib.native().decode_attn(query_states, cache, capacity, -1, group_size, None, key_states, value_states, 0, cache.length_counter)
     if out is not None:
         return out
     a, out, keep = _decode_args(query_states, cache, capacity, group_size, None, key_states, value_states,

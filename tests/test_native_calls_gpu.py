@@ -82,8 +82,9 @@ def test_errors_come_from_the_general_path():
     q = torch.zeros(1, 8, 1, 128, device=d, dtype=torch.bfloat16)
     with pytest.raises(ValueError, match="outside"):
         ia._decode_attention(q, kv, 17, 4, 32)
-    with pytest.raises(ValueError, match="query heads"):
-        ia._decode_attention(q, kv, 4, 2, 32)
+    for groups in (2, 0, -1):
+        with pytest.raises(ValueError, match="query heads"):
+            ia._decode_attention(q, kv, 4, groups, 32)
     with pytest.raises(ValueError, match="only supports 2D or 4D"):
         ia._decode_attention(q, kv, 4, 4, 32, attention_mask=torch.zeros(1, 1, 4, device=d))
     with pytest.raises(ValueError, match="do not match state"):
