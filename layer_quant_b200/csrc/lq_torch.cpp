@@ -66,6 +66,14 @@ bool as_long(PyObject* o, int64_t& v) {
   return overflow == 0;
 }
 
+// The truth value of an option; without one (a tensor of several elements) the call is not the ordinary case
+bool as_bool(PyObject* o, bool& v) {
+  const int r = o == nullptr ? -1 : PyObject_IsTrue(o);
+  if (r < 0) PyErr_Clear();
+  v = r == 1;
+  return r >= 0;
+}
+
 // Collects operands: every tensor has to be on one CUDA device and of a type the kernels read.
 struct Call {
   int device = -1;
@@ -155,9 +163,9 @@ PyObject* mx_update(PyObject*, PyObject* const* a, Py_ssize_t n) {
   Attr q(cache, N.q_state), e(cache, N.shared_exp), m(cache, N.micro_exp), bits_o(cache, N.format_bits), step_o(cache, N.step),
       layout_o(cache, N.layout), layer_o(cache, N.layer), counter_o(cache, N.step_counter);
   int64_t bits, step, layer;
-  bool packed;
+  bool packed, softplus, stochastic;
   if (!as_long(bits_o.o, bits) || !as_long(step_o.o, step) || !as_long(layer_o.o, layer) || !layout_of(layout_o.o, packed) ||
-      counter_o.o == nullptr || !PyLong_Check(a[11]) || !PyUnicode_Check(a[12]))
+      counter_o.o == nullptr || !as_bool(a[9], softplus) || !as_bool(a[10], stochastic) || !PyLong_Check(a[11]) || !PyUnicode_Check(a[12]))
     return none();
   Call c;
   lq_mx_update_args u = {};
@@ -175,13 +183,13 @@ PyObject* mx_update(PyObject*, PyObject* const* a, Py_ssize_t n) {
   u.dt_bias_stride[0] = u.D ? u.D_stride[0] : 0;
   u.dt_bias_stride[1] = u.D ? u.D_stride[1] : 0;
   u.ngroups = B->size(1);
-  u.dt_softplus = PyObject_IsTrue(a[9]) == 1;
+  u.dt_softplus = softplus;
   lq_rounding& r = u.rounding;
   r.seed = PyLong_AsUnsignedLongLongMask(a[11]);
   r.layer = static_cast<uint32_t>(layer);
   r.step = static_cast<uint64_t>(step);
   r.rng_offset = static_cast<uint64_t>(step) * static_cast<uint64_t>(u.state.batch) * u.state.heads * u.state.dim * u.state.dstate;
-  if (PyObject_IsTrue(a[10]) != 1) {
+  if (!stochastic) {
     r.mode = LQ_ROUND_HALF_UP;
   } else if (PyUnicode_CompareWithASCIIString(a[12], "layered") == 0) {
     r.mode = LQ_ROUND_PHILOX_LAYERED;
@@ -196,6 +204,11 @@ PyObject* mx_update(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const at::Tensor* k = c.tensor(counter_o.o, 1);
     if (k == nullptr || k->scalar_type() != at::kLong || k->numel() != 1) return none();
     r.step_counter = static_cast<const uint64_t*>(k->data_ptr());
+  }
+  bool advances = false;
+  if (counter_o.o != Py_None) {
+    const Attr advances_o(cache, N.advances_counter);
+    if (!as_bool(advances_o.o, advances)) return none();
   }
   at::Tensor out;
   if (!output(c, a[13], *x, out)) return none();
@@ -214,8 +227,7 @@ PyObject* mx_update(PyObject*, PyObject* const* a, Py_ssize_t n) {
     }
     Py_DECREF(next);
   } else {
-    Attr advances(cache, N.advances_counter);
-    if (advances.o != nullptr && PyObject_IsTrue(advances.o) == 1 && L.counter_add(const_cast<uint64_t*>(r.step_counter), 1, stream) != LQ_OK) {
+    if (advances && L.counter_add(const_cast<uint64_t*>(r.step_counter), 1, stream) != LQ_OK) {
       PyErr_SetString(PyExc_RuntimeError, "the step counter could not be advanced");
       return nullptr;
     }
@@ -261,7 +273,8 @@ PyObject* mx_quantize(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   int64_t bits;
   if (n != 3 || L.mx_quantize == nullptr || !as_long(a[1], bits) || (bits != 8 && bits != 4)) return none();
-  const bool packed = PyObject_IsTrue(a[2]) == 1;
+  bool packed;
+  if (!as_bool(a[2], packed)) return none();
   Call c;
   const at::Tensor* src = c.tensor(a[0], 4);
   if (src == nullptr) return none();
@@ -522,7 +535,8 @@ PyObject* prefill_attn(PyObject*, PyObject* const* a, Py_ssize_t n) {
 // dense_update(state [B,H,P,N], x, dt, A, B, C, D, z, dt_bias, dt_softplus, out)
 PyObject* dense_update(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
-  if (n != 11 || L.dense_state_update == nullptr) return none();
+  bool softplus;
+  if (n != 11 || L.dense_state_update == nullptr || !as_bool(a[9], softplus)) return none();
   Call c;
   lq_dense_update_args u = {};
   const at::Tensor* state = c.operand(a[0], u.state, u.state_stride, u.state_dtype);
@@ -551,7 +565,7 @@ PyObject* dense_update(PyObject*, PyObject* const* a, Py_ssize_t n) {
   u.dim = p;
   u.dstate = w;
   u.ngroups = g;
-  u.dt_softplus = PyObject_IsTrue(a[9]) == 1;
+  u.dt_softplus = softplus;
   if (!c.ok) return none();
   const auto guard = c.current();
   if (L.dense_state_update(&u, c.stream()) != LQ_OK) return none();
@@ -562,7 +576,8 @@ PyObject* dense_update(PyObject*, PyObject* const* a, Py_ssize_t n) {
 // conv1d_update(x [B,C], conv_state [B,C,W], weight [C,W], bias, silu, out)
 PyObject* conv1d_update(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
-  if (n != 6 || L.causal_conv1d_update == nullptr) return none();
+  bool silu;
+  if (n != 6 || L.causal_conv1d_update == nullptr || !as_bool(a[4], silu)) return none();
   Call c;
   lq_conv1d_update_args u = {};
   const at::Tensor* x = c.operand(a[0], u.x, u.x_stride, u.x_dtype);
@@ -581,7 +596,7 @@ PyObject* conv1d_update(PyObject*, PyObject* const* a, Py_ssize_t n) {
   u.batch = b;
   u.channels = ch;
   u.width = w;
-  u.silu = PyObject_IsTrue(a[4]) == 1;
+  u.silu = silu;
   if (!c.ok) return none();
   const auto guard = c.current();
   if (L.causal_conv1d_update(&u, c.stream()) != LQ_OK) return none();

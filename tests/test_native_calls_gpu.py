@@ -77,6 +77,11 @@ def test_errors_come_from_the_general_path():
     x = torch.zeros(1, 2, 16, device=d)
     with pytest.raises(ValueError, match="unknown rng_stream"):
         mk.mx_state_selective_update(cache, x, x, A, B, B, rng_stream="other")
+    for option in ("dt_softplus", "stochastic"):  # an option without a truth value
+        with pytest.raises(RuntimeError, match="ambiguous"):
+            mk.mx_state_selective_update(cache, x, x, A, B, B, **{option: torch.ones(2)})
+    with pytest.raises(RuntimeError, match="ambiguous"):
+        dense_state.selective_state_update(torch.zeros(1, 2, 16, 128, device=d), x, x, A, B, B, dt_softplus=torch.ones(2))
     assert cache.step == 0
     kv = ia._allocate_layer_cache(1, 2, 16, 128, 4, torch.device(d))
     q = torch.zeros(1, 8, 1, 128, device=d, dtype=torch.bfloat16)
