@@ -231,6 +231,8 @@ class MxUpdatePlan:
         if z is not None and z.ndim != 3:
             raise ValueError("Expected z [batch, heads, dim].")
         self.device = _lib.require_cuda(cache.q_state, x, dt, A, B, C, D, z, dt_bias, rand_words, h_out, out, step_counter)
+        if out is not None and out.shape != x.shape:
+            raise ValueError(f"Expected out shape {tuple(x.shape)}, got {tuple(out.shape)}")
         self.cache = cache
         self.out = torch.empty_like(x) if out is None else out
         self._keep = (x, dt, A, B, C, D, z, dt_bias, rand_words, h_out, step_counter)

@@ -82,6 +82,11 @@ def test_errors_come_from_the_general_path():
             mk.mx_state_selective_update(cache, x, x, A, B, B, **{option: torch.ones(2)})
     with pytest.raises(RuntimeError, match="ambiguous"):
         dense_state.selective_state_update(torch.zeros(1, 2, 16, 128, device=d), x, x, A, B, B, dt_softplus=torch.ones(2))
+    for shape in ((1, 2, 8), (1, 1, 16), (2, 2, 16), (2, 16)):  # the kernel would write with these strides
+        with pytest.raises(ValueError, match="Expected out shape"):
+            mk.mx_state_selective_update(cache, x, x, A, B, B, out=torch.zeros(shape, device=d))
+        with pytest.raises(ValueError, match="Expected out shape"):
+            mk.MxUpdatePlan(cache, x, x, A, B, B, out=torch.zeros(shape, device=d))
     assert cache.step == 0
     kv = ia._allocate_layer_cache(1, 2, 16, 128, 4, torch.device(d))
     q = torch.zeros(1, 8, 1, 128, device=d, dtype=torch.bfloat16)
