@@ -6,8 +6,7 @@
 // Here a call is one foreign function with positional arguments; what is left is the output's allocation and the launch.
 //
 // Every function handles the ordinary case only and returns None for anything else (operands on several devices or none, an unexpected
-// shape or type, a status other than LQ_OK from the library).  The operands' device is current while the library is called: a
-// kernel goes to the device that is current, whatever the stream.  The Python caller then takes its general path, which
+// shape or type, a status other than LQ_OK from the library).  The Python caller then takes its general path, which
 // makes the same launch through ctypes or raises the error that belongs to it, so error behaviour has one home.
 #include <ATen/ATen.h>
 #include <c10/cuda/CUDAException.h>
@@ -106,7 +105,6 @@ struct Call {
     type = dtype(*t);
     return t;
   }
-  c10::cuda::CUDAGuard current() const { return c10::cuda::CUDAGuard(static_cast<c10::DeviceIndex>(device)); }
   void* stream() const { return c10::cuda::getCurrentCUDAStream(static_cast<c10::DeviceIndex>(device)).stream(); }
 
  private:
@@ -115,6 +113,18 @@ struct Call {
     return nullptr;
   }
 };
+
+// f(stream) with `device` current, which is where the library's kernels go, and with other Python threads free to run: a launch
+// blocks for as long as the queue of launches is full.
+template <class F>
+int launch(int device, F f) {
+  const c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(device));
+  void* const stream = c10::cuda::getCurrentCUDAStream(static_cast<c10::DeviceIndex>(device)).stream();
+  PyThreadState* const thread = PyEval_SaveThread();
+  const int status = f(stream);
+  PyEval_RestoreThread(thread);
+  return status;
+}
 
 // out: the caller's tensor (shaped like `like`) or a fresh one; returns a new reference in `ref`
 bool output(Call& c, PyObject* given, const at::Tensor& like, at::Tensor& out) {
@@ -216,9 +226,7 @@ PyObject* mx_update(PyObject*, PyObject* const* a, Py_ssize_t n) {
   for (int i = 0; i < 3; ++i) u.out_stride[i] = out.stride(i);
   u.out_dtype = c.dtype(out);
   if (!c.ok) return none();
-  const auto guard = c.current();
-  void* stream = c.stream();
-  if (L.mx_state_update(&u, stream) != LQ_OK) return none();
+  if (launch(c.device, [&](void* stream) { return L.mx_state_update(&u, stream); }) != LQ_OK) return none();
   if (r.step_counter == nullptr) {
     PyObject* next = PyLong_FromLongLong(step + 1);
     if (next == nullptr || PyObject_SetAttr(cache, N.step, next) != 0) {
@@ -227,7 +235,7 @@ PyObject* mx_update(PyObject*, PyObject* const* a, Py_ssize_t n) {
     }
     Py_DECREF(next);
   } else {
-    if (advances && L.counter_add(const_cast<uint64_t*>(r.step_counter), 1, stream) != LQ_OK) {
+    if (advances && launch(c.device, [&](void* stream) { return L.counter_add(const_cast<uint64_t*>(r.step_counter), 1, stream); }) != LQ_OK) {
       PyErr_SetString(PyExc_RuntimeError, "the step counter could not be advanced");
       return nullptr;
     }
@@ -248,8 +256,7 @@ PyObject* mx_plan_run(PyObject*, PyObject* const* a, Py_ssize_t n) {
   lq_mx_update_args& u = *static_cast<lq_mx_update_args*>(address);
   u.rounding.step = static_cast<uint64_t>(step);
   u.rounding.rng_offset = static_cast<uint64_t>(step) * static_cast<uint64_t>(u.state.batch) * u.state.heads * u.state.dim * u.state.dstate;
-  const c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(device));
-  return PyLong_FromLong(L.mx_state_update(&u, c10::cuda::getCurrentCUDAStream(static_cast<c10::DeviceIndex>(device)).stream()));
+  return PyLong_FromLong(launch(static_cast<int>(device), [&](void* stream) { return L.mx_state_update(&u, stream); }));
   END_HANDLE_TH_ERRORS
 }
 
@@ -262,9 +269,7 @@ PyObject* int4_plan_launch(PyObject*, PyObject* const* a, Py_ssize_t n) {
     if (!PyErr_Occurred()) PyErr_SetString(PyExc_TypeError, "int4_plan_launch(address, device)");
     return nullptr;
   }
-  const c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(device));
-  return PyLong_FromLong(L.int4_decode_attn(static_cast<const lq_int4_decode_args*>(address),
-                                            c10::cuda::getCurrentCUDAStream(static_cast<c10::DeviceIndex>(device)).stream()));
+  return PyLong_FromLong(launch(static_cast<int>(device), [&](void* stream) { return L.int4_decode_attn(static_cast<const lq_int4_decode_args*>(address), stream); }));
   END_HANDLE_TH_ERRORS
 }
 
@@ -305,8 +310,7 @@ PyObject* mx_quantize(PyObject*, PyObject* const* a, Py_ssize_t n) {
   s.layout = packed ? LQ_MX_LAYOUT_PACKED : LQ_MX_LAYOUT_REFERENCE;
   lq_rounding r = {};
   r.mode = LQ_ROUND_HALF_EVEN;
-  const auto guard = c.current();
-  if (L.mx_quantize(&s, src->data_ptr(), type, width, &r, c.stream()) != LQ_OK) return none();
+  if (launch(c.device, [&](void* stream) { return L.mx_quantize(&s, src->data_ptr(), type, width, &r, stream); }) != LQ_OK) return none();
   PyObject* out = PyTuple_New(3);
   if (out == nullptr) return nullptr;
   PyTuple_SET_ITEM(out, 0, THPVariable_Wrap(std::move(q)));
@@ -459,19 +463,21 @@ PyObject* decode_attn(PyObject*, PyObject* const* a, Py_ssize_t n) {
     if (k == nullptr || k->scalar_type() != at::kLong || k->numel() != 1) return none();
     d.seq_len_counter = static_cast<const uint64_t*>(k->data_ptr());
   }
-  const auto guard = c.current();
-  if (splits <= 0) splits = L.int4_decode_auto_splits(batch, d.cache.kv_heads, std::max<int64_t>(seq_len - (d.k_new ? 1 : 0), 1));
+  if (splits <= 0) {
+    const c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(c.device));  // the rule asks for its number of SMs
+    splits = L.int4_decode_auto_splits(batch, d.cache.kv_heads, std::max<int64_t>(seq_len - (d.k_new ? 1 : 0), 1));
+  }
   d.splits = static_cast<int32_t>(std::min<int64_t>(splits, INT32_MAX));
-  void* stream = c.stream();
+  at::Tensor ws;  // held until the launch is in the stream
   if (splits > 1) {
-    const at::Tensor ws = workspace(c.device, stream, L.int4_decode_workspace_bytes(batch, heads, d.cache.kv_heads, dim, d.splits));
+    ws = workspace(c.device, c.stream(), L.int4_decode_workspace_bytes(batch, heads, d.cache.kv_heads, dim, d.splits));
     d.workspace = ws.data_ptr();
     d.workspace_bytes = ws.numel();
   }
   at::Tensor out = at::empty({batch, heads, dim}, q->options());
   d.out = out.data_ptr();
   for (int i = 0; i < 3; ++i) d.out_stride[i] = out.stride(i);
-  if (L.int4_decode_attn(&d, stream) != LQ_OK) return none();
+  if (launch(c.device, [&](void* stream) { return L.int4_decode_attn(&d, stream); }) != LQ_OK) return none();
   return THPVariable_Wrap(std::move(out));
   END_HANDLE_TH_ERRORS
 }
@@ -489,10 +495,11 @@ PyObject* pack_kv(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (!c.ok || k->sizes() != v->sizes() || k->scalar_type() != v->scalar_type() || pos->scalar_type() != at::kLong || !pos->is_contiguous() ||
       pos->size(0) != k->size(2) || k->size(0) != s.batch || k->size(1) != s.kv_heads || k->size(3) != s.head_dim)
     return none();
-  const auto guard = c.current();
-  if (L.int4_kv_append(&s, k->data_ptr(), k->strides().data(), v->data_ptr(), v->strides().data(), type,
-                       static_cast<const int64_t*>(pos->data_ptr()), static_cast<int32_t>(k->size(2)), c.stream()) != LQ_OK)
-    return none();
+  const auto append = [&](void* stream) {
+    return L.int4_kv_append(&s, k->data_ptr(), k->strides().data(), v->data_ptr(), v->strides().data(), type,
+                            static_cast<const int64_t*>(pos->data_ptr()), static_cast<int32_t>(k->size(2)), stream);
+  };
+  if (launch(c.device, append) != LQ_OK) return none();
   Py_RETURN_TRUE;
   END_HANDLE_TH_ERRORS
 }
@@ -525,8 +532,7 @@ PyObject* prefill_attn(PyObject*, PyObject* const* a, Py_ssize_t n) {
   p.q_heads = q->size(1);
   p.q_len = q->size(2);
   p.first_len = static_cast<int32_t>(first_len);
-  const auto guard = c.current();
-  if (L.int4_prefill_attn(&p, c.stream()) != LQ_OK) return none();
+  if (launch(c.device, [&](void* stream) { return L.int4_prefill_attn(&p, stream); }) != LQ_OK) return none();
   return give_back(a[5], std::move(out));
   END_HANDLE_TH_ERRORS
 }
@@ -566,9 +572,7 @@ PyObject* dense_update(PyObject*, PyObject* const* a, Py_ssize_t n) {
   u.dstate = w;
   u.ngroups = g;
   u.dt_softplus = softplus;
-  if (!c.ok) return none();
-  const auto guard = c.current();
-  if (L.dense_state_update(&u, c.stream()) != LQ_OK) return none();
+  if (!c.ok || launch(c.device, [&](void* stream) { return L.dense_state_update(&u, stream); }) != LQ_OK) return none();
   return give_back(a[10], std::move(out));
   END_HANDLE_TH_ERRORS
 }
@@ -597,9 +601,7 @@ PyObject* conv1d_update(PyObject*, PyObject* const* a, Py_ssize_t n) {
   u.channels = ch;
   u.width = w;
   u.silu = silu;
-  if (!c.ok) return none();
-  const auto guard = c.current();
-  if (L.causal_conv1d_update(&u, c.stream()) != LQ_OK) return none();
+  if (!c.ok || launch(c.device, [&](void* stream) { return L.causal_conv1d_update(&u, stream); }) != LQ_OK) return none();
   return give_back(a[5], std::move(out));
   END_HANDLE_TH_ERRORS
 }

@@ -145,3 +145,32 @@ def test_recorded_decode_owns_its_scratch():
         held += [torch.full((1 << 20,), 1, dtype=torch.uint8, device=dev()) for _ in range(64)]
     check()
     assert held
+
+
+def test_other_threads_run_during_a_launch(tmp_path):
+    """A launch blocks while CUDA's queue is full.  Here a stand-in for the library blocks in every call; another thread keeps running."""
+    import ctypes
+    import subprocess
+    import threading
+    import time
+    from layer_quant_b200 import _lib
+    names = ("mx_state_update", "mx_quantize", "counter_add", "int4_kv_append", "int4_decode_attn", "int4_decode_workspace_bytes",
+             "int4_decode_auto_splits", "int4_prefill_attn", "dense_state_update", "causal_conv1d_update")
+    source = tmp_path / "slow.c"
+    source.write_text("int usleep(unsigned);\n" + "".join(f"int lq_{n}(void) {{ usleep(400000); return 0; }}\n" for n in names))
+    subprocess.run(["gcc", "-shared", "-fPIC", str(source), "-o", str(tmp_path / "slow.so")], check=True)
+    native, block = _lib.native(), ctypes.create_string_buffer(4096)
+    address, index = ctypes.addressof(block), dev().index
+    native.bind(str(tmp_path / "slow.so"))
+    try:
+        for call in (lambda: native.mx_plan_run(address, index, 0), lambda: native.int4_plan_launch(address, index)):
+            thread = threading.Thread(target=call)
+            longest, last = 0.0, time.perf_counter()
+            thread.start()
+            while thread.is_alive():
+                time.sleep(0.001)
+                now = time.perf_counter()
+                longest, last = max(longest, now - last), now
+            assert longest < 0.2
+    finally:
+        native.bind(str(_lib.LIB_PATH))
