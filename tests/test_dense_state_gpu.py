@@ -144,12 +144,10 @@ def test_dense_update_against_reference_mx_fixtures(golden_dir, name):
         np.testing.assert_allclose(state.cpu().numpy(), g["h0"], rtol=3e-6, atol=1e-7)
 
 
-@pytest.mark.parametrize("state_dtype", [torch.bfloat16, torch.float16, torch.float32])
-@pytest.mark.parametrize("shape", [(1, 1, 4, 128, 1), (1, 3, 4, 128, 1), (3, 5, 12, 128, 5), (2, 7, 20, 128, 7), (9, 32, 64, 128, 8)])
-def test_rows_kernel_edges(state_dtype, shape):
-    """One step of four rows, an odd number of steps, runs across heads, groups and sequences.  Bound on the state: its own
-    rounding (one ulp; 2**-22 for fp32's few roundings) and, because h exp(A dt) + B dt x can cancel, 2**-17 of the operands: dt moves
-    by 2**-23 / dt when exp() differs in its last bit, through exp(A dt) with |A| <= 16 that is a few 2**-19 of them."""
+def check_update_edges(state_dtype, shape):
+    """Bound on the state: its own rounding (one ulp; 2**-22 for fp32's few roundings) and, because h exp(A dt) + B dt x can cancel,
+    2**-17 of the operands: dt moves by 2**-23 / dt when exp() differs in its last bit, through exp(A dt) with |A| <= 16 that is a few
+    2**-19 of them."""
     b, h, p, n, g = shape
     d = make_update_case(11, b, h, p, n, g)
     state = t(d["state"], state_dtype)
@@ -161,6 +159,22 @@ def test_rows_kernel_edges(state_dtype, shape):
     ulp = {torch.bfloat16: 2.0 ** -7, torch.float16: 2.0 ** -10, torch.float32: 2.0 ** -22}[state_dtype]
     error = np.abs(state.float().cpu().numpy() - want_h)
     assert (error <= ulp * np.abs(want_h) + 2.0 ** -17 * (np.abs(start) + np.abs(want_h)) + 1e-7).all()
+
+
+@pytest.mark.parametrize("state_dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("shape", [(1, 1, 16, 128, 1), (3, 5, 48, 128, 5), (2, 7, 80, 128, 7), (9, 32, 64, 128, 8), (37, 40, 80, 128, 8),
+                                   (61, 35, 48, 128, 7)])
+def test_rows_kernel_edges(state_dtype, shape):
+    """Dims that are multiples of 16 are the rows kernel's: the smallest launch, warps of one and two steps, and (the last two, 12.5 and
+    10.8 steps per warp) runs of several batches that start and end inside one and cross heads, groups and sequences."""
+    check_update_edges(state_dtype, shape)
+
+
+@pytest.mark.parametrize("state_dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("shape", [(1, 1, 4, 128, 1), (1, 3, 4, 128, 1), (3, 5, 12, 128, 5), (2, 7, 20, 128, 7)])
+def test_ring_kernel_edges(state_dtype, shape):
+    """Other dims are the ring kernel's, whatever the batch."""
+    check_update_edges(state_dtype, shape)
 
 
 def test_both_sides_of_the_batch_rule():
