@@ -405,12 +405,17 @@ def test_prefill_tensor_core_edges(ratio, tq, first, k_size, v_size):
     cache = fill_cache(m, k, v, gs, capacity=(total + 15) // 16 * 16)
     ref = oracle.int4_prefill_attention(q, *cache_np(cache), first, gs)
     for dtype in (torch.bfloat16, torch.float16):
-        if dtype == torch.float16 and v_size == 1e20:
-            continue  # beyond the output type
         out = m._prefill_attention(t(q, dtype), cache, ratio, gs, first_len=first)
-        if dtype == torch.float16 and v_size in (1e-7, 1e5):  # subnormal outputs / outputs past 65504
+        if dtype == torch.bfloat16:
+            assert_out_close(out, ref)
             continue
-        assert_out_close(out, ref)
+        # fp16 outputs may be subnormal (half a unit of 2**-24) or past 65504 (infinite); those near that edge may be either
+        inside = np.abs(ref) <= 65504.0
+        got = out.float().cpu().numpy().astype(np.float64)
+        scale = max(np.abs(ref).max(), 1e-30)
+        bound = 2.0 ** -10 * np.abs(ref) + 1e-4 * min(scale, 65504.0) + 2.0 ** -25
+        assert (np.abs(got - ref) <= bound)[inside & np.isfinite(got)].all()
+        assert np.array_equal(np.isfinite(got), inside) or (np.abs(ref)[np.isfinite(got) != inside] > 0.998 * 65504.0).all()
     from layer_quant_b200 import _lib
     assert _lib.device_status() == 0
 
@@ -423,14 +428,12 @@ def test_append_divisions_exhaustively(dtype):
     bits, exps = (7, 5) if dtype == torch.bfloat16 else (10, 5)
     n = 1 << bits
     mant = 1.0 + np.arange(n) / n
-    step = 1 if dtype == torch.bfloat16 else 3  # a third of the fp16 maxima (the scale depends on nothing else)
     cols = 126  # values beside the maximum and its negative in a row of one group
     vals = (mant[None, :] * 2.0 ** -np.arange(exps)[:, None]).reshape(-1)
     pad = -len(vals) % cols
     vals = np.concatenate([vals, np.zeros(pad)]).reshape(-1, cols)
-    amax = mant[::step]
-    for at in range(0, len(amax), 64):
-        a = amax[at:at + 64]
+    for at in range(0, n, 64):
+        a = mant[at:at + 64]
         x = np.empty((len(a), len(vals), 128), np.float32)
         x[:, :, 0] = a[:, None] * 2
         x[:, :, 1] = -a[:, None] * 2
@@ -446,6 +449,28 @@ def test_append_divisions_exhaustively(dtype):
             assert torch.equal(getattr(got, name), getattr(ref, name)), name
     q, s = oracle.int4_encode(x.reshape(1, 1, -1, 128), 128)
     assert np.array_equal(got.k_packed.cpu().numpy(), oracle.int4_pack_nibbles(q)) and np.array_equal(got.k_scale.cpu().numpy(), s)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_append_divisions_by_the_scale_floor(dtype):
+    """Groups whose largest value is below 7e-8 are divided by the floor of 1e-8: every such value of the type, subnormals included."""
+    m = ia()
+    bits = torch.arange(1 << 15, dtype=torch.int16).view(dtype).float()
+    vals = bits[bits <= 7e-8]
+    vals = torch.cat([vals, -vals])
+    rows = -(-len(vals) // 128)
+    k = torch.zeros(rows * 128)
+    k[:len(vals)] = vals
+    k = k.to(dtype).reshape(1, 1, rows, 128)
+    assert torch.equal(k.float().flatten()[:len(vals)], vals)
+    pos = torch.arange(rows, device=dev())
+    for gs in (32, 128):
+        cache = m._allocate_layer_cache(1, 1, rows, 128, 128 // gs, dev())
+        m._pack_kv_into_cache(cache, k.to(dev()), -k.to(dev()), pos, gs)
+        for src, packed, scale in ((k, cache.k_packed, cache.k_scale), (-k, cache.v_packed, cache.v_scale)):
+            q, s = oracle.int4_encode(src.float().numpy(), gs)
+            assert (s == np.float32(1e-8)).all()
+            assert np.array_equal(packed.cpu().numpy(), oracle.int4_pack_nibbles(q)) and np.array_equal(scale.cpu().numpy(), s)
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
