@@ -719,13 +719,17 @@ LQ_EXPORT int lq_dense_state_update(const lq_dense_update_args* args, void* cuda
   const size_t esz = a.state_dtype == LQ_F32 ? 4 : 2;
   d.vector_ok = reinterpret_cast<uintptr_t>(a.state) % 16 == 0 && (a.state_stride[0] * esz) % 16 == 0 &&
                 (a.state_stride[1] * esz) % 16 == 0 && (a.state_stride[2] * esz) % 16 == 0;
-  // the usual shape: rows dealt evenly to the warps of one resident wave.  Beyond 400 steps per warp (about batch 460) the ring kernel,
-  // whose CTAs keep more bytes in flight, is the faster one: batch 256 177 / 178 us, batch 1024 689 / 671 us.
+  // The usual shape: rows dealt evenly to the warps of one resident wave.  The longer the launch the less the even deal and the early start
+  // are worth, and the ring kernel keeps more bytes in flight.  us a launch, rows / ring, 128 heads of 64 rows a sequence:
+  //   bf16  batch 64 47.9 / 56.7, 128 91.6 / 99.9, 192 133 / 141, 256 177 / 176, 288 200 / 204, 320 218 / 216, 512 353 / 351, 1024 692 / 671
+  //   fp16  64 48.8 / 58.0, 192 134 / 143, 256 178 / 178, 288 200 / 206, 320 223 / 220, 1024 703 / 670
+  //   fp32  64 93.7 / 102, 72 103 / 109, 80 114 / 109, 104 154 / 142, 128 181 / 177, 256 354 / 337 (its steps have twice the bytes)
+  const uint64_t most_steps = a.state_dtype == LQ_F32 ? 64 : 256;  // per warp: batch 74 and 296
   const int batch_rows = a.state_dtype == LQ_F32 ? 8 : 16;
   const uint64_t steps = static_cast<uint64_t>(a.batch) * a.heads * a.dim / 4;
   if (d.vector_ok && d.dt_uniform && d.a_scalar && a.dstate == 128 && a.dim % 16 == 0 && a.state_stride[2] == 128 &&
       a.state_stride[1] == 128ll * a.dim && a.state_stride[0] == 128ll * a.dim * a.heads &&
-      steps <= 400ull * sm_count() * kRowsCtasPerSm * (kRowsThreads / 32)) {
+      steps <= most_steps * sm_count() * kRowsCtasPerSm * (kRowsThreads / 32)) {
     DenseRowsDerived r;
     const uint64_t warps = std::min<uint64_t>((steps + 1) / 2 * 2, static_cast<uint64_t>(sm_count()) * kRowsCtasPerSm * (kRowsThreads / 32));
     r.steps_per_warp = static_cast<uint32_t>(steps / warps);

@@ -177,20 +177,22 @@ def test_ring_kernel_edges(state_dtype, shape):
     check_update_edges(state_dtype, shape)
 
 
-def test_both_sides_of_the_batch_rule():
-    """A batch just large enough for the ring kernel equals its two halves, which the rows kernel takes: the update is the
-    same fp32 expression (a 16-bit state may differ by one rounding, 2**-8 relative), y a sum of 128 terms in another order."""
-    b, h, p, n, g = 464, 128, 64, 128, 8
+@pytest.mark.parametrize("state_dtype,b", [(torch.bfloat16, 464), (torch.float16, 300), (torch.float32, 80)])
+def test_both_sides_of_the_batch_rule(state_dtype, b):
+    """A batch large enough for the ring kernel equals its two halves, which the rows kernel takes: the update is the
+    same fp32 expression (a 16-bit state may differ by one rounding, 2**-8 or 2**-11 relative), y a sum of 128 terms in another order."""
+    h, p, n, g = 128, 64, 128, 8
     gen = torch.Generator(device=dev()).manual_seed(1)
     rnd = lambda *s: torch.randn(*s, generator=gen, device=dev()).to(torch.bfloat16)
-    state, x, dt, B, C = rnd(b, h, p, n), rnd(b, h, p), rnd(b, h), rnd(b, g, n), rnd(b, g, n)
+    state, x, dt, B, C = rnd(b, h, p, n).to(state_dtype), rnd(b, h, p), rnd(b, h), rnd(b, g, n), rnd(b, g, n)
     A = -torch.ones(h, device=dev())
     halves = state.clone()
     run = lambda s, r: ds().selective_state_update(s, x[r], dt[r][..., None].expand(-1, h, p), A[:, None, None].expand(h, p, n), B[r], C[r],
                                                    dt_softplus=True)
     y = run(state, slice(0, b))
-    yh = torch.cat([run(halves[:232], slice(0, 232)), run(halves[232:], slice(232, b))])
-    assert ((state.float() - halves.float()).abs() <= 2.0 ** -7 * halves.float().abs() + 1e-7).all()
+    yh = torch.cat([run(halves[:b // 2], slice(0, b // 2)), run(halves[b // 2:], slice(b // 2, b))])
+    ulp = {torch.bfloat16: 2.0 ** -7, torch.float16: 2.0 ** -10, torch.float32: 2.0 ** -22}[state_dtype]
+    assert ((state.float() - halves.float()).abs() <= ulp * halves.float().abs() + 1e-7).all()
     assert_out_close(y, yh.float().cpu().numpy())
 
 
