@@ -736,8 +736,10 @@ static int pick_splits(int batch, int kv_heads, int ctx_len) {
     const int64_t waves = (per_sm + 2) / 3;
     const double cost = 3.5 + (s > 1 ? 3.2 + 0.016 * s : 0.0) + tps * ((per_sm / 3) * kTileUs[3] + kTileUs[per_sm % 3]) + 4.0 * (waves - 1) +
                         1.1 * std::min<int64_t>(per_sm, 3);
-    // ties go to fewer splits; in launches of 200 us and more HBM evens out what the deal to the SMs leaves uneven
-    if (cost < best_cost * (best_cost > 200.0 ? 0.98 : 0.999)) {
+    // Ties go to fewer splits; in launches of 250 us and more HBM evens out what the deal to the SMs leaves uneven: us with the choice of
+    // 0.98 / of 0.999: batch 16 x 65536 269 / 278, 32 x 32768 281 / 289, 56 x 32768 456 / 477, 64 x 32768 511 / 535; below, 48 x 16384 (cost
+    // 203) 236 / 214, 96 x 8192 (207) 233 / 220.
+    if (cost < best_cost * (best_cost > 250.0 ? 0.98 : 0.999)) {
       best_cost = cost;
       best = s;
     }

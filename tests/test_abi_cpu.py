@@ -94,3 +94,9 @@ def test_no_fallback_when_library_missing(monkeypatch, tmp_path):
     monkeypatch.setattr(_lib, "LIB_PATH", tmp_path / "missing.so")
     with pytest.raises(RuntimeError, match="no CPU or Triton fallback"):
         _lib.lib()
+
+
+def test_split_count_in_launches_around_250_us(lib):
+    """Fewer splits win ties only in the longest launches (148 SMs, as on the GPU the rule was measured on and as without one)."""
+    for batch, tokens, splits in ((48, 16383, 3), (96, 8191, 2), (16, 65535, 8), (32, 32767, 4), (64, 32767, 2)):
+        assert lib.lq_int4_decode_auto_splits(batch, 8, tokens) == splits
