@@ -175,7 +175,8 @@ __global__ void int4_append_kernel(const AppendParams p, int64_t total_chunks, i
 
 // x / d, with inv the rounded reciprocal of d: an approximate quotient and one correction from its exact remainder (Markstein,
 // "Computation of elementary functions on the IBM RISC System/6000 processor", 1990).  For x of a 16-bit type this is the
-// correctly rounded quotient wherever the codec can tell (every pair of values is tried in the tests); finite x and d only.
+// correctly rounded quotient wherever the codec can tell (the tests try every mantissa of the group's largest value with every mantissa
+// of the others, at every exponent that matters, and every value under the scale's floor); finite x and d only.
 __device__ __forceinline__ float quotient16(float x, float d, float inv) {
   const float q = x * inv;
   return fmaf(fmaf(-q, d, x), inv, q);

@@ -24,8 +24,10 @@
 // What remains relative to the largest: inside a token the group scales below 2^-15 of its largest lose bits, and a weight times
 // V counts with the row's largest (first item), whichever group that is in.
 //
-// What bounds it: the five products take 5/2 of the tensor time of a bf16 attention.  Per 256 x 64 tile that is 2620 cycles;
-// shared memory moves 230 KB meanwhile (1800 cycles), which is why Q is an operand in TMEM, and the exp2 take 1024.
+// What bounds it: per 256 x 64 tile the five products take 2620 tensor cycles (5/2 of a bf16 attention; 1.33 us at 1965 MHz), shared memory
+// moves 230 KB (1800 cycles, which is why Q is an operand in TMEM) and the exp2 take 1024; a tile takes 2.05 us.  No pipe is full: within a
+// softmax group S, softmax, P, the products with V and the next S follow one another (P replaces S), and two groups fill one another's
+// gaps only in part (tensor pipe active in 53 % of the cycles at 8 x 1024).
 #pragma once
 
 #include "lq_common.cuh"
@@ -738,8 +740,7 @@ __device__ __forceinline__ void softmax_blocks(const Params& p, Shared& sh) {
 
 // One CTA per SM works through a list of row blocks, and a block's start overlaps the end of the one before: its first tiles are
 // unpacked, its query rows loaded and its first scores made while the last products run and the output is stored.  A tile
-// takes 2.05 us (five products at 91 % of the measured dense rate); as one CTA per block, start and end added 8 to 9 us to every
-// block.  8 x 1024 tokens: 185 -> 160 us; 2 x 2000 behind 6001: 884 -> 855; 16 x 256: 53 -> 43; 1 x 128 behind 4000 (halves): 135 -> 110.
+// takes 2.05 us; as one CTA per block, start and end added 8 to 9 us to every block.  8 x 1024 tokens: 185 -> 160 us; 2 x 2000 behind 6001: 884 -> 855; 16 x 256: 53 -> 43; 1 x 128 behind 4000 (halves): 135 -> 110.
 // Dropped: two score buffers of 32 tokens per group, which would let the tensor pipe run ahead of the softmax (a product of 32 columns
 // takes as long as one of 64: 2.31 us a tile), and starting the products of a tile's first half while its second is made (2.1 us).
 __global__ void __launch_bounds__(kThreads, 1) int4_prefill_kernel(const __grid_constant__ Params p) {

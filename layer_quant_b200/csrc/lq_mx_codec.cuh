@@ -201,7 +201,8 @@ __device__ __forceinline__ void mx_encode_block(const float (&h)[16], const MxRo
 // Association as in the reference kernel (mamba_state_8b_kernel.py:158, dB = B * dt, then state * dA + dB * x):
 // dB rounded (by the caller), t = dB * x rounded, then fma(h, dA, t), which is what a compiler that contracts the reference's
 // expression produces; the read-out keeps four partial sums over i mod 4, added as (y0 + y1) + (y2 + y3).
-// h is given as q * s with s a power of two: fma(h, dA, t) = fma(q, s dA, t), for s dA is exact.  sd: s dA of the pairs,
+// h is given as q * s with s a power of two: fma(h, dA, t) = fma(q, s dA, t), for s dA is exact unless it is subnormal (then a term below
+// 2^-119 is off by part of itself: nothing that a code, whose unit is 2^-99 at least, or a normal y can show).  sd: s dA of the pairs,
 // ONE: of the whole block (sd[0]).
 template <bool ONE>
 __device__ __forceinline__ float mx_update_readout16(float (&hv)[16], const float (&dB)[16], const float (&Cv)[16], const float (&sd)[8],
@@ -228,7 +229,7 @@ __device__ __forceinline__ float mx_update_readout16(float (&hv)[16], const floa
   return (ya.x + ya.y) + (yb.x + yb.y);
 }
 
-// What a stored block and dA = exp(A dt) give the update: q[i] and sd with h dA = q[i] sd of the pair, both exact.
+// What a stored block and dA = exp(A dt) give the update: q[i] and sd with h dA = q[i] sd of the pair, exact unless sd is subnormal.
 // Byte codes: q the code, sd = 2^(e - 127 + micro) dA.  The factor 1 or 2 of four pairs comes from a 16-entry table in shared memory
 // (two 128-bit loads in place of a mask, a multiply and a multiply per pair).  Packed nibbles: the micro-exponent doubles
 // the code instead, in bytes of unsigned integers (q + 16 or 2 q + 16), so one factor serves the block; `table` holds

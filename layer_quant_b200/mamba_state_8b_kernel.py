@@ -205,7 +205,7 @@ def allocate_state_kernel_cache(ssm_state_4d: torch.Tensor, group_size: int = MX
 
 class MxUpdatePlan:
     """A prepared ``mx_state_selective_update`` call: shapes are checked and the argument block of
-    the C entry point is filled once, so that repeating the step costs one ctypes call.  The
+    the C entry point is filled once, so that repeating the step costs one native call.  The
     tensors handed in must stay alive and in place (the plan keeps references).
 
     ``step_counter`` (a 1-element int64 CUDA tensor) makes the launch replayable from a CUDA
@@ -286,19 +286,6 @@ class MxUpdatePlan:
         self._address = ct.addressof(a)
         self._device_index = self.device.index
         self._counts_on_device = step_counter is not None
-        self._out_sig = (self.out.data_ptr(), self.out.stride(), self.out.dtype)
-
-    def rebind_out(self, out: torch.Tensor) -> None:
-        """Point the prepared call at another output tensor (shape and dtype of ``x``)."""
-        sig = (out.data_ptr(), out.stride(), out.dtype)
-        self.out = out
-        if sig == self._out_sig:
-            return
-        self._out_sig = sig
-        a = self.args
-        a.out = sig[0]
-        a.out_stride[0], a.out_stride[1], a.out_stride[2] = sig[1]
-        a.out_dtype = _lib.dtype_code(out)
 
     def run(self) -> torch.Tensor:
         cache = self.cache
