@@ -18,6 +18,7 @@
 #include <atomic>
 #include <cstdlib>
 #include <cstring>
+#include <type_traits>
 
 #include "lq_common.cuh"
 
@@ -1001,10 +1002,20 @@ static int launch_prefill_tc(const lq_int4_prefill_args& a, int ratio, cudaStrea
   const int sms = sm_count(), rest = static_cast<int>(blocks % sms);
   p.whole = static_cast<int>(blocks) - (2 * rest <= sms ? rest : 0);
   p.entries = p.whole + 2 * (static_cast<int>(blocks) - p.whole);
-  LQ_SET_SMEM_ONCE(prefill::int4_prefill_kernel, prefill::kSmemBytes);
-  prefill::int4_prefill_kernel<<<static_cast<unsigned>(std::min(p.entries, sms)), prefill::kThreads, prefill::kSmemBytes, st>>>(p);
-  LQ_CHECK_CUDA(cudaGetLastError());
-  return LQ_OK;
+  const auto launch = [&](auto lead) -> int {
+    constexpr int LEAD = decltype(lead)::value;
+    LQ_SET_SMEM_ONCE(prefill::int4_prefill_kernel<LEAD>, prefill::kSmemBytes);
+    prefill::int4_prefill_kernel<LEAD><<<static_cast<unsigned>(std::min(p.entries, sms)), prefill::kThreads, prefill::kSmemBytes, st>>>(p);
+    LQ_CHECK_CUDA(cudaGetLastError());
+    return LQ_OK;
+  };
+  // Token factors save products, for which they cost the softmax some 100 instructions per thread and tile.  With every SM busy the products
+  // (and the power they draw) count: 2 x 2000 behind 6001 tokens, groups of 64, 949 -> 875 us in long runs; 1 x 3000 167 -> 153; 3 x 700 behind
+  // 100, groups of 128, 46.8 -> 45.0.  Where the list is halves of one softmax group only, the softmax counts: 1 x 128 behind 4000 112 -> 116 us.
+  // In groups of 32 only a quarter of the dims would lead, and the tensor core takes N in steps that save nothing there.
+  if (p.whole > 0 && a.cache.group_size == 64) return launch(std::integral_constant<int, 64>{});
+  if (p.whole > 0 && a.cache.group_size == 128) return launch(std::integral_constant<int, 128>{});
+  return launch(std::integral_constant<int, 0>{});
 }
 
 LQ_EXPORT int lq_int4_prefill_attn(const lq_int4_prefill_args* args, void* cuda_stream) {

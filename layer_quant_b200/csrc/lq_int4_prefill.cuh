@@ -14,6 +14,11 @@
 // the same way: 2^-22 of a weight or 2^-35 of the row's largest, whichever is more.  (The mma.sync kernel keeps 2^-17 of every
 // weight.  The absolute part adds up to less than that over 2^17 tokens.)  Q is exact in fp16 for 16-bit queries.
 // S = Q Khi + Q Klo, O = Phi Vhi + Plo Vhi + Phi Vlo: five products per tile pair, all in fp32 accumulators.
+// Token factors (LEAD, the dims of the first group, 64 or 128): where all of a CTA's SM is busy a group's scale is worth more outside the products.
+// The mantissa of a token's first scale goes to the softmax, which multiplies the scores (K) and the weights after their sum is taken (V) by it in
+// fp32; the first group's operands are then a code times a power of two, exact in fp16, and need no lo part, the other groups' scales are divided by
+// it.  Groups of 64: four products per tile pair in place of five, of 128: three.  The error against 64 bits goes down with the lo parts: outputs that are
+// not the correctly rounded fp16 value 1.1 % -> 0.8 % (groups of 64) and 0.27 % (128) of 2 x 700 tokens.
 // Range.  Powers of two are taken out of every row of Q and of the K and V scales of every 16 tokens, so the
 // fp16 operands sit at the top of their range; the exponents come back for free, in the factor and the offset of the
 // exp2 argument.  With p' = 2^(s + Ev - m) the V exponent Ev is part of the running maximum m.
@@ -24,7 +29,9 @@
 // What remains relative to the largest: inside a token the group scales below 2^-15 of its largest lose bits, and a weight times
 // V counts with the row's largest (first item), whichever group that is in.
 //
-// What bounds it: per 256 x 64 tile the five products take 2620 tensor cycles (5/2 of a bf16 attention; 1.33 us at 1965 MHz), shared memory
+// What bounds it: in long runs the board's power (the five products run at 1365 TFLOP/s where cuBLAS sustains 1395: other schedules of the same
+// products, such as a third score buffer per pair of groups, took less cycles per tile, 3650 for 4030, at a clock lower by as much).  In short
+// runs: per 256 x 64 tile the five products take 2620 tensor cycles (5/2 of a bf16 attention; 1.33 us at 1965 MHz), shared memory
 // moves 230 KB (1800 cycles, which is why Q is an operand in TMEM) and the exp2 take 1024; a tile takes 2.05 us.  No pipe is full: within a
 // softmax group S, softmax, P, the products with V and the next S follow one another (P replaces S), and two groups fill one another's
 // gaps only in part (tensor pipe active in 53 % of the cycles at 8 x 1024).
@@ -49,7 +56,10 @@ constexpr float kScaleFloor = 1.0e-8f;        // of the codec
 // fp16 cannot hold is the absolute 2^-24, so the top of its range has to be used.  2^(kSlack + kLift) must stay below 65504.  A wider slack
 // raises the maximum less often and leaves less lift: with 8 and 0 weights below 2^-25 of the largest were lost altogether, at 969 us
 // against 977 for 2 x 2000 tokens behind 6001.
-constexpr float kSlack = 4.0f, kLift = 11.0f;
+// With token factors (below 2) on the weights the slack is a quarter less: 2^15.75.
+constexpr float kLift = 11.0f;
+template <int LEAD>
+constexpr float kSlack = LEAD ? 3.75f : 4.0f;
 // A score and the maximum part in one FMA, so the rounding of the maximum is in the difference; beyond scores of 2^24 that would
 // overflow P.  Queries below kLargeQ and K scales below kLargeK (values below 8 kLargeK) keep scores below 2^21.3; larger ones are rounded
 // before the difference is taken, in the pass that wide tiles take.
@@ -161,6 +171,7 @@ __device__ __forceinline__ void mma_commit(uint64_t* bar) {
 // fp16 inputs, fp32 accumulators, M = 128; K tile: N = 64 tokens, dims contiguous; V tile: N = 128 dims, dims contiguous (N-major)
 constexpr uint32_t kIdescS = (1u << 4) | ((64u / 8) << 17) | ((128u / 16) << 24);
 constexpr uint32_t kIdescO = (1u << 4) | (1u << 16) | ((128u / 8) << 17) | ((128u / 16) << 24);
+constexpr uint32_t kIdescO64 = (1u << 4) | (1u << 16) | ((64u / 8) << 17) | ((128u / 16) << 24);
 // Shared-memory matrix descriptor, 128-byte swizzle.  Stride offset 1024: the next eight rows of 128 bytes; lbo: the next
 // 64 dims of an N-major tile.
 __device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo) {
@@ -176,6 +187,7 @@ struct Shared {
   uint64_t k_first, full[2], empty[2], s_done[2], p_ready[2], q_ready[2];
   // Per 16 tokens: 2^Ek, Ev and 2^-Ev of the tile, four tiles deep (they are written a unit ahead of V)
   float k_factor[5][4], v_exp[5][4], v_inv[5][4];  // slot 4: 1, 0, 0
+  alignas(16) float k_lead[4][kTok], v_lead[4][kTok];  // token factors, where there are any
   // A byte per 16 tokens, bit 0: they are wide, bit 1: large K scales.  Then for wide ones the same per token (k_factor NaN: the
   // scale is not finite), and the 32-dim chunks of V whose scale is not finite, a bit each
   uint32_t wide[4];
@@ -259,9 +271,14 @@ __device__ __forceinline__ Exponents exponents_of(float (&sc)[2]) {
   return r;
 }
 
-// 32 dims of one token -> shared memory: 64 bytes of the hi part and of the lo part
-__device__ __forceinline__ void store_chunk(uint8_t* part_hi, int token, int chunk, const uint4& raw, float scale, int e) {
-  const float s = scale * pow2_of(-e);
+// The token factor of a scale (its exponent taken out) of the leading group: its mantissa, so that the rest is a power of two
+__device__ __forceinline__ float lead_of(float s) {
+  const uint32_t b = __float_as_uint(s);
+  return b < 0x00800000u ? 1.0f : __uint_as_float((b & 0x007FFFFFu) | 0x3F800000u);
+}
+// 32 dims of one token -> shared memory: 64 bytes of the hi part and, unless s is a power of two, of the lo part
+template <bool LO>
+__device__ __forceinline__ void store_chunk(uint8_t* part_hi, int token, int chunk, const uint4& raw, float s, bool lo_too) {
   const __half2 hi = __float2half2_rn(__uint_as_float(__float_as_uint(s) & 0xFFFF0000u));
   const __half2 lo = __float2half2_rn(s - __low2float(hi));
   const uint32_t words[4] = {raw.x, raw.y, raw.z, raw.w};
@@ -275,14 +292,15 @@ __device__ __forceinline__ void store_chunk(uint8_t* part_hi, int token, int chu
     for (int i = 0; i < 4; ++i) {
       const __half2 a = __hmul2(n[i], hi), b = __hmul2(n[i], lo);
       h[i] = *reinterpret_cast<const uint32_t*>(&a);
-      l[i] = *reinterpret_cast<const uint32_t*>(&b);
+      if (LO) l[i] = *reinterpret_cast<const uint32_t*>(&b);
     }
     uint8_t* dst = row + ((((chunk & 1) * 4 + w) ^ (token & 7)) << 4);
     *reinterpret_cast<uint4*>(dst) = make_uint4(h[0], h[1], h[2], h[3]);
-    *reinterpret_cast<uint4*>(dst + kPart) = make_uint4(l[0], l[1], l[2], l[3]);
+    if (LO && lo_too) *reinterpret_cast<uint4*>(dst + kPart) = make_uint4(l[0], l[1], l[2], l[3]);
   }
 }
 
+template <int LEAD>
 __device__ __forceinline__ void unpack_tiles(const Params& p, Shared& sh, uint8_t* smem) {
   const lq_int4_cache& c = p.a.cache;
   const int warp = (threadIdx.x >> 5) & 3, lane = threadIdx.x & 31;
@@ -348,9 +366,21 @@ __device__ __forceinline__ void unpack_tiles(const Params& p, Shared& sh, uint8_
       }
     }
   };
-  auto store = [&](int stage, const uint4 (&raw)[2], const float (&sc)[2], const int (&e)[2]) {
+  // Takes the exponent out of the lane's two scales, and the token's factor, which goes to `lead` of the tile
+  auto take_out = [&](float (&sc)[2], const int (&e)[2], float* lead) {
 #pragma unroll
-    for (int i = 0; i < 2; ++i) store_chunk(smem + stage * kStageBytes, row + 8 * i, chunk, raw[i], sc[i], e[i]);
+    for (int i = 0; i < 2; ++i) {
+      sc[i] *= pow2_of(-e[i]);
+      if (LEAD) {
+        const float f = lead_of(__shfl_sync(0xFFFFFFFFu, sc[i], lane & 7));
+        sc[i] = chunk < LEAD / 32 ? __uint_as_float(__float_as_uint(sc[i]) & 0x7F800000u) : __fdividef(sc[i], f);
+        if (chunk == 0) lead[row + 8 * i] = f;
+      }
+    }
+  };
+  auto store = [&](int stage, const uint4 (&raw)[2], const float (&s)[2]) {
+#pragma unroll
+    for (int i = 0; i < 2; ++i) store_chunk<LEAD != 128>(smem + stage * kStageBytes, row + 8 * i, chunk, raw[i], s[i], chunk >= LEAD / 32);
   };
   auto arrive = [&](uint64_t* bar) {
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -358,7 +388,7 @@ __device__ __forceinline__ void unpack_tiles(const Params& p, Shared& sh, uint8_
     if (lane == 0) mbar_arrive(bar);
   };
   uint4 k[2], v[2], k_next[2], v_next[2];
-  float ks_cur[2], vs_cur[2], vs_ahead[2], ks_next[2], vs_next[2];  // scales of k and v above; of V one tile further
+  float ks_cur[2], vs_cur[2], vs_ahead[2], ks_next[2], vs_next[2];  // scales of k and v above (of v with its exponents taken out); of V one tile further
   open_block();
   fetch(kp, tok, k);
   fetch_scales(ks, tok, ks_cur);
@@ -368,13 +398,12 @@ __device__ __forceinline__ void unpack_tiles(const Params& p, Shared& sh, uint8_
   fetch(kp, tok, k_next);
   fetch_scales(ks, tok, ks_next);
   fetch_scales(vs, tok, vs_ahead);
-  int ev[2];
   {
-    const Exponents ek = exponents_of(ks_cur), ev_first = exponents_of(vs_cur);
-    ev[0] = ev_first.e[0];
-    ev[1] = ev_first.e[1];
-    publish(0, ek, ev_first);
-    store(0, k, ks_cur, ek.e);
+    const Exponents ek = exponents_of(ks_cur), ev = exponents_of(vs_cur);
+    publish(0, ek, ev);
+    take_out(ks_cur, ek.e, sh.k_lead[0]);
+    take_out(vs_cur, ev.e, sh.v_lead[0]);
+    store(0, k, ks_cur);
     arrive(&sh.k_first);
   }
   int total = 0;  // tiles of all blocks of this CTA
@@ -394,12 +423,13 @@ __device__ __forceinline__ void unpack_tiles(const Params& p, Shared& sh, uint8_
     // iteration j - 2 is done (its last products are S of tile j - 1); unit 0 finds its stages empty, unit 1 waits for S of tile 0
     if (!wait_bar(&sh.empty[j & 1], ((j >> 1) ^ j ^ 1) & 1)) return;
     publish(j + 1, ek, ev_ahead);
-    store(2 + (j & 1), v, vs_cur, ev);
-    if (j + 1 < total) store((j + 1) & 1, k, ks_cur, ek.e);
+    take_out(ks_cur, ek.e, sh.k_lead[(j + 1) & 3]);
+    take_out(vs_ahead, ev_ahead.e, sh.v_lead[(j + 1) & 3]);
+    store(2 + (j & 1), v, vs_cur);
+    if (j + 1 < total) store((j + 1) & 1, k, ks_cur);
     arrive(&sh.full[j & 1]);
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
-      ev[i] = ev_ahead.e[i];
       v[i] = v_next[i];
       vs_cur[i] = vs_ahead[i];
       vs_ahead[i] = vs_next[i];
@@ -408,16 +438,17 @@ __device__ __forceinline__ void unpack_tiles(const Params& p, Shared& sh, uint8_
 }
 
 // ---- products --------------------------------------------------------------------------------------------------------
+template <int LEAD>
 __device__ __forceinline__ void issue_products(const Params& p, Shared& sh, uint8_t* smem) {
   const uint64_t k_desc = smem_desc(smem_u32(smem), 16), v_desc = smem_desc(smem_u32(smem) + 2 * kStageBytes, kPart / 2);
-  // S = Q Khi + Q Klo; 16 dims per product: 32 bytes inside a half of 64 dims
+  // S = Q Khi + Q Klo; 16 dims per product: 32 bytes inside a half of 64 dims.  The leading dims have no lo part
   auto issue_s = [&](int g, int j) {
     const uint32_t tm = g * kColsPerGroup;
     const uint64_t d = k_desc + (j & 1) * (kStageBytes >> 4);
 #pragma unroll
     for (int hl = 0; hl < 2; ++hl)
 #pragma unroll
-      for (int k = 0; k < 8; ++k)
+      for (int k = hl ? LEAD / 16 : 0; k < 8; ++k)
         mma_ts(tm + kColS, tm + kColQ + 8 * k, d + ((hl * kPart + (k >> 2) * (kPart / 2) + (k & 3) * 32) >> 4), kIdescS, hl + k > 0);
   };
   // O += Phi Vhi + Plo Vhi + Phi Vlo; 16 tokens per product: 2048 bytes
@@ -427,8 +458,12 @@ __device__ __forceinline__ void issue_products(const Params& p, Shared& sh, uint
 #pragma unroll
     for (int t = 0; t < 3; ++t)
 #pragma unroll
-      for (int k = 0; k < 4; ++k)
-        mma_ts(tm + kColO, tm + kColS + (t == 1 ? 32 : 0) + 8 * k, d + (((t == 2 ? kPart : 0) + k * 2048) >> 4), kIdescO, !first || t + k > 0);
+      for (int k = 0; k < 4; ++k) {
+        if (t < 2 || LEAD == 0)
+          mma_ts(tm + kColO, tm + kColS + (t == 1 ? 32 : 0) + 8 * k, d + (((t == 2 ? kPart : 0) + k * 2048) >> 4), kIdescO, !first || t + k > 0);
+        else if (LEAD == 64)  // the upper 64 dims
+          mma_ts(tm + kColO + 64, tm + kColS + 8 * k, d + ((kPart + kPart / 2 + k * 2048) >> 4), kIdescO64, true);
+      }
   };
   uint32_t p_parity = 0, q_parity = 0;  // bit g
   // S of a block's first tile, once the groups have put their query rows into TMEM
@@ -576,6 +611,7 @@ __device__ __forceinline__ void store_output(const lq_int4_prefill_args& a, int6
 // One row of scores of one block, a tile at a time: S -> P in place, running maximum and sum.  tile: the block's first, counted over
 // all blocks; parity: of the next wait for products of this group; l_run: the sum; bad: the 32-dim chunks for which the row has
 // attended to a V that is not finite.  False after a wait that ran out.
+template <int LEAD>
 __device__ __forceinline__ bool softmax_rows(const Params& p, Shared& sh, int pos0, int ntiles, int tile, uint32_t& parity, float cq, uint32_t large_q,
                                              float& l_run, uint32_t& bad) {
   const lq_int4_prefill_args& a = p.a;
@@ -597,6 +633,15 @@ __device__ __forceinline__ bool softmax_rows(const Params& p, Shared& sh, int po
     const uint32_t wide = sh.wide[f] | large_q;
     uint32_t s[64];
     tmem_load64(s, tm + kColS);
+    if (LEAD) {
+#pragma unroll
+      for (int i = 0; i < 64; i += 4) {
+        const float4 k = *reinterpret_cast<const float4*>(&sh.k_lead[f][i]);
+        const float2 a = __fmul2_rn(make_float2(__uint_as_float(s[i]), __uint_as_float(s[i + 1])), make_float2(k.x, k.y));
+        const float2 b = __fmul2_rn(make_float2(__uint_as_float(s[i + 2]), __uint_as_float(s[i + 3])), make_float2(k.z, k.w));
+        s[i] = __float_as_uint(a.x); s[i + 1] = __float_as_uint(a.y); s[i + 2] = __float_as_uint(b.x); s[i + 3] = __float_as_uint(b.y);
+      }
+    }
     // Rare cases share the branches that are there anyway: with branches of their own 1 x 128 behind 4000 took 115 us instead of 109.
     if (tok0 + kTok > warp_limit || wide != 0u) {
       if (wide != 0u) {  // the finished score of every token in place of the raw one
@@ -609,7 +654,7 @@ __device__ __forceinline__ bool softmax_rows(const Params& p, Shared& sh, int po
           tmem_load16(raw, tm + kColS + 16 * w);
 #pragma unroll
           for (int i = 0; i < 16; ++i) {
-            raw[i] = __float_as_uint(fmaf(__uint_as_float(raw[i]), cq * kf[own ? i : 0], ve[own ? i : 0]));
+            raw[i] = __float_as_uint(fmaf(__uint_as_float(raw[i]) * (LEAD ? sh.k_lead[f][16 * w + i] : 1.0f), cq * kf[own ? i : 0], ve[own ? i : 0]));
             if (own && tok0 + 16 * w + i < limit) bad |= sh.v_bad_tok[f][16 * w + i];
           }
           tmem_store16(tm + kColS + 16 * w, raw);
@@ -637,7 +682,7 @@ __device__ __forceinline__ bool softmax_rows(const Params& p, Shared& sh, int po
     if (j == 0) {
       m_run = m_tile;  // every row sees token 0
     }
-    if (__any_sync(0xFFFFFFFFu, m_tile > m_run + kSlack || wide != 0u)) {
+    if (__any_sync(0xFFFFFFFFu, m_tile > m_run + kSlack<LEAD> || wide != 0u)) {
       if (j > 0) {
         // rare: the running sums of this warp's rows move to a larger maximum (the products into O of the tile before are done)
         const float m_new = fmaxf(m_run, m_tile), alpha = exp2f(m_run - m_new);
@@ -674,8 +719,9 @@ __device__ __forceinline__ bool softmax_rows(const Params& p, Shared& sh, int po
       for (int i = 0; i < 8; ++i) {
         const float2 x = __ffma2_rn(make_float2(__uint_as_float(s[16 * w + 2 * i]), __uint_as_float(s[16 * w + 2 * i + 1])), make_float2(cw[w], cw[w]),
                                     make_float2(off, off));
-        const float2 pr = make_float2(mma::fast_exp2(x.x), mma::fast_exp2(x.y));
+        float2 pr = make_float2(mma::fast_exp2(x.x), mma::fast_exp2(x.y));
         sum = __fadd2_rn(sum, pr);
+        if (LEAD) pr = __fmul2_rn(pr, *reinterpret_cast<const float2*>(&sh.v_lead[f][16 * w + 2 * i]));
         // leading 11 bits by truncation (exact in fp16 from 2^-14 on), the rest rounded to fp16
         const float2 top = make_float2(__uint_as_float(__float_as_uint(pr.x) & 0xFFFFE000u), __uint_as_float(__float_as_uint(pr.y) & 0xFFFFE000u));
         const float2 rest = __ffma2_rn(top, make_float2(-1.0f, -1.0f), pr);
@@ -694,6 +740,7 @@ __device__ __forceinline__ bool softmax_rows(const Params& p, Shared& sh, int po
   return true;
 }
 
+template <int LEAD>
 __device__ __forceinline__ void softmax_blocks(const Params& p, Shared& sh) {
   const lq_int4_prefill_args& a = p.a;
   const int group = threadIdx.x >> 7, warp = (threadIdx.x >> 5) & 3, lane = threadIdx.x & 31;
@@ -723,7 +770,7 @@ __device__ __forceinline__ void softmax_blocks(const Params& p, Shared& sh) {
   for (int r = 0; entry_of(r) < p.entries; ++r) {
     const Block k = block_at(p, entry_of(r));
     if (group < k.groups) {
-      if (!softmax_rows(p, sh, k.pos0, k.ntiles, tile, parity, cq, large_q, l_run, bad)) return;
+      if (!softmax_rows<LEAD>(p, sh, k.pos0, k.ntiles, tile, parity, cq, large_q, l_run, bad)) return;
       const bool more = load_next(r + 1);  // all S of this block are done; its last products run meanwhile
       // the wait stands before the arrival that lets the next S be asked for: s_done is never two phases ahead of a warp
       if (!wait_bar(&sh.s_done[group], parity)) return;
@@ -743,6 +790,7 @@ __device__ __forceinline__ void softmax_blocks(const Params& p, Shared& sh) {
 // takes 2.05 us; as one CTA per block, start and end added 8 to 9 us to every block.  8 x 1024 tokens: 185 -> 160 us; 2 x 2000 behind 6001: 884 -> 855; 16 x 256: 53 -> 43; 1 x 128 behind 4000 (halves): 135 -> 110.
 // Dropped: two score buffers of 32 tokens per group, which would let the tensor pipe run ahead of the softmax (a product of 32 columns
 // takes as long as one of 64: 2.31 us a tile), and starting the products of a tile's first half while its second is made (2.1 us).
+template <int LEAD>
 __global__ void __launch_bounds__(kThreads, 1) int4_prefill_kernel(const __grid_constant__ Params p) {
   extern __shared__ uint8_t smem_raw[];
   __shared__ Shared sh;
@@ -772,11 +820,11 @@ __global__ void __launch_bounds__(kThreads, 1) int4_prefill_kernel(const __grid_
   fence_after();
   if (warp >= 8) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 88;");
-    if (warp < 12) unpack_tiles(p, sh, smem);
-    else if (warp == 12) issue_products(p, sh, smem);
+    if (warp < 12) unpack_tiles<LEAD>(p, sh, smem);
+    else if (warp == 12) issue_products<LEAD>(p, sh, smem);
   } else {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 168;");
-    softmax_blocks(p, sh);
+    softmax_blocks<LEAD>(p, sh);
   }
   fence_before();
   __syncthreads();

@@ -593,3 +593,36 @@ def test_prefill_huge_scores(size):
     cache = fill_cache(m, k, v, gs, dtype=torch.float32)
     ref = oracle.int4_prefill_attention(q, *cache_np(cache), 1, gs)
     assert_out_close(m._prefill_attention(t(q, torch.bfloat16), cache, 4, gs), ref)
+
+
+@pytest.mark.parametrize("gs", [64, 128])
+@pytest.mark.parametrize("ratio,tq,first", [(4, 3, 1), (4, 65, 1), (8, 19, 40), (2, 129, 63)])
+def test_prefill_token_factors(gs, ratio, tq, first):
+    """More than half as many row blocks as SMs and groups of 64 or 128: the kernel that keeps the first group's operands exact and multiplies by the
+    token's factor.  Sequence 0 as it comes, 1 and 2 with a first group far below and far above the others, 3 with a huge key and an infinite
+    value in the last token, which the rows before it must not notice."""
+    m = ia()
+    hkv, total = 2, first + tq - 1
+    b = 40 + torch.cuda.get_device_properties(0).multi_processor_count // (4 * -(-tq * ratio // 256))
+    k, v = (np.repeat(x, b, 0) for x in make_kv(91 + tq, 1, hkv, total))
+    for x in (k, v):
+        x[1, ..., :64] *= 2.0 ** -9
+        x[2, ..., :64] *= 2.0 ** 9
+    k[2] *= 2.0 ** -6
+    k[3, :, -1, 5], v[3, :, -1, 70] = 1e6, np.inf
+    q = np.repeat(bf16r(np.random.default_rng(tq).standard_normal((1, hkv * ratio, tq, 128)) * 0.5), b, 0)
+    cache = fill_cache(m, bf16r(k), bf16r(v), gs, capacity=(total + 15) // 16 * 16)
+    out = m._prefill_attention(t(q, torch.bfloat16), cache, ratio, gs, first_len=first)
+    parts = [x[:4] for x in cache_np(cache)]
+    with np.errstate(all="ignore"):
+        ref = oracle.int4_prefill_attention(q[:4], *parts, first, gs)
+        if tq > 1:  # the oracle's product of a zero weight and an infinity
+            ref[3, :, :-1] = oracle.int4_prefill_attention(q[3:4, :, :-1], *(x[3:4] for x in parts), first, gs)[0]
+    for i in range(3):
+        assert_out_close(out[i], ref[i])
+    assert_out_close(out[3, :, :-1], ref[3, :, :-1])
+    last = torch.from_numpy(np.isfinite(ref[3, :, -1]))
+    assert not torch.isfinite(out[3, :, -1][~last]).any()
+    assert torch.equal(out[4:], out[:1].expand(b - 4, -1, -1, -1))  # the others are sequence 0 once more
+    from layer_quant_b200 import _lib
+    assert _lib.device_status() == 0
