@@ -45,6 +45,7 @@ struct MxRoundCtx {
   uint32_t wrap32;       // PHILOX_REF: counters are taken modulo 2^32 with a zero high word
   uint32_t step, layer;  // PHILOX_LAYERED
   const uint32_t* words; // SUPPLIED / SUPPLIED_FIXED: 16 words of this block
+  const uint32_t* drawn = nullptr;       // PHILOX_REF: the block's 16 words, where the caller has drawn them
   const PhiloxStream* stream = nullptr;  // the layered modes: where the caller carries the generator along, used instead of the counter
 };
 
@@ -172,7 +173,7 @@ __device__ __forceinline__ void mx_encode_block(const float (&h)[16], const MxRo
             w = rnd[i];
           } else {  // the reference's stream: one Philox block per value, word 0
             const uint64_t c = ctx.counter + i;
-            w = philox4x32_10(static_cast<uint32_t>(c), ctx.wrap32 ? 0u : static_cast<uint32_t>(c >> 32), 0u, 0u, keys).w0;
+            w = ctx.drawn ? ctx.drawn[i] : philox4x32_10(static_cast<uint32_t>(c), ctx.wrap32 ? 0u : static_cast<uint32_t>(c >> 32), 0u, 0u, keys).w0;
           }
           const float fl = floorf(a);
           lvl = fl + set_gt(a - fl, word_to_uniform(w));  // (u < a - fl) ? 1 : 0

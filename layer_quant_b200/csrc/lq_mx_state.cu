@@ -336,6 +336,8 @@ __global__ void __launch_bounds__(kUpdateThreads, 4) mx_state_update_kernel(cons
 // current head and C of the current group are kept in registers.
 // NBLK_T = dstate / 16 when known at compile time (8 for Nemotron-H: all lane and address arithmetic
 // folds to constants), 0 = taken from the arguments.
+// kRefAnyOffset: PHILOX_REF with an offset that is no multiple of 16 (a caller's own).  A block's counters may pass 2^32, so every word is drawn by itself.
+constexpr int kRefAnyOffset = 64;
 constexpr int kRingSteps = 4, kRingStages = 2;
 constexpr int kPartialStride = 36;  // floats of a step's read-out partials: 32 and a shift of one 16-byte bank column
 template <int BITS, int LAYOUT>
@@ -572,6 +574,7 @@ __global__ void __launch_bounds__(kFastThreads, kFastCtasPerSm) mx_state_update_
   const MxRoundBase rb = make_round_base(a.rounding, static_cast<uint64_t>(s.batch) * H * P * dstate);
   // layered modes: the counters of the whole state fit 32 bits (fast_update_applies), so the stream carries them
   constexpr bool kStream = MODE == LQ_ROUND_PHILOX_LAYERED || MODE == LQ_ROUND_PHILOX_LAYERED4;
+  constexpr bool kDrawn = MODE == LQ_ROUND_PHILOX_REF;  // a block's 16 counters do not pass 2^32 (kRefAnyOffset otherwise)
   PhiloxStream stream;
   if (kStream) stream.init(static_cast<uint32_t>(lin), 0u, rb.step, rb.layer, d.keys);
 
@@ -633,11 +636,24 @@ __global__ void __launch_bounds__(kFastThreads, kFastCtasPerSm) mx_state_update_
       if (kAhead && k + 1 < kRingSteps) cur = Ring::read(buf, k + 1, lane);  // a step that does not exist: stale bytes, not used
       if (left == 0) next_head();
       --left;
+      // The reference's stream: the block's words first, four chains at a time, while few registers are in use.  (Drawn where they are used,
+      // the chains ran almost one behind the other: 1 / 4 / 32 sequences 8.3 / 19.1 / 113 -> 7.6 / 17.5 / 103 us a launch.)
+      uint32_t words[16];
+      if (kDrawn) {
+        const MxRoundCtx rc = round_ctx_at<MODE>(rb, lin);
+        PhiloxWords0 words0;
+        words0.init(static_cast<uint32_t>(rc.counter), rc.wrap32 ? 0u : static_cast<uint32_t>(rc.counter >> 32), d.keys);
+#pragma unroll
+        for (int i = 0; i < 16; i += 4) words0.draw<4>(i, d.keys, words + i);
+#pragma unroll
+        for (int i = 0; i < 16; ++i) asm volatile("" : "+r"(words[i]));  // stay here
+      }
       float hv[16], sd[8];
       mx_decode_scaled(now.q, now.e, now.mic, dA, e_max, table, hv, sd);
       float y = mx_update_readout16<IO::kNibbles>(hv, dB, Cv, sd, xp[k * rows_per_step]);  // h' = h exp(A dt) + (B dt) x
       MxRoundCtx ctx = round_ctx_at<MODE>(rb, lin);
       if (kStream) ctx.stream = &stream;
+      if (kDrawn) ctx.drawn = words;
       uint32_t codes[4], e_new, mic_new;
       mx_encode_block<BITS, MODE, IO::kNibbles>(hv, ctx, d.keys, codes, e_new, mic_new);
       IO::store_ptr(qptr + k * Ring::kQ, eptr + k * Ring::kE, mptr + k * Ring::kM, codes, e_new, mic_new);
@@ -927,7 +943,9 @@ static void launch_update_mode(const lq_mx_update_args& a, const MxUpdateDerived
     switch (a.rounding.mode) {
       case LQ_ROUND_HALF_UP: LQ_FAST_LAUNCH(LQ_ROUND_HALF_UP); break;
       case LQ_ROUND_HALF_EVEN: LQ_FAST_LAUNCH(LQ_ROUND_HALF_EVEN); break;
-      case LQ_ROUND_PHILOX_REF: LQ_FAST_LAUNCH(LQ_ROUND_PHILOX_REF); break;
+      case LQ_ROUND_PHILOX_REF:  // the state's size, by which a step counter moves the offset, is a multiple of 16
+        if (a.rounding.rng_offset % 16 == 0) LQ_FAST_LAUNCH(LQ_ROUND_PHILOX_REF); else LQ_FAST_LAUNCH(kRefAnyOffset);
+        break;
       case LQ_ROUND_SUPPLIED: LQ_FAST_LAUNCH(LQ_ROUND_SUPPLIED); break;
       case LQ_ROUND_PHILOX_LAYERED: LQ_FAST_LAUNCH(LQ_ROUND_PHILOX_LAYERED); break;
       case LQ_ROUND_PHILOX_LAYERED4: LQ_FAST_LAUNCH(LQ_ROUND_PHILOX_LAYERED4); break;

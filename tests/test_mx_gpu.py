@@ -465,3 +465,24 @@ def test_dense_quantiser_equals_strided(bits, layout, rows, dtype):
         caches.append(cache)
     a, c = caches
     assert torch.equal(a.q_state, c.q_state) and torch.equal(a.shared_exp, c.shared_exp) and torch.equal(a.micro_exp, c.micro_exp)
+
+
+@pytest.mark.parametrize("bits", [8, 4])
+@pytest.mark.parametrize("offset", [0, 5, 2**32 - 64, 2**32 - 7, 2**32 + 3, 2**33 - 64, 2**33 - 40, 2**63 + 16])
+def test_reference_stream_offsets_equal_general_kernel(bits, offset):
+    """The slab kernel draws a block's 16 words together where the offset is a multiple of 16 and one by one where it is not; counters that pass
+    2**32 between blocks and inside one, modulo 2**32 (offset below it) and as 64 bits.  The general kernel draws every word by itself."""
+    import ctypes
+    from layer_quant_b200 import _lib
+    m = mk()
+    d = make_update_case(41, 2, 4, 16, 128, 2)
+    x, dt, A, B, C, D, _, bias = expand_update_operands(d)
+    res = []
+    for h_out in (None, torch.empty((2, 4, 16, 128), dtype=torch.float32, device=dev())):
+        cache = m.allocate_state_kernel_cache(t(d["state"]), 16, bits)
+        plan = m.MxUpdatePlan(cache, x, dt, A, B, C, D=D, dt_bias=bias, stochastic=True, seed=77, rng_stream="reference", h_out=h_out)
+        plan.args.rounding.rng_offset = offset
+        _lib.launch(plan.device, _lib.lib().lq_mx_state_update, ctypes.byref(plan.args))
+        res.append((plan.out, cache.q_state, cache.shared_exp, cache.micro_exp))
+    for got, want in zip(*res):
+        assert torch.equal(got, want)
