@@ -626,3 +626,30 @@ def test_prefill_token_factors(gs, ratio, tq, first):
     assert torch.equal(out[4:], out[:1].expand(b - 4, -1, -1, -1))  # the others are sequence 0 once more
     from layer_quant_b200 import _lib
     assert _lib.device_status() == 0
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("gs", [32, 64, 128])
+@pytest.mark.parametrize("tq,offset", [(1, 0), (31, 0), (33, 4), (5, 12)])
+def test_append_vector_path_rows_and_alignment(gs, tq, offset, dtype):
+    """A CTA takes 32 rows and a thread sixteen values: row counts around that, and code rows that start on 4 bytes but not on 8 (two stores in
+    place of one).  The same values through strided rows take the general kernel."""
+    m = ia()
+    gen = torch.Generator(device=dev()).manual_seed(tq)
+    b, hkv, cap = 1, 3, 64
+    k, v = (torch.randn(b, hkv, tq, 128, generator=gen, device=dev()).to(dtype) for _ in range(2))
+    pos = torch.randperm(cap, generator=gen, device=dev())[:tq]
+    caches = []
+    for shift in (offset, 0):
+        cache = m._allocate_layer_cache(b, hkv, cap, 128, 128 // gs, dev())
+        for name in ("k_packed", "v_packed"):
+            raw = torch.zeros(b * hkv * cap * 64 + 16, dtype=torch.uint8, device=dev())
+            setattr(cache, name, raw[shift:shift + b * hkv * cap * 64].view(b, hkv, cap, 64))
+        for x in (cache.k_scale, cache.v_scale):
+            x.zero_()
+        caches.append(cache)
+    wide = [torch.empty(b, hkv, tq, 256, dtype=dtype, device=dev())[..., ::2].copy_(x) for x in (k, v)]
+    m._pack_kv_into_cache(caches[0], k, v, pos, gs)
+    m._pack_kv_into_cache(caches[1], *wide, pos, gs)
+    for name in ("k_packed", "v_packed", "k_scale", "v_scale"):
+        assert torch.equal(getattr(caches[0], name), getattr(caches[1], name)), name
