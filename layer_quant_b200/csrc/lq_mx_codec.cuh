@@ -62,12 +62,16 @@ __device__ __forceinline__ float set_gt(float a, float b) {
   return r;
 }
 
-// Byte 1 of four words -> one word (byte k from word k): three byte-permutes.
-__device__ __forceinline__ uint32_t gather_byte1(uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
-  const uint32_t ab = __byte_perm(a, b, 0x0051);  // [a.1, b.1, a.0, a.0]
-  const uint32_t cd = __byte_perm(c, d, 0x0051);
+// Byte BYTE (0 or 1) of four words -> one word (byte k from word k): three byte-permutes.
+template <int BYTE>
+__device__ __forceinline__ uint32_t gather_byte(uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+  const uint32_t ab = __byte_perm(a, b, BYTE ? 0x0051 : 0x0040);  // [a.BYTE, b.BYTE, ...]
+  const uint32_t cd = __byte_perm(c, d, BYTE ? 0x0051 : 0x0040);
   return __byte_perm(ab, cd, 0x5410);             // [ab.0, ab.1, cd.0, cd.1]
 }
+
+// floor(a) for 0 <= a < 2^22 by two additions: the rounding instruction has an eighth of their rate
+__device__ __forceinline__ float floor_small(float a) { return __fadd_rd(a, 8388608.0f) - 8388608.0f; }
 
 constexpr float kByteMagic = 49152.0f;  // 1.5 * 2^15: ulp 2^-8, mantissa bits 8..15 = integer part mod 256
 
@@ -136,7 +140,7 @@ __device__ __forceinline__ void mx_encode_block(const float (&h)[16], const MxRo
   }
 
   float macc = 0.0f;  // sum of 2^j over pairs with the micro-exponent set (exact)
-  uint32_t tb[16];    // bit patterns whose byte 1 is the code
+  uint32_t tb[16];    // bit patterns whose byte 1 (HALF_EVEN: byte 0) is the code
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
     const float micf = set_gt(pa[j], thresh);
@@ -162,35 +166,37 @@ __device__ __forceinline__ void mx_encode_block(const float (&h)[16], const MxRo
       float t;
       {
         const float a = fminf(fabsf(h[i]) * inv, M);
-        float lvl;
-        if (MODE == LQ_ROUND_HALF_UP) {
-          lvl = floorf(a + 0.5f);
-        } else if (MODE == LQ_ROUND_HALF_EVEN) {
-          lvl = rintf(a);
+        if (MODE == LQ_ROUND_HALF_EVEN) {  // rounded by the addition itself; byte 0 = two's complement of the signed level
+          t = copysignf(a, h[i]) + 12582912.0f;
         } else {
-          uint32_t w;
-          if (MODE == LQ_ROUND_SUPPLIED || MODE == LQ_ROUND_PHILOX_LAYERED4) {
-            w = rnd[i];
-          } else {  // the reference's stream: one Philox block per value, word 0
-            const uint64_t c = ctx.counter + i;
-            w = ctx.drawn ? ctx.drawn[i] : philox4x32_10(static_cast<uint32_t>(c), ctx.wrap32 ? 0u : static_cast<uint32_t>(c >> 32), 0u, 0u, keys).w0;
+          float lvl;  // never above M: a is not, and only what is below its next integer is raised to it
+          if (MODE == LQ_ROUND_HALF_UP) {
+            lvl = floor_small(a + 0.5f);
+          } else {
+            uint32_t w;
+            if (MODE == LQ_ROUND_SUPPLIED || MODE == LQ_ROUND_PHILOX_LAYERED4) {
+              w = rnd[i];
+            } else {  // the reference's stream: one Philox block per value, word 0
+              const uint64_t c = ctx.counter + i;
+              w = ctx.drawn ? ctx.drawn[i] : philox4x32_10(static_cast<uint32_t>(c), ctx.wrap32 ? 0u : static_cast<uint32_t>(c >> 32), 0u, 0u, keys).w0;
+            }
+            const float fl = floor_small(a);
+            lvl = fl + set_gt(a - fl, word_to_uniform(w));  // (u < a - fl) ? 1 : 0
           }
-          const float fl = floorf(a);
-          lvl = fl + set_gt(a - fl, word_to_uniform(w));  // (u < a - fl) ? 1 : 0
+          t = copysignf(lvl, h[i]) + kByteMagic;  // exact; byte 1 = two's complement of the signed level
         }
-        lvl = fminf(lvl, M);
-        t = copysignf(lvl, h[i]) + kByteMagic;  // exact; byte 1 = two's complement of the signed level
       }
       tb[i] = __float_as_uint(t);
     }
   }
+  constexpr int kByte = MODE == LQ_ROUND_HALF_EVEN ? 0 : 1;
 #pragma unroll
   for (int w = 0; w < 4; ++w) {
     if (!PACKED_NIBBLES) {
-      codes[w] = gather_byte1(tb[4 * w], tb[4 * w + 1], tb[4 * w + 2], tb[4 * w + 3]);
+      codes[w] = gather_byte<kByte>(tb[4 * w], tb[4 * w + 1], tb[4 * w + 2], tb[4 * w + 3]);
     } else if (w < 2) {  // even values to the low nibbles, odd ones to the high
-      const uint32_t ev = gather_byte1(tb[8 * w], tb[8 * w + 2], tb[8 * w + 4], tb[8 * w + 6]);
-      const uint32_t od = gather_byte1(tb[8 * w + 1], tb[8 * w + 3], tb[8 * w + 5], tb[8 * w + 7]);
+      const uint32_t ev = gather_byte<kByte>(tb[8 * w], tb[8 * w + 2], tb[8 * w + 4], tb[8 * w + 6]);
+      const uint32_t od = gather_byte<kByte>(tb[8 * w + 1], tb[8 * w + 3], tb[8 * w + 5], tb[8 * w + 7]);
       codes[w] = (ev & 0x0F0F0F0Fu) | ((od << 4) & 0xF0F0F0F0u);
     }
   }
