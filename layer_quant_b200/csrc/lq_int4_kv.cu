@@ -307,6 +307,7 @@ struct DecodeParams {
   int32_t splits;          // >= 1
   int32_t tiles_per_split;
   int32_t ctx_len;         // tokens read from the cache ring: seq_len, minus the fused new token
+  int32_t dependent = 0;   // launched as a programmatic dependent
   int32_t* counters;       // [B * Hkv] tickets (workspace)
   float* part_ml;          // [B * Hq * splits * 2]
   float* part_acc;         // [B * Hq * splits * 128]
@@ -771,6 +772,17 @@ static int pick_splits(int batch, int kv_heads, int ctx_len) {
     }                                                                                                               \
   } while (0)
 
+// Whether a launch is a programmatic dependent.  One hides launch, set-up and the way to the first tiles (2 us of a launch of 8 to 10), but is
+// placed around its predecessor's CTAs, several to the SMs that have room, and then takes as long as the fullest SM (16 x 8191, one split: 94 instead of
+// 50 us).  So: CTAs for which the predecessor leaves an SM each, and short ones, whose time is memory round trips whatever their SM holds.  us of four
+// launches of the same size, ordinary -> dependent, at tiles per CTA x CTAs: 5 x 8 33.2 -> 25.0, 8 x 64 41.0 -> 31.4, 16 x 64 49.4 -> 41.5, 8 x 96 41.2 -> 37.3;
+// 1 x 128 41.3 -> 34.8, 3 x 128 33.1 -> 27.0, but 4 x 128 41.4 -> 42.1 and 5 x 128 33.2 -> 35.0; 5 x 192 41.3 -> 35.2, 5 x 512 74.2 -> 67.1, 4 x 1600
+// 140 -> 128, but 7 x 192 41.5 -> 41.4 and 14 x 288 78.0 -> 81.9.
+static bool dependent_pays(int tiles, int64_t ctas) {
+  const int sms = sm_count();
+  return tiles <= (3 * ctas <= 2 * sms ? 16 : ctas <= sms ? 3 : 5);
+}
+
 template <int R, int GS>
 static int launch_decode(const DecodeParams& p, cudaStream_t st) {
   using L = StageLayout<GS>;
@@ -788,16 +800,17 @@ static int launch_decode(const DecodeParams& p, cudaStream_t st) {
 }
 
 template <int R, int GS>
-static int launch_decode_mma(const DecodeParams& p, cudaStream_t st) {
+static int launch_decode_mma(DecodeParams p, cudaStream_t st) {
   constexpr size_t smem = mma::WarpStage<GS>::kSmem;
   const dim3 grid(p.splits, p.a.cache.kv_heads, p.a.cache.batch);
 #define LQ_MMA_LAUNCH(MASK_, QM_)                                                                                   \
   do {                                                                                                              \
     LQ_SET_SMEM_ONCE((mma::int4_decode_warp_kernel<R, GS, MASK_, QM_>), smem);                                      \
-    mma::int4_decode_warp_kernel<R, GS, MASK_, QM_><<<grid, mma::kThreadsM, smem, st>>>(p);                    \
+    if (p.dependent) LQ_CHECK_CUDA(launch_dependent(mma::int4_decode_warp_kernel<R, GS, MASK_, QM_>, grid, mma::kThreadsM, smem, st, p)); \
+    else mma::int4_decode_warp_kernel<R, GS, MASK_, QM_><<<grid, mma::kThreadsM, smem, st>>>(p);                    \
   } while (0)
-  // Not a programmatic dependent launch: its CTAs would be placed around the predecessor's, several to the SMs that have room, and
-  // the launch would take as long as the fullest SM (16 x 8191, one split: 94 instead of 50 us).
+  // (with a device counter the tiles are not known here)
+  p.dependent = p.a.seq_len_counter == nullptr && dependent_pays(p.tiles_per_split, static_cast<int64_t>(grid.x) * grid.y * grid.z);
   if (p.a.mask) {
     if (p.a.dtype == LQ_BF16) LQ_MMA_LAUNCH(true, mma::kQBf16); else if (p.a.dtype == LQ_F16) LQ_MMA_LAUNCH(true, mma::kQF16); else LQ_MMA_LAUNCH(true, mma::kQF32);
   } else {

@@ -653,3 +653,30 @@ def test_append_vector_path_rows_and_alignment(gs, tq, offset, dtype):
     m._pack_kv_into_cache(caches[1], *wide, pos, gs)
     for name in ("k_packed", "v_packed", "k_scale", "v_scale"):
         assert torch.equal(getattr(caches[0], name), getattr(caches[1], name)), name
+
+
+@pytest.mark.parametrize("batch,start,splits", [(1, 70, 1), (1, 1000, 16), (9, 250, 1), (16, 120, 1), (16, 300, 1), (40, 190, 1), (40, 500, 3)])
+def test_decode_launches_follow_one_another(batch, start, splits):
+    """Launches with few or short CTAs are programmatic dependents, others are not; each appends a row that the next one attends to and shares the
+    scratch of the split merge.  A row of launches must equal the same launches waited for one by one."""
+    m = ia()
+    hkv, gs, steps = 8, 32, 12
+    k, v = make_kv(101, 1, hkv, start)
+    gen = torch.Generator(device=dev()).manual_seed(start)
+    rows = [[torch.randn(batch, h, 1, 128, generator=gen, device=dev()).to(torch.bfloat16) for h in (4 * hkv, hkv, hkv)] for _ in range(steps)]
+    res = []
+    for wait in (True, False):
+        cache = fill_cache(m, np.repeat(k, batch, 0), np.repeat(v, batch, 0), gs, capacity=start + steps)
+        plans = [m.Int4DecodePlan(q, cache, start + i + 1, gs, k_new=kn, v_new=vn, splits=splits) for i, (q, kn, vn) in enumerate(rows)]
+        outs = []
+        for plan in plans:
+            outs.append(plan.launch())
+            if wait:
+                torch.cuda.synchronize()
+        res.append((outs, cache))
+    for a, b in zip(res[0][0], res[1][0]):
+        assert torch.equal(a, b)
+    for name in ("k_packed", "v_packed", "k_scale", "v_scale"):
+        assert torch.equal(getattr(res[0][1], name), getattr(res[1][1], name)), name
+    from layer_quant_b200 import _lib
+    assert _lib.device_status() == 0
