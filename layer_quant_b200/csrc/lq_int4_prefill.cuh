@@ -14,8 +14,7 @@
 // the same way: 2^-22 of a weight or 2^-35 of the row's largest, whichever is more.  (The mma.sync kernel keeps 2^-17 of every
 // weight.  The absolute part adds up to less than that over 2^17 tokens.)  Q is exact in fp16 for 16-bit queries.
 // S = Q Khi + Q Klo, O = Phi Vhi + Plo Vhi + Phi Vlo: five products per tile pair, all in fp32 accumulators.
-// Token factors (LEAD, the dims of the first group, 64 or 128): where all of a CTA's SM is busy a group's scale is worth more outside the products.
-// The mantissa of a token's first scale goes to the softmax, which multiplies the scores (K) and the weights after their sum is taken (V) by it in
+// Token factors (LEAD, the dims of the first group, 64 or 128; 0: none): the mantissa of a token's first scale goes to the softmax, which multiplies the scores (K) and the weights after their sum is taken (V) by it in
 // fp32; the first group's operands are then a code times a power of two, exact in fp16, and need no lo part, the other groups' scales are divided by
 // it.  Groups of 64: four products per tile pair in place of five, of 128: three.  The error against 64 bits goes down with the lo parts: outputs that are
 // not the correctly rounded fp16 value 1.1 % -> 0.8 % (groups of 64) and 0.27 % (128) of 2 x 700 tokens.

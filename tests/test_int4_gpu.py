@@ -595,15 +595,14 @@ def test_prefill_huge_scores(size):
     assert_out_close(m._prefill_attention(t(q, torch.bfloat16), cache, 4, gs), ref)
 
 
-@pytest.mark.parametrize("gs", [64, 128])
-@pytest.mark.parametrize("ratio,tq,first", [(4, 3, 1), (4, 65, 1), (8, 19, 40), (2, 129, 63)])
+@pytest.mark.parametrize("gs,ratio,tq,first", [(128, 4, 3, 1), (128, 4, 65, 1), (128, 8, 19, 40), (128, 2, 129, 63), (64, 4, 2, 2000), (64, 4, 65, 2000)])
 def test_prefill_token_factors(gs, ratio, tq, first):
-    """More than half as many row blocks as SMs and groups of 64 or 128: the kernel that keeps the first group's operands exact and multiplies by the
-    token's factor.  Sequence 0 as it comes, 1 and 2 with a first group far below and far above the others, 3 with a huge key and an infinite
+    """The kernel that keeps the first group's operands exact and multiplies by the token's factor: groups of 128, and of 64 in launches that keep every SM
+    busy for long.  Sequence 0 as it comes, 1 and 2 with a first group far below and far above the others, 3 with a huge key and an infinite
     value in the last token, which the rows before it must not notice."""
     m = ia()
     hkv, total = 2, first + tq - 1
-    b = 40 + torch.cuda.get_device_properties(0).multi_processor_count // (4 * -(-tq * ratio // 256))
+    b = 5 if gs == 128 else torch.cuda.get_device_properties(0).multi_processor_count // -(-tq * ratio // 256) + 1
     k, v = (np.repeat(x, b, 0) for x in make_kv(91 + tq, 1, hkv, total))
     for x in (k, v):
         x[1, ..., :64] *= 2.0 ** -9
