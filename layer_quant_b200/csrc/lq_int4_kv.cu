@@ -1028,7 +1028,9 @@ static int launch_prefill_tc(const lq_int4_prefill_args& a, int ratio, cudaStrea
   const auto launch = [&](auto lead) -> int {
     constexpr int LEAD = decltype(lead)::value;
     LQ_SET_SMEM_ONCE(prefill::int4_prefill_kernel<LEAD>, prefill::kSmemBytes);
-    prefill::int4_prefill_kernel<LEAD><<<static_cast<unsigned>(std::min(p.entries, sms)), prefill::kThreads, prefill::kSmemBytes, st>>>(p);
+    // Dependent: its CTAs take all registers of an SM, so they cannot crowd, and launch, barriers and tensor memory are ready when the packing ends.
+    // With it, packing and attention: 1 x 24 tokens 13.0 -> 9.6 us, 1 x 100 14.9 -> 11.7, 2 x 300 24.5 -> 21.8, 16 x 256 56.1 -> 53.
+    LQ_CHECK_CUDA(launch_dependent(prefill::int4_prefill_kernel<LEAD>, static_cast<unsigned>(std::min(p.entries, sms)), prefill::kThreads, prefill::kSmemBytes, st, p));
     LQ_CHECK_CUDA(cudaGetLastError());
     return LQ_OK;
   };

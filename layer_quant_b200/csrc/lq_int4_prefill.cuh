@@ -793,6 +793,7 @@ template <int LEAD>
 __global__ void __launch_bounds__(kThreads, 1) int4_prefill_kernel(const __grid_constant__ Params p) {
   extern __shared__ uint8_t smem_raw[];
   __shared__ Shared sh;
+  pdl_launch_dependents();
   uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
   const int warp = threadIdx.x >> 5;
   if (warp == 12) {
@@ -817,6 +818,7 @@ __global__ void __launch_bounds__(kThreads, 1) int4_prefill_kernel(const __grid_
   fence_before();
   __syncthreads();
   fence_after();
+  pdl_wait();  // nothing above reads memory; below, what the predecessor has written (the packed rows as a rule) is read
   if (warp >= 8) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 88;");
     if (warp < 12) unpack_tiles<LEAD>(p, sh, smem);
