@@ -1037,7 +1037,8 @@ static int launch_prefill_tc(const lq_int4_prefill_args& a, int ratio, cudaStrea
   // Token factors save products and lo parts, for which they cost the softmax some 100 instructions per thread and tile.  Groups of 128 lose two products
   // of five: always (us without -> with: 1 x 1000 tokens 45.8 -> 41.7, 2 x 500 behind 3000 129.9 -> 111.2, 1 x 128 behind 4000 117.8 -> 105.3).  Groups of 64
   // lose one, which only pays where the products draw the board's full power, with every SM busy for long (2 x 2000 behind 6001 949 -> 875 us
-  // in a row of launches, 1 x 3000 167 -> 153; but 1 x 1000 45.9 -> 47.9, 2 x 500 behind 3000 129.9 -> 136.8, 1 x 2000 83.1 -> 85.6).  In groups
+  // in a row of launches, 1 x 3000 167 -> 153, though six launches on a cool board 864 -> 907;
+  // but 1 x 1000 45.9 -> 47.9, 2 x 500 behind 3000 129.9 -> 136.8, 1 x 2000 83.1 -> 85.6).  In groups
   // of 32 a quarter of the dims would lead, and the tensor core takes N in steps that save nothing there.
   const bool full_power = blocks >= 2 * sms && blocks * (a.first_len + a.q_len / 2) / prefill::kTok >= 60ll * sms;
   if (a.cache.group_size == 64 && full_power) return launch(std::integral_constant<int, 64>{});
