@@ -1025,25 +1025,19 @@ static int launch_prefill_tc(const lq_int4_prefill_args& a, int ratio, cudaStrea
   const int sms = sm_count(), rest = static_cast<int>(blocks % sms);
   p.whole = static_cast<int>(blocks) - (2 * rest <= sms ? rest : 0);
   p.entries = p.whole + 2 * (static_cast<int>(blocks) - p.whole);
-  const auto launch = [&](auto lead) -> int {
-    constexpr int LEAD = decltype(lead)::value;
-    LQ_SET_SMEM_ONCE(prefill::int4_prefill_kernel<LEAD>, prefill::kSmemBytes);
+  const auto launch = [&](auto factors) -> int {
+    constexpr bool FACTORS = decltype(factors)::value;
+    LQ_SET_SMEM_ONCE(prefill::int4_prefill_kernel<FACTORS>, prefill::kSmemBytes);
     // Dependent: its CTAs take all registers of an SM, so they cannot crowd, and launch, barriers and tensor memory are ready when the packing ends.
     // With it, packing and attention: 1 x 24 tokens 13.0 -> 9.6 us, 1 x 100 14.9 -> 11.7, 2 x 300 24.5 -> 21.8, 16 x 256 56.1 -> 53.
-    LQ_CHECK_CUDA(launch_dependent(prefill::int4_prefill_kernel<LEAD>, static_cast<unsigned>(std::min(p.entries, sms)), prefill::kThreads, prefill::kSmemBytes, st, p));
+    LQ_CHECK_CUDA(launch_dependent(prefill::int4_prefill_kernel<FACTORS>, static_cast<unsigned>(std::min(p.entries, sms)), prefill::kThreads, prefill::kSmemBytes, st, p));
     LQ_CHECK_CUDA(cudaGetLastError());
     return LQ_OK;
   };
   // Token factors save products and lo parts, for which they cost the softmax some 100 instructions per thread and tile.  Groups of 128 lose two products
-  // of five: always (us without -> with: 1 x 1000 tokens 45.8 -> 41.7, 2 x 500 behind 3000 129.9 -> 111.2, 1 x 128 behind 4000 117.8 -> 105.3).  Groups of 64
-  // lose one, which only pays where the products draw the board's full power, with every SM busy for long (2 x 2000 behind 6001 949 -> 875 us
-  // in a row of launches, 1 x 3000 167 -> 153, though six launches on a cool board 864 -> 907;
-  // but 1 x 1000 45.9 -> 47.9, 2 x 500 behind 3000 129.9 -> 136.8, 1 x 2000 83.1 -> 85.6).  In groups
-  // of 32 a quarter of the dims would lead, and the tensor core takes N in steps that save nothing there.
-  const bool full_power = blocks >= 2 * sms && blocks * (a.first_len + a.q_len / 2) / prefill::kTok >= 60ll * sms;
-  if (a.cache.group_size == 64 && full_power) return launch(std::integral_constant<int, 64>{});
-  if (a.cache.group_size == 128) return launch(std::integral_constant<int, 128>{});
-  return launch(std::integral_constant<int, 0>{});
+  // of five (us without -> with: 1 x 1000 tokens 45.8 -> 41.7, 2 x 500 behind 3000 129.9 -> 111.2, 1 x 128 behind 4000 117.8 -> 105.3).  The group size
+  // alone decides: a sequence's bits do not depend on what shares its launch.
+  return a.cache.group_size == 128 ? launch(std::true_type{}) : launch(std::false_type{});
 }
 
 LQ_EXPORT int lq_int4_prefill_attn(const lq_int4_prefill_args* args, void* cuda_stream) {

@@ -14,10 +14,11 @@
 // the same way: 2^-22 of a weight or 2^-35 of the row's largest, whichever is more.  (The mma.sync kernel keeps 2^-17 of every
 // weight.  The absolute part adds up to less than that over 2^17 tokens.)  Q is exact in fp16 for 16-bit queries.
 // S = Q Khi + Q Klo, O = Phi Vhi + Plo Vhi + Phi Vlo: five products per tile pair, all in fp32 accumulators.
-// Token factors (LEAD, the dims of the first group, 64 or 128; 0: none): the mantissa of a token's first scale goes to the softmax, which multiplies the scores (K) and the weights after their sum is taken (V) by it in
-// fp32; the first group's operands are then a code times a power of two, exact in fp16, and need no lo part, the other groups' scales are divided by
-// it.  Groups of 64: four products per tile pair in place of five, of 128: three.  The error against 64 bits goes down with the lo parts: outputs that are
-// not the correctly rounded fp16 value 1.1 % -> 0.8 % (groups of 64) and 0.27 % (128) of 2 x 700 tokens.
+// Token factors (FACTORS, groups of 128, where a token has one scale): the mantissa of the scale goes to the softmax, which multiplies the scores (K) and
+// the weights after their sum is taken (V) by it in fp32; the operands are then a code times a power of two, exact in fp16, and need no lo part: three
+// products per tile pair in place of five.  The error against 64 bits goes down with the lo parts: outputs that are
+// not the correctly rounded fp16 value 1.1 % -> 0.27 % of 2 x 700 tokens.  (Groups of 64 could leave out one product of five, Phi Vlo and Q Klo of the first group.
+// Dropped: it pays only in rows of long launches, and a rule on the launch's size made a sequence's bits depend on what shares its launch.)
 // Range.  Powers of two are taken out of every row of Q and of the K and V scales of every 16 tokens, so the
 // fp16 operands sit at the top of their range; the exponents come back for free, in the factor and the offset of the
 // exp2 argument.  With p' = 2^(s + Ev - m) the V exponent Ev is part of the running maximum m.
@@ -57,8 +58,8 @@ constexpr float kScaleFloor = 1.0e-8f;        // of the codec
 // against 977 for 2 x 2000 tokens behind 6001.
 // With token factors (below 2) on the weights the slack is a quarter less: 2^15.75.
 constexpr float kLift = 11.0f;
-template <int LEAD>
-constexpr float kSlack = LEAD ? 3.75f : 4.0f;
+template <bool FACTORS>
+constexpr float kSlack = FACTORS ? 3.75f : 4.0f;
 // A score and the maximum part in one FMA, so the rounding of the maximum is in the difference; beyond scores of 2^24 that would
 // overflow P.  Queries below kLargeQ and K scales below kLargeK (values below 8 kLargeK) keep scores below 2^21.3; larger ones are rounded
 // before the difference is taken, in the pass that wide tiles take.
@@ -170,7 +171,6 @@ __device__ __forceinline__ void mma_commit(uint64_t* bar) {
 // fp16 inputs, fp32 accumulators, M = 128; K tile: N = 64 tokens, dims contiguous; V tile: N = 128 dims, dims contiguous (N-major)
 constexpr uint32_t kIdescS = (1u << 4) | ((64u / 8) << 17) | ((128u / 16) << 24);
 constexpr uint32_t kIdescO = (1u << 4) | (1u << 16) | ((128u / 8) << 17) | ((128u / 16) << 24);
-constexpr uint32_t kIdescO64 = (1u << 4) | (1u << 16) | ((64u / 8) << 17) | ((128u / 16) << 24);
 // Shared-memory matrix descriptor, 128-byte swizzle.  Stride offset 1024: the next eight rows of 128 bytes; lbo: the next
 // 64 dims of an N-major tile.
 __device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo) {
@@ -270,14 +270,14 @@ __device__ __forceinline__ Exponents exponents_of(float (&sc)[2]) {
   return r;
 }
 
-// The token factor of a scale (its exponent taken out) of the leading group: its mantissa, so that the rest is a power of two
+// The token factor of a scale (its exponent taken out): its mantissa, so that the rest is a power of two
 __device__ __forceinline__ float lead_of(float s) {
   const uint32_t b = __float_as_uint(s);
   return b < 0x00800000u ? 1.0f : __uint_as_float((b & 0x007FFFFFu) | 0x3F800000u);
 }
 // 32 dims of one token -> shared memory: 64 bytes of the hi part and, unless s is a power of two, of the lo part
 template <bool LO>
-__device__ __forceinline__ void store_chunk(uint8_t* part_hi, int token, int chunk, const uint4& raw, float s, bool lo_too) {
+__device__ __forceinline__ void store_chunk(uint8_t* part_hi, int token, int chunk, const uint4& raw, float s) {
   const __half2 hi = __float2half2_rn(__uint_as_float(__float_as_uint(s) & 0xFFFF0000u));
   const __half2 lo = __float2half2_rn(s - __low2float(hi));
   const uint32_t words[4] = {raw.x, raw.y, raw.z, raw.w};
@@ -295,11 +295,11 @@ __device__ __forceinline__ void store_chunk(uint8_t* part_hi, int token, int chu
     }
     uint8_t* dst = row + ((((chunk & 1) * 4 + w) ^ (token & 7)) << 4);
     *reinterpret_cast<uint4*>(dst) = make_uint4(h[0], h[1], h[2], h[3]);
-    if (LO && lo_too) *reinterpret_cast<uint4*>(dst + kPart) = make_uint4(l[0], l[1], l[2], l[3]);
+    if (LO) *reinterpret_cast<uint4*>(dst + kPart) = make_uint4(l[0], l[1], l[2], l[3]);
   }
 }
 
-template <int LEAD>
+template <bool FACTORS>
 __device__ __forceinline__ void unpack_tiles(const Params& p, Shared& sh, uint8_t* smem) {
   const lq_int4_cache& c = p.a.cache;
   const int warp = (threadIdx.x >> 5) & 3, lane = threadIdx.x & 31;
@@ -370,16 +370,15 @@ __device__ __forceinline__ void unpack_tiles(const Params& p, Shared& sh, uint8_
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
       sc[i] *= pow2_of(-e[i]);
-      if (LEAD) {
-        const float f = lead_of(__shfl_sync(0xFFFFFFFFu, sc[i], lane & 7));
-        sc[i] = chunk < LEAD / 32 ? __uint_as_float(__float_as_uint(sc[i]) & 0x7F800000u) : __fdividef(sc[i], f);
-        if (chunk == 0) lead[row + 8 * i] = f;
+      if (FACTORS) {
+        if (chunk == 0) lead[row + 8 * i] = lead_of(sc[i]);
+        sc[i] = __uint_as_float(__float_as_uint(sc[i]) & 0x7F800000u);
       }
     }
   };
   auto store = [&](int stage, const uint4 (&raw)[2], const float (&s)[2]) {
 #pragma unroll
-    for (int i = 0; i < 2; ++i) store_chunk<LEAD != 128>(smem + stage * kStageBytes, row + 8 * i, chunk, raw[i], s[i], chunk >= LEAD / 32);
+    for (int i = 0; i < 2; ++i) store_chunk<!FACTORS>(smem + stage * kStageBytes, row + 8 * i, chunk, raw[i], s[i]);
   };
   auto arrive = [&](uint64_t* bar) {
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -437,17 +436,17 @@ __device__ __forceinline__ void unpack_tiles(const Params& p, Shared& sh, uint8_
 }
 
 // ---- products --------------------------------------------------------------------------------------------------------
-template <int LEAD>
+template <bool FACTORS>
 __device__ __forceinline__ void issue_products(const Params& p, Shared& sh, uint8_t* smem) {
   const uint64_t k_desc = smem_desc(smem_u32(smem), 16), v_desc = smem_desc(smem_u32(smem) + 2 * kStageBytes, kPart / 2);
-  // S = Q Khi + Q Klo; 16 dims per product: 32 bytes inside a half of 64 dims.  The leading dims have no lo part
+  // S = Q Khi + Q Klo; 16 dims per product: 32 bytes inside a half of 64 dims.  With token factors there is no lo part
   auto issue_s = [&](int g, int j) {
     const uint32_t tm = g * kColsPerGroup;
     const uint64_t d = k_desc + (j & 1) * (kStageBytes >> 4);
 #pragma unroll
-    for (int hl = 0; hl < 2; ++hl)
+    for (int hl = 0; hl < (FACTORS ? 1 : 2); ++hl)
 #pragma unroll
-      for (int k = hl ? LEAD / 16 : 0; k < 8; ++k)
+      for (int k = 0; k < 8; ++k)
         mma_ts(tm + kColS, tm + kColQ + 8 * k, d + ((hl * kPart + (k >> 2) * (kPart / 2) + (k & 3) * 32) >> 4), kIdescS, hl + k > 0);
   };
   // O += Phi Vhi + Plo Vhi + Phi Vlo; 16 tokens per product: 2048 bytes
@@ -455,14 +454,10 @@ __device__ __forceinline__ void issue_products(const Params& p, Shared& sh, uint
     const uint32_t tm = g * kColsPerGroup;
     const uint64_t d = v_desc + (j & 1) * (kStageBytes >> 4);
 #pragma unroll
-    for (int t = 0; t < 3; ++t)
+    for (int t = 0; t < (FACTORS ? 2 : 3); ++t)
 #pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        if (t < 2 || LEAD == 0)
-          mma_ts(tm + kColO, tm + kColS + (t == 1 ? 32 : 0) + 8 * k, d + (((t == 2 ? kPart : 0) + k * 2048) >> 4), kIdescO, !first || t + k > 0);
-        else if (LEAD == 64)  // the upper 64 dims
-          mma_ts(tm + kColO + 64, tm + kColS + 8 * k, d + ((kPart + kPart / 2 + k * 2048) >> 4), kIdescO64, true);
-      }
+      for (int k = 0; k < 4; ++k)
+        mma_ts(tm + kColO, tm + kColS + (t == 1 ? 32 : 0) + 8 * k, d + (((t == 2 ? kPart : 0) + k * 2048) >> 4), kIdescO, !first || t + k > 0);
   };
   uint32_t p_parity = 0, q_parity = 0;  // bit g
   // S of a block's first tile, once the groups have put their query rows into TMEM
@@ -610,7 +605,7 @@ __device__ __forceinline__ void store_output(const lq_int4_prefill_args& a, int6
 // One row of scores of one block, a tile at a time: S -> P in place, running maximum and sum.  tile: the block's first, counted over
 // all blocks; parity: of the next wait for products of this group; l_run: the sum; bad: the 32-dim chunks for which the row has
 // attended to a V that is not finite.  False after a wait that ran out.
-template <int LEAD>
+template <bool FACTORS>
 __device__ __forceinline__ bool softmax_rows(const Params& p, Shared& sh, int pos0, int ntiles, int tile, uint32_t& parity, float cq, uint32_t large_q,
                                              float& l_run, uint32_t& bad) {
   const lq_int4_prefill_args& a = p.a;
@@ -632,7 +627,7 @@ __device__ __forceinline__ bool softmax_rows(const Params& p, Shared& sh, int po
     const uint32_t wide = sh.wide[f] | large_q;
     uint32_t s[64];
     tmem_load64(s, tm + kColS);
-    if (LEAD) {
+    if (FACTORS) {
 #pragma unroll
       for (int i = 0; i < 64; i += 4) {
         const float4 k = *reinterpret_cast<const float4*>(&sh.k_lead[f][i]);
@@ -653,7 +648,7 @@ __device__ __forceinline__ bool softmax_rows(const Params& p, Shared& sh, int po
           tmem_load16(raw, tm + kColS + 16 * w);
 #pragma unroll
           for (int i = 0; i < 16; ++i) {
-            raw[i] = __float_as_uint(fmaf(__uint_as_float(raw[i]) * (LEAD ? sh.k_lead[f][16 * w + i] : 1.0f), cq * kf[own ? i : 0], ve[own ? i : 0]));
+            raw[i] = __float_as_uint(fmaf(__uint_as_float(raw[i]) * (FACTORS ? sh.k_lead[f][16 * w + i] : 1.0f), cq * kf[own ? i : 0], ve[own ? i : 0]));
             if (own && tok0 + 16 * w + i < limit) bad |= sh.v_bad_tok[f][16 * w + i];
           }
           tmem_store16(tm + kColS + 16 * w, raw);
@@ -681,7 +676,7 @@ __device__ __forceinline__ bool softmax_rows(const Params& p, Shared& sh, int po
     if (j == 0) {
       m_run = m_tile;  // every row sees token 0
     }
-    if (__any_sync(0xFFFFFFFFu, m_tile > m_run + kSlack<LEAD> || wide != 0u)) {
+    if (__any_sync(0xFFFFFFFFu, m_tile > m_run + kSlack<FACTORS> || wide != 0u)) {
       if (j > 0) {
         // rare: the running sums of this warp's rows move to a larger maximum (the products into O of the tile before are done)
         const float m_new = fmaxf(m_run, m_tile), alpha = exp2f(m_run - m_new);
@@ -720,7 +715,7 @@ __device__ __forceinline__ bool softmax_rows(const Params& p, Shared& sh, int po
                                     make_float2(off, off));
         float2 pr = make_float2(mma::fast_exp2(x.x), mma::fast_exp2(x.y));
         sum = __fadd2_rn(sum, pr);
-        if (LEAD) pr = __fmul2_rn(pr, *reinterpret_cast<const float2*>(&sh.v_lead[f][16 * w + 2 * i]));
+        if (FACTORS) pr = __fmul2_rn(pr, *reinterpret_cast<const float2*>(&sh.v_lead[f][16 * w + 2 * i]));
         // leading 11 bits by truncation (exact in fp16 from 2^-14 on), the rest rounded to fp16
         const float2 top = make_float2(__uint_as_float(__float_as_uint(pr.x) & 0xFFFFE000u), __uint_as_float(__float_as_uint(pr.y) & 0xFFFFE000u));
         const float2 rest = __ffma2_rn(top, make_float2(-1.0f, -1.0f), pr);
@@ -739,7 +734,7 @@ __device__ __forceinline__ bool softmax_rows(const Params& p, Shared& sh, int po
   return true;
 }
 
-template <int LEAD>
+template <bool FACTORS>
 __device__ __forceinline__ void softmax_blocks(const Params& p, Shared& sh) {
   const lq_int4_prefill_args& a = p.a;
   const int group = threadIdx.x >> 7, warp = (threadIdx.x >> 5) & 3, lane = threadIdx.x & 31;
@@ -769,7 +764,7 @@ __device__ __forceinline__ void softmax_blocks(const Params& p, Shared& sh) {
   for (int r = 0; entry_of(r) < p.entries; ++r) {
     const Block k = block_at(p, entry_of(r));
     if (group < k.groups) {
-      if (!softmax_rows<LEAD>(p, sh, k.pos0, k.ntiles, tile, parity, cq, large_q, l_run, bad)) return;
+      if (!softmax_rows<FACTORS>(p, sh, k.pos0, k.ntiles, tile, parity, cq, large_q, l_run, bad)) return;
       const bool more = load_next(r + 1);  // all S of this block are done; its last products run meanwhile
       // the wait stands before the arrival that lets the next S be asked for: s_done is never two phases ahead of a warp
       if (!wait_bar(&sh.s_done[group], parity)) return;
@@ -789,7 +784,7 @@ __device__ __forceinline__ void softmax_blocks(const Params& p, Shared& sh) {
 // takes 2.05 us; as one CTA per block, start and end added 8 to 9 us to every block.  8 x 1024 tokens: 185 -> 160 us; 2 x 2000 behind 6001: 884 -> 855; 16 x 256: 53 -> 43; 1 x 128 behind 4000 (halves): 135 -> 110.
 // Dropped: two score buffers of 32 tokens per group, which would let the tensor pipe run ahead of the softmax (a product of 32 columns
 // takes as long as one of 64: 2.31 us a tile), and starting the products of a tile's first half while its second is made (2.1 us).
-template <int LEAD>
+template <bool FACTORS>
 __global__ void __launch_bounds__(kThreads, 1) int4_prefill_kernel(const __grid_constant__ Params p) {
   extern __shared__ uint8_t smem_raw[];
   __shared__ Shared sh;
@@ -821,11 +816,11 @@ __global__ void __launch_bounds__(kThreads, 1) int4_prefill_kernel(const __grid_
   pdl_wait();  // nothing above reads memory; below, what the predecessor has written (the packed rows as a rule) is read
   if (warp >= 8) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 88;");
-    if (warp < 12) unpack_tiles<LEAD>(p, sh, smem);
-    else if (warp == 12) issue_products<LEAD>(p, sh, smem);
+    if (warp < 12) unpack_tiles<FACTORS>(p, sh, smem);
+    else if (warp == 12) issue_products<FACTORS>(p, sh, smem);
   } else {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 168;");
-    softmax_blocks<LEAD>(p, sh);
+    softmax_blocks<FACTORS>(p, sh);
   }
   fence_before();
   __syncthreads();

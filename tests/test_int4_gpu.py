@@ -534,6 +534,28 @@ def test_prefill_work_list_equals_single_sequences(batch, tq, first):
     assert _lib.device_status() == 0
 
 
+@pytest.mark.parametrize("gs", [32, 64, 128])
+def test_prefill_bits_do_not_depend_on_the_size_of_the_launch(gs):
+    """More than two row blocks per SM behind a long context, 16-bit outputs fine enough to show another choice of products: each sequence
+    equals, bit for bit, a launch of its own."""
+    m = ia()
+    gen = torch.Generator(device=dev()).manual_seed(gs)
+    tq, first = 65, 2000
+    batch = torch.cuda.get_device_properties(0).multi_processor_count // 2 + 1  # four blocks a sequence
+    total = first + tq - 1
+    k, v = (torch.randn(batch, 2, total, 128, generator=gen, device=dev()).half() for _ in range(2))
+    q = torch.randn(batch, 8, tq, 128, generator=gen, device=dev()).half()
+    cache = m._allocate_layer_cache(batch, 2, 2080, 128, 128 // gs, dev())
+    m._pack_kv_into_cache(cache, k, v, torch.arange(total, device=dev()), gs)
+    out = m._prefill_attention(q, cache, 4, gs, first_len=first)
+    for b in range(0, batch, 9):
+        one = m._allocate_layer_cache(1, 2, 2080, 128, 128 // gs, dev())
+        m._pack_kv_into_cache(one, k[b:b + 1], v[b:b + 1], torch.arange(total, device=dev()), gs)
+        assert torch.equal(out[b:b + 1], m._prefill_attention(q[b:b + 1], one, 4, gs, first_len=first))
+    from layer_quant_b200 import _lib
+    assert _lib.device_status() == 0
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("delta", [9.3, 16.45, 20.4, 22.7, 24.4, 26.3])
 def test_prefill_keeps_small_weights(delta, dtype):
@@ -597,8 +619,7 @@ def test_prefill_huge_scores(size):
 
 @pytest.mark.parametrize("gs,ratio,tq,first", [(128, 4, 3, 1), (128, 4, 65, 1), (128, 8, 19, 40), (128, 2, 129, 63), (64, 4, 2, 2000), (64, 4, 65, 2000)])
 def test_prefill_token_factors(gs, ratio, tq, first):
-    """The kernel that keeps the first group's operands exact and multiplies by the token's factor: groups of 128, and of 64 in launches that keep every SM
-    busy for long.  Sequence 0 as it comes, 1 and 2 with a first group far below and far above the others, 3 with a huge key and an infinite
+    """Groups of 128 keep the operands exact and multiply by the token's factor; large launches with groups of 64 behind a long context.  Sequence 0 as it comes, 1 and 2 with a first group far below and far above the others, 3 with a huge key and an infinite
     value in the last token, which the rows before it must not notice."""
     m = ia()
     hkv, total = 2, first + tq - 1
