@@ -239,7 +239,7 @@ struct Exponents {
 };
 __device__ __forceinline__ Exponents exponents_of(float (&sc)[2]) {
   Exponents r;
-  const uint32_t b[2] = {__float_as_uint(sc[0]), __float_as_uint(sc[1])};  // scales are positive or zero
+  const uint32_t b[2] = {__float_as_uint(sc[0]), __float_as_uint(sc[1])};  // a negative scale counts as out of range here; its tokens are wide
   const uint32_t hi = __reduce_max_sync(0xFFFFFFFFu, max(b[0], b[1]));
   r.e[0] = r.e[1] = exponent_of(hi);
   r.bad[0] = r.bad[1] = 0u;
@@ -270,10 +270,11 @@ __device__ __forceinline__ Exponents exponents_of(float (&sc)[2]) {
   return r;
 }
 
-// The token factor of a scale (its exponent taken out): its mantissa, so that the rest is a power of two
+// The token factor of a scale (its exponent taken out): its mantissa, so that the rest is a power of two.  The sign stays with the power: the codec
+// writes positive scales, a caller's own cache may hold others
 __device__ __forceinline__ float lead_of(float s) {
   const uint32_t b = __float_as_uint(s);
-  return b < 0x00800000u ? 1.0f : __uint_as_float((b & 0x007FFFFFu) | 0x3F800000u);
+  return (b & 0x7FFFFFFFu) < 0x00800000u ? 1.0f : __uint_as_float((b & 0x007FFFFFu) | 0x3F800000u);
 }
 // 32 dims of one token -> shared memory: 64 bytes of the hi part and, unless s is a power of two, of the lo part
 template <bool LO>
@@ -372,7 +373,7 @@ __device__ __forceinline__ void unpack_tiles(const Params& p, Shared& sh, uint8_
       sc[i] *= pow2_of(-e[i]);
       if (FACTORS) {
         if (chunk == 0) lead[row + 8 * i] = lead_of(sc[i]);
-        sc[i] = __uint_as_float(__float_as_uint(sc[i]) & 0x7F800000u);
+        sc[i] = __uint_as_float(__float_as_uint(sc[i]) & 0xFF800000u);
       }
     }
   };

@@ -604,6 +604,23 @@ def test_prefill_rows_do_not_depend_on_later_tokens(size, which, gs):
                 assert_out_close(got[torch.from_numpy(finite)], want[finite])
 
 
+@pytest.mark.parametrize("gs", [32, 64, 128])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_prefill_negative_scales(gs, dtype):
+    """A caller's own cache may hold scales of either sign: some groups of K and of V here, first groups among them."""
+    m = ia()
+    tq = 150
+    k, v = make_kv(81, 1, 2, tq)
+    q = bf16r(np.random.default_rng(82).standard_normal((1, 8, tq, 128)) * 0.5)
+    cache = fill_cache(m, k, v, gs)
+    gen = torch.Generator(device=dev()).manual_seed(gs)
+    for x in (cache.k_scale, cache.v_scale):
+        x.copy_(torch.where(torch.rand(x.shape, generator=gen, device=dev()) < 0.3, -x, x))
+    assert (cache.k_scale[:, :, :tq, 0] < 0).any() and (cache.v_scale[:, :, :tq, 0] < 0).any()
+    ref = oracle.int4_prefill_attention(q, *cache_np(cache), 1, gs)
+    assert_out_close(m._prefill_attention(t(q, dtype), cache, 4, gs), ref)
+
+
 @pytest.mark.parametrize("size", [3e5, 1e7, 1e9, 1e30])
 def test_prefill_huge_scores(size):
     """Keys so large that a score's last bit is worth more than the softmax has range: each row is one token's V, as in fp64."""
