@@ -335,15 +335,16 @@ __device__ __forceinline__ void unpack_tiles(const Params& p, Shared& sh, uint8_
       open_block();
     }
   };
-  // 16 bytes (32 dims) of this lane's two tokens of a tile, and their scales
+  // 16 bytes (32 dims) of this lane's two tokens of a tile, and their scales.  Ordinary loads, here and of the query: the non-coherent ones are for
+  // data that nobody writes while the kernel lives, and a dependent launch lives while its predecessor writes these
   auto fetch = [&](const uint8_t* codes, int token, uint4 (&raw)[2]) {
 #pragma unroll
     for (int i = 0; i < 2; ++i)
-      raw[i] = token + 8 * i < p.kv_len ? __ldg(reinterpret_cast<const uint4*>(codes + static_cast<int64_t>(token + 8 * i) * 64)) : make_uint4(0, 0, 0, 0);
+      raw[i] = token + 8 * i < p.kv_len ? *reinterpret_cast<const uint4*>(codes + static_cast<int64_t>(token + 8 * i) * 64) : make_uint4(0, 0, 0, 0);
   };
   auto fetch_scales = [&](const float* scales, int token, float (&sc)[2]) {
 #pragma unroll
-    for (int i = 0; i < 2; ++i) sc[i] = token + 8 * i < p.kv_len ? __ldg(scales + (static_cast<int64_t>(token + 8 * i) << groups_log2)) : 0.0f;
+    for (int i = 0; i < 2; ++i) sc[i] = token + 8 * i < p.kv_len ? scales[static_cast<int64_t>(token + 8 * i) << groups_log2] : 0.0f;
   };
   auto publish = [&](int tile, const Exponents& ek, const Exponents& ev) {
     const int f = tile & 3;
@@ -511,7 +512,7 @@ __device__ __forceinline__ void load_query_row(const lq_int4_prefill_args& a, in
     const uint4* src = reinterpret_cast<const uint4*>(static_cast<const uint16_t*>(a.q) + base);
 #pragma unroll
     for (int i = 0; i < 16; ++i) {
-      const uint4 v = __ldg(src + i);
+      const uint4 v = src[i];
       raw[4 * i] = v.x; raw[4 * i + 1] = v.y; raw[4 * i + 2] = v.z; raw[4 * i + 3] = v.w;
     }
   } else {

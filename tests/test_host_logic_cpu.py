@@ -319,3 +319,15 @@ def test_launch_makes_the_operands_device_current(monkeypatch, current, status):
     else:
         _lib.launch(torch.device("cuda", 1), entry_point, "a")
     assert state["seen"] == [("a", 101, 1)] and state["device"] == current
+
+
+@pytest.mark.parametrize("name", ["lq_int4_prefill.cuh"])
+def test_kernels_launched_as_dependents_read_operands_with_ordinary_loads(name):
+    """Such a kernel is alive while its predecessor still writes the operands; non-coherent loads (__ldg, ld.global.nc) ask for data that nobody
+    writes in that time."""
+    import re
+    from pathlib import Path
+    import layer_quant_b200
+    text = (Path(layer_quant_b200.__file__).parent / "csrc" / name).read_text()
+    code = re.sub(r"//[^\n]*|/\*.*?\*/", "", text, flags=re.S)
+    assert [line for line in code.splitlines() if "__ldg" in line or "ld.global.nc" in line] == []

@@ -621,6 +621,38 @@ def test_prefill_negative_scales(gs, dtype):
     assert_out_close(m._prefill_attention(t(q, dtype), cache, 4, gs), ref)
 
 
+@pytest.mark.parametrize("gs", [32, 64, 128])
+def test_prefill_chunks_follow_one_another(gs):
+    """Short chunks packed and attended over in a row, each launch in the way of the one before: the rows that one writes share sectors with
+    rows that the launch before reads, and the queries are written by the launch before too.  Equal to the same calls waited for one by one."""
+    m = ia()
+    chunks = [3, 5, 24, 1, 7, 24, 2, 61, 3, 5, 24, 8] * 2
+    gen = torch.Generator(device=dev()).manual_seed(gs)
+    rows = [[torch.randn(2, h, n, 128, generator=gen, device=dev()).to(torch.bfloat16) for h in (8, 2, 2)] for n in chunks]
+    positions = [torch.arange(at, at + n, device=dev()) for at, n in zip(np.cumsum([0] + chunks).tolist(), chunks)]
+    res = []
+    for wait in (True, False):
+        step = torch.cuda.synchronize if wait else lambda: None
+        cache = fill_cache(m, *(np.zeros((2, 2, 0, 128), np.float32),) * 2, gs, capacity=512)
+        outs, at = [], 0
+        for (q, k, v), pos in zip(rows, positions):
+            m._pack_kv_into_cache(cache, k, v, pos, gs, known_len=at + q.shape[2])
+            step()
+            outs.append(m._prefill_attention(q, cache, 4, gs, first_len=at + 1))
+            step()
+            outs.append(m._prefill_attention(outs[-1], cache, 4, gs, first_len=at + 1))  # queries that the launch before has just written
+            step()
+            at += q.shape[2]
+        torch.cuda.synchronize()
+        res.append((outs, cache))
+    for a, b in zip(res[0][0], res[1][0]):
+        assert torch.isfinite(a).all() and torch.equal(a, b)
+    for name in ("k_packed", "v_packed"):
+        assert torch.equal(getattr(res[0][1], name), getattr(res[1][1], name)), name
+    from layer_quant_b200 import _lib
+    assert _lib.device_status() == 0
+
+
 @pytest.mark.parametrize("size", [3e5, 1e7, 1e9, 1e30])
 def test_prefill_huge_scores(size):
     """Keys so large that a score's last bit is worth more than the softmax has range: each row is one token's V, as in fp64."""
