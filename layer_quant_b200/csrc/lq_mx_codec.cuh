@@ -118,7 +118,7 @@ __device__ __forceinline__ void mx_encode_block(const float (&h)[16], const MxRo
     const uint4* w4 = reinterpret_cast<const uint4*>(ctx.words);
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      const uint4 v = __ldg(w4 + i);
+      const uint4 v = w4[i];  // an ordinary load: a dependent launch lives while its predecessor may still write them
       rnd[4 * i] = v.x; rnd[4 * i + 1] = v.y; rnd[4 * i + 2] = v.z; rnd[4 * i + 3] = v.w;
     }
   }

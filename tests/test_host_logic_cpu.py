@@ -321,13 +321,14 @@ def test_launch_makes_the_operands_device_current(monkeypatch, current, status):
     assert state["seen"] == [("a", 101, 1)] and state["device"] == current
 
 
-@pytest.mark.parametrize("name", ["lq_int4_prefill.cuh"])
+@pytest.mark.parametrize("name", ["lq_int4_prefill.cuh", "lq_int4_decode.cuh", "lq_int4_mma.cuh", "lq_int4_kv.cu", "lq_mx_codec.cuh", "lq_mx_state.cu",
+                                  "lq_ssm_operands.cuh", "lq_dense_state.cu", "lq_common.cuh"])
 def test_kernels_launched_as_dependents_read_operands_with_ordinary_loads(name):
     """Such a kernel is alive while its predecessor still writes the operands; non-coherent loads (__ldg, ld.global.nc) ask for data that nobody
-    writes in that time."""
+    writes in that time, such as the codec's constant table."""
     import re
     from pathlib import Path
     import layer_quant_b200
     text = (Path(layer_quant_b200.__file__).parent / "csrc" / name).read_text()
     code = re.sub(r"//[^\n]*|/\*.*?\*/", "", text, flags=re.S)
-    assert [line for line in code.splitlines() if "__ldg" in line or "ld.global.nc" in line] == []
+    assert [line for line in code.splitlines() if "__ldg" in line or "ld.global.nc" in line and "mx_exp_cut_table" not in line] == []

@@ -486,3 +486,33 @@ def test_reference_stream_offsets_equal_general_kernel(bits, offset):
         res.append((plan.out, cache.q_state, cache.shared_exp, cache.micro_exp))
     for got, want in zip(*res):
         assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("stream", ["reference", "layered"])
+def test_supplied_words_written_by_the_launch_before(stream):
+    """The update reads its random words where the launch before, in whose way it starts, has just written them (the codes of an INT4 append serve as
+    words).  Equal to the same calls waited for one by one."""
+    from layer_quant_b200 import int4_8b_attention as ia
+    m = mk()
+    d = make_update_case(51, 1, 4, 16, 128, 2)
+    x, dt, A, B, C, D, _, bias = expand_update_operands(d)
+    gen = torch.Generator(device=dev()).manual_seed(3)
+    steps = [torch.randn(2, 1, 2, 256, 128, generator=gen, device=dev()).to(torch.bfloat16) for _ in range(12)]
+    pos = torch.arange(256, device=dev())
+    res = []
+    for wait in (True, False):
+        kv = ia._allocate_layer_cache(1, 2, 256, 128, 4, dev())
+        words = kv.k_packed.view(torch.int32).view(1, 4, 16, 128)
+        cache = m.allocate_state_kernel_cache(t(d["state"]), 16, 8)
+        outs = []
+        for k, v in steps:
+            ia._pack_kv_into_cache(kv, k, v, pos, 32, known_len=256)
+            if wait:
+                torch.cuda.synchronize()
+            outs.append(m.mx_state_selective_update(cache, x, dt, A, B, C, D=D, dt_bias=bias, dt_softplus=True, rng_stream=stream, rand_words=words))
+            outs.append(cache.q_state.clone())
+            if wait:
+                torch.cuda.synchronize()
+        res.append(outs + [cache.shared_exp, cache.micro_exp])
+    for a, b in zip(*res):
+        assert torch.equal(a, b)
