@@ -1028,9 +1028,16 @@ static int launch_prefill_tc(const lq_int4_prefill_args& a, int ratio, cudaStrea
   const auto launch = [&](auto factors) -> int {
     constexpr bool FACTORS = decltype(factors)::value;
     LQ_SET_SMEM_ONCE(prefill::int4_prefill_kernel<FACTORS>, prefill::kSmemBytes);
-    // Dependent: its CTAs take all registers of an SM, so they cannot crowd, and launch, barriers and tensor memory are ready when the packing ends.
-    // With it, packing and attention: 1 x 24 tokens 13.0 -> 9.6 us, 1 x 100 14.9 -> 11.7, 2 x 300 24.5 -> 21.8, 16 x 256 56.1 -> 53.
-    LQ_CHECK_CUDA(launch_dependent(prefill::int4_prefill_kernel<FACTORS>, static_cast<unsigned>(std::min(p.entries, sms)), prefill::kThreads, prefill::kSmemBytes, st, p));
+    // A dependent launch has barriers and tensor memory ready when the packing ends, 1.5 to 3 us (recorded in a graph 0 to 2), but runs up to 4 % longer where the
+    // predecessor's CTAs leave the SMs one by one.  us of the packing and this launch, ordinary / dependent: 1 x 24 11.4 / 9.1, 1 x 100 13.9 / 11.4, 16 x 100
+    // 26.5 / 22.7, 2 x 600 33.2 / 30.9, 12 x 76 behind 506 (11 tiles per SM) 52.1 / 48.6; 1 x 1500 (15) 59.2 / 58.1 (recorded 56.7 / 57.4), 30 x 256 (13) 92.9 / 95.3, 3 x 1000
+    // (20) 73.7 / 75.6, 8 x 1024 (29) 188.8 / 192.4 (183.7 / 191.2).  Behind a state update of batch 8: 8 x 300 (5) 45.5 / 43.5, 1 x 1000 (7) 51.4 / 50.2,
+    // 30 x 256 100.6 / 101.4, 9 x 666 (28) 120.3 / 123.0.  Dependents of this kernel do not start early (no trigger): with one at the start,
+    // 8 x 300 and an append took 36.0 us in place of 32.8, 2 x 1500 and a decode launch 109 in place of 99, 8 x 1024 and its packing 8 us more.
+    const unsigned grid = static_cast<unsigned>(std::min(p.entries, sms));
+    const int64_t tiles = blocks * (a.first_len + a.q_len / 2) / prefill::kTok;
+    if (tiles <= 12ll * sms) LQ_CHECK_CUDA(launch_dependent(prefill::int4_prefill_kernel<FACTORS>, grid, prefill::kThreads, prefill::kSmemBytes, st, p));
+    else prefill::int4_prefill_kernel<FACTORS><<<grid, prefill::kThreads, prefill::kSmemBytes, st>>>(p);
     LQ_CHECK_CUDA(cudaGetLastError());
     return LQ_OK;
   };

@@ -789,8 +789,7 @@ __device__ __forceinline__ void softmax_blocks(const Params& p, Shared& sh) {
 template <bool FACTORS>
 __global__ void __launch_bounds__(kThreads, 1) int4_prefill_kernel(const __grid_constant__ Params p) {
   extern __shared__ uint8_t smem_raw[];
-  __shared__ Shared sh;
-  pdl_launch_dependents();
+  __shared__ Shared sh;  // no early trigger: dependents that start as this kernel's CTAs leave cost 1 to 4 % of a launch of many blocks (lq_int4_kv.cu)
   uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
   const int warp = threadIdx.x >> 5;
   if (warp == 12) {
