@@ -68,7 +68,6 @@ __global__ void __launch_bounds__(kThreadsM, (R <= 4 && QM != kQF32) ? 3 : 2) in
   const bool is_lo = DUP && t >= 2;
   const uint32_t lo_mul = is_lo ? 65536u : 0u, lo_mask = is_lo ? 0xFFFF0000u : 0u;
   uint8_t* const newtile = smem + L::kSmem - N::kNewBytes;
-  pdl_launch_dependents();
   if (p.dependent && threadIdx.x < 4) {  // the CTA's codes and scales, asked for in L2 while the predecessor still runs (a prefetch reads nothing)
     const int first = min(split * p.tiles_per_split * kTileTok, p.ctx_len);
     const uint32_t tokens = static_cast<uint32_t>(min(first + p.tiles_per_split * kTileTok, p.ctx_len) - first);

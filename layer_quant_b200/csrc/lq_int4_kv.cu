@@ -772,15 +772,22 @@ static int pick_splits(int batch, int kv_heads, int ctx_len) {
     }                                                                                                               \
   } while (0)
 
-// Whether a launch is a programmatic dependent.  One hides launch, set-up and the way to the first tiles (2 us of a launch of 8 to 10), but is
-// placed around its predecessor's CTAs, several to the SMs that have room, and then takes as long as the fullest SM (16 x 8191, one split: 94 instead of
-// 50 us).  So: CTAs for which the predecessor leaves an SM each, and short ones, whose time is memory round trips whatever their SM holds.  us of four
-// launches of the same size, ordinary -> dependent, at tiles per CTA x CTAs: 5 x 8 33.2 -> 25.0, 8 x 64 41.0 -> 31.4, 16 x 64 49.4 -> 41.5, 8 x 96 41.2 -> 37.3;
-// 1 x 128 41.3 -> 34.8, 3 x 128 33.1 -> 27.0, but 4 x 128 41.4 -> 42.1 and 5 x 128 33.2 -> 35.0; 5 x 192 41.3 -> 35.2, 5 x 512 74.2 -> 67.1, 4 x 1600
-// 140 -> 128, but 7 x 192 41.5 -> 41.4 and 14 x 288 78.0 -> 81.9.
+// Whether a decode launch is a programmatic dependent.  One hides launch, set-up and the way to the first tiles (2 us of a launch of 8 to 10).
+// Left to itself it loses more than that: its CTAs are placed where the predecessor leaves room, several to an SM, and the launch takes as long as the fullest
+// SM.  So it asks for so much shared memory that an SM holds no more of its CTAs than an even deal puts there (kHoldsOne, kHoldsTwo; three are
+// what it holds anyway).  us of a pair of launches, a predecessor and 8 x 1024 in one split (16 tiles x 64 CTAs): ordinary / dependent / dependent with an SM
+// each, behind a state update of batch 8 22.7 / 28.6 / 21.4, an append of 8 x 1024 22.6 / 24.2 / 20.1, an unquantised update of batch 32 40.2 / 44.7 / 38.1,
+// a GEMM 21.6 / 19.6 / 19.7, 16 x 8191 61.5 / 61.5 / 57.9, itself 12.4 / 10.8 / 10.6; 24 x 320 (5 x 192, two per SM) behind the update of batch 8
+// 20.6 / 20.0 / 18.7, itself 10.3 / 9.3 / 8.2; 40 x 200 (4 x 320) 20.6 / - / 18.8 and 10.3 / - / 8.4.  Recorded in a graph the gain is smaller, and behind long
+// kernels without a trigger a dependent costs up to 0.5 us more than it saves at 5 tiles, 0.8 at 16 tiles x 64 CTAs (behind 16 x 8191 55.8 -> 56.6), 1.0 at
+// 12 x 96, but up to 1.9 at 16 x 96, 2.0 at 8 x 128, 2.4 at 8 x 288: hence the tiles.  Short CTAs in any number even out (103 x 19, 1 x 824, behind the update of
+// batch 8 22.7 -> 20.7, 200 x 320, 5 x 1600, 51.9 -> 50.2, themselves 12.4 -> 10.6 and 40.9 -> 39.2).
+// Dependents of a decode launch do not start early (no trigger): they would lie around it in the same way (16 x 8191 and a dependent of 64 CTAs
+// 55.5 -> 60.1 recorded, 1 x 1024 and a state update of batch 60 59.2 -> 61.9, 200 x 256 and an update of batch 250 230.6 -> 233.5).
+constexpr size_t kHoldsOne = 116 * 1024, kHoldsTwo = 77 * 1024;  // of an SM's 228 KB, with 1 KB for each CTA
 static bool dependent_pays(int tiles, int64_t ctas) {
   const int sms = sm_count();
-  return tiles <= (3 * ctas <= 2 * sms ? 16 : ctas <= sms ? 3 : 5);
+  return tiles <= (2 * ctas <= sms ? 16 : 3 * ctas <= 2 * sms ? 12 : 5);
 }
 
 template <int R, int GS>
@@ -801,16 +808,18 @@ static int launch_decode(const DecodeParams& p, cudaStream_t st) {
 
 template <int R, int GS>
 static int launch_decode_mma(DecodeParams p, cudaStream_t st) {
-  constexpr size_t smem = mma::WarpStage<GS>::kSmem;
+  static_assert(mma::WarpStage<GS>::kSmem <= kHoldsTwo, "the sizes for one and two CTAs are not smaller than what the kernel uses");
   const dim3 grid(p.splits, p.a.cache.kv_heads, p.a.cache.batch);
+  const int64_t ctas = static_cast<int64_t>(grid.x) * grid.y * grid.z;
+  // (with a device counter the tiles are not known here)
+  p.dependent = p.a.seq_len_counter == nullptr && dependent_pays(p.tiles_per_split, ctas);
+  const size_t smem = !p.dependent || ctas > 2 * sm_count() ? mma::WarpStage<GS>::kSmem : ctas > sm_count() ? kHoldsTwo : kHoldsOne;
 #define LQ_MMA_LAUNCH(MASK_, QM_)                                                                                   \
   do {                                                                                                              \
-    LQ_SET_SMEM_ONCE((mma::int4_decode_warp_kernel<R, GS, MASK_, QM_>), smem);                                      \
+    LQ_SET_SMEM_ONCE((mma::int4_decode_warp_kernel<R, GS, MASK_, QM_>), kHoldsOne);                                 \
     if (p.dependent) LQ_CHECK_CUDA(launch_dependent(mma::int4_decode_warp_kernel<R, GS, MASK_, QM_>, grid, mma::kThreadsM, smem, st, p)); \
     else mma::int4_decode_warp_kernel<R, GS, MASK_, QM_><<<grid, mma::kThreadsM, smem, st>>>(p);                    \
   } while (0)
-  // (with a device counter the tiles are not known here)
-  p.dependent = p.a.seq_len_counter == nullptr && dependent_pays(p.tiles_per_split, static_cast<int64_t>(grid.x) * grid.y * grid.z);
   if (p.a.mask) {
     if (p.a.dtype == LQ_BF16) LQ_MMA_LAUNCH(true, mma::kQBf16); else if (p.a.dtype == LQ_F16) LQ_MMA_LAUNCH(true, mma::kQF16); else LQ_MMA_LAUNCH(true, mma::kQF32);
   } else {

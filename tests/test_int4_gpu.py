@@ -749,3 +749,49 @@ def test_decode_launches_follow_one_another(batch, start, splits):
         assert torch.equal(getattr(res[0][1], name), getattr(res[1][1], name)), name
     from layer_quant_b200 import _lib
     assert _lib.device_status() == 0
+
+
+PAIRS = """
+import sys, torch
+from tests.util import dev, expand_update_operands, make_update_case
+from layer_quant_b200 import int4_8b_attention as ia, mamba_state_8b_kernel as mk
+x, dt, A, B, C, D, _, bias = expand_update_operands(make_update_case(1, 8, 128, 64, 128, 8))
+state = mk.allocate_state_kernel_cache(torch.randn(8, 128, 64, 128, device=dev()), 16, 8)
+update = mk.MxUpdatePlan(state, x, dt, A, B, C, D=D, dt_bias=bias, dt_softplus=True, rng_stream="layered")
+plans = []
+for batch, length, splits in ((8, 1024, 1), (1, 2048, 2)):
+    cache = ia._allocate_layer_cache(batch, 8, length, 128, 4, dev())
+    k, v = (torch.randn(batch, 8, length, 128, device=dev()).bfloat16() for _ in range(2))
+    ia._pack_kv_into_cache(cache, k, v, torch.arange(length, device=dev()), 32)
+    q = torch.randn(batch, 32, 1, 128, device=dev()).bfloat16()
+    plans.append(ia.Int4DecodePlan(q, cache, length, 32, splits=splits))
+for plan in plans:
+    update.run(), plan.launch()
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        keep = [(update.run(), plan.launch()) for _ in range(50)]
+    best = 1e9
+    for _ in range(12):
+        e = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+        e[0].record(); g.replay(); e[1].record(); e[1].synchronize()
+        best = min(best, e[0].elapsed_time(e[1]) * 20)
+    print(best)
+"""
+
+
+def test_dependent_decode_launches_do_not_crowd():
+    """Few long CTAs behind a state update, whose CTAs leave the SMs one by one: placed several to an SM they take a quarter longer than ordinary
+    launches (27.6 for 20.9 us a pair), with an SM each they do not."""
+    import os
+    import subprocess
+    import sys
+    from pathlib import Path
+    us = []
+    for pdl in "01":
+        run = subprocess.run([sys.executable, "-c", PAIRS], env=dict(os.environ, LQ_MX_PDL=pdl), cwd=Path(__file__).resolve().parents[1],
+                             capture_output=True, text=True, timeout=300)
+        assert run.returncode == 0, run.stderr[-2000:]
+        us.append([float(x) for x in run.stdout.split()])
+    for ordinary, dependent in zip(*us):
+        assert dependent < 1.08 * ordinary, us
