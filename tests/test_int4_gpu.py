@@ -668,8 +668,9 @@ def test_prefill_huge_scores(size):
 
 @pytest.mark.parametrize("gs,ratio,tq,first", [(128, 4, 3, 1), (128, 4, 65, 1), (128, 8, 19, 40), (128, 2, 129, 63), (64, 4, 2, 2000), (64, 4, 65, 2000)])
 def test_prefill_token_factors(gs, ratio, tq, first):
-    """Groups of 128 keep the operands exact and multiply by the token's factor; large launches with groups of 64 behind a long context.  Sequence 0 as it comes, 1 and 2 with a first group far below and far above the others, 3 with a huge key and an infinite
-    value in the last token, which the rows before it must not notice."""
+    """Groups of 128, whose operands are exact beside a factor of the token, and large launches with groups of 64 behind a long context.  Sequence 0 as it
+    comes, 1 and 2 with a first half far below and far above the other, 3 with a huge key and an infinite value in the last token, which the
+    rows before it must not notice, nor the groups beside the infinite one."""
     m = ia()
     hkv, total = 2, first + tq - 1
     b = 5 if gs == 128 else torch.cuda.get_device_properties(0).multi_processor_count // -(-tq * ratio // 256) + 1
@@ -692,9 +693,60 @@ def test_prefill_token_factors(gs, ratio, tq, first):
     assert_out_close(out[3, :, :-1], ref[3, :, :-1])
     last = torch.from_numpy(np.isfinite(ref[3, :, -1]))
     assert not torch.isfinite(out[3, :, -1][~last]).any()
+    assert last.any() == (gs == 64)
+    if gs == 64:
+        assert_out_close(out[3, :, -1][last], ref[3, :, -1][last.numpy()])
     assert torch.equal(out[4:], out[:1].expand(b - 4, -1, -1, -1))  # the others are sequence 0 once more
     from layer_quant_b200 import _lib
     assert _lib.device_status() == 0
+
+
+@pytest.mark.parametrize("gs", [32, 64, 128])
+@pytest.mark.parametrize("tq,first", [(1, 100), (40, 100), (150, 80)])
+def test_prefill_keeps_all_bits_of_the_scales(gs, tq, first):
+    """Scales with all low mantissa bits set, two tokens that share the weight of every row at scores near 20, fp16 outputs.  An output is the correctly
+    rounded one, give or take what the operands lose: 2^-20 of a K operand moves a score by 20 * 2^-20 and its weight by as much, fp32 sums of 128 terms
+    of that size and the exponent's argument (below 32, ulp 2^-19) no more again; 2^-20 of V and 2^-22 of the weights are less.  That the
+    low bits of K or of V are in the result shows in the oracle without them, which is outside."""
+    m = ia()
+    total = first + tq - 1
+    rng = np.random.default_rng(gs + tq)
+    u = np.sign(rng.standard_normal((1, 2, 1, 128)))
+    k, v = make_kv(83 + tq, 1, 2, total)
+    for token in (3, 70):
+        k[:, :, token] = bf16r(1.5 * u + 0.3 * rng.standard_normal(u.shape))[:, :, 0]
+    q = np.float16(1.2 * np.repeat(u, 4, 1) + 0.1 * rng.standard_normal((1, 8, tq, 128)))
+    cache = fill_cache(m, k, v, gs)
+    for x in (cache.k_scale, cache.v_scale):
+        x.view(torch.int32).bitwise_or_(0xFFFF)
+    kp, vp, ks, vs = cache_np(cache)
+    ref = oracle.int4_prefill_attention(q, kp, vp, ks, vs, first, gs)
+    size = np.abs(oracle.int4_decode(oracle.int4_unpack_nibbles(vp[:, :, [3, 70]]), vs[:, :, [3, 70]], gs)).max()
+
+    def close(x):
+        return (np.abs(x - ref) <= 2.0 ** -11 * np.abs(ref) + 2.0 ** -24 + 3 * 20 * 2.0 ** -20 * size).all()
+
+    assert close(m._prefill_attention(t(q), cache, 4, gs, first_len=first).double().cpu().numpy())
+    cut = [(x.view(np.uint32) & np.uint32(0xFFFF0000)).view(np.float32) for x in (ks, vs)]
+    assert not close(oracle.int4_prefill_attention(q, kp, vp, cut[0], vs, first, gs))
+    assert not close(oracle.int4_prefill_attention(q, kp, vp, ks, cut[1], first, gs))
+
+
+@pytest.mark.parametrize("gs,limit", [(32, 0.02), (64, 0.02), (128, 0.006)])
+def test_prefill_share_of_outputs_not_correctly_rounded(gs, limit):
+    """Of a prompt of 700 tokens, fp16 outputs against the 64-bit oracle rounded to fp16.  With an error of e in the largest values V of a row, a share of
+    about 2 e / (2^-11 |out|) is rounded the other way: 2^-20 of V beside outputs a fifth of it gives 2 %, and without the lo parts (groups of 128) the
+    2^-22 of the weights are what remains."""
+    m = ia()
+    tq = 700
+    k, v = make_kv(95, 1, 2, tq)
+    q = np.float16(np.random.default_rng(96).standard_normal((1, 8, tq, 128)))
+    cache = fill_cache(m, k, v, gs)
+    ref = oracle.int4_prefill_attention(q, *cache_np(cache), 1, gs)
+    got = m._prefill_attention(t(q), cache, 4, gs).cpu().numpy()
+    share = (got != ref.astype(np.float16)).mean()
+    print(f"groups of {gs}: {100 * share:.2f} %")
+    assert share < limit
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
