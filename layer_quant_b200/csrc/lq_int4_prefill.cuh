@@ -16,8 +16,8 @@
 // S = Q Khi + Q Klo, O = Phi Vhi + Plo Vhi + Phi Vlo: five products per tile pair, all in fp32 accumulators.
 // Token factors (FACTORS, groups of 128, where a token has one scale): the mantissa of the scale goes to the softmax, which multiplies the scores (K) and
 // the weights after their sum is taken (V) by it in fp32; the operands are then a code times a power of two, exact in fp16, and need no lo part: three
-// products per tile pair in place of five.  The error against 64 bits goes down with the lo parts: outputs that are
-// not the correctly rounded fp16 value 1.1 % -> 0.27 % of 2 x 700 tokens.  (Groups of 64 could leave out one product of five, Phi Vlo and Q Klo of the first group.
+// products per tile pair in place of five.  The error against 64 bits goes down with the lo parts: fp16 outputs that are
+// not the correctly rounded value 1.08 % -> 0.27 % of 2 x 700 tokens, 3.9 -> 1.5 % of 2 x 500 behind 3000, 8.1 -> 3.6 % of 1 x 300 behind 8000.  (Groups of 64 could leave out one product of five, Phi Vlo and Q Klo of the first group.
 // Dropped: it pays only in rows of long launches, and a rule on the launch's size made a sequence's bits depend on what shares its launch.)
 // Range.  Powers of two are taken out of every row of Q and of the K and V scales of every 16 tokens, so the
 // fp16 operands sit at the top of their range; the exponents come back for free, in the factor and the offset of the
@@ -29,12 +29,13 @@
 // What remains relative to the largest: inside a token the group scales below 2^-15 of its largest lose bits, and a weight times
 // V counts with the row's largest (first item), whichever group that is in.
 //
-// What bounds it: in long runs the board's power (the five products run at 1365 TFLOP/s where cuBLAS sustains 1395: other schedules of the same
-// products, such as a third score buffer per pair of groups, took less cycles per tile, 3650 for 4030, at a clock lower by as much).  In short
-// runs: per 256 x 64 tile the five products take 2620 tensor cycles (5/2 of a bf16 attention; 1.33 us at 1965 MHz), shared memory
-// moves 230 KB (1800 cycles, which is why Q is an operand in TMEM) and the exp2 take 1024; a tile takes 2.05 us.  No pipe is full: within a
+// What bounds it: the chain of a softmax group.  Per 256 x 64 tile the five products take 2620 tensor cycles (5/2 of a bf16 attention), shared memory
+// moves 230 KB (1800 cycles, which is why Q is an operand in TMEM) and the exp2 take 1024; a tile takes 4230 cycles in 2 x 2000 tokens behind 6001, starts and
+// ends of blocks included, and with token factors, 1570 tensor cycles, still 3630.  No pipe is full: within a
 // softmax group S, softmax, P, the products with V and the next S follow one another (P replaces S), and two groups fill one another's
-// gaps only in part (tensor pipe active in 53 % of the cycles at 8 x 1024).
+// gaps only in part (tensor pipe active in 53 % of the cycles at 8 x 1024).  In long rows of launches the board's power limit comes on top: five products at
+// 1243 TFLOP/s (of measured 1425 sustained) run at 1695 MHz, 954 us in place of 844 for a few launches on a cool board; three products hold 1942 MHz, 715 us
+// and 710.  Other schedules of the five, such as a third score buffer for the two groups, took less cycles per tile (3650) at a clock lower by as much.
 #pragma once
 
 #include "lq_common.cuh"
