@@ -190,8 +190,8 @@ __device__ __forceinline__ float max_nan(float a, float b) {
 
 // The usual case: 16-bit K and V with contiguous, 16-byte aligned rows, group size 32, 64 or 128, head dim 128.  A thread takes 32 bytes
 // (sixteen values, two 32-bit words of codes) of a row of K and of the same row of V, eight threads a row.
-// Bound by instruction issue (152 instructions per eight values when a thread took 16 bytes of two rows, a fifth of them addresses): so one
-// scale, one set of addresses and one position per sixteen values, divisions as multiplications on pairs (quotient16, packed fp32x2),
+// Such a kernel is bound by instruction issue (152 instructions per eight values when a thread took 16 bytes of two rows, a fifth of them addresses; 88
+// now, and the ramp of the launch shows): so one scale, one set of addresses and one position per sixteen values, divisions as multiplications on pairs (quotient16, packed fp32x2),
 // and codes gathered by one shift-and-add each, the magic number's share of the sum taken off at the end.  8 x 1024 tokens, group 64: 38 -> 14.7 us as
 // 16-byte threads, 11.2 us now.
 constexpr int kAppendRows = 32;  // rows per CTA
