@@ -47,7 +47,15 @@ struct MxRoundCtx {
   const uint32_t* words; // SUPPLIED / SUPPLIED_FIXED: 16 words of this block
   const uint32_t* drawn = nullptr;       // PHILOX_REF: the block's 16 words, where the caller has drawn them
   const PhiloxStream* stream = nullptr;  // the layered modes: where the caller carries the generator along, used instead of the counter
+  const uint32_t* exp_step = nullptr;    // MxExpSteps of the format in shared memory, where the caller has staged them
 };
+
+// What added to the bits of a block maximum makes its exponent field step up where the shared exponent does, per exponent field.
+// (Infinity keeps its field.)
+template <int BITS>
+__device__ __forceinline__ uint32_t mx_exp_step(int field) {
+  return 0x7FFFFFu - (field == 255 ? MxFormat<BITS>::kCutFirst : mx_exp_cut_table<BITS>()[field]);
+}
 
 __device__ __forceinline__ float max3(float a, float b, float c) {  // one three-input instruction (sm_100)
   float r;
@@ -99,11 +107,16 @@ __device__ __forceinline__ void mx_encode_block(const float (&h)[16], const MxRo
   // on the exponent (the rounded logarithm), but always lies in [kCutFirst, kCutLast] (below field 34 it makes no
   // difference): only a maximum in that sliver, one in 200,000, has to look it up.
   const uint32_t abits = __float_as_uint(amax);
-  uint32_t up = (abits + (0x7FFFFFu - MxFormat<BITS>::kCutFirst)) >> 23;
-  if (up != (abits + (0x7FFFFFu - MxFormat<BITS>::kCutLast)) >> 23) {
-    uint32_t cut;  // volatile: a branch, not a load that every block waits for
-    asm volatile("ld.global.nc.u32 %0, [%1];" : "=r"(cut) : "l"(mx_exp_cut_table<BITS>() + (abits >> 23)));
-    up = (abits >> 23) + ((abits & 0x7FFFFFu) > cut ? 1u : 0u);
+  uint32_t up;
+  if (ctx.exp_step) {
+    up = (abits + ctx.exp_step[abits >> 23]) >> 23;
+  } else {
+    up = (abits + (0x7FFFFFu - MxFormat<BITS>::kCutFirst)) >> 23;
+    if (up != (abits + (0x7FFFFFu - MxFormat<BITS>::kCutLast)) >> 23) {
+      uint32_t cut;  // volatile: a branch, not a load that every block waits for
+      asm volatile("ld.global.nc.u32 %0, [%1];" : "=r"(cut) : "l"(mx_exp_cut_table<BITS>() + (abits >> 23)));
+      up = (abits >> 23) + ((abits & 0x7FFFFFu) > cut ? 1u : 0u);
+    }
   }
   int biased = static_cast<int>(up) - MxFormat<BITS>::kShift;
   biased = biased < 28 ? 28 : biased;
@@ -139,35 +152,38 @@ __device__ __forceinline__ void mx_encode_block(const float (&h)[16], const MxRo
     pw[0] = r.w0; pw[1] = r.w1; pw[2] = r.w2; pw[3] = r.w3;
   }
 
-  float macc = 0.0f;  // sum of 2^j over pairs with the micro-exponent set (exact)
+  float2 macc = make_float2(0.0f, 0.0f);  // sums of 4^k over the even pairs 2 k (x) and the odd ones 2 k + 1 (y) with the micro-exponent set (exact)
   uint32_t tb[16];    // bit patterns whose byte 1 (HALF_EVEN: byte 0) is the code
+  // Two pairs at a time: packed instructions take a value of either pair, so that their factors are the two pairs' own and none is needed twice.
 #pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    const float micf = set_gt(pa[j], thresh);
-    const float inv = fmaf(micf, neg_half_inv0, inv0);  // 1 / (base * 2^micro), exact
-    macc = fmaf(micf, static_cast<float>(1 << j), macc);
-    if (kFixed) {  // the pair shares 1 / scale: one packed fp32x2 FMA for both values
-      float cf[2];
+  for (int j = 6; j >= 0; j -= 2) {
+    const float2 micf = make_float2(set_gt(pa[j], thresh), set_gt(pa[j + 1], thresh));
+    const float2 inv2 = __ffma2_rn(micf, make_float2(neg_half_inv0, neg_half_inv0), make_float2(inv0, inv0));  // 1 / (base * 2^micro), exact
+    macc = j == 6 ? micf : __ffma2_rn(macc, make_float2(4.0f, 4.0f), micf);
 #pragma unroll
-      for (int k = 0; k < 2; ++k) {
-        const int i = 2 * j + k;
-        const uint32_t c = (MODE == LQ_ROUND_SUPPLIED_FIXED) ? (0x47400000u | (rnd[i] & 0xFFu))
-                                                             : __byte_perm(pw[i >> 2], 0x47400000u, 0x7650 + (i & 3));
-        cf[k] = __uint_as_float(c);
-      }
-      const float2 t2 = __ffma2_rn(make_float2(h[2 * j], h[2 * j + 1]), make_float2(inv, inv), make_float2(cf[0], cf[1]));
-      tb[2 * j] = __float_as_uint(t2.x);
-      tb[2 * j + 1] = __float_as_uint(t2.y);
-      continue;
-    }
-#pragma unroll
-    for (int k = 0; k < 2; ++k) {
+    for (int k = 0; k < 2; ++k) {  // values i of pair j and i + 2 of pair j + 1
       const int i = 2 * j + k;
-      float t;
-      {
-        const float a = fminf(fabsf(h[i]) * inv, M);
+      if (kFixed) {
+        float cf[2];
+#pragma unroll
+        for (int l = 0; l < 2; ++l) {
+          const int n = i + 2 * l;
+          const uint32_t c = (MODE == LQ_ROUND_SUPPLIED_FIXED) ? (0x47400000u | (rnd[n] & 0xFFu))
+                                                               : __byte_perm(pw[n >> 2], 0x47400000u, 0x7650 + (n & 3));
+          cf[l] = __uint_as_float(c);
+        }
+        const float2 t2 = __ffma2_rn(make_float2(h[i], h[i + 2]), inv2, make_float2(cf[0], cf[1]));
+        tb[i] = __float_as_uint(t2.x);
+        tb[i + 2] = __float_as_uint(t2.y);
+        continue;
+      }
+#pragma unroll
+      for (int l = 0; l < 2; ++l) {
+        const int n = i + 2 * l;
+        float t;
+        const float a = fminf(fabsf(h[n]) * (l ? inv2.y : inv2.x), M);
         if (MODE == LQ_ROUND_HALF_EVEN) {  // rounded by the addition itself; byte 0 = two's complement of the signed level
-          t = copysignf(a, h[i]) + 12582912.0f;
+          t = copysignf(a, h[n]) + 12582912.0f;
         } else {
           float lvl;  // never above M: a is not, and only what is below its next integer is raised to it
           if (MODE == LQ_ROUND_HALF_UP) {
@@ -175,18 +191,18 @@ __device__ __forceinline__ void mx_encode_block(const float (&h)[16], const MxRo
           } else {
             uint32_t w;
             if (MODE == LQ_ROUND_SUPPLIED || MODE == LQ_ROUND_PHILOX_LAYERED4) {
-              w = rnd[i];
+              w = rnd[n];
             } else {  // the reference's stream: one Philox block per value, word 0
-              const uint64_t c = ctx.counter + i;
-              w = ctx.drawn ? ctx.drawn[i] : philox4x32_10(static_cast<uint32_t>(c), ctx.wrap32 ? 0u : static_cast<uint32_t>(c >> 32), 0u, 0u, keys).w0;
+              const uint64_t c = ctx.counter + n;
+              w = ctx.drawn ? ctx.drawn[n] : philox4x32_10(static_cast<uint32_t>(c), ctx.wrap32 ? 0u : static_cast<uint32_t>(c >> 32), 0u, 0u, keys).w0;
             }
             const float fl = floor_small(a);
             lvl = fl + set_gt(a - fl, word_to_uniform(w));  // (u < a - fl) ? 1 : 0
           }
-          t = copysignf(lvl, h[i]) + kByteMagic;  // exact; byte 1 = two's complement of the signed level
+          t = copysignf(lvl, h[n]) + kByteMagic;  // exact; byte 1 = two's complement of the signed level
         }
+        tb[n] = __float_as_uint(t);
       }
-      tb[i] = __float_as_uint(t);
     }
   }
   constexpr int kByte = MODE == LQ_ROUND_HALF_EVEN ? 0 : 1;
@@ -200,7 +216,7 @@ __device__ __forceinline__ void mx_encode_block(const float (&h)[16], const MxRo
       codes[w] = (ev & 0x0F0F0F0Fu) | ((od << 4) & 0xF0F0F0F0u);
     }
   }
-  micro_bits = __float_as_uint(macc + 8388608.0f) & 0xFFu;
+  micro_bits = __float_as_uint(fmaf(macc.y, 2.0f, macc.x + 8388608.0f)) & 0xFFu;  // exact
 }
 
 // h' = h * dA + (B * dt) * x on 16 values and the block's share of <h', C>, with packed fp32x2 instructions
@@ -211,29 +227,26 @@ __device__ __forceinline__ void mx_encode_block(const float (&h)[16], const MxRo
 // h is given as q * s with s a power of two: fma(h, dA, t) = fma(q, s dA, t), for s dA is exact unless it is subnormal (then a term below
 // 2^-119 is off by part of itself: nothing that a code, whose unit is 2^-99 at least, or a normal y can show).  sd: s dA of the pairs,
 // ONE: of the whole block (sd[0]).
+// A packed instruction takes value i of one pair and i + 2 of the next: their factors are two neighbours of sd, and no register holds one twice.
 template <bool ONE>
 __device__ __forceinline__ float mx_update_readout16(float (&hv)[16], const float (&dB)[16], const float (&Cv)[16], const float (&sd)[8],
                                                      float x) {
   const float2 x2 = make_float2(x, x);
-  float2 ya = make_float2(0.0f, 0.0f), yb = make_float2(0.0f, 0.0f);
+  float2 y[2] = {make_float2(0.0f, 0.0f), make_float2(0.0f, 0.0f)};  // sums over i mod 4: (0, 2) and (1, 3)
 #pragma unroll
   for (int i = 0; i < 16; i += 4) {
-    const float s0 = sd[ONE ? 0 : i / 2], s1 = sd[ONE ? 0 : i / 2 + 1];
-    const float2 t0 = __fmul2_rn(make_float2(dB[i], dB[i + 1]), x2);
-    const float2 t1 = __fmul2_rn(make_float2(dB[i + 2], dB[i + 3]), x2);
-    float2 h0, h1;
-    if (ONE) {
-      h0 = __ffma2_rn(make_float2(hv[i], hv[i + 1]), make_float2(s0, s0), t0);
-      h1 = __ffma2_rn(make_float2(hv[i + 2], hv[i + 3]), make_float2(s1, s1), t1);
-    } else {  // scalar: a packed operand would need each pair's factor twice
-      h0 = make_float2(fmaf(hv[i], s0, t0.x), fmaf(hv[i + 1], s0, t0.y));
-      h1 = make_float2(fmaf(hv[i + 2], s1, t1.x), fmaf(hv[i + 3], s1, t1.y));
+    const float2 s2 = make_float2(sd[ONE ? 0 : i / 2], sd[ONE ? 0 : i / 2 + 1]);
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const float2 t = __fmul2_rn(make_float2(dB[i + k], dB[i + k + 2]), x2);
+      const float2 h = __ffma2_rn(make_float2(hv[i + k], hv[i + k + 2]), s2, t);
+      hv[i + k] = h.x;
+      hv[i + k + 2] = h.y;
+      y[k] = __ffma2_rn(h, make_float2(Cv[i + k], Cv[i + k + 2]), y[k]);
     }
-    hv[i] = h0.x; hv[i + 1] = h0.y; hv[i + 2] = h1.x; hv[i + 3] = h1.y;
-    ya = __ffma2_rn(h0, make_float2(Cv[i], Cv[i + 1]), ya);
-    yb = __ffma2_rn(h1, make_float2(Cv[i + 2], Cv[i + 3]), yb);
   }
-  return (ya.x + ya.y) + (yb.x + yb.y);
+  const float2 s = __fadd2_rn(y[0], y[1]);
+  return s.x + s.y;  // (y0 + y1) + (y2 + y3)
 }
 
 // What a stored block and dA = exp(A dt) give the update: q[i] and sd with h dA = q[i] sd of the pair, exact unless sd is subnormal.
@@ -262,24 +275,32 @@ struct MxPairMasks {
 __device__ __forceinline__ void mx_decode_block(const uint32_t (&codes)[4], uint32_t e, uint32_t micro_bits, float (&h)[16]);
 __device__ __forceinline__ void mx4_nibbles_to_bytes(uint32_t lo, uint32_t hi, uint32_t (&codes)[4]);
 
+// KNOWN: the caller has seen that every lane's e lies in [1, e_max + 1].
+template <bool KNOWN>
 __device__ __forceinline__ void mx_decode_scaled(const uint4& raw, uint32_t e, uint32_t micro_bits, float dA, uint32_t e_max, const MxPairFactors& table,
                                                  float (&q)[16], float (&sd)[8]) {
   const uint32_t codes[4] = {raw.x, raw.y, raw.z, raw.w};
-  if (__all_sync(0xFFFFFFFFu, e - 1u <= e_max)) {
+  if (KNOWN || __all_sync(0xFFFFFFFFu, e - 1u <= e_max)) {
     const float4 f0 = table.f[micro_bits & 15u], f1 = table.f[micro_bits >> 4];
     const float base = __uint_as_float(e << 23) * dA;
-    sd[0] = f0.x * base; sd[1] = f0.y * base; sd[2] = f0.z * base; sd[3] = f0.w * base;
-    sd[4] = f1.x * base; sd[5] = f1.y * base; sd[6] = f1.z * base; sd[7] = f1.w * base;
+    const float2 base2 = make_float2(base, base);
+    const float2 p[4] = {__fmul2_rn(make_float2(f0.x, f0.y), base2), __fmul2_rn(make_float2(f0.z, f0.w), base2),
+                         __fmul2_rn(make_float2(f1.x, f1.y), base2), __fmul2_rn(make_float2(f1.z, f1.w), base2)};
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      sd[2 * j] = p[j].x;
+      sd[2 * j + 1] = p[j].y;
+    }
 #pragma unroll
     for (int w = 0; w < 4; ++w) {
       const uint32_t biased = codes[w] ^ 0x80808080u;  // q + 128 as unsigned bytes
 #pragma unroll
-      for (int k = 0; k < 4; k += 2) {
+      for (int k = 0; k < 2; ++k) {
         const float2 r = __fadd2_rn(make_float2(__uint_as_float(__byte_perm(biased, 0x47000000u, 0x7604 | (k << 4))),
-                                                __uint_as_float(__byte_perm(biased, 0x47000000u, 0x7604 | ((k + 1) << 4)))),
+                                                __uint_as_float(__byte_perm(biased, 0x47000000u, 0x7604 | ((k + 2) << 4)))),
                                     make_float2(-32896.0f, -32896.0f));
         q[4 * w + k] = r.x;
-        q[4 * w + k + 1] = r.y;
+        q[4 * w + k + 2] = r.y;
       }
     }
   } else {
@@ -289,9 +310,10 @@ __device__ __forceinline__ void mx_decode_scaled(const uint4& raw, uint32_t e, u
   }
 }
 
+template <bool KNOWN>
 __device__ __forceinline__ void mx_decode_scaled(const uint4& raw, uint32_t e, uint32_t micro_bits, float dA, uint32_t e_max, const MxPairMasks& table,
                                                  float (&q)[16], float (&sd)[8]) {
-  if (__all_sync(0xFFFFFFFFu, e - 1u <= e_max)) {
+  if (KNOWN || __all_sync(0xFFFFFFFFu, e - 1u <= e_max)) {
     sd[0] = __uint_as_float(e << 23) * dA;
     const uint2 mask = table.m[micro_bits];
 #pragma unroll
@@ -300,12 +322,16 @@ __device__ __forceinline__ void mx_decode_scaled(const uint4& raw, uint32_t e, u
       const uint32_t ev = (x & 0x0F0F0F0Fu) ^ 0x08080808u, od = ((x >> 4) & 0x0F0F0F0Fu) ^ 0x08080808u;  // q + 8; byte k = pair k
       const uint32_t ev2 = ev + ((m & ev) | (~m & 0x08080808u)), od2 = od + ((m & od) | (~m & 0x08080808u));
 #pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const float2 r = __fadd2_rn(make_float2(__uint_as_float(__byte_perm(ev2, 0x47000000u, 0x7604 | (k << 4))),
-                                                __uint_as_float(__byte_perm(od2, 0x47000000u, 0x7604 | (k << 4)))),
-                                    make_float2(-32784.0f, -32784.0f));
-        q[8 * w + 2 * k] = r.x;
-        q[8 * w + 2 * k + 1] = r.y;
+      for (int k = 0; k < 4; k += 2) {
+#pragma unroll
+        for (int l = 0; l < 2; ++l) {
+          const uint32_t half = l ? od2 : ev2;
+          const float2 r = __fadd2_rn(make_float2(__uint_as_float(__byte_perm(half, 0x47000000u, 0x7604 | (k << 4))),
+                                                  __uint_as_float(__byte_perm(half, 0x47000000u, 0x7604 | ((k + 1) << 4)))),
+                                      make_float2(-32784.0f, -32784.0f));
+          q[8 * w + 2 * k + l] = r.x;
+          q[8 * w + 2 * k + l + 2] = r.y;
+        }
       }
     }
   } else {

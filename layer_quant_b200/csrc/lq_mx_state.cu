@@ -7,9 +7,12 @@
 // wave of two-warp CTAs; mx_state_update_kernel takes any strides, per-row dt and ragged shapes, one CTA per
 // (batch, head).
 //
-// Both are bound by instruction issue and latency, not by HBM: at 18 bytes per block read and written the memory
+// Both are bound by the dispatch of instructions, not by HBM or by latency: at 18 bytes per block read and written the memory
 // system could deliver one value every ~12 issue slots per SM sub-partition, and decode + update + read-out +
-// exponent + rounding + random bits need more than that.
+// exponent + rounding + random bits need more than that.  What an instruction costs there was measured in random mixes of independent chains
+// (the same for two, four and six warps per scheduler): 2 cycles of the logic pipe for byte permutes, logic, shifts and compares, one slot for a
+// scalar FMA, two for a packed one (beside byte permutes it takes 3.1 cycles, as two scalar ones do; a packed product with two register operands
+// 2.1), and 2.4 cycles of the logic pipe for a wide multiply.
 #include <algorithm>
 #include <cstdlib>
 #include <type_traits>
@@ -331,15 +334,20 @@ __global__ void __launch_bounds__(kUpdateThreads, 4) mx_state_update_kernel(cons
 // staging fits in shared memory.
 //
 // The state comes through a ring of two stages of four steps per warp (cp.async: a warp synchronises with itself only), so that a
-// step has no global address arithmetic, no copies of prefetched registers, and its loads are one to two stages old.
-// B and C of the slab's (batch, group)s wait in shared memory as [quarter][block] float4; dB = B dt of the
-// current head and C of the current group are kept in registers.
+// step has no global address arithmetic for its loads, no copies of prefetched registers, and its loads are one to two stages old.
+// B and C of the slab's (batch, group)s and dB = B dt of a warp's current head wait in shared memory as [quarter][block] float4 and are read in every
+// step: eight 128-bit loads that share addresses between rows and cost next to nothing beside the arithmetic, for 32 registers.
+// A warp's first stage is as long as makes the others start where heads do.  A whole stage of one head with ordinary exponents asks nothing per
+// step and takes two steps at a time; anything else goes step by step.
+// 272 -> 248 instructions per 16 values (with set-up) and the packed operands of lq_mx_codec.cuh: MX8 1522 -> 1361 us (batch 250, eight layers),
+// 422 -> 381 (64), deterministic rounding 402 -> 354 (60), MX4 417 -> 392 (64).  Four steps at a time, or two copies of two, run slower (1455, 1515).
 // NBLK_T = dstate / 16 when known at compile time (8 for Nemotron-H: all lane and address arithmetic
 // folds to constants), 0 = taken from the arguments.
 // kRefAnyOffset: PHILOX_REF with an offset that is no multiple of 16 (a caller's own).  A block's counters may pass 2^32, so every word is drawn by itself.
 constexpr int kRefAnyOffset = 64;
 constexpr int kRingSteps = 4, kRingStages = 2;
 constexpr int kPartialStride = 36;  // floats of a step's read-out partials: 32 and a shift of one 16-byte bank column
+constexpr int kPartials = (kFastThreads / 32) * kRingSteps * kPartialStride;  // floats of a stage's, per CTA
 template <int BITS, int LAYOUT>
 struct MxRing {
   using IO = MxBlockIO<BITS, LAYOUT>;
@@ -365,8 +373,25 @@ struct MxRing {
   __device__ __forceinline__ static void cp16(uint32_t dst, const uint8_t* src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
   }
+  // WHOLE: with a form of its own for whole stages (MX8, batch 250: 1412 -> 1361 us; the shorter stages of MX4 and the few of the reference's
+  // stream lose a little by the second copy)
+  template <bool WHOLE>
   __device__ __forceinline__ static void issue(Source& s, uint32_t stage, uint32_t lane, int left, int advance = kRingSteps) {
     const uint32_t off = stage * kStage;
+    if (WHOLE && left >= kRingSteps) {  // a whole stage: nothing to ask per chunk
+#pragma unroll
+      for (uint32_t c = 0; c < kRingSteps * kQ / 16; c += 32) cp16(s.dst_q + off + c * 16, s.q + c * 16);
+      if (LAYOUT != LQ_MX_LAYOUT_PACKED) {
+#pragma unroll
+        for (uint32_t c = 0; c < kRingSteps * kM / 16; c += 32) cp16(s.dst_q + off + kOffM + c * 16, s.m + c * 16);
+      }
+      if (lane < (LAYOUT == LQ_MX_LAYOUT_PACKED ? 2 * kEChunks : kEChunks)) cp16(s.dst_em + off, s.em);
+      if (LAYOUT != LQ_MX_LAYOUT_PACKED) s.m += advance * kM;
+      asm volatile("cp.async.commit_group;" ::: "memory");
+      s.q += advance * kQ;
+      s.em += advance * kE;
+      return;
+    }
 #pragma unroll
     for (uint32_t c = 0; c < kRingSteps * kQ / 16; c += 32)
       if (static_cast<int>(((c + lane) * 16) / kQ) < left) cp16(s.dst_q + off + c * 16, s.q + c * 16);
@@ -381,21 +406,20 @@ struct MxRing {
     s.q += advance * kQ;
     s.em += advance * kE;
   }
-  // this lane's block of step k
-  __device__ __forceinline__ static MxRaw read(const uint8_t* stage, uint32_t k, uint32_t lane) {
+  // this lane's block of the step whose mantissas start at `q` + lane * kQBytes and whose exponents at `e` + lane; d: steps further on
+  __device__ __forceinline__ static MxRaw read(const uint8_t* q, const uint8_t* e, const uint8_t* m, uint32_t d) {
     MxRaw r;
-    const uint8_t* q = stage + k * kQ + lane * IO::kQBytes;
     if (IO::kNibbles) {
-      const uint2 v = *reinterpret_cast<const uint2*>(q);
+      const uint2 v = *reinterpret_cast<const uint2*>(q + d * kQ);
       r.q = make_uint4(v.x, v.y, 0u, 0u);
     } else {
-      r.q = *reinterpret_cast<const uint4*>(q);
+      r.q = *reinterpret_cast<const uint4*>(q + d * kQ);
     }
-    r.e = stage[kOffE + k * kE + lane];
+    r.e = e[d * kE];
     if (LAYOUT == LQ_MX_LAYOUT_PACKED) {
-      r.mic = stage[kOffM + k * kM + lane];
+      r.mic = e[kOffM - kOffE + d * kM];
     } else {
-      const uint2 mm = *reinterpret_cast<const uint2*>(stage + kOffM + k * kM + lane * 8);
+      const uint2 mm = *reinterpret_cast<const uint2*>(m + d * kM);
       r.mic = (((mm.x & 0x01010101u) * 0x10204080u) >> 28) | ((((mm.y & 0x01010101u) * 0x10204080u) >> 28) << 4);
     }
     return r;
@@ -406,11 +430,11 @@ template <int BITS, int LAYOUT, int MODE, int NBLK_T>
 __global__ void __launch_bounds__(kFastThreads, kFastCtasPerSm) mx_state_update_fast_kernel(const lq_mx_update_args a, const MxUpdateDerived d) {
   using IO = MxBlockIO<BITS, LAYOUT>;
   using Ring = MxRing<BITS, LAYOUT>;
-  // MX8: a first stage of one step lets every warp start before the other stages queue up in memory (batch 8: 11.0 -> 10.7 us),
-  // and a block is read where it is used (batch 250: 192 -> 190 us, six copies less per step).  MX4 moves half the bytes and is
-  // better off the other way (batch 64: 53.3 -> 51.7 us).
-  constexpr int kFirstSteps = BITS == 8 ? 1 : kRingSteps;
-  constexpr bool kAhead = BITS == 4;
+  // whole stages two steps at a time; the reference's stream draws sixteen words a step, which leaves nothing to gain by a second copy (batch 32: 795 us
+  // against 878)
+  constexpr bool kWhole = MODE != LQ_ROUND_PHILOX_REF && MODE != kRefAnyOffset;
+  constexpr bool kWholeIssue = kWhole && BITS == 8;
+  constexpr int kUnroll = 2;
   extern __shared__ __align__(16) uint8_t smem_fast[];
   const lq_mx_state& s = a.state;
   const int H = s.heads, P = s.dim;
@@ -424,6 +448,9 @@ __global__ void __launch_bounds__(kFastThreads, kFastCtasPerSm) mx_state_update_
   const uint32_t steps_per_head = static_cast<uint32_t>(P / rows_per_step);
   const int heads_per_group = H / a.ngroups;
 
+  uint32_t steps[256 / kFastThreads];  // of the module's constants, which no kernel writes
+#pragma unroll
+  for (int i = 0; i < 256 / kFastThreads; ++i) steps[i] = mx_exp_step<BITS>(threadIdx.x + i * kFastThreads);
   // this CTA's slab: units [u0, u1), rows [R0, R1) of the [batch * heads * dim] row space; the first units_rem CTAs
   // take one unit more than the others
   const uint32_t u0 = blockIdx.x * d.units_per_cta + min(blockIdx.x, d.units_rem);
@@ -440,11 +467,13 @@ __global__ void __launch_bounds__(kFastThreads, kFastCtasPerSm) mx_state_update_
   const int n_heads = static_cast<int>(bh_last - bh_first) + 1;
   const int n_bg = static_cast<int>(fast_div(bh_last, d.div_heads_per_group) - bg_first) + 1;
   float* const bc = reinterpret_cast<float*>(smem_fast + Ring::kBytes);  // per (batch, group): B, then C
-  float* const sx = bc + n_bg * 2 * dstate;  // x of the slab's rows
-  // read-out of the slab's rows: one partial sum per 16-value block when a row spans eight lanes (added up when
-  // the slab's y is written, in the order a butterfly over the eight lanes would add them), else the row's sum
-  float* const sy = sx + n_rows;
-  float* const sdt = sy + (NBLK_T == 8 ? static_cast<int>(n_units) * 2 * kPartialStride : n_rows);   // per touched head
+  float* const sdB = bc + n_bg * 2 * dstate;   // per warp: B dt of its current head, laid out as B
+  // read-out of a stage's rows where a row spans eight lanes: one partial sum per 16-value block, added up when the stage has been worked
+  // through, in the order a butterfly over the eight lanes would add them
+  float* const spart = sdB + (kFastThreads / 32) * dstate;
+  float* const sx = spart + (NBLK_T == 8 ? kPartials : 0);  // x of the slab's rows
+  float* const sy = sx + n_rows;   // <h', C> of the slab's rows
+  float* const sdt = sy + n_rows;  // per touched head
   float* const sdA = sdt + n_heads;
 
   // (batch, head, row) of the slab's first row, once per CTA
@@ -464,6 +493,10 @@ __global__ void __launch_bounds__(kFastThreads, kFastCtasPerSm) mx_state_update_
   const uint32_t my_step0 = step_first + warp * n_units;
   const int n_mine = static_cast<int>(n_units);
   const uint64_t block0 = static_cast<uint64_t>(my_step0) * 32;
+  // its first head, the steps left of it, and the steps of its first stage: what is over stages that start where heads do (if heads are whole stages)
+  const uint32_t bh_mine = fast_div(my_step0, d.div_steps_per_head);
+  int left = static_cast<int>(steps_per_head - (my_step0 - bh_mine * steps_per_head));
+  const int first = ((left - 1) & (kRingSteps - 1)) + 1;
   uint8_t* qptr = static_cast<uint8_t*>(s.q_state) + (block0 + lane) * IO::kQBytes;
   uint8_t* eptr = s.shared_exp + block0 + lane;
   uint8_t* mptr = s.micro_exp + (block0 + lane) * IO::kMicroBytes;
@@ -474,22 +507,18 @@ __global__ void __launch_bounds__(kFastThreads, kFastCtasPerSm) mx_state_update_
   using Table = std::conditional_t<IO::kNibbles, MxPairMasks, MxPairFactors>;
   __shared__ Table table;
   for (int i = threadIdx.x; i < (IO::kNibbles ? 256 : 16); i += kFastThreads) table.fill(i);
+  __shared__ uint32_t exp_step[256];
   uint8_t* const ring = smem_fast + warp * (kRingStages * Ring::kStage);
   typename Ring::Source source(static_cast<uint32_t>(__cvta_generic_to_shared(ring)), static_cast<const uint8_t*>(s.q_state) + block0 * IO::kQBytes,
                                s.shared_exp + block0, s.micro_exp + block0 * IO::kMicroBytes, lane);
   // what the first stages will read, asked for in L2 while the predecessor still runs (a prefetch reads nothing): 10.6 -> 10.1 us at
-  // batch 8
+  // batch 8, ...
   if (lane == 0) {
     const uint32_t ahead = min(n_units, static_cast<uint32_t>(kRingSteps));
     asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(static_cast<const uint8_t*>(s.q_state) + block0 * IO::kQBytes), "r"(ahead * Ring::kQ) : "memory");
     asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(s.shared_exp + block0), "r"(ahead * Ring::kE) : "memory");
     asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(s.micro_exp + block0 * IO::kMicroBytes), "r"(ahead * Ring::kM) : "memory");
   }
-  // everything above is arithmetic on the arguments; from here on memory the predecessor may have written is read
-  pdl_wait();
-  // the first stages travel while the operands below are staged
-  Ring::issue(source, 0, lane, min(n_mine, kFirstSteps), kFirstSteps);
-
   // B / C of (batch, group) bgi, block kb; `which` 0: B, 1: C
   const int n_bc = n_bg * nblk * 2;
   auto bc_source = [&](int i, const void*& base, const int64_t*& st, int& dtype, int& b, int& g, int& kb) {
@@ -506,7 +535,7 @@ __global__ void __launch_bounds__(kFastThreads, kFastCtasPerSm) mx_state_update_
     const int kb = (i >> 1) & (nblk - 1);
     float4* dst = reinterpret_cast<float4*>(bc + ((i >> (lpr_log2 + 1)) * 2 + (i & 1)) * dstate) + kb;
 #pragma unroll
-    for (int k = 0; k < 4; ++k) dst[k * nblk] = make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
+    for (int k = 0; k < 4; ++k) dst[k * nblk] = make_float4(v[4 * k], v[4 * k + 2], v[4 * k + 1], v[4 * k + 3]);
   };
   auto stage_bc = [&](int i) {
     const void* base; const int64_t* st; int dtype, b, g, kb;
@@ -531,6 +560,35 @@ __global__ void __launch_bounds__(kFastThreads, kFastCtasPerSm) mx_state_update_
     sdA[i] = expf(A * dt);
   };
   const int tid = threadIdx.x;
+  // ... and the first round of every operand (batch 8: 10.2 -> 9.9 us a launch in a graph whose operands come from HBM)
+  const auto ask = [](const void* p, int64_t i, int dtype) {  // a hint: nothing is read
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(static_cast<const uint8_t*>(p) + i * (dtype == LQ_F32 ? 4 : 2)) : "memory");
+  };
+  if (tid < n_heads) {
+    const unsigned hh = static_cast<unsigned>(h_first + tid);
+    const unsigned bq = fast_div(hh, d.div_heads);
+    const int h = static_cast<int>(hh - bq * static_cast<unsigned>(H)), b = b_first + static_cast<int>(bq);
+    ask(a.dt, b * a.dt_stride[0] + h * a.dt_stride[1], a.dt_dtype);
+    if (a.dt_bias) ask(a.dt_bias, h * a.dt_bias_stride[0], a.dt_bias_dtype);
+    ask(a.A, h * a.A_stride[0], a.A_dtype);
+  }
+  if (4 * tid < n_rows) {
+    int b, h, p;
+    row_coords(4 * tid, b, h, p);
+    ask(a.x, b * a.x_stride[0] + h * a.x_stride[1] + p * a.x_stride[2], a.x_dtype);
+  }
+  if (tid < n_bc) {
+    const void* base; const int64_t* st; int dtype, b, g, kb;
+    bc_source(tid, base, st, dtype, b, g, kb);
+    ask(base, b * st[0] + g * st[1] + kb * 16 * st[2], dtype);
+  }
+#pragma unroll
+  for (int i = 0; i < 256 / kFastThreads; ++i) exp_step[threadIdx.x + i * kFastThreads] = steps[i];
+  // everything above is arithmetic on the arguments; from here on memory the predecessor may have written is read
+  pdl_wait();
+  // the first stages travel while the operands below are staged
+  Ring::template issue<kWholeIssue>(source, 0, lane, min(n_mine, first), first);
+
   if (NBLK_T == 8 && d.vec) {
     // 16-bit operands in vectors.  The first round of every kind is requested before any of it is used: one latency, not three
     auto x_vec = [&](int i) {
@@ -578,35 +636,36 @@ __global__ void __launch_bounds__(kFastThreads, kFastCtasPerSm) mx_state_update_
   PhiloxStream stream;
   if (kStream) stream.init(static_cast<uint32_t>(lin), 0u, rb.step, rb.layer, d.keys);
 
-  for (int i = 1; i < kRingStages; ++i) Ring::issue(source, i, lane, n_mine - kFirstSteps - (i - 1) * kRingSteps);
+  for (int i = 1; i < kRingStages; ++i) Ring::template issue<kWholeIssue>(source, i, lane, n_mine - first - (i - 1) * kRingSteps);
   __syncthreads();
 
   // current head of this warp: its operands, and the steps left in it
-  const uint32_t bh_mine = fast_div(my_step0, d.div_steps_per_head);
-  uint32_t left = steps_per_head - (my_step0 - bh_mine * steps_per_head);
   const float* head = sdt + (bh_mine - bh_first);
   const uint32_t bg_mine = fast_div(bh_mine, d.div_heads_per_group);
   int h_in_group = static_cast<int>(bh_mine - bg_mine * static_cast<uint32_t>(heads_per_group));
-  const float4* bcp = reinterpret_cast<const float4*>(bc + (bg_mine - bg_first) * 2 * dstate) + blk;
-  float dB[16], Cv[16], dA;
+  const float4* bcp = reinterpret_cast<const float4*>(bc + (bg_mine - bg_first) * 2 * dstate);
+  float4* const dBp = reinterpret_cast<float4*>(sdB + warp * dstate);
+  float dA;
   uint32_t e_max;
   auto read16 = [&](const float4* src, float (&v)[16]) {
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
       const float4 f = src[k * nblk];
-      v[4 * k] = f.x; v[4 * k + 1] = f.y; v[4 * k + 2] = f.z; v[4 * k + 3] = f.w;
+      v[4 * k] = f.x; v[4 * k + 2] = f.y; v[4 * k + 1] = f.z; v[4 * k + 3] = f.w;
     }
   };
   auto load_head = [&]() {
     const float dt = head[0];
     dA = head[n_heads];
     e_max = dA <= 1048576.0f ? 228u : 0u;
-    read16(bcp, dB);
-#pragma unroll
-    for (int i = 0; i < 16; ++i) dB[i] = __fmul_rn(dB[i], dt);
+    __syncwarp();  // the head before has been read
+    for (int i = lane; i < dstate / 4; i += 32) {
+      const float4 f = bcp[i];
+      dBp[i] = make_float4(__fmul_rn(f.x, dt), __fmul_rn(f.y, dt), __fmul_rn(f.z, dt), __fmul_rn(f.w, dt));
+    }
+    __syncwarp();
   };
   load_head();
-  read16(bcp + dstate / 4, Cv);
 
   auto next_head = [&]() {  // B / C change only with the (batch, group)
     left = steps_per_head;
@@ -614,77 +673,114 @@ __global__ void __launch_bounds__(kFastThreads, kFastCtasPerSm) mx_state_update_
     if (++h_in_group == heads_per_group) {
       h_in_group = 0;
       bcp += dstate / 2;
-      read16(bcp + dstate / 4, Cv);
     }
     load_head();
   };
 
   const float* xp = sx + warp * n_mine * rows_per_step + (lane >> lpr_log2);
-  float* yp = NBLK_T == 8 ? sy + warp * n_mine * kPartialStride + lane : sy + warp * n_mine * rows_per_step + (lane >> lpr_log2);
+  float* yp = sy + warp * n_mine * rows_per_step + (NBLK_T == 8 ? lane : lane >> lpr_log2);
+  float* const part = spart + warp * (kRingSteps * kPartialStride);
   uint32_t stage = 0;
+  // One step, the k-th from where the running pointers are: this lane's block; returns its share of <h', C>.
+  const uint8_t *rq = ring, *re = ring, *rm = ring;  // where the current step's block lies in the ring
+  auto step = [&](auto known, int k) {
+    const MxRaw now = Ring::read(rq, re, rm, k);
+    // The reference's stream: the block's words first, four chains at a time, while few registers are in use.  (Drawn where they are used,
+    // the chains ran almost one behind the other: 1 / 4 / 32 sequences 8.3 / 19.1 / 113 -> 7.6 / 17.5 / 103 us a launch.)
+    uint32_t words[16];
+    if (kDrawn) {
+      const MxRoundCtx rc = round_ctx_at<MODE>(rb, lin);
+      PhiloxWords0 words0;
+      words0.init(static_cast<uint32_t>(rc.counter), rc.wrap32 ? 0u : static_cast<uint32_t>(rc.counter >> 32), d.keys);
+#pragma unroll
+      for (int i = 0; i < 16; i += 4) words0.draw<4>(i, d.keys, words + i);
+#pragma unroll
+      for (int i = 0; i < 16; ++i) asm volatile("" : "+r"(words[i]));  // stay here
+    }
+    float hv[16], sd[8], dB[16], Cv[16];
+    mx_decode_scaled<decltype(known)::value>(now.q, now.e, now.mic, dA, e_max, table, hv, sd);
+    read16(dBp + blk, dB);
+    read16(bcp + dstate / 4 + blk, Cv);
+    const float y = mx_update_readout16<IO::kNibbles>(hv, dB, Cv, sd, xp[k * rows_per_step]);  // h' = h exp(A dt) + (B dt) x
+    MxRoundCtx ctx = round_ctx_at<MODE>(rb, lin);
+    ctx.exp_step = exp_step;
+    if (kStream) ctx.stream = &stream;
+    if (kDrawn) ctx.drawn = words;
+    uint32_t codes[4], e_new, mic_new;
+    mx_encode_block<BITS, MODE, IO::kNibbles>(hv, ctx, d.keys, codes, e_new, mic_new);
+    IO::store_ptr(qptr + k * Ring::kQ, eptr + k * Ring::kE, mptr + k * Ring::kM, codes, e_new, mic_new);
+    if (kStream) stream.pa += static_cast<uint64_t>(kPhiloxM0) * dl; else lin += dl;
+    return y;
+  };
+  float* part_k = part;
+  auto advance = [&](int k) {
+    rq += k * Ring::kQ; re += k * Ring::kE; rm += k * Ring::kM;
+    qptr += k * Ring::kQ; eptr += k * Ring::kE; mptr += k * Ring::kM;
+    xp += k * rows_per_step;
+    part_k += k * kPartialStride;
+    if (NBLK_T != 8) yp += k * rows_per_step;
+  };
+  auto put_y = [&](int k, float y) {
+    if (NBLK_T == 8) {
+      part_k[k * kPartialStride] = y;
+    } else {
+      for (int o = nblk >> 1; o > 0; o >>= 1) y += __shfl_xor_sync(0xFFFFFFFFu, y, o);
+      if (blk == 0) yp[k * rows_per_step] = y;
+    }
+  };
 #pragma unroll 1
-  for (int todo = n_mine, len = kFirstSteps; todo > 0; todo -= len, len = kRingSteps) {  // steps to do from this stage on, steps in it
+  for (int todo = n_mine, len = first; todo > 0; todo -= len, len = kRingSteps) {  // steps to do from this stage on, steps in it
     asm volatile("cp.async.wait_group %0;" ::"n"(kRingStages - 1) : "memory");
     __syncwarp();
     const uint8_t* const buf = ring + stage * Ring::kStage;
-    MxRaw cur = {make_uint4(0u, 0u, 0u, 0u), 0u, 0u};
-    if (kAhead) cur = Ring::read(buf, 0, lane);
+    rq = buf + lane * IO::kQBytes;
+    re = buf + Ring::kOffE + lane;
+    rm = buf + Ring::kOffM + lane * IO::kMicroBytes;
+    part_k = part + lane;
+    const int n = min(len, todo);
+    if (left == 0) next_head();
+    // A whole stage of one head whose stored exponents are ordinary (four a lane: nonzero, the two top bits not both set; dA likewise) needs no
+    // question per step.
+    const uint32_t e4 = reinterpret_cast<const uint32_t*>(buf + Ring::kOffE)[lane];
+    const bool odd = ((((e4 - 0x01010101u) & ~e4) | (e4 & (e4 << 1))) & 0x80808080u) != 0u;
+    if (kWhole && n == kRingSteps && left >= kRingSteps && e_max != 0u && !__any_sync(0xFFFFFFFFu, odd)) {
+      left -= kRingSteps;
 #pragma unroll 1
-    for (int k = 0; k < kRingSteps; ++k) {
-      if (k >= min(len, todo)) break;
-      const MxRaw now = kAhead ? cur : Ring::read(buf, k, lane);
-      if (kAhead && k + 1 < kRingSteps) cur = Ring::read(buf, k + 1, lane);  // a step that does not exist: stale bytes, not used
-      if (left == 0) next_head();
-      --left;
-      // The reference's stream: the block's words first, four chains at a time, while few registers are in use.  (Drawn where they are used,
-      // the chains ran almost one behind the other: 1 / 4 / 32 sequences 8.3 / 19.1 / 113 -> 7.6 / 17.5 / 103 us a launch.)
-      uint32_t words[16];
-      if (kDrawn) {
-        const MxRoundCtx rc = round_ctx_at<MODE>(rb, lin);
-        PhiloxWords0 words0;
-        words0.init(static_cast<uint32_t>(rc.counter), rc.wrap32 ? 0u : static_cast<uint32_t>(rc.counter >> 32), d.keys);
+      for (int k0 = 0; k0 < kRingSteps; k0 += kUnroll) {
+        float y[kUnroll];
 #pragma unroll
-        for (int i = 0; i < 16; i += 4) words0.draw<4>(i, d.keys, words + i);
+        for (int k = 0; k < kUnroll; ++k) y[k] = step(std::true_type{}, k);
 #pragma unroll
-        for (int i = 0; i < 16; ++i) asm volatile("" : "+r"(words[i]));  // stay here
+        for (int k = 0; k < kUnroll; ++k) put_y(k, y[k]);
+        advance(kUnroll);
       }
-      float hv[16], sd[8];
-      mx_decode_scaled(now.q, now.e, now.mic, dA, e_max, table, hv, sd);
-      float y = mx_update_readout16<IO::kNibbles>(hv, dB, Cv, sd, xp[k * rows_per_step]);  // h' = h exp(A dt) + (B dt) x
-      MxRoundCtx ctx = round_ctx_at<MODE>(rb, lin);
-      if (kStream) ctx.stream = &stream;
-      if (kDrawn) ctx.drawn = words;
-      uint32_t codes[4], e_new, mic_new;
-      mx_encode_block<BITS, MODE, IO::kNibbles>(hv, ctx, d.keys, codes, e_new, mic_new);
-      IO::store_ptr(qptr + k * Ring::kQ, eptr + k * Ring::kE, mptr + k * Ring::kM, codes, e_new, mic_new);
-      if (NBLK_T == 8) {
-        yp[k * kPartialStride] = y;
-      } else {
-        for (int o = nblk >> 1; o > 0; o >>= 1) y += __shfl_xor_sync(0xFFFFFFFFu, y, o);
-        if (blk == 0) yp[k * rows_per_step] = y;
+    } else {
+#pragma unroll 1
+      for (int k = 0; k < n; ++k) {
+        if (left == 0) next_head();
+        --left;
+        put_y(0, step(std::false_type{}, 0));
+        advance(1);
       }
-      if (kStream) stream.pa += static_cast<uint64_t>(kPhiloxM0) * dl; else lin += dl;
     }
     __syncwarp();  // the stage has been read
-    Ring::issue(source, stage, lane, todo - len - (kRingStages - 1) * kRingSteps);
-    qptr += len * Ring::kQ; eptr += len * Ring::kE; mptr += len * Ring::kM;
-    xp += len * rows_per_step;
-    yp += len * (NBLK_T == 8 ? kPartialStride : rows_per_step);
+    if (NBLK_T == 8 && lane < 4 * kRingSteps) {  // row lane & 3 of step lane / 4; of steps that do not exist: stale sums into rows that do not
+      const float4* p = reinterpret_cast<const float4*>(part + (lane >> 2) * kPartialStride + (lane & 3) * 8);
+      const float4 p0 = p[0], p1 = p[1];
+      if (static_cast<int>(lane >> 2) < n) yp[0] = ((p0.x + p1.x) + (p0.z + p1.z)) + ((p0.y + p1.y) + (p0.w + p1.w));
+    }
+    Ring::template issue<kWholeIssue>(source, stage, lane, todo - len - (kRingStages - 1) * kRingSteps);
+    if (NBLK_T == 8) yp += n * rows_per_step;
     stage ^= 1u;
   }
   __syncthreads();
   // y = <h', C> + D x (* z), stored for the whole slab at once
-  const auto row_sum = [](const float4& p0, const float4& p1) {  // in the butterfly's order
-    return ((p0.x + p1.x) + (p0.z + p1.z)) + ((p0.y + p1.y) + (p0.w + p1.w));
-  };
   if (NBLK_T == 8 && d.vec) {  // a thread takes the four rows of a step
     for (int i = tid; 4 * i < n_rows; i += kFastThreads) {
       int b, h, p;
       row_coords(4 * i, b, h, p);
-      const float4* part = reinterpret_cast<const float4*>(sy + i * kPartialStride);
-      float y[4];
-#pragma unroll
-      for (int r = 0; r < 4; ++r) y[r] = row_sum(part[2 * r], part[2 * r + 1]);
+      const float4 sum = reinterpret_cast<const float4*>(sy)[i];
+      float y[4] = {sum.x, sum.y, sum.z, sum.w};
       if (a.D) {
         const float D = load_as_float(a.D, h * a.D_stride[0], a.D_dtype);
         const float4 x = reinterpret_cast<const float4*>(sx)[i];
@@ -705,13 +801,7 @@ __global__ void __launch_bounds__(kFastThreads, kFastCtasPerSm) mx_state_update_
   for (int i = tid; i < n_rows; i += kFastThreads) {
     int b, h, p;
     row_coords(i, b, h, p);
-    float y;
-    if (NBLK_T == 8) {
-      const float4* part = reinterpret_cast<const float4*>(sy + (i >> 2) * kPartialStride + (i & 3) * 8);
-      y = row_sum(part[0], part[1]);
-    } else {
-      y = sy[i];
-    }
+    float y = sy[i];
     if (a.D) y += sx[i] * load_as_float(a.D, h * a.D_stride[0] + p * a.D_stride[1], a.D_dtype);
     if (a.z) y *= load_as_float(a.z, b * a.z_stride[0] + h * a.z_stride[1] + p * a.z_stride[2], a.z_dtype);
     store_from_float(a.out, b * a.out_stride[0] + h * a.out_stride[1] + p * a.out_stride[2], a.out_dtype, y);
@@ -906,17 +996,18 @@ template <int BITS, int LAYOUT>
 static void launch_update_mode(const lq_mx_update_args& a, const MxUpdateDerived& d, cudaStream_t st) {
   using IO = MxBlockIO<BITS, LAYOUT>;
   if (fast_update_applies<BITS, LAYOUT>(a, d)) {
-    // One wave of resident CTAs when a CTA's slab stays within max_units units (its x / y staging: 40 bytes per row, as much as
-    // lets kFastCtasPerSm CTAs share an SM's 228 KB); more waves of equally sized slabs otherwise.
+    // One wave of resident CTAs when a CTA's slab stays within max_units units (its x / y staging: 8 bytes per row, as much as
+    // lets kFastCtasPerSm CTAs share an SM's 228 KB); more waves of equally sized slabs otherwise.  Longer slabs have less set-up: batch 250
+    // 1385 us with 64 units at most, 1372 with 80 to 192.
     const int rows_per_pass = (32 >> d.lpr_log2) * (kFastThreads / 32);
-    const size_t row_bytes = sizeof(float) * (d.nblk == 8 ? 1 + kPartialStride / 4 : 2);
     const auto smem_of = [&](uint64_t units) {
       const uint64_t heads = units / (a.state.dim / rows_per_pass) + 2, groups = heads / (a.state.heads / a.ngroups) + 2;
-      return MxRing<BITS, LAYOUT>::kBytes + row_bytes * units * rows_per_pass + sizeof(float) * (2 * heads + 2 * a.state.dstate * groups);
+      return MxRing<BITS, LAYOUT>::kBytes + sizeof(float) * (2 * units * rows_per_pass + 2 * heads + a.state.dstate * (2 * groups + kFastThreads / 32) +
+                                                             (d.nblk == 8 ? kPartials : 0));
     };
-    const size_t budget = 228 * 1024 / kFastCtasPerSm - 1024 - (IO::kNibbles ? sizeof(MxPairMasks) : sizeof(MxPairFactors));
-    uint64_t max_units = 64;
-    if (const char* env = getenv("LQ_MX_MAX_UNITS")) max_units = std::min(80, std::max(1, atoi(env)));  // tuning aid
+    const size_t budget = 228 * 1024 / kFastCtasPerSm - 1024 - 1024 - (IO::kNibbles ? sizeof(MxPairMasks) : sizeof(MxPairFactors));
+    uint64_t max_units = 192;
+    if (const char* env = getenv("LQ_MX_MAX_UNITS")) max_units = std::min(400, std::max(1, atoi(env)));  // tuning aid
     while (max_units > 1 && smem_of(max_units) > budget) --max_units;
     MxUpdateDerived dd = d;
     const auto vec16 = [](const void* p, int dtype, const int64_t* st, int mult) {  // 16-bit, innermost contiguous, `mult` elements aligned

@@ -516,3 +516,39 @@ def test_supplied_words_written_by_the_launch_before(stream):
         res.append(outs + [cache.shared_exp, cache.micro_exp])
     for a, b in zip(*res):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("bits,layout", [(8, "packed"), (8, "reference"), (4, "packed"), (4, "reference")])
+@pytest.mark.parametrize("stochastic", [True, False])
+@pytest.mark.parametrize("shape", [
+    (3, 4, 64, 128, 2),      # heads of four whole ring stages, slabs that start anywhere in one
+    (7, 16, 24, 128, 4),     # heads of six steps: a stage holds the end of one and the start of the next
+    (40, 24, 40, 128, 8),    # heads of ten steps, slabs of several heads
+    (2, 5, 32, 64, 5),       # rows of four blocks: sums by shuffles
+    (224, 128, 64, 128, 8),  # more than one wave of slabs
+])
+def test_whole_stages_equal_general_kernel(bits, layout, stochastic, shape):
+    """Ring stages that are worked through without a question per step, beside stages that are not: stored exponents on either side of what
+    counts as ordinary, a factor exp(A dt) beyond 2**20 and heads that end inside a stage.  The fp32 dump sends the second run to the general kernel."""
+    m = mk()
+    b, h, p, n, g = shape
+    gen = torch.Generator(device=dev()).manual_seed(b + p)
+    rnd = lambda *s: torch.randn(*s, generator=gen, device=dev())
+    first = m.allocate_state_kernel_cache(rnd(b, h, p, n).to(torch.bfloat16), 16, bits, layout=layout)
+    odd = torch.tensor([0, 1, 191, 192, 229, 230, 255], dtype=torch.uint8, device=dev())
+    flat = first.shared_exp.view(-1)
+    where = torch.randint(0, flat.numel(), (min(200, flat.numel() // 300 + 1),), generator=gen, device=dev())
+    flat[where] = odd[torch.arange(where.numel(), device=dev()) % odd.numel()]
+    x, B, C = (v.to(torch.bfloat16) for v in (rnd(b, h, p), rnd(b, g, n), rnd(b, g, n)))
+    dt = rnd(b, h).to(torch.bfloat16)[..., None].expand(b, h, p)
+    A = -torch.exp(rnd(h))
+    A[h // 2] = 60.0  # exp(A dt) beyond 2**20 wherever softplus(dt) is above 0.24
+    A = A[:, None, None].expand(h, p, n)
+    res = []
+    for general in (False, True):
+        cache = m.MambaStateKernelCache(first.q_state.clone(), first.shared_exp.clone(), first.micro_exp.clone(), format_bits=bits, layout=first.layout)
+        extra = dict(h_out=torch.empty((b, h, p, n), dtype=torch.float32, device=dev())) if general else {}
+        y = m.mx_state_selective_update(cache, x, dt, A, B, C, dt_softplus=True, stochastic=stochastic, seed=9, rng_stream="layered" if stochastic else None, **extra)
+        res.append((y.view(torch.int16), cache.q_state, cache.shared_exp, cache.micro_exp))
+    for got, want in zip(*res):
+        assert torch.equal(got, want)
