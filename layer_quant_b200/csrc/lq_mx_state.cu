@@ -438,7 +438,9 @@ __global__ void __launch_bounds__(kFastThreads, kFastCtasPerSm) mx_state_update_
   extern __shared__ __align__(16) uint8_t smem_fast[];
   const lq_mx_state& s = a.state;
   const int H = s.heads, P = s.dim;
-  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  // the warp's number from one lane: the compiler keeps what follows from it in uniform registers (24 layers of batch 1 of the reference's stream
+  // 175 -> 172 us, eight of batch 60 with deterministic rounding 354 -> 345)
+  const uint32_t lane = threadIdx.x & 31, warp = __shfl_sync(0xFFFFFFFFu, threadIdx.x >> 5, 0);
   const int nblk = NBLK_T ? NBLK_T : d.nblk;
   const int lpr_log2 = NBLK_T == 8 ? 3 : d.lpr_log2;
   const int dstate = NBLK_T ? NBLK_T * 16 : s.dstate;

@@ -552,3 +552,23 @@ def test_whole_stages_equal_general_kernel(bits, layout, stochastic, shape):
         res.append((y.view(torch.int16), cache.q_state, cache.shared_exp, cache.micro_exp))
     for got, want in zip(*res):
         assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("layout", ["reference", "packed"])
+@pytest.mark.parametrize("bits", [8, 4])
+def test_micro_exponent_edges(bits, layout):
+    """Pair maxima at M base and one unit in the last place on either side, over the exponents a quantiser emits, against the oracle."""
+    m, top = (63.0, 100.0) if bits == 8 else (7.0, 11.0)  # a block maximum of `top` units has the unit as its base
+    rows = []
+    for e in [*range(-96, 116, 4), 115, 116, 117, 118, 119]:
+        edge = np.float32(m * 2.0 ** e)
+        row = np.zeros(16, np.float32)
+        row[15] = top * 2.0 ** e
+        row[[0, 3, 5, 6, 8, 11]] = [edge, np.nextafter(edge, np.float32(np.inf)), np.nextafter(edge, np.float32(0)), -edge,
+                                    -np.nextafter(edge, np.float32(np.inf)), -np.nextafter(edge, np.float32(0))]
+        rows.append(row)
+    vals = np.stack(rows)
+    q, e, mi, _ = quantize(vals, bits, layout, 1)  # half even
+    for got, want in zip((q, e, mi), oracle.mx_encode(vals, int(m), "half_even")):
+        assert np.array_equal(got, want)
+    assert mi[:, :8].tolist() == [[0, 1, 0, 0, 1, 0, 0, 1]] * len(rows)
