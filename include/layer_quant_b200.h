@@ -217,7 +217,8 @@ int lq_int4_decode_attn(const lq_int4_decode_args* args, void* cuda_stream);
  * A buffer may be reused for any problem it is large enough for.                               */
 size_t lq_int4_decode_workspace_bytes(int32_t batch, int32_t q_heads, int32_t kv_heads, int32_t head_dim,
                                       int32_t max_splits);
-/* The split count the library would pick for this problem on the current device (>= 1). */
+/* Room for the split count that the library picks for this problem on the current device with splits = 0 (>= 1): the most over its
+ * kernels, so a workspace of this many splits is always enough. */
 int32_t lq_int4_decode_auto_splits(int32_t batch, int32_t kv_heads, int32_t seq_len);
 
 /* Causal attention of q_len consecutive query positions over the packed cache, which already holds

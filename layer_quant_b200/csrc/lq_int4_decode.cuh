@@ -1,5 +1,5 @@
-// q_len = 1 GQA decode attention over the packed INT4 KV cache: one CTA (4 warps) per (split, kv head, batch), each warp on a
-// contiguous quarter of the CTA's tokens with a ring of its own.
+// q_len = 1 GQA decode attention over the packed INT4 KV cache: one CTA per (split, kv head, batch), of four warps or, where an SM gets one CTA anyway, of as
+// many as an SM holds, each warp on a contiguous part of the CTA's tokens with a ring of its own.
 //
 // The arithmetic of a 16-token step is that of lq_int4_mma.cuh (S^T = K Q^T and O^T = V^T (P v_scale)^T on mma.sync, the unpacked
 // nibbles as A operand in registers); what differs is everything around it.  A warp stages 32 tokens at a time with cp.async and
@@ -16,15 +16,15 @@ namespace mma {
 
 constexpr int kStageTok = 32, kStagesD = 3;
 
-template <int GS>
+template <int GS, int NW>
 struct WarpStage {
   static constexpr int kG = kD / GS;
   static constexpr int kCodeBytes = kStageTok * 64, kScaleBytes = kStageTok * kG * 4;
   static constexpr int kKc = 0, kVc = kCodeBytes, kKs = 2 * kCodeBytes, kVs = kKs + kScaleBytes;
   static constexpr int kBytes = kVs + kScaleBytes;
   static constexpr int kWarp = kStagesD * kBytes;
-  static constexpr int kMergeBytes = kWarpsM * 8 * kD * 4;  // [warps][heads][128] floats, later the split factors
-  static constexpr int kSmem = (kWarpsM * kWarp > kMergeBytes ? kWarpsM * kWarp : kMergeBytes) + TileLayout<GS>::kNewBytes;
+  static constexpr int kMergeBytes = NW * 8 * kD * 4;  // [warps][heads][128] floats, later the split factors
+  static constexpr int kSmem = (NW * kWarp > kMergeBytes ? NW * kWarp : kMergeBytes) + TileLayout<GS>::kNewBytes;
 };
 
 __device__ __forceinline__ void mma_f16_from(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1,
@@ -53,11 +53,15 @@ __device__ __forceinline__ uint32_t nib_pair_f16_plus72(uint32_t x) { return and
 enum QueryMode { kQBf16 = 0, kQF16 = 1, kQF32 = 2 };
 
 // QM: a bf16 query is multiplied as it is; an fp16 query with the K codes in fp16; an fp32 query as bf16 hi + lo (two products).
-template <int R, int GS, bool HAS_MASK, int QM>
-__global__ void __launch_bounds__(kThreadsM, (R <= 4 && QM != kQF32) ? 3 : 2) int4_decode_warp_kernel(const DecodeParams p) {
+// NW: warps of the CTA, 4, or as many as an SM holds (kWideWarps; the rule and what it gives stand at wide_pays).
+template <int R, int QM>
+constexpr int kWideWarps = R <= 4 && QM != kQF32 ? 12 : 8;
+template <int R, int GS, bool HAS_MASK, int QM, int NW>
+__global__ void __launch_bounds__(NW * 32, kWideWarps<R, QM> / NW) int4_decode_warp_kernel(const DecodeParams p) {
   static_assert(R <= 8, "at most eight head columns");
+  constexpr int kWarpsM = NW, kThreadsM = NW * 32;
   constexpr bool QSPLIT = QM == kQF32;
-  using L = WarpStage<GS>;
+  using L = WarpStage<GS, NW>;
   using N = TileLayout<GS>;
   constexpr int G = L::kG;
   extern __shared__ __align__(128) uint8_t smem[];
@@ -100,7 +104,8 @@ __global__ void __launch_bounds__(kThreadsM, (R <= 4 && QM != kQF32) ? 3 : 2) in
   {
     const int cta_begin = min(split * rl.tiles_per_split * kTileTok, rl.ctx_len);
     const int cta_end = min(cta_begin + rl.tiles_per_split * kTileTok, rl.ctx_len);
-    const int steps = (cta_end - cta_begin + 15) >> 4, each = steps >> 2, more = steps & 3;
+    const unsigned steps = static_cast<unsigned>(cta_end - cta_begin + 15) >> 4;
+    const int each = static_cast<int>(steps / NW), more = static_cast<int>(steps % NW);
     tok = cta_begin + 16 * (warp * each + min(warp, more));
     tok_end = min(tok + 16 * (each + (warp < more ? 1 : 0)), cta_end);
   }

@@ -728,11 +728,49 @@ static size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 constexpr size_t kMaxTickets = 65536;
 constexpr size_t kTicketBytes = kMaxTickets * sizeof(int32_t);
 
+// Whether a decode launch is a programmatic dependent.  One hides launch, set-up and the way to the first tiles (2 us of a launch of 8 to 10).
+// Left to itself it loses more than that: its CTAs are placed where the predecessor leaves room, several to an SM, and the launch takes as long as the fullest
+// SM.  So it asks for so much shared memory that an SM holds no more of its CTAs than an even deal puts there (kHoldsOne, kHoldsTwo; three are
+// what it holds anyway).  us of a pair of launches, a predecessor and 8 x 1024 in one split (16 tiles x 64 CTAs): ordinary / dependent / dependent with an SM
+// each, behind a state update of batch 8 22.7 / 28.6 / 21.4, an append of 8 x 1024 22.6 / 24.2 / 20.1, an unquantised update of batch 32 40.2 / 44.7 / 38.1,
+// a GEMM 21.6 / 19.6 / 19.7, 16 x 8191 61.5 / 61.5 / 57.9, itself 12.4 / 10.8 / 10.6; 24 x 320 (5 x 192, two per SM) behind the update of batch 8
+// 20.6 / 20.0 / 18.7, itself 10.3 / 9.3 / 8.2; 40 x 200 (4 x 320) 20.6 / - / 18.8 and 10.3 / - / 8.4.  Recorded in a graph the gain is smaller, and behind long
+// kernels without a trigger a dependent costs up to 0.5 us more than it saves at 5 tiles, 0.8 at 16 tiles x 64 CTAs (behind 16 x 8191 55.8 -> 56.6), 1.0 at
+// 12 x 96, but up to 1.9 at 16 x 96, 2.0 at 8 x 128, 2.4 at 8 x 288: hence the tiles.  Short CTAs in any number even out (103 x 19, 1 x 824, behind the update of
+// batch 8 22.7 -> 20.7, 200 x 320, 5 x 1600, 51.9 -> 50.2, themselves 12.4 -> 10.6 and 40.9 -> 39.2).
+// Dependents of a decode launch do not start early (no trigger): they would lie around it in the same way (16 x 8191 and a dependent of 64 CTAs
+// 55.5 -> 60.1 recorded, 1 x 1024 and a state update of batch 60 59.2 -> 61.9, 200 x 256 and an update of batch 250 230.6 -> 233.5).
+constexpr size_t kHoldsOne = 116 * 1024, kHoldsTwo = 77 * 1024;  // of an SM's 228 KB, with 1 KB for each CTA
+static bool dependent_pays(int tiles, int64_t ctas) {
+  const int sms = sm_count();
+  return tiles <= (2 * ctas <= sms ? 16 : 3 * ctas <= 2 * sms ? 12 : 5);
+}
+
+// The tensor-pipe kernel covers group sizes 32 / 64 / 128 (a 16-byte chunk of a row never straddles
+// two groups); group size 16 stays on the CUDA-core kernel.  LQ_INT4_KERNEL=cuda_core forces the
+// latter (A/B measurements).
+static bool use_mma_kernel(int gs) {
+  static const bool forced_off = [] {
+    const char* e = getenv("LQ_INT4_KERNEL");
+    return e != nullptr && strcmp(e, "cuda_core") == 0;
+  }();
+  return !forced_off && (gs == 32 || gs == 64 || gs == 128);
+}
+
+// Whether a decode launch has CTAs of as many warps as an SM holds in place of four: where an SM gets one CTA anyway and its warps have work.  A tile then
+// takes 0.255 us in place of 0.352, and one split of a (batch, kv head) does where three shared an SM and were merged.  us, four warps with the best split
+// count / as many as an SM holds: 16 x 8191 46.1 / 43.0, 18 x 20000 99.0 / 90.2, 18 x 4000 28.8 / 26.7, 1 x 131072 45.0 / 43.0, 7 x 500 (8 tiles) 7.5 / 7.0, 1 x 300
+// (5) 6.4 / 5.9; with fewer tiles the other way: 7 x 200 (4) 5.9 / 6.2, 1 x 1024 in eight splits (2) 7.6 / 8.2.
+static bool wide_pays(int tiles, int64_t ctas) { return tiles >= 5 && ctas <= sm_count(); }
+
 // Split count from a cost model in microseconds, fitted to 360 measurements on B200 (batch 1 to 200, 33 to 131072 tokens, 1 to 64
-// splits; 6 % rms, the choice within 1 % of the best on average).  An SM holds three CTAs; a 64-token tile of one, two or
-// three at a time takes 0.35, 0.57 and 0.77 us; a further wave of CTAs pays its set-up again, more CTAs per SM start
-// later, and more than one split pays the merge.
-static int pick_splits(int batch, int kv_heads, int ctx_len) {
+// splits; 6 % rms, the choice within 1 % of the best on average) and to 290 more with CTAs of twelve warps (batch 1 to 18, 200 to 131072 tokens).  An SM holds
+// three CTAs; a 64-token tile of one, two or
+// three at a time takes 0.35, 0.57 and 0.77 us, of one of twelve warps 0.255; a further wave of CTAs pays its set-up again, more CTAs per SM start
+// later, and more than one split pays the merge.  A dependent launch hides about 1.5 us: 4 x 2048 in eight splits 9.95 us, in the four chosen without this
+// 12.3; 2 x 4096 in 16 10.2 (12.3 in eight), 1 x 8192 in 32 10.6 (12.3 in 18).
+// tensor: of the tensor-pipe kernel; the CUDA-core kernel has neither.
+static int pick_splits(int batch, int kv_heads, int ctx_len, bool tensor) {
   const int ntiles = std::max(1, (ctx_len + kTile - 1) / kTile);
   const int sms = sm_count();
   const int64_t base = static_cast<int64_t>(batch) * kv_heads;
@@ -745,8 +783,10 @@ static int pick_splits(int batch, int kv_heads, int ctx_len) {
     if ((ntiles + tps - 1) / tps != s) continue;  // would leave empty splits
     const int64_t per_sm = (base * s + sms - 1) / sms;  // CTAs on the busiest SM
     const int64_t waves = (per_sm + 2) / 3;
-    const double cost = 3.5 + (s > 1 ? 3.2 + 0.016 * s : 0.0) + tps * ((per_sm / 3) * kTileUs[3] + kTileUs[per_sm % 3]) + 4.0 * (waves - 1) +
-                        1.1 * std::min<int64_t>(per_sm, 3);
+    double cost = 3.5 + (s > 1 ? 3.2 + 0.016 * s : 0.0);
+    if (tensor && wide_pays(tps, base * s)) cost += 0.255 * tps + std::min(2.2, 0.1 * tps) + 1.1;
+    else cost += tps * ((per_sm / 3) * kTileUs[3] + kTileUs[per_sm % 3]) + 4.0 * (waves - 1) + 1.1 * std::min<int64_t>(per_sm, 3);
+    if (tensor && dependent_pays(tps, base * s)) cost -= 1.5;
     // Ties go to fewer splits; in launches of 250 us and more HBM evens out what the deal to the SMs leaves uneven: us with the choice of
     // 0.98 / of 0.999: batch 16 x 65536 269 / 278, 32 x 32768 281 / 289, 56 x 32768 456 / 477, 64 x 32768 511 / 535; below, 48 x 16384 (cost
     // 203) 236 / 214, 96 x 8192 (207) 233 / 220.
@@ -772,24 +812,6 @@ static int pick_splits(int batch, int kv_heads, int ctx_len) {
     }                                                                                                               \
   } while (0)
 
-// Whether a decode launch is a programmatic dependent.  One hides launch, set-up and the way to the first tiles (2 us of a launch of 8 to 10).
-// Left to itself it loses more than that: its CTAs are placed where the predecessor leaves room, several to an SM, and the launch takes as long as the fullest
-// SM.  So it asks for so much shared memory that an SM holds no more of its CTAs than an even deal puts there (kHoldsOne, kHoldsTwo; three are
-// what it holds anyway).  us of a pair of launches, a predecessor and 8 x 1024 in one split (16 tiles x 64 CTAs): ordinary / dependent / dependent with an SM
-// each, behind a state update of batch 8 22.7 / 28.6 / 21.4, an append of 8 x 1024 22.6 / 24.2 / 20.1, an unquantised update of batch 32 40.2 / 44.7 / 38.1,
-// a GEMM 21.6 / 19.6 / 19.7, 16 x 8191 61.5 / 61.5 / 57.9, itself 12.4 / 10.8 / 10.6; 24 x 320 (5 x 192, two per SM) behind the update of batch 8
-// 20.6 / 20.0 / 18.7, itself 10.3 / 9.3 / 8.2; 40 x 200 (4 x 320) 20.6 / - / 18.8 and 10.3 / - / 8.4.  Recorded in a graph the gain is smaller, and behind long
-// kernels without a trigger a dependent costs up to 0.5 us more than it saves at 5 tiles, 0.8 at 16 tiles x 64 CTAs (behind 16 x 8191 55.8 -> 56.6), 1.0 at
-// 12 x 96, but up to 1.9 at 16 x 96, 2.0 at 8 x 128, 2.4 at 8 x 288: hence the tiles.  Short CTAs in any number even out (103 x 19, 1 x 824, behind the update of
-// batch 8 22.7 -> 20.7, 200 x 320, 5 x 1600, 51.9 -> 50.2, themselves 12.4 -> 10.6 and 40.9 -> 39.2).
-// Dependents of a decode launch do not start early (no trigger): they would lie around it in the same way (16 x 8191 and a dependent of 64 CTAs
-// 55.5 -> 60.1 recorded, 1 x 1024 and a state update of batch 60 59.2 -> 61.9, 200 x 256 and an update of batch 250 230.6 -> 233.5).
-constexpr size_t kHoldsOne = 116 * 1024, kHoldsTwo = 77 * 1024;  // of an SM's 228 KB, with 1 KB for each CTA
-static bool dependent_pays(int tiles, int64_t ctas) {
-  const int sms = sm_count();
-  return tiles <= (2 * ctas <= sms ? 16 : 3 * ctas <= 2 * sms ? 12 : 5);
-}
-
 template <int R, int GS>
 static int launch_decode(const DecodeParams& p, cudaStream_t st) {
   using L = StageLayout<GS>;
@@ -806,39 +828,36 @@ static int launch_decode(const DecodeParams& p, cudaStream_t st) {
   return LQ_OK;
 }
 
-template <int R, int GS>
+template <int R, int GS, bool MASK, int QM>
 static int launch_decode_mma(DecodeParams p, cudaStream_t st) {
-  static_assert(mma::WarpStage<GS>::kSmem <= kHoldsTwo, "the sizes for one and two CTAs are not smaller than what the kernel uses");
   const dim3 grid(p.splits, p.a.cache.kv_heads, p.a.cache.batch);
   const int64_t ctas = static_cast<int64_t>(grid.x) * grid.y * grid.z;
   // (with a device counter the tiles are not known here)
   p.dependent = p.a.seq_len_counter == nullptr && dependent_pays(p.tiles_per_split, ctas);
-  const size_t smem = !p.dependent || ctas > 2 * sm_count() ? mma::WarpStage<GS>::kSmem : ctas > sm_count() ? kHoldsTwo : kHoldsOne;
-#define LQ_MMA_LAUNCH(MASK_, QM_)                                                                                   \
-  do {                                                                                                              \
-    LQ_SET_SMEM_ONCE((mma::int4_decode_warp_kernel<R, GS, MASK_, QM_>), kHoldsOne);                                 \
-    if (p.dependent) LQ_CHECK_CUDA(launch_dependent(mma::int4_decode_warp_kernel<R, GS, MASK_, QM_>, grid, mma::kThreadsM, smem, st, p)); \
-    else mma::int4_decode_warp_kernel<R, GS, MASK_, QM_><<<grid, mma::kThreadsM, smem, st>>>(p);                    \
-  } while (0)
-  if (p.a.mask) {
-    if (p.a.dtype == LQ_BF16) LQ_MMA_LAUNCH(true, mma::kQBf16); else if (p.a.dtype == LQ_F16) LQ_MMA_LAUNCH(true, mma::kQF16); else LQ_MMA_LAUNCH(true, mma::kQF32);
-  } else {
-    if (p.a.dtype == LQ_BF16) LQ_MMA_LAUNCH(false, mma::kQBf16); else if (p.a.dtype == LQ_F16) LQ_MMA_LAUNCH(false, mma::kQF16); else LQ_MMA_LAUNCH(false, mma::kQF32);
-  }
-#undef LQ_MMA_LAUNCH
-  LQ_CHECK_CUDA(cudaGetLastError());
-  return LQ_OK;
+  const auto launch = [&](auto warps) {
+    constexpr int NW = decltype(warps)::value;
+    constexpr size_t kSmem = mma::WarpStage<GS, NW>::kSmem;
+    static_assert(NW > 4 || kSmem <= kHoldsTwo, "the sizes for one and two CTAs are not smaller than what the kernel uses");
+    const size_t smem = NW > 4 || !p.dependent || ctas > 2 * sm_count() ? kSmem : ctas > sm_count() ? kHoldsTwo : kHoldsOne;
+    const auto kernel = mma::int4_decode_warp_kernel<R, GS, MASK, QM, NW>;
+    LQ_SET_SMEM_ONCE(kernel, std::max(kSmem, kHoldsOne));
+    if (p.dependent) LQ_CHECK_CUDA(launch_dependent(kernel, grid, NW * 32, smem, st, p));
+    else kernel<<<grid, NW * 32, smem, st>>>(p);
+    LQ_CHECK_CUDA(cudaGetLastError());
+    return static_cast<int>(LQ_OK);
+  };
+  if (wide_pays(p.tiles_per_split, ctas)) return launch(std::integral_constant<int, mma::kWideWarps<R, QM>>{});
+  return launch(std::integral_constant<int, 4>{});
 }
 
-// The tensor-pipe kernel covers group sizes 32 / 64 / 128 (a 16-byte chunk of a row never straddles
-// two groups); group size 16 stays on the CUDA-core kernel.  LQ_INT4_KERNEL=cuda_core forces the
-// latter (A/B measurements).
-static bool use_mma_kernel(int gs) {
-  static const bool forced_off = [] {
-    const char* e = getenv("LQ_INT4_KERNEL");
-    return e != nullptr && strcmp(e, "cuda_core") == 0;
-  }();
-  return !forced_off && (gs == 32 || gs == 64 || gs == 128);
+template <int R, int GS>
+static int launch_decode_mma(const DecodeParams& p, cudaStream_t st) {
+  if (p.a.mask) {
+    if (p.a.dtype == LQ_BF16) return launch_decode_mma<R, GS, true, mma::kQBf16>(p, st);
+    return p.a.dtype == LQ_F16 ? launch_decode_mma<R, GS, true, mma::kQF16>(p, st) : launch_decode_mma<R, GS, true, mma::kQF32>(p, st);
+  }
+  if (p.a.dtype == LQ_BF16) return launch_decode_mma<R, GS, false, mma::kQBf16>(p, st);
+  return p.a.dtype == LQ_F16 ? launch_decode_mma<R, GS, false, mma::kQF16>(p, st) : launch_decode_mma<R, GS, false, mma::kQF32>(p, st);
 }
 
 template <int R>
@@ -922,7 +941,7 @@ LQ_EXPORT size_t lq_int4_decode_workspace_bytes(int32_t batch, int32_t q_heads, 
 
 LQ_EXPORT int32_t lq_int4_decode_auto_splits(int32_t batch, int32_t kv_heads, int32_t seq_len) {
   if (batch <= 0 || kv_heads <= 0 || seq_len <= 0) return 1;
-  return pick_splits(batch, kv_heads, seq_len);
+  return std::max(pick_splits(batch, kv_heads, seq_len, true), pick_splits(batch, kv_heads, seq_len, false));
 }
 
 LQ_EXPORT int lq_int4_decode_attn(const lq_int4_decode_args* args, void* cuda_stream) {
@@ -959,7 +978,7 @@ LQ_EXPORT int lq_int4_decode_attn(const lq_int4_decode_args* args, void* cuda_st
   p.a = a;
   p.ctx_len = a.seq_len - (a.k_new ? 1 : 0);
   const int ntiles = std::max(1, (p.ctx_len + kTile - 1) / kTile);
-  int splits = a.splits > 0 ? a.splits : pick_splits(c.batch, c.kv_heads, std::max(p.ctx_len, 1));
+  int splits = a.splits > 0 ? a.splits : pick_splits(c.batch, c.kv_heads, std::max(p.ctx_len, 1), use_mma_kernel(c.group_size));
   splits = std::max(1, std::min(std::min(splits, ntiles), mma::kMaxSplitsM));  // the merge holds one factor per split in shared memory
   int tps = (ntiles + splits - 1) / splits;
   splits = (ntiles + tps - 1) / tps;  // no empty splits
@@ -1158,7 +1177,7 @@ LQ_EXPORT int lq_int4_decode_attn_static(const lq_int4_decode_args* args, void* 
   int splits = a.splits;
   const int ctx_len = std::max(a.seq_len - (a.k_new ? 1 : 0), 1);
   if (splits <= 0) {  // library's choice, kept inside what the built-in scratch can hold
-    splits = pick_splits(c.batch, c.kv_heads, ctx_len);
+    splits = pick_splits(c.batch, c.kv_heads, ctx_len, use_mma_kernel(c.group_size));
     if (splits > max_splits) splits = static_cast<int>(std::max<int64_t>(max_splits, 1));
   } else {
     // an explicit count is used as lq_int4_decode_attn would use it: never more splits than 64-token tiles, nor than 128

@@ -464,14 +464,14 @@ PyObject* decode_attn(PyObject*, PyObject* const* a, Py_ssize_t n) {
     if (k == nullptr || k->scalar_type() != at::kLong || k->numel() != 1) return none();
     d.seq_len_counter = static_cast<const uint64_t*>(k->data_ptr());
   }
+  d.splits = static_cast<int32_t>(std::min<int64_t>(std::max<int64_t>(splits, 0), INT32_MAX));  // 0: the library's choice, for which the scratch below has room
   if (splits <= 0) {
     const c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(c.device));  // the rule asks for its number of SMs
     splits = L.int4_decode_auto_splits(batch, d.cache.kv_heads, std::max<int64_t>(seq_len - (d.k_new ? 1 : 0), 1));
   }
-  d.splits = static_cast<int32_t>(std::min<int64_t>(splits, INT32_MAX));
   at::Tensor ws;  // held until the launch is in the stream
   if (splits > 1) {
-    ws = workspace(c.device, c.stream(), L.int4_decode_workspace_bytes(batch, heads, d.cache.kv_heads, dim, d.splits));
+    ws = workspace(c.device, c.stream(), L.int4_decode_workspace_bytes(batch, heads, d.cache.kv_heads, dim, static_cast<int32_t>(std::min<int64_t>(splits, INT32_MAX))));
     d.workspace = ws.data_ptr();
     d.workspace_bytes = ws.numel();
   }

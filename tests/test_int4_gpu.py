@@ -848,3 +848,40 @@ def test_dependent_decode_launches_do_not_crowd():
         us.append([float(x) for x in run.stdout.split()])
     for ordinary, dependent in zip(*us):
         assert dependent < 1.08 * ordinary, us
+
+
+@pytest.mark.parametrize("tlen", [256, 257, 320, 321, 833, 1601])  # five tiles are the fewest for CTAs of twelve (eight) warps; steps per warp even and not
+@pytest.mark.parametrize("ratio,gs,dtype", [(4, 32, torch.bfloat16), (4, 64, torch.float16), (1, 128, torch.bfloat16), (2, 32, torch.float16),
+                                            (8, 64, torch.bfloat16), (4, 32, torch.float32)])
+def test_decode_with_all_warps_of_an_sm_in_one_cta(tlen, ratio, gs, dtype):
+    """No more CTAs than SMs: one split and two, with and without a mask, the new token appended, against the oracle."""
+    m = ia()
+    b, hkv = 3, 2
+    k, v = make_kv(tlen, b, hkv, tlen)
+    q = bf16r(np.random.default_rng(tlen + ratio).standard_normal((b, hkv * ratio, 1, 128)))
+    full = fill_cache(m, k, v, gs, capacity=2048)
+    keep = np.random.default_rng(tlen).random((b, tlen)) < 0.8
+    keep[:, 0] = True
+    for splits in (1, 2):
+        for mask in (None, keep):
+            cache = fill_cache(m, k[:, :, : tlen - 1], v[:, :, : tlen - 1], gs, capacity=2048)
+            bias = None if mask is None else oracle.decode_attention_mask(mask.astype(np.int64), b, tlen)
+            ref = oracle.int4_decode_attention(q[:, :, 0], *cache_np(full), tlen, gs, *(() if bias is None else (bias,)))
+            out = m._append_decode_attention(t(q, dtype), t(k[:, :, tlen - 1:], dtype), t(v[:, :, tlen - 1:], dtype), cache, tlen, ratio, gs,
+                                             attention_mask=None if mask is None else torch.from_numpy(mask.astype(np.int64)).to(dev()), splits=splits)
+            assert_out_close(out, ref)
+            for name in ("k_packed", "v_packed", "k_scale", "v_scale"):
+                assert torch.equal(getattr(cache, name)[:, :, :tlen], getattr(full, name)[:, :, :tlen]), name
+
+
+def test_library_choice_fits_the_room_it_asks_for():
+    """A workspace of lq_int4_decode_auto_splits splits is enough for splits = 0 on every kernel."""
+    m = ia()
+    for b, tlen, gs in ((1, 1000, 16), (1, 1000, 32), (4, 2000, 16), (4, 2000, 128), (16, 2000, 16), (16, 2000, 32), (2, 4000, 64)):
+        k, v = make_kv(b + gs, 1, 8, tlen)
+        cache = fill_cache(m, np.repeat(k, b, 0), np.repeat(v, b, 0), gs)
+        q = t(bf16r(np.random.default_rng(b).standard_normal((b, 32, 1, 128))), torch.bfloat16)
+        want = m._decode_attention(q, cache, tlen, 4, gs, splits=1)
+        plan = m.Int4DecodePlan(q, cache, tlen, gs)
+        for out in (m._decode_attention(q, cache, tlen, 4, gs), plan.launch()):
+            assert (out.float() - want.float()).abs().max().item() <= 2.0 ** -7 * want.float().abs().max().item()
