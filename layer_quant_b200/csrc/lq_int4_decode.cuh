@@ -79,17 +79,8 @@ __global__ void __launch_bounds__(NW * 32, kWideWarps<R, QM> / NW) int4_decode_w
   const bool is_lo = DUP && t >= 2;
   const uint32_t lo_mul = is_lo ? 65536u : 0u, lo_mask = is_lo ? 0xFFFF0000u : 0u;
   uint8_t* const newtile = smem + L::kSmem - N::kNewBytes;
-  if (p.dependent && threadIdx.x < 4) {  // the CTA's codes and scales, asked for in L2 while the predecessor still runs (a prefetch reads nothing)
-    const int first = min(split * p.tiles_per_split * kTileTok, p.ctx_len);
-    const uint32_t tokens = static_cast<uint32_t>(min(first + p.tiles_per_split * kTileTok, p.ctx_len) - first);
-    const bool v = threadIdx.x & 1, scales = threadIdx.x & 2;
-    const int64_t* const st = scales ? (v ? c.vs_stride : c.ks_stride) : (v ? c.vp_stride : c.kp_stride);
-    const int64_t base = b * st[0] + kvh * st[1];
-    const uint8_t* const from = scales ? reinterpret_cast<const uint8_t*>((v ? c.v_scale : c.k_scale) + base + static_cast<int64_t>(first) * G)
-                                       : (v ? c.v_packed : c.k_packed) + base + static_cast<int64_t>(first) * 64;
-    const uint32_t bytes = (tokens * (scales ? G * 4u : 64u)) & ~15u;
-    if (bytes) asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(from), "r"(bytes) : "memory");
-  }
+  // Nothing is asked for in L2 ahead of the wait: it took longer than the loads themselves at every size (us with / without: 64 x 600 24.7 / 21.3, 24 x 1000 17.3 / 15.2,
+  // 16 x 1000 9.7 / 9.6, 200 x 600 53.2 / 47.2).
   pdl_wait();
   const RunLengths rl = run_lengths(p);
   const bool do_new = a.k_new != nullptr && split == p.splits - 1;

@@ -728,22 +728,31 @@ static size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 constexpr size_t kMaxTickets = 65536;
 constexpr size_t kTicketBytes = kMaxTickets * sizeof(int32_t);
 
-// Whether a decode launch is a programmatic dependent.  One hides launch, set-up and the way to the first tiles (2 us of a launch of 8 to 10).
-// Left to itself it loses more than that: its CTAs are placed where the predecessor leaves room, several to an SM, and the launch takes as long as the fullest
+// Decode launches are programmatic dependents: launch, set-up and the way to the first tiles (2 to 3 us) lie behind the predecessor's end.
+// Left to itself a dependent loses by its CTAs being placed where the predecessor leaves room, several to an SM, for the launch takes as long as the fullest
 // SM.  So it asks for so much shared memory that an SM holds no more of its CTAs than an even deal puts there (kHoldsOne, kHoldsTwo; three are
 // what it holds anyway).  us of a pair of launches, a predecessor and 8 x 1024 in one split (16 tiles x 64 CTAs): ordinary / dependent / dependent with an SM
 // each, behind a state update of batch 8 22.7 / 28.6 / 21.4, an append of 8 x 1024 22.6 / 24.2 / 20.1, an unquantised update of batch 32 40.2 / 44.7 / 38.1,
-// a GEMM 21.6 / 19.6 / 19.7, 16 x 8191 61.5 / 61.5 / 57.9, itself 12.4 / 10.8 / 10.6; 24 x 320 (5 x 192, two per SM) behind the update of batch 8
-// 20.6 / 20.0 / 18.7, itself 10.3 / 9.3 / 8.2; 40 x 200 (4 x 320) 20.6 / - / 18.8 and 10.3 / - / 8.4.  Recorded in a graph the gain is smaller, and behind long
-// kernels without a trigger a dependent costs up to 0.5 us more than it saves at 5 tiles, 0.8 at 16 tiles x 64 CTAs (behind 16 x 8191 55.8 -> 56.6), 1.0 at
-// 12 x 96, but up to 1.9 at 16 x 96, 2.0 at 8 x 128, 2.4 at 8 x 288: hence the tiles.  Short CTAs in any number even out (103 x 19, 1 x 824, behind the update of
-// batch 8 22.7 -> 20.7, 200 x 320, 5 x 1600, 51.9 -> 50.2, themselves 12.4 -> 10.6 and 40.9 -> 39.2).
+// a GEMM 21.6 / 19.6 / 19.7, itself 12.4 / 10.8 / 10.6.  Of all sizes, ordinary / dependent, behind itself, an update of batch 8, one of batch 60 and an
+// unquantised one of batch 32: 12 x 300 8.2 / 6.2, 18.6 / 16.7, 56.2 / 53.8, 32.2 / 30.0; 24 x 3001 32.5 / 29.1, 45.2 / 40.1, 79.9 / 77.1, 57.8 / 55.8;
+// 16 x 8191 43.1 / 40.7, 55.0 / 52.3, 90.2 / 87.8, 68.3 / 66.6; 1 x 131072 51.1 / 45.9, 57.4 / 55.6, 92.6 / 90.7, 70.2 / 69.0; 200 x 320 43.6 / 43.8,
+// 53.1 / 51.1, 90.7 / 87.8, 69.2 / 65.8.  (What made long ones slower as dependents was that a CTA asked for its tiles in L2 ahead of its loads.)
+// A recorded launch has no latency left to hide, and dependents behind one another cost up to 8 % there (16 x 8191 40.7 / 43.7, 24 x 3001 30.5 / 33.1):
+// recorded_dependent_pays keeps them to short and to few CTAs (8 x 300 7.7 / 6.2, 100 x 120 14.9 / 13.6).
 // Dependents of a decode launch do not start early (no trigger): they would lie around it in the same way (16 x 8191 and a dependent of 64 CTAs
 // 55.5 -> 60.1 recorded, 1 x 1024 and a state update of batch 60 59.2 -> 61.9, 200 x 256 and an update of batch 250 230.6 -> 233.5).
 constexpr size_t kHoldsOne = 116 * 1024, kHoldsTwo = 77 * 1024;  // of an SM's 228 KB, with 1 KB for each CTA
-static bool dependent_pays(int tiles, int64_t ctas) {
+static bool recorded_dependent_pays(int tiles, int64_t ctas) {
   const int sms = sm_count();
   return tiles <= (2 * ctas <= sms ? 16 : 3 * ctas <= 2 * sms ? 12 : 5);
+}
+static bool recording(cudaStream_t st) {
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &status) != cudaSuccess) {  // the legacy stream while another records: the launch itself will say so
+    cudaGetLastError();
+    return false;
+  }
+  return status != cudaStreamCaptureStatusNone;
 }
 
 // The tensor-pipe kernel covers group sizes 32 / 64 / 128 (a 16-byte chunk of a row never straddles
@@ -758,18 +767,17 @@ static bool use_mma_kernel(int gs) {
 }
 
 // Whether a decode launch has CTAs of as many warps as an SM holds in place of four: where an SM gets one CTA anyway and its warps have work.  A tile then
-// takes 0.255 us in place of 0.352, and one split of a (batch, kv head) does where three shared an SM and were merged.  us, four warps with the best split
+// takes 0.26 us in place of 0.35, and one split of a (batch, kv head) does where three shared an SM and were merged.  us, four warps with the best split
 // count / as many as an SM holds: 16 x 8191 46.1 / 43.0, 18 x 20000 99.0 / 90.2, 18 x 4000 28.8 / 26.7, 1 x 131072 45.0 / 43.0, 7 x 500 (8 tiles) 7.5 / 7.0, 1 x 300
 // (5) 6.4 / 5.9; with fewer tiles the other way: 7 x 200 (4) 5.9 / 6.2, 1 x 1024 in eight splits (2) 7.6 / 8.2.
 static bool wide_pays(int tiles, int64_t ctas) { return tiles >= 5 && ctas <= sm_count(); }
 
 // Split count from a cost model in microseconds, fitted to 360 measurements on B200 (batch 1 to 200, 33 to 131072 tokens, 1 to 64
-// splits; 6 % rms, the choice within 1 % of the best on average) and to 290 more with CTAs of twelve warps (batch 1 to 18, 200 to 131072 tokens).  An SM holds
-// three CTAs; a 64-token tile of one, two or
-// three at a time takes 0.35, 0.57 and 0.77 us, of one of twelve warps 0.255; a further wave of CTAs pays its set-up again, more CTAs per SM start
-// later, and more than one split pays the merge.  A dependent launch hides about 1.5 us: 4 x 2048 in eight splits 9.95 us, in the four chosen without this
-// 12.3; 2 x 4096 in 16 10.2 (12.3 in eight), 1 x 8192 in 32 10.6 (12.3 in 18).
-// tensor: of the tensor-pipe kernel; the CUDA-core kernel has neither.
+// splits; 6 % rms).  An SM holds three CTAs; a 64-token tile of one, two or
+// three at a time takes 0.35, 0.57 and 0.77 us; a further wave of CTAs pays its set-up again, more CTAs per SM start
+// later, and more than one split pays the merge.
+// tensor: of the tensor-pipe kernel, whose launches are dependents and may have all warps of an SM in one CTA (0.262 us a tile); its merge and that CTA are fitted to 330
+// measurements (batch 1 to 100, 146 to 65536 tokens; the choice is 0.5 % above the best on average).
 static int pick_splits(int batch, int kv_heads, int ctx_len, bool tensor) {
   const int ntiles = std::max(1, (ctx_len + kTile - 1) / kTile);
   const int sms = sm_count();
@@ -778,15 +786,15 @@ static int pick_splits(int batch, int kv_heads, int ctx_len, bool tensor) {
   int best = 1;
   double best_cost = 1.0e300;
   const int max_splits = std::min(ntiles, 128);
-  for (int s = 1; s <= max_splits; ++s) {
+  int next = 1;
+  for (int s = 1; s <= max_splits; s = next) {
     const int tps = (ntiles + s - 1) / s;
-    if ((ntiles + tps - 1) / tps != s) continue;  // would leave empty splits
+    next = tps > 1 ? (ntiles + tps - 2) / (tps - 1) : max_splits + 1;  // counts in between would leave empty splits
     const int64_t per_sm = (base * s + sms - 1) / sms;  // CTAs on the busiest SM
     const int64_t waves = (per_sm + 2) / 3;
-    double cost = 3.5 + (s > 1 ? 3.2 + 0.016 * s : 0.0);
-    if (tensor && wide_pays(tps, base * s)) cost += 0.255 * tps + std::min(2.2, 0.1 * tps) + 1.1;
+    double cost = 3.5 + (s > 1 ? 3.2 + (tensor ? 0.006 : 0.016) * s : 0.0);
+    if (tensor && wide_pays(tps, base * s)) cost += 2.4 + 0.262 * tps;
     else cost += tps * ((per_sm / 3) * kTileUs[3] + kTileUs[per_sm % 3]) + 4.0 * (waves - 1) + 1.1 * std::min<int64_t>(per_sm, 3);
-    if (tensor && dependent_pays(tps, base * s)) cost -= 1.5;
     // Ties go to fewer splits; in launches of 250 us and more HBM evens out what the deal to the SMs leaves uneven: us with the choice of
     // 0.98 / of 0.999: batch 16 x 65536 269 / 278, 32 x 32768 281 / 289, 56 x 32768 456 / 477, 64 x 32768 511 / 535; below, 48 x 16384 (cost
     // 203) 236 / 214, 96 x 8192 (207) 233 / 220.
@@ -833,7 +841,7 @@ static int launch_decode_mma(DecodeParams p, cudaStream_t st) {
   const dim3 grid(p.splits, p.a.cache.kv_heads, p.a.cache.batch);
   const int64_t ctas = static_cast<int64_t>(grid.x) * grid.y * grid.z;
   // (with a device counter the tiles are not known here)
-  p.dependent = p.a.seq_len_counter == nullptr && dependent_pays(p.tiles_per_split, ctas);
+  p.dependent = p.a.seq_len_counter == nullptr && (!recording(st) || recorded_dependent_pays(p.tiles_per_split, ctas));
   const auto launch = [&](auto warps) {
     constexpr int NW = decltype(warps)::value;
     constexpr size_t kSmem = mma::WarpStage<GS, NW>::kSmem;
