@@ -495,10 +495,11 @@ __global__ void __launch_bounds__(kFastThreads, kFastCtasPerSm) mx_state_update_
   const uint32_t my_step0 = step_first + warp * n_units;
   const int n_mine = static_cast<int>(n_units);
   const uint64_t block0 = static_cast<uint64_t>(my_step0) * 32;
-  // its first head, the steps left of it, and the steps of its first stage: what is over stages that start where heads do (if heads are whole stages)
+  // its first head, the steps left of it, and the steps of its first stage: all of them if they fit one (batch 3 of the reference's stream 284 -> 273 us, 20
+  // layers), else what is over stages that start where heads do (if heads are whole stages)
   const uint32_t bh_mine = fast_div(my_step0, d.div_steps_per_head);
   int left = static_cast<int>(steps_per_head - (my_step0 - bh_mine * steps_per_head));
-  const int first = ((left - 1) & (kRingSteps - 1)) + 1;
+  const int first = n_units <= kRingSteps ? static_cast<int>(n_units) : ((left - 1) & (kRingSteps - 1)) + 1;
   uint8_t* qptr = static_cast<uint8_t*>(s.q_state) + (block0 + lane) * IO::kQBytes;
   uint8_t* eptr = s.shared_exp + block0 + lane;
   uint8_t* mptr = s.micro_exp + (block0 + lane) * IO::kMicroBytes;
