@@ -474,7 +474,8 @@ __global__ void __launch_bounds__(kDenseThreads, 4) dense_state_update_ring_kern
 // so every access is 512 contiguous bytes, goes straight to registers, and a lane keeps only its 8 or 4 values of B and C.
 // 4 KB (16 or 8 rows of one head: a batch) are requested while the batch before is worked on; 16 warps per SM do so independently
 // (more warps would spill), without shared memory or barriers.  Steps are dealt to the warps evenly: at batch 32 the even deal is worth what whole
-// heads per CTA lost in the last wave.  Launched as a programmatic dependent, its first batch asked for in L2 before the wait.
+// heads per CTA lost in the last wave.  Launched as a programmatic dependent, its first two batches asked for in
+// L2 before the wait (convolution and update of 24 layers of batch 32: 692 us with one, 679 with two, 718 with none; smaller batches the same with one and two).
 // With the convolution before it, batch 32, bf16: 35.8 -> 27.5 us a layer (5.1 TB/s).
 constexpr int kRowsThreads = 64, kRowsCtasPerSm = 8;
 struct DenseRowsDerived {
@@ -497,7 +498,7 @@ __global__ void __launch_bounds__(kRowsThreads, kRowsCtasPerSm) dense_state_upda
   uint4* const state = static_cast<uint4*>(a.state) + lane;
   if (lane == 0)
     asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(state + static_cast<uint64_t>(first) * kStep),
-                 "r"(min(end - first, static_cast<uint32_t>(S)) * kStep * 16) : "memory");
+                 "r"(min(end - first, 2u * S) * kStep * 16) : "memory");
   const uint32_t col = (lane * V) & 127;
   // after the reduction lane l holds a row's total; it keeps step l & 7 of the batch
   const uint32_t row_in_step = DT == LQ_F32 ? 2 * (lane >> 4) + ((lane >> 3) & 1) : (lane >> 4) + 2 * ((lane >> 3) & 1);
