@@ -742,8 +742,7 @@ constexpr size_t kTicketBytes = kMaxTickets * sizeof(int32_t);
 // Dependents of a decode launch do not start early (no trigger): they would lie around it in the same way (16 x 8191 and a dependent of 64 CTAs
 // 55.5 -> 60.1 recorded, 1 x 1024 and a state update of batch 60 59.2 -> 61.9, 200 x 256 and an update of batch 250 230.6 -> 233.5).
 constexpr size_t kHoldsOne = 116 * 1024, kHoldsTwo = 77 * 1024;  // of an SM's 228 KB, with 1 KB for each CTA
-static bool recorded_dependent_pays(int tiles, int64_t ctas) {
-  const int sms = sm_count();
+static bool recorded_dependent_pays(int tiles, int64_t ctas, int sms) {
   return tiles <= (2 * ctas <= sms ? 16 : 3 * ctas <= 2 * sms ? 12 : 5);
 }
 static bool recording(cudaStream_t st) {
@@ -770,7 +769,7 @@ static bool use_mma_kernel(int gs) {
 // takes 0.26 us in place of 0.35, and one split of a (batch, kv head) does where three shared an SM and were merged.  us, four warps with the best split
 // count / as many as an SM holds: 16 x 8191 46.1 / 43.0, 18 x 20000 99.0 / 90.2, 18 x 4000 28.8 / 26.7, 1 x 131072 45.0 / 43.0, 7 x 500 (8 tiles) 7.5 / 7.0, 1 x 300
 // (5) 6.4 / 5.9; with fewer tiles the other way: 7 x 200 (4) 5.9 / 6.2, 1 x 1024 in eight splits (2) 7.6 / 8.2.
-static bool wide_pays(int tiles, int64_t ctas) { return tiles >= 5 && ctas <= sm_count(); }
+static bool wide_pays(int tiles, int64_t ctas, int sms) { return tiles >= 5 && ctas <= sms; }
 
 // Split count from a cost model in microseconds, fitted to 360 measurements on B200 (batch 1 to 200, 33 to 131072 tokens, 1 to 64
 // splits; 6 % rms).  An SM holds three CTAs; a 64-token tile of one, two or
@@ -793,7 +792,7 @@ static int pick_splits(int batch, int kv_heads, int ctx_len, bool tensor) {
     const int64_t per_sm = (base * s + sms - 1) / sms;  // CTAs on the busiest SM
     const int64_t waves = (per_sm + 2) / 3;
     double cost = 3.5 + (s > 1 ? 3.2 + (tensor ? 0.006 : 0.016) * s : 0.0);
-    if (tensor && wide_pays(tps, base * s)) cost += 2.4 + 0.262 * tps;
+    if (tensor && wide_pays(tps, base * s, sms)) cost += 2.4 + 0.262 * tps;
     else cost += tps * ((per_sm / 3) * kTileUs[3] + kTileUs[per_sm % 3]) + 4.0 * (waves - 1) + 1.1 * std::min<int64_t>(per_sm, 3);
     // Ties go to fewer splits; in launches of 250 us and more HBM evens out what the deal to the SMs leaves uneven: us with the choice of
     // 0.98 / of 0.999: batch 16 x 65536 269 / 278, 32 x 32768 281 / 289, 56 x 32768 456 / 477, 64 x 32768 511 / 535; below, 48 x 16384 (cost
@@ -840,13 +839,14 @@ template <int R, int GS, bool MASK, int QM>
 static int launch_decode_mma(DecodeParams p, cudaStream_t st) {
   const dim3 grid(p.splits, p.a.cache.kv_heads, p.a.cache.batch);
   const int64_t ctas = static_cast<int64_t>(grid.x) * grid.y * grid.z;
+  const int sms = sm_count();
   // (with a device counter the tiles are not known here)
-  p.dependent = p.a.seq_len_counter == nullptr && (!recording(st) || recorded_dependent_pays(p.tiles_per_split, ctas));
+  p.dependent = p.a.seq_len_counter == nullptr && (!recording(st) || recorded_dependent_pays(p.tiles_per_split, ctas, sms));
   const auto launch = [&](auto warps) {
     constexpr int NW = decltype(warps)::value;
     constexpr size_t kSmem = mma::WarpStage<GS, NW>::kSmem;
     static_assert(NW > 4 || kSmem <= kHoldsTwo, "the sizes for one and two CTAs are not smaller than what the kernel uses");
-    const size_t smem = NW > 4 || !p.dependent || ctas > 2 * sm_count() ? kSmem : ctas > sm_count() ? kHoldsTwo : kHoldsOne;
+    const size_t smem = NW > 4 || !p.dependent || ctas > 2 * sms ? kSmem : ctas > sms ? kHoldsTwo : kHoldsOne;
     const auto kernel = mma::int4_decode_warp_kernel<R, GS, MASK, QM, NW>;
     LQ_SET_SMEM_ONCE(kernel, std::max(kSmem, kHoldsOne));
     if (p.dependent) LQ_CHECK_CUDA(launch_dependent(kernel, grid, NW * 32, smem, st, p));
@@ -854,7 +854,7 @@ static int launch_decode_mma(DecodeParams p, cudaStream_t st) {
     LQ_CHECK_CUDA(cudaGetLastError());
     return static_cast<int>(LQ_OK);
   };
-  if (wide_pays(p.tiles_per_split, ctas)) return launch(std::integral_constant<int, mma::kWideWarps<R, QM>>{});
+  if (wide_pays(p.tiles_per_split, ctas, sms)) return launch(std::integral_constant<int, mma::kWideWarps<R, QM>>{});
   return launch(std::integral_constant<int, 4>{});
 }
 
