@@ -57,7 +57,7 @@ __device__ __forceinline__ uint32_t fast_div(uint32_t n, const FastDiv& f) { ret
 
 // Programmatic dependent launch: the kernel may be scheduled while its predecessor in the stream is still running (its CTAs take
 // the slots the predecessor's CTAs leave); before its griddepcontrol.wait, which returns once the predecessor has completed and its writes
-// are visible, it reads and writes no global memory and only asks for lines in L2 (a prefetch reads nothing).
+// are visible, it reads and writes no global memory but the module's own constants, and only asks for lines in L2 (a prefetch reads nothing).
 // Behind the wait operands are read with ordinary loads (the non-coherent ones are for data that nobody writes while the kernel lives).  Whether a kernel lets its own dependents
 // start early (pdl_launch_dependents) is a separate choice: the decode and prefill kernels do not.  LQ_MX_PDL=0 switches it off.
 bool use_pdl();  // lq_api.cu

@@ -5,8 +5,9 @@
 // nibbles as A operand in registers); what differs is everything around it.  A warp stages 32 tokens at a time with cp.async and
 // synchronises with itself only, so the warps of a CTA drift apart and their unpacking (ALU), exponentials and products overlap, and
 // the per-stage work (addresses, waits, issue) is shared by two steps.
-// What bounds it: issue and latency of about 320 instructions per 16 tokens with three warps per scheduler, then HBM.
-// Batch 64 x 32768, group 32: 541 -> 468 us (5.74 TB/s); batch 16 x 8191: 51 -> 45 us; fp16 query, 200 x 8000, group 128: 461 -> 348 us.
+// What bounds it: about 320 instructions per 16 tokens, half of them on the integer pipe (73 logic operations and 48 shifts unpack bf16 nibbles; moves and multiplies
+// share its cycles) with three warps per scheduler, then HBM.
+// Batch 64 x 32768, group 32: 541 -> 468 us (5.74 TB/s); batch 16 x 8191: 51 -> 45 -> 40 us; fp16 query, 200 x 8000, group 128: 461 -> 348 us.
 #pragma once
 
 #include "lq_int4_mma.cuh"
