@@ -217,6 +217,11 @@ int lq_int4_decode_attn(const lq_int4_decode_args* args, void* cuda_stream);
  * A buffer may be reused for any problem it is large enough for.                               */
 size_t lq_int4_decode_workspace_bytes(int32_t batch, int32_t q_heads, int32_t kv_heads, int32_t head_dim,
                                       int32_t max_splits);
+/* The split count that lq_int4_decode_attn uses for these arguments on the current device (>= 1): with splits = 0 the
+ * library's choice, which takes longer to make than a launch's other checks.  A caller that repeats a launch asks once,
+ * sizes the workspace by the answer and sets `splits` to it.  Reads cache.batch / kv_heads / group_size, seq_len, splits
+ * and whether k_new is set; follows no pointer.                                                */
+int32_t lq_int4_decode_split_count(const lq_int4_decode_args* args);
 /* Room for the split count that the library picks for this problem on the current device with splits = 0 (>= 1): the most over its
  * kernels, so a workspace of this many splits is always enough. */
 int32_t lq_int4_decode_auto_splits(int32_t batch, int32_t kv_heads, int32_t seq_len);

@@ -141,6 +141,8 @@ def lib() -> C.CDLL:
     l.lq_int4_static_scratch_bytes.restype = C.c_size_t
     l.lq_int4_decode_workspace_bytes.argtypes = [C.c_int32] * 5
     l.lq_int4_decode_workspace_bytes.restype = C.c_size_t
+    l.lq_int4_decode_split_count.argtypes = [C.POINTER(Int4DecodeArgs)]
+    l.lq_int4_decode_split_count.restype = C.c_int32
     l.lq_int4_decode_auto_splits.argtypes = [C.c_int32] * 3
     l.lq_int4_decode_auto_splits.restype = C.c_int32
     l.lq_dense_state_update.argtypes = [C.POINTER(DenseUpdateArgs), C.c_void_p]

@@ -805,6 +805,18 @@ static int pick_splits(int batch, int kv_heads, int ctx_len, bool tensor) {
   return best;
 }
 
+// The split count that a decode launch uses and the tiles of a split.  An explicit count is used as given, up to the tiles and to kMaxSplitsM (the merge
+// holds one factor per split in shared memory); no split is empty, and dealing a dealt count again changes nothing.
+static int deal_splits(const lq_int4_decode_args& a, int* tiles_per_split) {
+  const int ctx_len = std::max(a.seq_len - (a.k_new ? 1 : 0), 1);
+  const int ntiles = (ctx_len + kTile - 1) / kTile;
+  const int asked = a.splits > 0 ? a.splits : pick_splits(a.cache.batch, a.cache.kv_heads, ctx_len, use_mma_kernel(a.cache.group_size));
+  const int splits = std::max(1, std::min(std::min(asked, ntiles), mma::kMaxSplitsM));
+  const int tps = (ntiles + splits - 1) / splits;
+  if (tiles_per_split) *tiles_per_split = tps;
+  return (ntiles + tps - 1) / tps;
+}
+
 // Raises a kernel's dynamic shared-memory limit once per device and process instead of on every launch (the
 // attribute belongs to the function on a device; each expansion site has its own record, one bit per device).
 #define LQ_SET_SMEM_ONCE(KERNEL_, BYTES_)                                                                          \
@@ -841,7 +853,7 @@ static int launch_decode_mma(DecodeParams p, cudaStream_t st) {
   const int64_t ctas = static_cast<int64_t>(grid.x) * grid.y * grid.z;
   const int sms = sm_count();
   // (with a device counter the tiles are not known here)
-  p.dependent = p.a.seq_len_counter == nullptr && (!recording(st) || recorded_dependent_pays(p.tiles_per_split, ctas, sms));
+  p.dependent = p.a.seq_len_counter == nullptr && (recorded_dependent_pays(p.tiles_per_split, ctas, sms) || !recording(st));
   const auto launch = [&](auto warps) {
     constexpr int NW = decltype(warps)::value;
     constexpr size_t kSmem = mma::WarpStage<GS, NW>::kSmem;
@@ -952,6 +964,11 @@ LQ_EXPORT int32_t lq_int4_decode_auto_splits(int32_t batch, int32_t kv_heads, in
   return std::max(pick_splits(batch, kv_heads, seq_len, true), pick_splits(batch, kv_heads, seq_len, false));
 }
 
+LQ_EXPORT int32_t lq_int4_decode_split_count(const lq_int4_decode_args* args) {
+  if (args == nullptr || args->cache.batch <= 0 || args->cache.kv_heads <= 0 || args->seq_len <= 0) return 1;
+  return deal_splits(*args, nullptr);
+}
+
 LQ_EXPORT int lq_int4_decode_attn(const lq_int4_decode_args* args, void* cuda_stream) {
   LQ_CHECK_ARG(args != nullptr, "lq_int4_decode_attn: null args");
   const lq_int4_decode_args& a = *args;
@@ -985,13 +1002,7 @@ LQ_EXPORT int lq_int4_decode_attn(const lq_int4_decode_args* args, void* cuda_st
   DecodeParams p;
   p.a = a;
   p.ctx_len = a.seq_len - (a.k_new ? 1 : 0);
-  const int ntiles = std::max(1, (p.ctx_len + kTile - 1) / kTile);
-  int splits = a.splits > 0 ? a.splits : pick_splits(c.batch, c.kv_heads, std::max(p.ctx_len, 1), use_mma_kernel(c.group_size));
-  splits = std::max(1, std::min(std::min(splits, ntiles), mma::kMaxSplitsM));  // the merge holds one factor per split in shared memory
-  int tps = (ntiles + splits - 1) / splits;
-  splits = (ntiles + tps - 1) / tps;  // no empty splits
-  p.splits = splits;
-  p.tiles_per_split = tps;
+  const int splits = p.splits = deal_splits(a, &p.tiles_per_split);
   p.counters = nullptr; p.part_ml = nullptr; p.part_acc = nullptr;
   if (splits > 1) {
     const size_t need = lq_int4_decode_workspace_bytes(c.batch, a.q_heads, c.kv_heads, c.head_dim, splits);

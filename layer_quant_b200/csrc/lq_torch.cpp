@@ -33,7 +33,7 @@ struct Library {
                         int32_t, void*) = nullptr;
   int (*int4_decode_attn)(const lq_int4_decode_args*, void*) = nullptr;
   size_t (*int4_decode_workspace_bytes)(int32_t, int32_t, int32_t, int32_t, int32_t) = nullptr;
-  int32_t (*int4_decode_auto_splits)(int32_t, int32_t, int32_t) = nullptr;
+  int32_t (*int4_decode_split_count)(const lq_int4_decode_args*) = nullptr;
   int (*int4_prefill_attn)(const lq_int4_prefill_args*, void*) = nullptr;
   int (*dense_state_update)(const lq_dense_update_args*, void*) = nullptr;
   int (*causal_conv1d_update)(const lq_conv1d_update_args*, void*) = nullptr;
@@ -428,7 +428,7 @@ bool decode_mask(Call& c, PyObject* o, int64_t batch, int64_t seq_len, lq_int4_d
 PyObject* decode_attn(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   int64_t seq_len, ratio, group, splits;
-  if (n != 10 || L.int4_decode_attn == nullptr || !as_long(a[2], seq_len) || !as_long(a[3], ratio) || !as_long(a[4], group) ||
+  if (n != 10 || L.int4_decode_attn == nullptr || L.int4_decode_split_count == nullptr || !as_long(a[2], seq_len) || !as_long(a[3], ratio) || !as_long(a[4], group) ||
       !as_long(a[8], splits))
     return none();
   Call c;
@@ -464,14 +464,14 @@ PyObject* decode_attn(PyObject*, PyObject* const* a, Py_ssize_t n) {
     if (k == nullptr || k->scalar_type() != at::kLong || k->numel() != 1) return none();
     d.seq_len_counter = static_cast<const uint64_t*>(k->data_ptr());
   }
-  d.splits = static_cast<int32_t>(std::min<int64_t>(std::max<int64_t>(splits, 0), INT32_MAX));  // 0: the library's choice, for which the scratch below has room
-  if (splits <= 0) {
+  if (splits <= 0) {  // the library's choice, made here once: it costs 0.1 to 0.8 us
     const c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(c.device));  // the rule asks for its number of SMs
-    splits = L.int4_decode_auto_splits(batch, d.cache.kv_heads, std::max<int64_t>(seq_len - (d.k_new ? 1 : 0), 1));
+    splits = L.int4_decode_split_count(&d);
   }
+  d.splits = static_cast<int32_t>(std::min<int64_t>(splits, INT32_MAX));
   at::Tensor ws;  // held until the launch is in the stream
   if (splits > 1) {
-    ws = workspace(c.device, c.stream(), L.int4_decode_workspace_bytes(batch, heads, d.cache.kv_heads, dim, static_cast<int32_t>(std::min<int64_t>(splits, INT32_MAX))));
+    ws = workspace(c.device, c.stream(), L.int4_decode_workspace_bytes(batch, heads, d.cache.kv_heads, dim, d.splits));
     d.workspace = ws.data_ptr();
     d.workspace_bytes = ws.numel();
   }
@@ -630,11 +630,12 @@ PyObject* bind(PyObject*, PyObject* path_o) {
   find(L.int4_kv_append, "lq_int4_kv_append");
   find(L.int4_decode_attn, "lq_int4_decode_attn");
   find(L.int4_decode_workspace_bytes, "lq_int4_decode_workspace_bytes");
-  find(L.int4_decode_auto_splits, "lq_int4_decode_auto_splits");
   find(L.int4_prefill_attn, "lq_int4_prefill_attn");
   find(L.dense_state_update, "lq_dense_state_update");
   find(L.causal_conv1d_update, "lq_causal_conv1d_update");
   if (!ok) return nullptr;
+  // (the ctypes binding has seen that the library has it; a stand-in may not, and leaves decode_attn to the general path)
+  L.int4_decode_split_count = reinterpret_cast<decltype(L.int4_decode_split_count)>(dlsym(h, "lq_int4_decode_split_count"));
   Py_RETURN_NONE;
 }
 

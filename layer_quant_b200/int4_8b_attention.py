@@ -229,9 +229,10 @@ def _decode_args(query_states, cache, seq_len, group_size, mask, k_new=None, v_n
             raise TypeError("seq_len_counter must be a one-element int64 CUDA tensor")
         a.seq_len_counter = seq_len_counter.data_ptr()
     l = _lib.lib()
-    a.splits = max(splits, 0)  # 0: the library's choice, for which the scratch below has room
-    if splits <= 0:
-        splits = l.lq_int4_decode_auto_splits(batch, a.cache.kv_heads, max(seq_len - (1 if k_new is not None else 0), 1))
+    if splits <= 0:  # the library's choice, made once for all launches of this block
+        with torch.cuda.device(dev):  # by the number of SMs
+            splits = l.lq_int4_decode_split_count(ct.byref(a))
+    a.splits = splits
     ws = None
     if splits > 1:
         need = l.lq_int4_decode_workspace_bytes(batch, n_heads, a.cache.kv_heads, head_dim, splits)

@@ -88,6 +88,30 @@ def test_workspace_size_and_split_heuristic(lib):
     assert lib.lq_int4_decode_auto_splits(256, 8, 131072) <= 4
 
 
+def decode_args(batch, seq_len, gs=32, append=False, splits=0, kv_heads=8, ratio=4):
+    """What the split count depends on (nothing here is launched: no pointer is set but the one that says whether a row is appended)."""
+    from layer_quant_b200 import _lib
+    a = _lib.Int4DecodeArgs()
+    a.cache.batch, a.cache.kv_heads, a.cache.capacity, a.cache.head_dim, a.cache.group_size = batch, kv_heads, seq_len, 128, gs
+    a.q_heads, a.seq_len, a.splits, a.dtype = ratio * kv_heads, seq_len, splits, _lib.LQ_BF16
+    if append:
+        a.k_new = a.v_new = 256
+    return a
+
+
+def test_split_count_is_the_launchs_own(lib):
+    """Of either kernel (group size 16: CUDA cores), on both sides of where a CTA gets all warps of an SM; given back as `splits` it stays."""
+    choice = lambda *a, **k: lib.lq_int4_decode_split_count(ct.byref(decode_args(*a, **k)))
+    assert choice(16, 8192, append=True) == 1 and choice(16, 8192, gs=16, append=True) == 3
+    assert choice(1, 131072) == 18 and choice(18, 4000) == 1 and choice(24, 3001) == 2
+    for b, n, gs in ((1, 1, 32), (1, 1024, 32), (1, 1024, 16), (3, 5000, 64), (64, 32768, 128), (200, 320, 32)):
+        s = choice(b, n, gs=gs)
+        assert 1 <= s <= 128 and choice(b, n, gs=gs, splits=s) == s
+    assert choice(2, 130, splits=100) == 3 and choice(2, 640, splits=7) == 5 and choice(1, 131072, splits=500) == 128  # never an empty split
+    assert choice(1, 1, append=True) == 1
+    assert lib.lq_int4_decode_split_count(None) == 1 and choice(0, 100) == 1 and choice(1, 0) == 1
+
+
 def test_no_fallback_when_library_missing(monkeypatch, tmp_path):
     from layer_quant_b200 import _lib
     monkeypatch.setattr(_lib, "_lib", None)

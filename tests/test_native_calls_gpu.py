@@ -147,6 +147,38 @@ def test_recorded_decode_owns_its_scratch():
     assert held
 
 
+def test_split_count_is_chosen_once(tmp_path):
+    """A call asks for the library's choice once and launches with it; a prepared launch has asked when it was made."""
+    import ctypes
+    import subprocess
+    from pathlib import Path
+    from layer_quant_b200 import _lib
+    from layer_quant_b200 import int4_8b_attention as m
+    include = Path(_lib.__file__).resolve().parents[1] / "include"
+    names = ("mx_state_update", "mx_quantize", "counter_add", "int4_kv_append", "int4_decode_auto_splits", "int4_prefill_attn",
+             "dense_state_update", "causal_conv1d_update")
+    source = tmp_path / "counts.c"
+    source.write_text('#include "layer_quant_b200.h"\nint asked, launched;\n' + "".join(f"int stand_in_{n}(void) __asm__(\"lq_{n}\");\nint stand_in_{n}(void) {{ return 0; }}\n" for n in names) +
+                      "int32_t lq_int4_decode_split_count(const lq_int4_decode_args* a) { asked += 1; return a->splits ? -1 : 3; }\n"
+                      "size_t lq_int4_decode_workspace_bytes(int32_t b, int32_t q, int32_t k, int32_t d, int32_t s) { return s == 3 ? 4096 : 0; }\n"
+                      "int lq_int4_decode_attn(const lq_int4_decode_args* a, void* s) { launched = a->workspace_bytes >= 4096 ? a->splits : -1; return 0; }\n")
+    subprocess.run(["gcc", "-shared", "-fPIC", "-I", str(include), str(source), "-o", str(tmp_path / "counts.so")], check=True)
+    cache = m._allocate_layer_cache(2, 2, 256, 128, 4, dev())
+    q = torch.zeros(2, 8, 1, 128, dtype=torch.bfloat16, device=dev())
+    native, counts = _lib.native(), ctypes.CDLL(str(tmp_path / "counts.so"))
+    asked, launched = (ctypes.c_int.in_dll(counts, n) for n in ("asked", "launched"))
+    native.bind(str(tmp_path / "counts.so"))
+    try:
+        m._decode_attention(q, cache, 200, 4, 32)
+        assert (asked.value, launched.value) == (1, 3)
+        plan = m.Int4DecodePlan(q, cache, 200, 32)
+        assert plan.args.splits == _lib.lib().lq_int4_decode_split_count(ctypes.byref(plan.args)) >= 1
+        plan.launch()
+        assert asked.value == 1
+    finally:
+        native.bind(str(_lib.LIB_PATH))
+
+
 def test_other_threads_run_during_a_launch(tmp_path):
     """A launch blocks while CUDA's queue is full.  Here a stand-in for the library blocks in every call; another thread keeps running."""
     import ctypes
