@@ -222,8 +222,9 @@ size_t lq_int4_decode_workspace_bytes(int32_t batch, int32_t q_heads, int32_t kv
  * sizes the workspace by the answer and sets `splits` to it.  Reads cache.batch / kv_heads / group_size, seq_len, splits
  * and whether k_new is set; follows no pointer.                                                */
 int32_t lq_int4_decode_split_count(const lq_int4_decode_args* args);
-/* Room for the split count that the library picks for this problem on the current device with splits = 0 (>= 1): the most over its
- * kernels, so a workspace of this many splits is always enough. */
+/* Room for the split count that the library picks on the current device with splits = 0 and this seq_len in the argument
+ * block (>= 1): the most over its kernels, with and without a new row, so a workspace of this many splits is enough for
+ * any of them.  The count itself is lq_int4_decode_split_count's.                               */
 int32_t lq_int4_decode_auto_splits(int32_t batch, int32_t kv_heads, int32_t seq_len);
 
 /* Causal attention of q_len consecutive query positions over the packed cache, which already holds

@@ -961,7 +961,8 @@ LQ_EXPORT size_t lq_int4_decode_workspace_bytes(int32_t batch, int32_t q_heads, 
 
 LQ_EXPORT int32_t lq_int4_decode_auto_splits(int32_t batch, int32_t kv_heads, int32_t seq_len) {
   if (batch <= 0 || kv_heads <= 0 || seq_len <= 0) return 1;
-  return std::max(pick_splits(batch, kv_heads, seq_len, true), pick_splits(batch, kv_heads, seq_len, false));
+  const auto most = [&](int ctx_len) { return std::max(pick_splits(batch, kv_heads, ctx_len, true), pick_splits(batch, kv_heads, ctx_len, false)); };
+  return std::max(most(seq_len), most(std::max(seq_len - 1, 1)));  // a launch that appends chooses for the tokens before the new one
 }
 
 LQ_EXPORT int32_t lq_int4_decode_split_count(const lq_int4_decode_args* args) {

@@ -112,6 +112,20 @@ def test_split_count_is_the_launchs_own(lib):
     assert lib.lq_int4_decode_split_count(None) == 1 and choice(0, 100) == 1 and choice(1, 0) == 1
 
 
+def test_room_is_enough_for_the_choice(lib):
+    """Around every length at which a tile begins, on either kernel, with and without a row appended: the choice is not monotonic in the length, and a launch
+    that appends chooses for one token less."""
+    for batch in (1, 2, 3, 5, 16, 18, 24, 39, 64):
+        for tile in [*range(1, 100), 256, 511, 1024, 2048]:
+            for n in (64 * tile - 1, 64 * tile, 64 * tile + 1, 64 * tile + 2):
+                room = lib.lq_int4_decode_auto_splits(batch, 8, n)
+                for gs in (16, 32):
+                    for append in (False, True):
+                        assert lib.lq_int4_decode_split_count(ct.byref(decode_args(batch, n, gs, append))) <= room, (batch, n, gs, append)
+    for n in (1, 2, 2 ** 31 - 65):
+        assert lib.lq_int4_decode_auto_splits(1, 8, n) >= 1
+
+
 def test_no_fallback_when_library_missing(monkeypatch, tmp_path):
     from layer_quant_b200 import _lib
     monkeypatch.setattr(_lib, "_lib", None)

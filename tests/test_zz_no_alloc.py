@@ -72,6 +72,29 @@ def _problem(m, b, hq, hkv, tlen, gs, gen, dev, capacity=None):
     return q, cache
 
 
+def test_room_for_the_librarys_choice_when_a_row_is_appended():
+    """The C call as the header describes it: a workspace of lq_int4_decode_auto_splits(seq_len) splits, splits = 0 and a new row, where the choice for
+    one token less is the larger one."""
+    from layer_quant_b200 import _lib
+    from layer_quant_b200 import int4_8b_attention as m
+    lib = _lib.lib()
+    dev = torch.device("cuda", torch.cuda.current_device())
+    gen = torch.Generator(device=dev).manual_seed(19)
+    for tlen in (1153, 2305, 4737):
+        q, cache = _problem(m, 1, 32, 8, tlen, 32, gen, dev, capacity=tlen + 15)
+        k, v = (torch.randn((1, 8, 128), generator=gen, device=dev).bfloat16() for _ in range(2))
+        ws = torch.zeros(lib.lq_int4_decode_workspace_bytes(1, 32, 8, 128, lib.lq_int4_decode_auto_splits(1, 8, tlen)), dtype=torch.uint8, device=dev)
+        outs = []
+        for splits in (0, 1):
+            outs.append(torch.empty((1, 32, 128), dtype=torch.bfloat16, device=dev))
+            a = _args(m, _lib, q, cache, tlen, 32, splits, outs[-1], ws)
+            a.k_new, a.v_new = k.data_ptr(), v.data_ptr()
+            for i in range(3):
+                a.k_new_stride[i], a.v_new_stride[i] = k.stride(i), v.stride(i)
+            _lib.check(lib.lq_int4_decode_attn(ct.byref(a), torch.cuda.current_stream(dev).cuda_stream))
+        assert (outs[0].float() - outs[1].float()).abs().max().item() <= 2.0 ** -7 * outs[1].float().abs().max().item()
+
+
 def test_static_scratch_limits():
     """The edges of the built-in scratch: exactly as many partial results as it holds, the library's own split count
     clamped to fit, a problem too wide for any splitting (one split is always accepted), and an explicit split count
