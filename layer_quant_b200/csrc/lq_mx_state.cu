@@ -434,6 +434,9 @@ __global__ void __launch_bounds__(kFastThreads, kFastCtasPerSm) mx_state_update_
   // against 878)
   constexpr bool kWhole = MODE != LQ_ROUND_PHILOX_REF && MODE != kRefAnyOffset;
   constexpr bool kWholeIssue = kWhole && BITS == 8;
+  // With four draws a block a step is long, and the second copy pays only in slabs that mostly stay in it (us of layered4 before there was one / always / from
+  // twelve units a CTA on: batch 6 13.3 / 13.9 / 12.8, 8 16.1 / 17.0 / 15.5, 12 22.2 / 22.3 / 21.1, 14 (twelve units) 25.1 / 23.5 / 23.4, 20 34.4 / 33.4 / 33.3).
+  const bool whole_pays = MODE != LQ_ROUND_PHILOX_LAYERED4 || d.units_per_cta >= 3 * kRingSteps;
   constexpr int kUnroll = 2;
   extern __shared__ __align__(16) uint8_t smem_fast[];
   const lq_mx_state& s = a.state;
@@ -746,7 +749,7 @@ __global__ void __launch_bounds__(kFastThreads, kFastCtasPerSm) mx_state_update_
     // question per step.
     const uint32_t e4 = reinterpret_cast<const uint32_t*>(buf + Ring::kOffE)[lane];
     const bool odd = ((((e4 - 0x01010101u) & ~e4) | (e4 & (e4 << 1))) & 0x80808080u) != 0u;
-    if (kWhole && n == kRingSteps && left >= kRingSteps && e_max != 0u && !__any_sync(0xFFFFFFFFu, odd)) {
+    if (kWhole && whole_pays && n == kRingSteps && left >= kRingSteps && e_max != 0u && !__any_sync(0xFFFFFFFFu, odd)) {
       left -= kRingSteps;
 #pragma unroll 1
       for (int k0 = 0; k0 < kRingSteps; k0 += kUnroll) {

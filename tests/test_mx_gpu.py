@@ -554,6 +554,28 @@ def test_whole_stages_equal_general_kernel(bits, layout, stochastic, shape):
         assert torch.equal(got, want)
 
 
+@pytest.mark.parametrize("bits,layout", [(8, "packed"), (4, "reference")])
+@pytest.mark.parametrize("batch", [2, 13, 14, 16])  # slabs of one, eleven, twelve and thirteen units on 148 SMs: whole stages from twelve on
+def test_layered4_slabs_equal_general_kernel(bits, layout, batch):
+    """The stream of four draws a block, in slabs on either side of where whole stages have a form of their own, against the general kernel."""
+    m = mk()
+    h, p, n, g = 128, 64, 128, 8
+    gen = torch.Generator(device=dev()).manual_seed(batch)
+    rnd = lambda *s: torch.randn(*s, generator=gen, device=dev())
+    first = m.allocate_state_kernel_cache(rnd(batch, h, p, n).to(torch.bfloat16), 16, bits, layout=layout)
+    x, B, C = (v.to(torch.bfloat16) for v in (rnd(batch, h, p), rnd(batch, g, n), rnd(batch, g, n)))
+    dt = rnd(batch, h).to(torch.bfloat16)[..., None].expand(batch, h, p)
+    A = (-torch.exp(rnd(h)))[:, None, None].expand(h, p, n)
+    res = []
+    for general in (False, True):
+        cache = m.MambaStateKernelCache(first.q_state.clone(), first.shared_exp.clone(), first.micro_exp.clone(), format_bits=bits, layout=first.layout)
+        extra = dict(h_out=torch.empty((batch, h, p, n), dtype=torch.float32, device=dev())) if general else {}
+        y = m.mx_state_selective_update(cache, x, dt, A, B, C, dt_softplus=True, seed=9, rng_stream="layered4", **extra)
+        res.append((y.view(torch.int16), cache.q_state, cache.shared_exp, cache.micro_exp))
+    for got, want in zip(*res):
+        assert torch.equal(got, want)
+
+
 @pytest.mark.parametrize("layout", ["reference", "packed"])
 @pytest.mark.parametrize("bits", [8, 4])
 def test_micro_exponent_edges(bits, layout):
