@@ -173,6 +173,7 @@ struct MxUpdateDerived {
   // first units_rem CTAs one more
   uint32_t units_per_cta, units_rem;
   FastDiv div_steps_per_head, div_heads, div_dim, div_heads_per_group, div_groups;
+  uint32_t ask_operands;  // fast path: x, dt, A, B and C are asked for in L2 ahead of the wait (last: ahead of the divisors it took them off their 8 bytes, 2 %)
 };
 
 // One CTA = `hpc` consecutive heads of one (batch, B/C group): B and C are fetched once and stay in
@@ -433,10 +434,11 @@ __global__ void __launch_bounds__(kFastThreads, kFastCtasPerSm) mx_state_update_
   // whole stages two steps at a time; the reference's stream draws sixteen words a step, which leaves nothing to gain by a second copy (batch 32: 795 us
   // against 878)
   constexpr bool kWhole = MODE != LQ_ROUND_PHILOX_REF && MODE != kRefAnyOffset;
+  constexpr bool kLongSteps = !kWhole || MODE == LQ_ROUND_PHILOX_LAYERED4;  // several draws a block
   constexpr bool kWholeIssue = kWhole && BITS == 8;
   // With four draws a block a step is long, and the second copy pays only in slabs that mostly stay in it (us of layered4 before there was one / always / from
   // twelve units a CTA on: batch 6 13.3 / 13.9 / 12.8, 8 16.1 / 17.0 / 15.5, 12 22.2 / 22.3 / 21.1, 14 (twelve units) 25.1 / 23.5 / 23.4, 20 34.4 / 33.4 / 33.3).
-  const bool whole_pays = MODE != LQ_ROUND_PHILOX_LAYERED4 || d.units_per_cta >= 3 * kRingSteps;
+  const bool whole_pays = !kLongSteps || d.units_per_cta >= 3 * kRingSteps;
   constexpr int kUnroll = 2;
   extern __shared__ __align__(16) uint8_t smem_fast[];
   const lq_mx_state& s = a.state;
@@ -566,27 +568,29 @@ __global__ void __launch_bounds__(kFastThreads, kFastCtasPerSm) mx_state_update_
     sdA[i] = expf(A * dt);
   };
   const int tid = threadIdx.x;
-  // ... and the first round of every operand (batch 8: 10.2 -> 9.9 us a launch in a graph whose operands come from HBM)
-  const auto ask = [](const void* p, int64_t i, int dtype) {  // a hint: nothing is read
-    asm volatile("prefetch.global.L2 [%0];" ::"l"(static_cast<const uint8_t*>(p) + i * (dtype == LQ_F32 ? 4 : 2)) : "memory");
-  };
-  if (tid < n_heads) {
-    const unsigned hh = static_cast<unsigned>(h_first + tid);
-    const unsigned bq = fast_div(hh, d.div_heads);
-    const int h = static_cast<int>(hh - bq * static_cast<unsigned>(H)), b = b_first + static_cast<int>(bq);
-    ask(a.dt, b * a.dt_stride[0] + h * a.dt_stride[1], a.dt_dtype);
-    if (a.dt_bias) ask(a.dt_bias, h * a.dt_bias_stride[0], a.dt_bias_dtype);
-    ask(a.A, h * a.A_stride[0], a.A_dtype);
-  }
-  if (4 * tid < n_rows) {
-    int b, h, p;
-    row_coords(4 * tid, b, h, p);
-    ask(a.x, b * a.x_stride[0] + h * a.x_stride[1] + p * a.x_stride[2], a.x_dtype);
-  }
-  if (tid < n_bc) {
-    const void* base; const int64_t* st; int dtype, b, g, kb;
-    bc_source(tid, base, st, dtype, b, g, kb);
-    ask(base, b * st[0] + g * st[1] + kb * 16 * st[2], dtype);
+  // ... and, where the launch says so, the first round of every operand (batch 8: 10.2 -> 9.9 us a launch in a graph whose operands come from HBM)
+  if (kLongSteps || d.ask_operands) {
+    const auto ask = [](const void* p, int64_t i, int dtype) {  // a hint: nothing is read
+      asm volatile("prefetch.global.L2 [%0];" ::"l"(static_cast<const uint8_t*>(p) + i * (dtype == LQ_F32 ? 4 : 2)) : "memory");
+    };
+    if (tid < n_heads) {
+      const unsigned hh = static_cast<unsigned>(h_first + tid);
+      const unsigned bq = fast_div(hh, d.div_heads);
+      const int h = static_cast<int>(hh - bq * static_cast<unsigned>(H)), b = b_first + static_cast<int>(bq);
+      ask(a.dt, b * a.dt_stride[0] + h * a.dt_stride[1], a.dt_dtype);
+      if (a.dt_bias) ask(a.dt_bias, h * a.dt_bias_stride[0], a.dt_bias_dtype);
+      ask(a.A, h * a.A_stride[0], a.A_dtype);
+    }
+    if (4 * tid < n_rows) {
+      int b, h, p;
+      row_coords(4 * tid, b, h, p);
+      ask(a.x, b * a.x_stride[0] + h * a.x_stride[1] + p * a.x_stride[2], a.x_dtype);
+    }
+    if (tid < n_bc) {
+      const void* base; const int64_t* st; int dtype, b, g, kb;
+      bc_source(tid, base, st, dtype, b, g, kb);
+      ask(base, b * st[0] + g * st[1] + kb * 16 * st[2], dtype);
+    }
   }
 #pragma unroll
   for (int i = 0; i < 256 / kFastThreads; ++i) exp_step[threadIdx.x + i * kFastThreads] = steps[i];
@@ -1030,6 +1034,11 @@ static void launch_update_mode(const lq_mx_update_args& a, const MxUpdateDerived
     }
     dd.units_per_cta = static_cast<uint32_t>(dd.units_total / ctas);
     dd.units_rem = static_cast<uint32_t>(dd.units_total % ctas);
+    // Several CTAs an SM of one unit each are through before their askings are, which then stand in the way, most of all where all ask for the same lines of B and
+    // C.  us with / without, operands in HBM: two sequences of 48 heads x 96 and one group 5.31 / 4.84 (MX4 5.34 / 4.63), one of 128 x 64 4.66 / 4.65 (MX4 4.41
+    // / 4.16); with one CTA an SM (24 x 40) 3.71 / 3.86.  (Streams of several draws a block ask in any case: their steps are long, the reference's
+    // 7.13 / 7.33.)
+    dd.ask_operands = dd.units_total > ctas || ctas <= static_cast<uint64_t>(sm_count());
     dd.div_steps_per_head = fast_div_of(static_cast<uint32_t>(2 * (a.state.dim / rows_per_pass)));
     dd.div_groups = fast_div_of(static_cast<uint32_t>(a.ngroups));
     dd.div_heads = fast_div_of(static_cast<uint32_t>(a.state.heads));
