@@ -219,12 +219,12 @@ size_t lq_int4_decode_workspace_bytes(int32_t batch, int32_t q_heads, int32_t kv
                                       int32_t max_splits);
 /* The split count that lq_int4_decode_attn uses for these arguments on the current device (>= 1): with splits = 0 the
  * library's choice, which takes longer to make than a launch's other checks.  A caller that repeats a launch asks once,
- * sizes the workspace by the answer and sets `splits` to it.  Reads cache.batch / kv_heads / group_size, seq_len, splits
- * and whether k_new is set; follows no pointer.                                                */
+ * sizes the workspace by the answer and sets `splits` to it.  Reads cache.batch / kv_heads / group_size, q_heads, dtype,
+ * seq_len, splits and whether k_new is set; follows no pointer.                                */
 int32_t lq_int4_decode_split_count(const lq_int4_decode_args* args);
 /* Room for the split count that the library picks on the current device with splits = 0 and this seq_len in the argument
- * block (>= 1): the most over its kernels, with and without a new row, so a workspace of this many splits is enough for
- * any of them.  The count itself is lq_int4_decode_split_count's.                               */
+ * block (>= 1): the most over its kernels, query types and head counts, with and without a new row, so a workspace of this
+ * many splits is enough for any of them.  The count itself is lq_int4_decode_split_count's.                               */
 int32_t lq_int4_decode_auto_splits(int32_t batch, int32_t kv_heads, int32_t seq_len);
 
 /* Causal attention of q_len consecutive query positions over the packed cache, which already holds

@@ -772,12 +772,27 @@ static bool use_mma_kernel(int gs) {
 static bool wide_pays(int tiles, int64_t ctas, int sms) { return tiles >= 5 && ctas <= sms; }
 
 // Split count from a cost model in microseconds, fitted to 360 measurements on B200 (batch 1 to 200, 33 to 131072 tokens, 1 to 64
-// splits; 6 % rms).  An SM holds three CTAs; a 64-token tile of one, two or
-// three at a time takes 0.35, 0.57 and 0.77 us; a further wave of CTAs pays its set-up again, more CTAs per SM start
-// later, and more than one split pays the merge.
-// tensor: of the tensor-pipe kernel, whose launches are dependents and may have all warps of an SM in one CTA (0.262 us a tile); its merge and that CTA are fitted to 330
-// measurements (batch 1 to 100, 146 to 65536 tokens; the choice is 0.5 % above the best on average).
-static int pick_splits(int batch, int kv_heads, int ctx_len, bool tensor) {
+// splits; 6 % rms).  A 64-token tile of one, two or three CTAs of an SM at a time takes 0.35, 0.57 and 0.77 us; a further wave of CTAs pays its set-up
+// again, more CTAs per SM start later, and more than one split pays the merge.  Three kernels differ in what an SM holds of them:
+//   the CUDA-core kernel;
+//   the tensor-pipe kernel, three CTAs of four warps: its launches are dependents and may have all warps of an SM in one CTA (twelve).  Merge and that CTA are fitted to 330
+//     measurements (batch 1 to 100, 146 to 65536 tokens; the choice is 0.5 % above the best on average);
+//   the same for fp32 queries or eight heads a kv head, two CTAs of four warps or one of eight: 830 measurements (batch 1 to 200, 500 to 131072 tokens, five kinds), the
+//     choice 0.7 % above the best.  (With the constants of three, 3 % above: 4 x 32768 with eight heads and fp16 in 13 splits 62.7 us, in nine 45.7; fp32
+//     24 x 12000 in two 96.8, in three 86.9, 4 x 1000 with eight heads in four 11.8, in one 9.5.)
+// even_us: in longer launches HBM evens out what the deal to the SMs leaves uneven, and a count has to be 2 % better than a smaller one.  us with the choice of
+// 0.98 / of 0.999: batch 16 x 65536 269 / 278, 32 x 32768 281 / 289, 56 x 32768 456 / 477, 64 x 32768 511 / 535; below, 48 x 16384 (cost
+// 203) 236 / 214, 96 x 8192 (207) 233 / 220.
+struct DecodeCosts {
+  int hold;              // CTAs of four warps per SM
+  double start, wave;    // per CTA of an SM's first wave; per further wave
+  double merge, merge_split;
+  double wide, wide_tile;  // a CTA of all warps of an SM, and its tile; 0: there is none
+  double even_us;
+};
+constexpr DecodeCosts kCudaCore = {3, 1.1, 4.0, 3.2, 0.016, 0.0, 0.0, 250.0}, kTensorThree = {3, 1.1, 4.0, 3.2, 0.006, 2.4, 0.262, 250.0},
+                      kTensorTwo = {2, 0.7, 3.5, 3.7, 0.05, 1.1, 0.282, 100.0};
+static int pick_splits(int batch, int kv_heads, int ctx_len, const DecodeCosts& c) {
   const int ntiles = std::max(1, (ctx_len + kTile - 1) / kTile);
   const int sms = sm_count();
   const int64_t base = static_cast<int64_t>(batch) * kv_heads;
@@ -790,14 +805,11 @@ static int pick_splits(int batch, int kv_heads, int ctx_len, bool tensor) {
     const int tps = (ntiles + s - 1) / s;
     next = tps > 1 ? (ntiles + tps - 2) / (tps - 1) : max_splits + 1;  // counts in between would leave empty splits
     const int64_t per_sm = (base * s + sms - 1) / sms;  // CTAs on the busiest SM
-    const int64_t waves = (per_sm + 2) / 3;
-    double cost = 3.5 + (s > 1 ? 3.2 + (tensor ? 0.006 : 0.016) * s : 0.0);
-    if (tensor && wide_pays(tps, base * s, sms)) cost += 2.4 + 0.262 * tps;
-    else cost += tps * ((per_sm / 3) * kTileUs[3] + kTileUs[per_sm % 3]) + 4.0 * (waves - 1) + 1.1 * std::min<int64_t>(per_sm, 3);
-    // Ties go to fewer splits; in launches of 250 us and more HBM evens out what the deal to the SMs leaves uneven: us with the choice of
-    // 0.98 / of 0.999: batch 16 x 65536 269 / 278, 32 x 32768 281 / 289, 56 x 32768 456 / 477, 64 x 32768 511 / 535; below, 48 x 16384 (cost
-    // 203) 236 / 214, 96 x 8192 (207) 233 / 220.
-    if (cost < best_cost * (best_cost > 250.0 ? 0.98 : 0.999)) {
+    const int64_t waves = (per_sm + c.hold - 1) / c.hold;
+    double cost = 3.5 + (s > 1 ? c.merge + c.merge_split * s : 0.0);
+    if (c.wide_tile > 0.0 && wide_pays(tps, base * s, sms)) cost += c.wide + c.wide_tile * tps;
+    else cost += tps * ((per_sm / c.hold) * kTileUs[c.hold] + kTileUs[per_sm % c.hold]) + c.wave * (waves - 1) + c.start * std::min<int64_t>(per_sm, c.hold);
+    if (cost < best_cost * (best_cost > c.even_us ? 0.98 : 0.999)) {  // ties go to fewer splits
       best_cost = cost;
       best = s;
     }
@@ -805,12 +817,20 @@ static int pick_splits(int batch, int kv_heads, int ctx_len, bool tensor) {
   return best;
 }
 
+// Of the kernel that these arguments go to.
+static const DecodeCosts& decode_costs(const lq_int4_decode_args& a) {
+  static_assert(mma::kWideWarps<4, mma::kQBf16> == 4 * kTensorThree.hold && mma::kWideWarps<4, mma::kQF16> == 4 * kTensorThree.hold &&
+                mma::kWideWarps<8, mma::kQBf16> == 4 * kTensorTwo.hold && mma::kWideWarps<4, mma::kQF32> == 4 * kTensorTwo.hold, "what an SM holds");
+  if (!use_mma_kernel(a.cache.group_size)) return kCudaCore;
+  return a.q_heads <= 4ll * a.cache.kv_heads && a.dtype != LQ_F32 ? kTensorThree : kTensorTwo;
+}
+
 // The split count that a decode launch uses and the tiles of a split.  An explicit count is used as given, up to the tiles and to kMaxSplitsM (the merge
 // holds one factor per split in shared memory); no split is empty, and dealing a dealt count again changes nothing.
 static int deal_splits(const lq_int4_decode_args& a, int* tiles_per_split) {
   const int ctx_len = std::max(a.seq_len - (a.k_new ? 1 : 0), 1);
   const int ntiles = (ctx_len + kTile - 1) / kTile;
-  const int asked = a.splits > 0 ? a.splits : pick_splits(a.cache.batch, a.cache.kv_heads, ctx_len, use_mma_kernel(a.cache.group_size));
+  const int asked = a.splits > 0 ? a.splits : pick_splits(a.cache.batch, a.cache.kv_heads, ctx_len, decode_costs(a));
   const int splits = std::max(1, std::min(std::min(asked, ntiles), mma::kMaxSplitsM));
   const int tps = (ntiles + splits - 1) / splits;
   if (tiles_per_split) *tiles_per_split = tps;
@@ -961,7 +981,11 @@ LQ_EXPORT size_t lq_int4_decode_workspace_bytes(int32_t batch, int32_t q_heads, 
 
 LQ_EXPORT int32_t lq_int4_decode_auto_splits(int32_t batch, int32_t kv_heads, int32_t seq_len) {
   if (batch <= 0 || kv_heads <= 0 || seq_len <= 0) return 1;
-  const auto most = [&](int ctx_len) { return std::max(pick_splits(batch, kv_heads, ctx_len, true), pick_splits(batch, kv_heads, ctx_len, false)); };
+  const auto most = [&](int ctx_len) {
+    int splits = 1;
+    for (const DecodeCosts* c : {&kCudaCore, &kTensorThree, &kTensorTwo}) splits = std::max(splits, pick_splits(batch, kv_heads, ctx_len, *c));
+    return splits;
+  };
   return std::max(most(seq_len), most(std::max(seq_len - 1, 1)));  // a launch that appends chooses for the tokens before the new one
 }
 
@@ -1197,7 +1221,8 @@ LQ_EXPORT int lq_int4_decode_attn_static(const lq_int4_decode_args* args, void* 
   int splits = a.splits;
   const int ctx_len = std::max(a.seq_len - (a.k_new ? 1 : 0), 1);
   if (splits <= 0) {  // library's choice, kept inside what the built-in scratch can hold
-    splits = pick_splits(c.batch, c.kv_heads, ctx_len, use_mma_kernel(c.group_size));
+    // (one choice for all query types and head counts: a caller who cannot size the scratch keeps the counts, and so the bits, that this entry has always given)
+    splits = pick_splits(c.batch, c.kv_heads, ctx_len, use_mma_kernel(c.group_size) ? kTensorThree : kCudaCore);
     if (splits > max_splits) splits = static_cast<int>(std::max<int64_t>(max_splits, 1));
   } else {
     // an explicit count is used as lq_int4_decode_attn would use it: never more splits than 64-token tiles, nor than 128

@@ -88,12 +88,12 @@ def test_workspace_size_and_split_heuristic(lib):
     assert lib.lq_int4_decode_auto_splits(256, 8, 131072) <= 4
 
 
-def decode_args(batch, seq_len, gs=32, append=False, splits=0, kv_heads=8, ratio=4):
+def decode_args(batch, seq_len, gs=32, append=False, splits=0, kv_heads=8, ratio=4, dtype=None):
     """What the split count depends on (nothing here is launched: no pointer is set but the one that says whether a row is appended)."""
     from layer_quant_b200 import _lib
     a = _lib.Int4DecodeArgs()
     a.cache.batch, a.cache.kv_heads, a.cache.capacity, a.cache.head_dim, a.cache.group_size = batch, kv_heads, seq_len, 128, gs
-    a.q_heads, a.seq_len, a.splits, a.dtype = ratio * kv_heads, seq_len, splits, _lib.LQ_BF16
+    a.q_heads, a.seq_len, a.splits, a.dtype = ratio * kv_heads, seq_len, splits, _lib.LQ_BF16 if dtype is None else dtype
     if append:
         a.k_new = a.v_new = 256
     return a
@@ -109,6 +109,11 @@ def test_split_count_is_the_launchs_own(lib):
         assert 1 <= s <= 128 and choice(b, n, gs=gs, splits=s) == s
     assert choice(2, 130, splits=100) == 3 and choice(2, 640, splits=7) == 5 and choice(1, 131072, splits=500) == 128  # never an empty split
     assert choice(1, 1, append=True) == 1
+    # fp32 queries and eight heads a kv head: CTAs of eight warps, two of four an SM, measured best or within a per cent of it at these sizes
+    from layer_quant_b200 import _lib
+    for kw in (dict(ratio=8), dict(ratio=8, dtype=_lib.LQ_F16), dict(dtype=_lib.LQ_F32), dict(ratio=1, dtype=_lib.LQ_F32)):
+        for batch, tokens, splits in ((4, 32768, 9), (24, 12000, 3), (64, 6000, 1), (16, 8191, 1), (1, 131072, 18)):
+            assert choice(batch, tokens, append=True, **kw) == splits, (batch, tokens, kw)
     assert lib.lq_int4_decode_split_count(None) == 1 and choice(0, 100) == 1 and choice(1, 0) == 1
 
 
@@ -119,9 +124,9 @@ def test_room_is_enough_for_the_choice(lib):
         for tile in [*range(1, 100), 256, 511, 1024, 2048]:
             for n in (64 * tile - 1, 64 * tile, 64 * tile + 1, 64 * tile + 2):
                 room = lib.lq_int4_decode_auto_splits(batch, 8, n)
-                for gs in (16, 32):
+                for gs, ratio in ((16, 4), (32, 4), (32, 8)):
                     for append in (False, True):
-                        assert lib.lq_int4_decode_split_count(ct.byref(decode_args(batch, n, gs, append))) <= room, (batch, n, gs, append)
+                        assert lib.lq_int4_decode_split_count(ct.byref(decode_args(batch, n, gs, append, ratio=ratio))) <= room, (batch, n, gs, ratio, append)
     for n in (1, 2, 2 ** 31 - 65):
         assert lib.lq_int4_decode_auto_splits(1, 8, n) >= 1
 
