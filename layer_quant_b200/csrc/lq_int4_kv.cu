@@ -730,10 +730,11 @@ constexpr size_t kTicketBytes = kMaxTickets * sizeof(int32_t);
 
 // Decode launches are programmatic dependents: launch, set-up and the way to the first tiles (2 to 3 us) lie behind the predecessor's end.
 // Left to itself a dependent loses by its CTAs being placed where the predecessor leaves room, several to an SM, for the launch takes as long as the fullest
-// SM.  So it asks for so much shared memory that an SM holds no more of its CTAs than an even deal puts there (kHoldsOne, kHoldsTwo; three are
-// what it holds anyway).  us of a pair of launches, a predecessor and 8 x 1024 in one split (16 tiles x 64 CTAs): ordinary / dependent / dependent with an SM
-// each, behind a state update of batch 8 22.7 / 28.6 / 21.4, an append of 8 x 1024 22.6 / 24.2 / 20.1, an unquantised update of batch 32 40.2 / 44.7 / 38.1,
-// a GEMM 21.6 / 19.6 / 19.7, itself 12.4 / 10.8 / 10.6.  Of all sizes, ordinary / dependent, behind itself, an update of batch 8, one of batch 60 and an
+// SM.  So it asks for so much shared memory that an SM holds no more of its CTAs than an even deal puts there (kHoldsOne, kHoldsTwo; three, or one of all
+// warps, are what it holds anyway).  us of a pair of recorded launches, ordinary / dependent / dependent with that, behind a state update of batch 8 and an append of 8 x 1024: one CTA an
+// SM, 7 x 200 (4 tiles x 56 CTAs) 15.7 / 16.7 / 15.6, 13.8 / 15.1 / 13.7, 12 x 250 (4 x 96) 16.4 / 17.4 / 15.9, 14.5 / 15.7 / 13.9; two, 24 x 320 (5 x 192) 17.7 / 18.8
+// / 17.0, 15.9 / 16.9 / 15.2; not recorded, 24 x 1000 (16 x 192) 26.8 / 27.9 / 23.9, 26.7 / 26.1 / 22.3, 36 x 600 (10 x 288) 24.6 / 23.1 / 20.6, 22.6 / 21.2 / 18.5.
+// Of all sizes, ordinary / dependent, behind itself, an update of batch 8, one of batch 60 and an
 // unquantised one of batch 32: 12 x 300 8.2 / 6.2, 18.6 / 16.7, 56.2 / 53.8, 32.2 / 30.0; 24 x 3001 32.5 / 29.1, 45.2 / 40.1, 79.9 / 77.1, 57.8 / 55.8;
 // 16 x 8191 43.1 / 40.7, 55.0 / 52.3, 90.2 / 87.8, 68.3 / 66.6; 1 x 131072 51.1 / 45.9, 57.4 / 55.6, 92.6 / 90.7, 70.2 / 69.0; 200 x 320 43.6 / 43.8,
 // 53.1 / 51.1, 90.7 / 87.8, 69.2 / 65.8.  (What made long ones slower as dependents was that a CTA asked for its tiles in L2 ahead of its loads.)

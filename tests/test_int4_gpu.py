@@ -850,6 +850,47 @@ def test_dependent_decode_launches_do_not_crowd():
         assert dependent < 1.08 * ordinary, us
 
 
+FOUR_WARPS = PAIRS.split("plans = []")[0] + """
+recorded, problems = sys.argv[1] == "recorded", [tuple(map(int, p.split("x"))) for p in sys.argv[2:]]
+for batch, length in problems:
+    cache = ia._allocate_layer_cache(batch, 8, (length + 15) // 16 * 16, 128, 4, dev())
+    k, v = (torch.randn(batch, 8, length, 128, device=dev()).bfloat16() for _ in range(2))
+    ia._pack_kv_into_cache(cache, k, v, torch.arange(length, device=dev()), 32)
+    plan = ia.Int4DecodePlan(torch.randn(batch, 32, 1, 128, device=dev()).bfloat16(), cache, length, 32, splits=1)
+    row = lambda: [(update.run(), plan.launch()) for _ in range(50)]
+    row(), torch.cuda.synchronize()
+    if recorded:
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g):
+            row()
+    best = 1e9
+    for _ in range(12):
+        e = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+        e[0].record(), (g.replay if recorded else row)(), e[1].record(), e[1].synchronize()
+        best = min(best, e[0].elapsed_time(e[1]) * 20)
+    print(best)
+"""
+
+
+@pytest.mark.parametrize("how,problems", [("recorded", ["7x200", "12x250", "24x320"]), ("unrecorded", ["24x1000"])])
+def test_dependent_launches_of_four_warps_do_not_crowd(how, problems):
+    """The launches that ask for more shared memory than they use, so that an SM holds one or two of their CTAs: fewer than five tiles in no more CTAs than SMs,
+    and up to twice as many CTAs as SMs.  Without that they take 1.04 to 1.07 of an ordinary launch's time behind a state update (us of a pair: 16.7 for 15.7, 17.4 for
+    16.4, 18.8 for 17.7; unrecorded 27.9 for 26.8), with it 0.89 to 1.0."""
+    import os
+    import subprocess
+    import sys
+    from pathlib import Path
+    us = []
+    for pdl in "01":
+        run = subprocess.run([sys.executable, "-c", FOUR_WARPS, how, *problems], env=dict(os.environ, LQ_MX_PDL=pdl),
+                             cwd=Path(__file__).resolve().parents[1], capture_output=True, text=True, timeout=300)
+        assert run.returncode == 0, run.stderr[-2000:]
+        us.append([float(x) for x in run.stdout.split()])
+    for ordinary, dependent in zip(*us):
+        assert dependent < 1.025 * ordinary, us
+
+
 @pytest.mark.parametrize("tlen", [256, 257, 320, 321, 833, 1601])  # five tiles are the fewest for CTAs of twelve (eight) warps; steps per warp even and not
 @pytest.mark.parametrize("ratio,gs,dtype", [(4, 32, torch.bfloat16), (4, 64, torch.float16), (1, 128, torch.bfloat16), (2, 32, torch.float16),
                                             (8, 64, torch.bfloat16), (4, 32, torch.float32)])
