@@ -307,7 +307,6 @@ struct DecodeParams {
   int32_t splits;          // >= 1
   int32_t tiles_per_split;
   int32_t ctx_len;         // tokens read from the cache ring: seq_len, minus the fused new token
-  int32_t dependent = 0;   // launched as a programmatic dependent
   int32_t* counters;       // [B * Hkv] tickets (workspace)
   float* part_ml;          // [B * Hq * splits * 2]
   float* part_acc;         // [B * Hq * splits * 128]
@@ -869,20 +868,20 @@ static int launch_decode(const DecodeParams& p, cudaStream_t st) {
 }
 
 template <int R, int GS, bool MASK, int QM>
-static int launch_decode_mma(DecodeParams p, cudaStream_t st) {
+static int launch_decode_mma(const DecodeParams& p, cudaStream_t st) {
   const dim3 grid(p.splits, p.a.cache.kv_heads, p.a.cache.batch);
   const int64_t ctas = static_cast<int64_t>(grid.x) * grid.y * grid.z;
   const int sms = sm_count();
   // (with a device counter the tiles are not known here)
-  p.dependent = p.a.seq_len_counter == nullptr && (recorded_dependent_pays(p.tiles_per_split, ctas, sms) || !recording(st));
+  const bool dependent = p.a.seq_len_counter == nullptr && (recorded_dependent_pays(p.tiles_per_split, ctas, sms) || !recording(st));
   const auto launch = [&](auto warps) {
     constexpr int NW = decltype(warps)::value;
     constexpr size_t kSmem = mma::WarpStage<GS, NW>::kSmem;
     static_assert(NW > 4 || kSmem <= kHoldsTwo, "the sizes for one and two CTAs are not smaller than what the kernel uses");
-    const size_t smem = NW > 4 || !p.dependent || ctas > 2 * sms ? kSmem : ctas > sms ? kHoldsTwo : kHoldsOne;
+    const size_t smem = NW > 4 || !dependent || ctas > 2 * sms ? kSmem : ctas > sms ? kHoldsTwo : kHoldsOne;
     const auto kernel = mma::int4_decode_warp_kernel<R, GS, MASK, QM, NW>;
     LQ_SET_SMEM_ONCE(kernel, std::max(kSmem, kHoldsOne));
-    if (p.dependent) LQ_CHECK_CUDA(launch_dependent(kernel, grid, NW * 32, smem, st, p));
+    if (dependent) LQ_CHECK_CUDA(launch_dependent(kernel, grid, NW * 32, smem, st, p));
     else kernel<<<grid, NW * 32, smem, st>>>(p);
     LQ_CHECK_CUDA(cudaGetLastError());
     return static_cast<int>(LQ_OK);

@@ -1002,6 +1002,15 @@ static bool fast_update_applies(const lq_mx_update_args& a, const MxUpdateDerive
          s.dim % rows_per_pass == 0 && aligned && units < (1ull << 30) && counters <= (1ull << 32);
 }
 
+// Units of a CTA's slab at most; LQ_MX_MAX_UNITS (a tuning aid) is read once.
+static uint64_t max_slab_units() {
+  static const uint64_t units = [] {
+    const char* env = getenv("LQ_MX_MAX_UNITS");
+    return static_cast<uint64_t>(env ? std::min(400, std::max(1, atoi(env))) : 192);
+  }();
+  return units;
+}
+
 template <int BITS, int LAYOUT>
 static void launch_update_mode(const lq_mx_update_args& a, const MxUpdateDerived& d, cudaStream_t st) {
   using IO = MxBlockIO<BITS, LAYOUT>;
@@ -1016,8 +1025,7 @@ static void launch_update_mode(const lq_mx_update_args& a, const MxUpdateDerived
                                                              (d.nblk == 8 ? kPartials : 0));
     };
     const size_t budget = 228 * 1024 / kFastCtasPerSm - 1024 - 1024 - (IO::kNibbles ? sizeof(MxPairMasks) : sizeof(MxPairFactors));
-    uint64_t max_units = 192;
-    if (const char* env = getenv("LQ_MX_MAX_UNITS")) max_units = std::min(400, std::max(1, atoi(env)));  // tuning aid
+    uint64_t max_units = max_slab_units();
     while (max_units > 1 && smem_of(max_units) > budget) --max_units;
     MxUpdateDerived dd = d;
     const auto vec16 = [](const void* p, int dtype, const int64_t* st, int mult) {  // 16-bit, innermost contiguous, `mult` elements aligned

@@ -107,6 +107,8 @@ def test_split_count_is_the_launchs_own(lib):
     for b, n, gs in ((1, 1, 32), (1, 1024, 32), (1, 1024, 16), (3, 5000, 64), (64, 32768, 128), (200, 320, 32)):
         s = choice(b, n, gs=gs)
         assert 1 <= s <= 128 and choice(b, n, gs=gs, splits=s) == s
+    for batch, tokens, s in ((48, 16383, 3), (96, 8191, 2), (16, 65535, 8), (32, 32767, 4), (64, 32767, 2)):
+        assert choice(batch, tokens) == choice(batch, tokens, gs=16) == s
     assert choice(2, 130, splits=100) == 3 and choice(2, 640, splits=7) == 5 and choice(1, 131072, splits=500) == 128  # never an empty split
     assert choice(1, 1, append=True) == 1
     # fp32 queries and eight heads a kv head: CTAs of eight warps, two of four an SM, measured best or within a per cent of it at these sizes
