@@ -340,8 +340,9 @@ __global__ void __launch_bounds__(kUpdateThreads, 4) mx_state_update_kernel(cons
 // step: eight 128-bit loads that share addresses between rows and cost next to nothing beside the arithmetic, for 32 registers.
 // A warp's first stage is as long as makes the others start where heads do.  A whole stage of one head with ordinary exponents asks nothing per
 // step and takes two steps at a time; anything else goes step by step.
-// 272 -> 248 instructions per 16 values (with set-up) and the packed operands of lq_mx_codec.cuh: MX8 1522 -> 1361 us (batch 250, eight layers),
-// 422 -> 381 (64), deterministic rounding 402 -> 354 (60), MX4 417 -> 392 (64).  Four steps at a time, or two copies of two, run slower (1455, 1515).
+// 272 -> 248 instructions per 16 values (with set-up) and the packed operands of lq_mx_codec.cuh: MX8 1522 -> 1361 us (batch 250, eight layers, a few passes at a
+// time; in long rows, at the board's power limit, 1520 -> 1403 to 1423), 422 -> 381 (64), deterministic rounding 402 -> 354 (60), MX4 417 -> 392 (64).  Four steps at a time,
+// or two copies of two, run slower (1455, 1515).
 // NBLK_T = dstate / 16 when known at compile time (8 for Nemotron-H: all lane and address arithmetic
 // folds to constants), 0 = taken from the arguments.
 // kRefAnyOffset: PHILOX_REF with an offset that is no multiple of 16 (a caller's own).  A block's counters may pass 2^32, so every word is drawn by itself.
