@@ -779,8 +779,8 @@ def test_append_vector_path_rows_and_alignment(gs, tq, offset, dtype):
 @pytest.mark.parametrize("batch,start,splits", [(1, 70, 1), (1, 1000, 16), (8, 1000, 1), (9, 250, 1), (12, 700, 1), (16, 120, 1), (16, 300, 1),
                                                 (24, 250, 1), (40, 190, 1), (40, 500, 3)])
 def test_decode_launches_follow_one_another(batch, start, splits):
-    """Launches with few or short CTAs are programmatic dependents, one or two CTAs to an SM where there are no more than that, others are not; each appends a row that the next one attends to and shares the
-    scratch of the split merge.  A row of launches must equal the same launches waited for one by one."""
+    """Launches are programmatic dependents, one or two CTAs to an SM where there are no more than that; each appends a row that the next one attends to and
+    shares the scratch of the split merge.  A row of launches must equal the same launches waited for one by one."""
     m = ia()
     hkv, gs, steps = 8, 32, 12
     k, v = make_kv(101, 1, hkv, start)
