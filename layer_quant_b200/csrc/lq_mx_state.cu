@@ -161,11 +161,13 @@ __device__ __forceinline__ MxRoundCtx round_ctx_at(const MxRoundBase& b, uint64_
 }
 
 struct MxUpdateDerived {
+  enum : int32_t { kVec = 1, kAsk = 2 };
   int32_t nblk;        // dstate / 16
   int32_t lpr_log2;    // lanes per row = 1 << lpr_log2 >= nblk
   int32_t dt_uniform;  // dt and dt_bias do not depend on the row (dim) index
   int32_t a_scalar;    // A depends on the head only
-  int32_t vec;         // x, out, B, C in 16 bits, aligned for vectors; D per head, no z; dim a multiple of 4
+  int32_t flags;       // kVec: x, out, B, C in 16 bits, aligned for vectors; D per head, no z; dim a multiple of 4.  kAsk: x, dt, A, B and C are asked for in
+                       // L2 ahead of the wait.  (One word: a field more is a launch 1 % longer.)
   int32_t heads_per_cta;  // consecutive heads of one B/C group handled by one CTA
   PhiloxKeys keys;        // round keys of rounding.seed
   uint64_t units_total;   // fast path: batch * heads * dim / rows per pass (< 2^31)
@@ -173,7 +175,6 @@ struct MxUpdateDerived {
   // first units_rem CTAs one more
   uint32_t units_per_cta, units_rem;
   FastDiv div_steps_per_head, div_heads, div_dim, div_heads_per_group, div_groups;
-  uint32_t ask_operands;  // fast path: x, dt, A, B and C are asked for in L2 ahead of the wait (last: ahead of the divisors it took them off their 8 bytes, 2 %)
 };
 
 // One CTA = `hpc` consecutive heads of one (batch, B/C group): B and C are fetched once and stay in
@@ -340,8 +341,8 @@ __global__ void __launch_bounds__(kUpdateThreads, 4) mx_state_update_kernel(cons
 // step: eight 128-bit loads that share addresses between rows and cost next to nothing beside the arithmetic, for 32 registers.
 // A warp's first stage is as long as makes the others start where heads do.  A whole stage of one head with ordinary exponents asks nothing per
 // step and takes two steps at a time; anything else goes step by step.
-// 272 -> 248 instructions per 16 values (with set-up) and the packed operands of lq_mx_codec.cuh: MX8 1522 -> 1361 us (batch 250, eight layers, a few passes at a
-// time; in long rows, at the board's power limit, 1520 -> 1403 to 1423), 422 -> 381 (64), deterministic rounding 402 -> 354 (60), MX4 417 -> 392 (64).  Four steps at a time,
+// 272 -> 248 instructions per 16 values (with set-up) and the packed operands of lq_mx_codec.cuh: MX8 1522 -> 1361 us (batch 250, eight layers; on boxes that are at their
+// power limit then, 1520 -> 1403 to 1423), 422 -> 381 (64), deterministic rounding 402 -> 354 (60), MX4 417 -> 392 (64).  Four steps at a time,
 // or two copies of two, run slower (1455, 1515).
 // NBLK_T = dstate / 16 when known at compile time (8 for Nemotron-H: all lane and address arithmetic
 // folds to constants), 0 = taken from the arguments.
@@ -569,29 +570,31 @@ __global__ void __launch_bounds__(kFastThreads, kFastCtasPerSm) mx_state_update_
     sdA[i] = expf(A * dt);
   };
   const int tid = threadIdx.x;
-  // ... and, where the launch says so, the first round of every operand (batch 8: 10.2 -> 9.9 us a launch in a graph whose operands come from HBM)
-  if (kLongSteps || d.ask_operands) {
-    const auto ask = [](const void* p, int64_t i, int dtype) {  // a hint: nothing is read
-      asm volatile("prefetch.global.L2 [%0];" ::"l"(static_cast<const uint8_t*>(p) + i * (dtype == LQ_F32 ? 4 : 2)) : "memory");
-    };
-    if (tid < n_heads) {
-      const unsigned hh = static_cast<unsigned>(h_first + tid);
-      const unsigned bq = fast_div(hh, d.div_heads);
-      const int h = static_cast<int>(hh - bq * static_cast<unsigned>(H)), b = b_first + static_cast<int>(bq);
-      ask(a.dt, b * a.dt_stride[0] + h * a.dt_stride[1], a.dt_dtype);
-      if (a.dt_bias) ask(a.dt_bias, h * a.dt_bias_stride[0], a.dt_bias_dtype);
-      ask(a.A, h * a.A_stride[0], a.A_dtype);
-    }
-    if (4 * tid < n_rows) {
-      int b, h, p;
-      row_coords(4 * tid, b, h, p);
-      ask(a.x, b * a.x_stride[0] + h * a.x_stride[1] + p * a.x_stride[2], a.x_dtype);
-    }
-    if (tid < n_bc) {
-      const void* base; const int64_t* st; int dtype, b, g, kb;
-      bc_source(tid, base, st, dtype, b, g, kb);
-      ask(base, b * st[0] + g * st[1] + kb * 16 * st[2], dtype);
-    }
+  // ... and, where the launch says so, the first round of every operand (batch 8: 10.2 -> 9.9 us a launch in a graph whose operands come from HBM).  The launch's word is
+  // a predicate of the instruction: as a branch around all of this it changed the code of the steps (MX8 0.8 % slower, MX4 1 to 2 % faster).
+  const int asks = d.flags & d.kAsk;
+  const auto ask = [&](const void* p, int64_t i, int dtype) {  // a hint: nothing is read
+    const uint8_t* const at = static_cast<const uint8_t*>(p) + i * (dtype == LQ_F32 ? 4 : 2);
+    if (kLongSteps) asm volatile("prefetch.global.L2 [%0];" ::"l"(at) : "memory");
+    else asm volatile("{\n.reg .pred p;\nsetp.ne.s32 p, %1, 0;\n@p prefetch.global.L2 [%0];\n}" ::"l"(at), "r"(asks) : "memory");
+  };
+  if (tid < n_heads) {
+    const unsigned hh = static_cast<unsigned>(h_first + tid);
+    const unsigned bq = fast_div(hh, d.div_heads);
+    const int h = static_cast<int>(hh - bq * static_cast<unsigned>(H)), b = b_first + static_cast<int>(bq);
+    ask(a.dt, b * a.dt_stride[0] + h * a.dt_stride[1], a.dt_dtype);
+    if (a.dt_bias) ask(a.dt_bias, h * a.dt_bias_stride[0], a.dt_bias_dtype);
+    ask(a.A, h * a.A_stride[0], a.A_dtype);
+  }
+  if (4 * tid < n_rows) {
+    int b, h, p;
+    row_coords(4 * tid, b, h, p);
+    ask(a.x, b * a.x_stride[0] + h * a.x_stride[1] + p * a.x_stride[2], a.x_dtype);
+  }
+  if (tid < n_bc) {
+    const void* base; const int64_t* st; int dtype, b, g, kb;
+    bc_source(tid, base, st, dtype, b, g, kb);
+    ask(base, b * st[0] + g * st[1] + kb * 16 * st[2], dtype);
   }
 #pragma unroll
   for (int i = 0; i < 256 / kFastThreads; ++i) exp_step[threadIdx.x + i * kFastThreads] = steps[i];
@@ -600,7 +603,7 @@ __global__ void __launch_bounds__(kFastThreads, kFastCtasPerSm) mx_state_update_
   // the first stages travel while the operands below are staged
   Ring::template issue<kWholeIssue>(source, 0, lane, min(n_mine, first), first);
 
-  if (NBLK_T == 8 && d.vec) {
+  if (NBLK_T == 8 && (d.flags & d.kVec)) {
     // 16-bit operands in vectors.  The first round of every kind is requested before any of it is used: one latency, not three
     auto x_vec = [&](int i) {
       int b, h, p;
@@ -786,7 +789,7 @@ __global__ void __launch_bounds__(kFastThreads, kFastCtasPerSm) mx_state_update_
   }
   __syncthreads();
   // y = <h', C> + D x (* z), stored for the whole slab at once
-  if (NBLK_T == 8 && d.vec) {  // a thread takes the four rows of a step
+  if (NBLK_T == 8 && (d.flags & d.kVec)) {  // a thread takes the four rows of a step
     for (int i = tid; 4 * i < n_rows; i += kFastThreads) {
       int b, h, p;
       row_coords(4 * i, b, h, p);
@@ -1032,7 +1035,7 @@ static void launch_update_mode(const lq_mx_update_args& a, const MxUpdateDerived
     const auto vec16 = [](const void* p, int dtype, const int64_t* st, int mult) {  // 16-bit, innermost contiguous, `mult` elements aligned
       return dtype != LQ_F32 && st[2] == 1 && st[0] % mult == 0 && st[1] % mult == 0 && reinterpret_cast<uintptr_t>(p) % (2 * mult) == 0;
     };
-    dd.vec = vec16(a.x, a.x_dtype, a.x_stride, 4) && vec16(a.out, a.out_dtype, a.out_stride, 4) && vec16(a.B, a.B_dtype, a.B_stride, 8) &&
+    const bool vec = vec16(a.x, a.x_dtype, a.x_stride, 4) && vec16(a.out, a.out_dtype, a.out_stride, 4) && vec16(a.B, a.B_dtype, a.B_stride, 8) &&
              vec16(a.C, a.C_dtype, a.C_stride, 8) && a.state.dim % 4 == 0 && !a.z && (!a.D || a.D_stride[1] == 0);
     dd.units_total = static_cast<uint64_t>(a.state.batch) * a.state.heads * (a.state.dim / rows_per_pass);
     const uint64_t wave = static_cast<uint64_t>(kFastCtasPerSm) * sm_count();
@@ -1044,10 +1047,11 @@ static void launch_update_mode(const lq_mx_update_args& a, const MxUpdateDerived
     dd.units_per_cta = static_cast<uint32_t>(dd.units_total / ctas);
     dd.units_rem = static_cast<uint32_t>(dd.units_total % ctas);
     // Several CTAs an SM of one unit each are through before their askings are, which then stand in the way, most of all where all ask for the same lines of B and
-    // C.  us with / without, operands in HBM: two sequences of 48 heads x 96 and one group 5.31 / 4.84 (MX4 5.34 / 4.63), one of 128 x 64 4.66 / 4.65 (MX4 4.41
-    // / 4.16); with one CTA an SM (24 x 40) 3.71 / 3.86.  (Streams of several draws a block ask in any case: their steps are long, the reference's
+    // C.  us with / without, operands in HBM: two sequences of 48 heads x 96 and one group 5.31 / 4.76 (MX4 5.32 / 4.74), one of 128 x 64 4.65 / 4.57 (MX4 4.39
+    // / 4.33); with one CTA an SM (24 x 40) 3.71 / 3.86.  (Streams of several draws a block ask in any case: their steps are long, the reference's
     // 7.13 / 7.33.)
-    dd.ask_operands = dd.units_total > ctas || ctas <= static_cast<uint64_t>(sm_count());
+    const bool ask = dd.units_total > ctas || ctas <= static_cast<uint64_t>(sm_count());
+    dd.flags = (vec ? dd.kVec : 0) | (ask ? dd.kAsk : 0);
     dd.div_steps_per_head = fast_div_of(static_cast<uint32_t>(2 * (a.state.dim / rows_per_pass)));
     dd.div_groups = fast_div_of(static_cast<uint32_t>(a.ngroups));
     dd.div_heads = fast_div_of(static_cast<uint32_t>(a.state.heads));
