@@ -576,6 +576,30 @@ def test_layered4_slabs_equal_general_kernel(bits, layout, batch):
         assert torch.equal(got, want)
 
 
+@pytest.mark.parametrize("a_dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("bits,p,n", [(8, 24, 128), (4, 7, 80), (8, 5, 16)])
+def test_dense_A_equals_A_per_head(bits, p, n, a_dtype):
+    """A of every row and column, contiguous and with strides of its own, where all of a head are the same: the bits of the update with A per head."""
+    m = mk()
+    b, h, g = 3, 4, 2
+    gen = torch.Generator(device=dev()).manual_seed(n)
+    rnd = lambda *s: torch.randn(*s, generator=gen, device=dev())
+    first = m.allocate_state_kernel_cache(rnd(b, h, p, n).to(torch.bfloat16), 16, bits)
+    x, B, C = (v.to(torch.bfloat16) for v in (rnd(b, h, p), rnd(b, g, n), rnd(b, g, n)))
+    dt = rnd(b, h).to(torch.bfloat16)[..., None].expand(b, h, p)
+    A = (-torch.exp(rnd(h))).to(a_dtype)[:, None, None].expand(h, p, n)
+    wide = torch.full((h, p, 2 * n + 3), 7.0, dtype=a_dtype, device=dev())
+    wide[..., 1:2 * n + 1:2] = A
+    res = []
+    for form in (A, A.contiguous(), wide[..., 1:2 * n + 1:2]):
+        cache = m.MambaStateKernelCache(first.q_state.clone(), first.shared_exp.clone(), first.micro_exp.clone(), format_bits=bits, layout=first.layout)
+        y = m.mx_state_selective_update(cache, x, dt, form, B, C, dt_softplus=True, seed=9, rng_stream="layered")
+        res.append((y.view(torch.int16), cache.q_state, cache.shared_exp, cache.micro_exp))
+    for other in res[1:]:
+        for got, want in zip(other, res[0]):
+            assert torch.equal(got, want)
+
+
 @pytest.mark.parametrize("layout", ["reference", "packed"])
 @pytest.mark.parametrize("bits", [8, 4])
 def test_micro_exponent_edges(bits, layout):
